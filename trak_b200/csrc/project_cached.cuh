@@ -30,6 +30,8 @@ __global__ void __launch_bounds__(128) materialize_kernel(uint16_t* __restrict__
     const uint32_t by = blockIdx.y;
     const uint32_t sel_lo = h ? 0x1054u : 0x5410u;
     const uint32_t sel_hi = h ? 0x3276u : 0x7632u;
+    SignBases<BF16> bases;
+    if (PTYPE == TB_RADEMACHER) bases.load();
     Xw st;
     xw_seed(st, seed + 658105236u * stream_col + 359124577u * by);
     uint4* row = reinterpret_cast<uint4*>(matrix + ((size_t)(blockIdx.x * tiles + by) * nst) * (CACHED_A_BYTES / 2u)) +
@@ -40,7 +42,7 @@ __global__ void __launch_bounds__(128) materialize_kernel(uint16_t* __restrict__
         for (uint32_t c = 0; c < 4; ++c) {
             uint32_t w[8];
             if (PTYPE == TB_RADEMACHER)
-                gen_rademacher<BF16>(st, h, w);
+                gen_rademacher<BF16>(st, h, sel_lo, bases, w);
             else
                 gen_normal<BF16>(st, h, sel_lo, sel_hi, w);
             row[2u * c] = make_uint4(w[0], w[1], w[2], w[3]);

@@ -92,6 +92,8 @@ project_wide_kernel(const __grid_constant__ CUtensorMap tmap, const ProjParams p
         const uint32_t stream_col = col0 + m;
         const uint32_t sel_lo = h ? 0x1054u : 0x5410u;
         const uint32_t sel_hi = h ? 0x3276u : 0x7632u;
+        SignBases<BF16> bases;
+        if (PTYPE == TB_RADEMACHER) bases.load();
         const uint32_t row_addr = smem_base + g * (SA * WIDE_A_BYTES) + m * 64u;
         const uint32_t sw = (m >> 1) & 3u;                 // 64-byte swizzle of this row
         bool ok = true;
@@ -118,7 +120,7 @@ project_wide_kernel(const __grid_constant__ CUtensorMap tmap, const ProjParams p
                     for (uint32_t c = 0; c < 2; ++c) {
                         uint32_t w[8];
                         if (PTYPE == TB_RADEMACHER)
-                            gen_rademacher<BF16>(st, h, w);
+                            gen_rademacher<BF16>(st, h, sel_lo, bases, w);
                         else
                             gen_normal<BF16>(st, h, sel_lo, sel_hi, w);
                         // features 16c .. 16c+15 of this column: 16-byte pieces 2c and 2c + 1 of the row
