@@ -251,6 +251,17 @@ int tb_project_static(int device, void *stream, const void *grads, int dtype, in
  * 32-bit range is what keeps the matrix bit-identical to the reference's. */
 int tb_selftest_sqrt(int device, void *stream, uint64_t first, uint64_t count, uint64_t *mismatches_dev);
 
+/* ---- pageable host memory (no counterpart in the reference) ---------------------
+ * Copies between pageable host memory (numpy memmaps, host accumulators) and the device through a small pinned
+ * ring per device and direction; several host threads share the host side, which runs under the PCIe copies.
+ * Both calls are ordered on `stream` and may be made from any thread.
+ *   tb_host_to_device  returns when `src` has been read; the last device copies may still be in flight.
+ *   tb_device_to_host  returns when `dst` is complete; with add_f32 the data are floats and `dst += data`.
+ *   tb_host_staging_release  frees the pinned rings (16 MB each; made again on the next use). */
+int tb_host_to_device(int device, void *stream, void *dst, const void *src, size_t bytes);
+int tb_device_to_host(int device, void *stream, void *dst, const void *src, size_t bytes, int add_f32);
+int tb_host_staging_release(void);
+
 /* ---- measurement aid (no counterpart in the reference) -------------------------
  * Arms the calling thread: the next tb_project call records the two events
  * (cudaEvent_t passed as void*) on its stream immediately before and after its

@@ -132,3 +132,12 @@ def test_segment_table_validation():
     assert lib.tb_project_segments(0, None, segs, 0, 0, 4, 0x3000, 512, 512, 0, 148, 0, 1.0, 0, 0x10000, big) == 4
     assert lib.tb_project_segments(0, None, segs, 2, 0, 4, 0x3000, 512, 500, 0, 148, 0, 1.0, 0, 0x10000, big) == 3
     assert lib.tb_project_segments_workspace_bytes(0, 4, 15, 512, 148, 2) > lib.tb_project_workspace_bytes(0, 4, 15, 512, 148)
+
+
+def test_host_copy_validation():
+    lib = _lib.lib()
+    assert lib.tb_host_to_device(0, None, None, None, 0) == 0
+    assert lib.tb_host_to_device(0, None, None, 0x1000, 8) == 4
+    assert lib.tb_host_to_device(-1, None, 0x1000, 0x1000, 8) == 4
+    assert lib.tb_device_to_host(0, None, 0x1000, None, 8, 0) == 4
+    assert lib.tb_device_to_host(0, None, 0x1000, 0x1000, 6, 1) == 4    # not whole floats

@@ -13,8 +13,8 @@ Here the loop is turned inside out: train rows are walked in blocks, and for one
   ``accumulate``), the checkpoints' feature rows arriving from their stores through pinned staging;
 * the checkpoints' out-to-loss weights of the block are summed on the device;
 * ``tb_finalize_scores`` applies ``(sum / M) * (sum_w / M)`` and casts to the store's dtype;
-* the finished block leaves the GPU once, through one of two pinned buffers, and the host writes it
-  into the memmap while the GPU works on the next block.
+* the finished block leaves the GPU once, on a stream of its own, and is written into the memmap while the
+  GPU works on the next block.
 
 No host array of the full size exists, every score crosses PCIe once, finished, and the host does
 one ``memcpy`` per block.  A rank that owns the train rows ``[lo, hi)`` finalizes only those.
@@ -54,17 +54,17 @@ def finalize_scores_block(score_sum: torch.Tensor, out_to_loss_sum: torch.Tensor
     return out
 
 
-def _rows_to_device(src, lo, hi, device, stager):
+def _rows_to_device(src, lo, hi, device):
     """Rows [lo, hi) of a feature store (numpy memmap / array, CPU or CUDA tensor) as a CUDA matrix."""
     if isinstance(src, torch.Tensor):
         return sc._as_device_matrix(src[lo:hi], device)
-    return sc._as_device_matrix(mmap_io.read_rows(src, lo, hi, device, stager), device)
+    return sc._as_device_matrix(mmap_io.read_rows(src, lo, hi, device), device)
 
 
 def _whole_to_device(src, device):
     if isinstance(src, torch.Tensor):
         return sc._as_device_matrix(src, device)
-    return sc._as_device_matrix(torch.from_numpy(np.array(src)), device)   # a copy: the store may be read-only
+    return sc._as_device_matrix(mmap_io.read_rows(src, 0, src.shape[0], device), device)
 
 
 class ScoreFinalizer:
@@ -79,7 +79,8 @@ class ScoreFinalizer:
     ``scores/<exp>.mmap`` memmap, fp16 or fp32, or a CPU tensor) and returns it.
     """
 
-    STAGE_BYTES = 256 << 20  # each of the two pinned buffers the finished blocks leave through
+    STAGE_BYTES = 256 << 20   # most bytes of a finished block
+    UPLOAD_BYTES = 64 << 20   # about so many of a host feature store are uploaded per block and checkpoint
 
     def __init__(self, features, target_grads, out_to_loss, device, row_block: int = 65_536):
         if not (len(features) == len(target_grads) == len(out_to_loss)) or len(features) == 0:
@@ -116,21 +117,30 @@ class ScoreFinalizer:
         dev, m, M = self.device, self.n_targets, self.num_models
         esize = 2 if out_dtype == torch.float16 else 4
         step = max(256, min(self.row_block, self.STAGE_BYTES // (esize * m) // 256 * 256))
+        host = [f for f in self.features if not (isinstance(f, torch.Tensor) and f.is_cuda)]
+        if host:
+            # blocks short enough that uploading one overlaps computing and writing out the one before
+            row_bytes = max(f.shape[1] * (f.element_size() if isinstance(f, torch.Tensor) else f.itemsize) for f in host)
+            step = min(step, max(4096, self.UPLOAD_BYTES // row_bytes // 256 * 256))
         step = min(step, max(1, hi - lo))
+        contiguous = scores_store.is_contiguous() and not scores_store.is_cuda if is_tensor \
+            else scores_store.flags.c_contiguous
         with torch.cuda.device(dev):
             acc = torch.empty(step, m, dtype=torch.float32, device=dev)
-            done = torch.empty(step, m, dtype=out_dtype, device=dev)
-            stage = [torch.empty(step, m, dtype=out_dtype).pin_memory() for _ in range(2)]
-            stagers = {}
+            done = [torch.empty(step, m, dtype=out_dtype, device=dev) for _ in range(2)]
+            out_stream = torch.cuda.Stream(dev)
             pending = None
 
             def flush(item):
-                r0, nrows, buf, event = item
-                event.synchronize()
-                if is_tensor:
-                    scores_store[r0:r0 + nrows] = buf[:nrows]
-                else:
-                    scores_store[r0:r0 + nrows] = buf[:nrows].numpy()
+                r0, block, event = item
+                rows = scores_store[r0:r0 + block.shape[0]]
+                out_stream.wait_event(event)
+                if contiguous:
+                    mmap_io.device_to_host(rows, block, out_stream)
+                    return
+                with torch.cuda.stream(out_stream):
+                    rows[...] = block.to(rows.device) if is_tensor else block.cpu().numpy()
+                out_stream.synchronize()
 
             for i, r0 in enumerate(range(lo, hi, step)):
                 r1 = min(hi, r0 + step)
@@ -138,14 +148,7 @@ class ScoreFinalizer:
                 w_sum = torch.zeros(nrows, dtype=torch.float32, device=dev)
                 for j in range(M):
                     src = self.features[j]
-                    stager = None
-                    if not isinstance(src, torch.Tensor):
-                        key = (src.dtype, src.shape[1])
-                        if key not in stagers:
-                            stagers[key] = mmap_io.PinnedStager(src.shape[1], mmap_io._TORCH[np.dtype(src.dtype)],
-                                                                min(16384, step))
-                        stager = stagers[key]
-                    blk = _rows_to_device(src, r0, r1, dev, stager)
+                    blk = _rows_to_device(src, r0, r1, dev)
                     tg = self.targets[j]
                     if tg.dtype != blk.dtype:
                         wide = torch.promote_types(tg.dtype, blk.dtype)
@@ -154,15 +157,13 @@ class ScoreFinalizer:
                     wj = self.out_to_loss[j]
                     wj = wj[r0:r1] if isinstance(wj, torch.Tensor) else torch.from_numpy(np.array(wj[r0:r1]))
                     w_sum += wj.to(dev, torch.float32, non_blocking=True).reshape(-1)
-                finalize_scores_block(acc[:nrows], w_sum, M, out=done[:nrows])
                 # buffer i % 2 was last read by the flush of block i - 2, which has returned
-                buf = stage[i % 2]
-                buf[:nrows].copy_(done[:nrows], non_blocking=True)
+                block = finalize_scores_block(acc[:nrows], w_sum, M, out=done[i % 2][:nrows])
                 event = torch.cuda.Event()
                 event.record(torch.cuda.current_stream(dev))
                 if pending is not None:
                     flush(pending)
-                pending = (r0, nrows, buf, event)
+                pending = (r0, block, event)
             if pending is not None:
                 flush(pending)
             _lib.device_status(dev.index)

@@ -8,8 +8,10 @@ example.  ``TRAKer`` moves whole arrays at once (``ch.as_tensor(memmap, device=.
 trak/traker.py:480-486,662-665) and writes results back through a pageable ``.cpu()``.
 
 The helpers here read and write *row ranges* of those same files, so a rank that owns the
-train rows ``[lo, hi)`` touches only its part, and they go through a reusable pair of pinned
-staging buffers in chunks, the host side of one chunk overlapping the device copy of the next.  The files stay byte-compatible with the reference: they are opened with
+train rows ``[lo, hi)`` touches only its part.  Transfers of a megabyte and more between a file and a GPU are the
+library's (``tb_host_to_device``, ``tb_device_to_host``: several host threads, a pinned ring); smaller ones and CPU
+targets go through a reusable pair of staging buffers, the host side of one chunk overlapping the device copy of the
+next.  The files stay byte-compatible with the reference: they are opened with
 the same numpy call, nothing else is written.
 """
 import os
@@ -17,6 +19,8 @@ import os
 import numpy as np
 import torch
 from numpy.lib.format import open_memmap
+
+from . import _lib
 
 _NP = {torch.float16: np.float16, torch.float32: np.float32, torch.int32: np.int32}
 _TORCH = {np.dtype(v): k for k, v in _NP.items()}
@@ -31,6 +35,35 @@ def create_store(path, shape, dtype=torch.float16) -> np.memmap:
 def open_store(path, mode="r+") -> np.memmap:
     """An existing store; shape and dtype come from its npy header."""
     return open_memmap(filename=str(path), mode=mode)
+
+
+# Transfers of pageable host memory go through the library's own threads and pinned ring from this size on.
+NATIVE_MIN_BYTES = 1 << 20
+
+
+def host_to_device(src, device) -> torch.Tensor:
+    """A copy of a C-contiguous numpy array or CPU tensor on a CUDA device, ordered on its current stream; ``src``
+    has been read when the call returns."""
+    device = torch.device(device)
+    if isinstance(src, np.ndarray):
+        dtype, ptr, nbytes = _TORCH[src.dtype], src.ctypes.data, src.nbytes
+    else:
+        dtype, ptr, nbytes = src.dtype, src.data_ptr(), src.numel() * src.element_size()
+    out = torch.empty(tuple(src.shape), dtype=dtype, device=device)
+    with torch.cuda.device(out.device):
+        _lib.check(_lib.lib().tb_host_to_device(out.device.index, torch.cuda.current_stream(out.device).cuda_stream,
+                                                out.data_ptr(), ptr, nbytes))
+    return out
+
+
+def device_to_host(dst, src: torch.Tensor, stream=None, add: bool = False) -> None:
+    """Copies a contiguous CUDA tensor over a C-contiguous host array or CPU tensor of the same size and dtype (or,
+    fp32 only, adds it), ordered on ``stream`` (default: the device's current one); complete on return."""
+    ptr = dst.ctypes.data if isinstance(dst, np.ndarray) else dst.data_ptr()
+    with torch.cuda.device(src.device):
+        stream = torch.cuda.current_stream(src.device) if stream is None else stream
+        _lib.check(_lib.lib().tb_device_to_host(src.device.index, stream.cuda_stream, ptr, src.data_ptr(),
+                                                src.numel() * src.element_size(), int(add)))
 
 
 class PinnedStager:
@@ -76,6 +109,9 @@ def read_rows(store: np.memmap, lo: int, hi: int, device, stager: PinnedStager =
     if store.ndim != 2 or not (0 <= lo <= hi <= store.shape[0]):
         raise ValueError("row range outside the store")
     dtype = _TORCH[store.dtype]
+    rows = store[lo:hi]
+    if torch.device(device).type == "cuda" and rows.flags.c_contiguous and rows.nbytes >= NATIVE_MIN_BYTES:
+        return host_to_device(rows, device)
     out = torch.empty((hi - lo, store.shape[1]), dtype=dtype, device=device)
     if stager is None:
         stager = PinnedStager(store.shape[1], dtype, min(16384, max(1, hi - lo)))
@@ -97,6 +133,10 @@ def write_rows(store: np.memmap, lo: int, values: torch.Tensor, stager: PinnedSt
             or lo + n > store.shape[0]:
         raise ValueError("row range or row length does not match the store")
     dtype = _TORCH[store.dtype]
+    rows = store[lo:lo + n]
+    if values.is_cuda and rows.flags.c_contiguous and rows.nbytes >= NATIVE_MIN_BYTES:
+        device_to_host(rows, values.to(dtype).contiguous())
+        return
     if stager is None:
         stager = PinnedStager(store.shape[1], dtype, min(16384, max(1, n)))
     pending = None  # (buffer index, first row, rows) whose copy has been enqueued but not yet written out

@@ -15,8 +15,8 @@ passed to an unmodified ``TRAKer(score_computer=B200ScoreComputer)``
   (one all-reduce of k x k fp32) -- rows sharded across GPUs, everything else
   local: the inverse is replicated, features and scores stay row-sharded;
 * ``get_scores`` takes an optional ``row_scale`` (the out-to-loss weights) that is
-  applied inside the GEMM epilogue, and streams the scores to a host accumulator through
-  two pinned buffers while the next block is being multiplied.
+  applied inside the GEMM epilogue, and streams the scores to a host accumulator while the
+  next block is being multiplied.
 
 There is no CPU path: tensors are moved to ``device`` and the CUDA library must load.
 """
@@ -24,7 +24,7 @@ import logging
 
 import torch
 
-from . import _lib
+from . import _lib, mmap_io
 
 _DTYPES = {torch.float16: _lib.TB_F16, torch.bfloat16: _lib.TB_BF16, torch.float32: _lib.TB_F32}
 _workspaces = {}
@@ -75,7 +75,11 @@ class StreamPair:
 
 
 def _as_device_matrix(t: torch.Tensor, device) -> torch.Tensor:
-    t = t.to(device, non_blocking=True)
+    if not t.is_cuda and t.dtype in _DTYPES and t.is_contiguous() and torch.device(device).type == "cuda" \
+            and t.numel() * t.element_size() >= mmap_io.NATIVE_MIN_BYTES and not t.is_pinned():
+        t = mmap_io.host_to_device(t, device)
+    else:
+        t = t.to(device, non_blocking=True)
     if t.dtype not in _DTYPES:
         t = t.float()
     if t.dim() != 2:
@@ -104,6 +108,13 @@ def gram(x: torch.Tensor, out: torch.Tensor = None, accumulate: bool = False) ->
 
 def spd_inverse_(a: torch.Tensor, lambda_reg: float = 0.0, rescale: bool = True) -> torch.Tensor:
     """In place: a <- inv(a + lambda I) [/ mean |entry|] for a CUDA fp32 [k, k] matrix."""
+    _launch_spd_inverse(a, lambda_reg, rescale)
+    _lib.device_status(a.device.index)  # raises NotPositiveDefinite / DeviceTimeout
+    return a
+
+
+def _launch_spd_inverse(a: torch.Tensor, lambda_reg: float, rescale: bool) -> None:
+    """``spd_inverse_`` without waiting for it: the caller checks ``device_status`` before it returns."""
     if a.dtype != torch.float32 or a.dim() != 2 or a.shape[0] != a.shape[1] or a.stride(1) != 1:
         raise RuntimeError("expected a square fp32 matrix with unit column stride")
     dev = a.device
@@ -113,8 +124,6 @@ def spd_inverse_(a: torch.Tensor, lambda_reg: float = 0.0, rescale: bool = True)
         ws = _workspace(dev, stream, lib.tb_spd_inverse_workspace_bytes(a.shape[0]))
         _lib.check(lib.tb_spd_inverse(dev.index, stream, a.data_ptr(), a.shape[0], a.stride(0),
                                       float(lambda_reg), int(rescale), None, ws.data_ptr(), ws.numel()))
-        _lib.device_status(dev.index)  # raises NotPositiveDefinite / DeviceTimeout
-    return a
 
 
 def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, row_scale: torch.Tensor = None,
@@ -170,7 +179,7 @@ class B200ScoreComputer:
         self.proj_dim = grads.shape[1]
         accs = [None, None]   # one partial Gram per stream of the pair (blocks alternate between them)
         with torch.cuda.device(self.device), self._pair() as pair:
-            for i, block in enumerate(b for b in torch.split(grads, self.CUDA_MAX_DIM_SIZE, dim=0) if b.shape[0]):
+            for i, block in enumerate(self._blocks(grads)):
                 with pair.stream(i):
                     blk = _as_device_matrix(block, self.device)
                     blk.record_stream(torch.cuda.current_stream(self.device))
@@ -191,30 +200,41 @@ class B200ScoreComputer:
 
     # -- trak/score_computers.py:157-177
     def get_x_xtx_inv(self, grads: torch.Tensor, xtx: torch.Tensor) -> torch.Tensor:
-        inv = xtx.to(self.device, torch.float32).clone()
-        spd_inverse_(inv, self.lambda_reg, rescale=True)
-        inv = inv.to(self.dtype)
-        result = torch.empty(grads.shape[0], inv.shape[1], dtype=self.dtype, device=self.device)
-        if grads.shape[0]:
-            probe = grads[:1]
-            in_dtype = probe.dtype if probe.dtype in _DTYPES else torch.float32
-            if in_dtype != inv.dtype:  # the narrower operand is promoted, never the inverse demoted
-                inv = inv.to(torch.promote_types(in_dtype, inv.dtype))
+        result = torch.empty(grads.shape[0], xtx.shape[1], dtype=self.dtype, device=self.device)
         start = 0
         with torch.cuda.device(self.device), self._pair() as pair:
-            for i, block in enumerate(b for b in torch.split(grads, self.CUDA_MAX_DIM_SIZE, dim=0) if b.shape[0]):
+            # the pair's streams do not wait for the inverse: the blocks are copied and converted meanwhile
+            inv = xtx.to(self.device, torch.float32, copy=True)
+            _launch_spd_inverse(inv, self.lambda_reg, rescale=True)
+            inv = inv.to(self.dtype)
+            in_dtype = grads.dtype if grads.dtype in _DTYPES else torch.float32
+            if in_dtype != inv.dtype:  # the narrower operand is promoted, never the inverse demoted
+                inv = inv.to(torch.promote_types(in_dtype, inv.dtype))
+            inverted = torch.cuda.Event()
+            inverted.record(torch.cuda.current_stream(self.device))
+            for i, block in enumerate(self._blocks(grads)):
                 rows = slice(start, start + block.shape[0])
                 start += block.shape[0]
                 with pair.stream(i):
                     blk = _as_device_matrix(block, self.device).to(inv.dtype)
                     blk.record_stream(torch.cuda.current_stream(self.device))
+                    torch.cuda.current_stream(self.device).wait_event(inverted)
                     # the inverse is symmetric, so block @ inv == block @ inv.T
                     if result.dtype == torch.float32:
                         gemm_nt(blk, inv, out=result[rows])
                     else:
                         result[rows] = gemm_nt(blk, inv).to(self.dtype)
-        _lib.device_status(self.device.index)
+        _lib.device_status(self.device.index)  # raises NotPositiveDefinite / DeviceTimeout
         return result
+
+    UPLOAD_BYTES = 96 << 20  # about so many bytes of a host matrix are uploaded at a time, under the work on the last
+
+    def _blocks(self, t: torch.Tensor, rows: int = None):
+        """The row blocks of ``t`` that are multiplied at a time; shorter ones for a matrix on the host."""
+        rows = self.CUDA_MAX_DIM_SIZE if rows is None else rows
+        if not t.is_cuda:
+            rows = min(rows, max(8192, self.UPLOAD_BYTES // max(1, t.shape[1] * t.element_size()) // 256 * 256))
+        return (b for b in torch.split(t, rows, dim=0) if b.shape[0])
 
     def _pair(self) -> StreamPair:
         pair = getattr(self, "_stream_pair", None)
@@ -227,10 +247,9 @@ class B200ScoreComputer:
                    row_scale: torch.Tensor = None) -> None:
         """``accumulator += features @ target_grads.T`` (times ``row_scale`` per train row when given).
 
-        TRAKer keeps the accumulator on the host (trak/traker.py:632): the product then leaves the GPU
-        through two pinned staging buffers of at most ``HOST_STAGE_BYTES`` each, the copy of one row block
-        overlapping the GEMM of the next and the host-side ``+=`` of the one before, instead of one
-        synchronous pageable copy per block."""
+        TRAKer keeps the accumulator on the host (trak/traker.py:632): the product then leaves the GPU in row
+        blocks of at most ``HOST_STAGE_BYTES``, copied and added by several host threads while the GPU multiplies
+        the next block, instead of one synchronous pageable copy per block."""
         self._accumulate_products(features, _as_device_matrix(target_grads, self.device), accumulator, row_scale)
 
     def get_scores_from_grads(self, grads: torch.Tensor, xtx: torch.Tensor, target_grads: torch.Tensor,
@@ -240,8 +259,8 @@ class B200ScoreComputer:
         ``xtx`` exactly as ``get_x_xtx_inv`` forms it (trak/score_computers.py:157-168).  One product over
         the train rows instead of two: ``2 k^2 m`` flop for ``inv @ target_grads.T`` replace the ``2 n k^2``
         of the features.  For callers that do not need the features themselves (TRAKer stores them)."""
-        inv = xtx.to(self.device, torch.float32).clone()
-        spd_inverse_(inv, self.lambda_reg, rescale=True)
+        inv = xtx.to(self.device, torch.float32, copy=True)
+        spd_inverse_(inv, self.lambda_reg, rescale=True)   # raises before anything is added to the accumulator
         targets = _as_device_matrix(target_grads, self.device)
         solved = gemm_nt(targets.float(), inv)  # [m, k] = target_grads @ inv  (inv is symmetric)
         self._accumulate_products(grads, solved, accumulator, row_scale)
@@ -252,17 +271,20 @@ class B200ScoreComputer:
         step = self.CUDA_MAX_DIM_SIZE
         if on_host:
             step = max(256, min(step, self.HOST_STAGE_BYTES // (4 * m) // 256 * 256))
-            stage = self._host_stage(min(step, features.shape[0]), m)
+            threaded = accumulator.dtype == torch.float32 and accumulator.is_contiguous()
         pending = None
 
         def flush(item):
-            rows, buf, event = item
-            event.synchronize()
-            accumulator[rows] += buf.to(accumulator.dtype)
+            rows, part, stream = item
+            if threaded:
+                mmap_io.device_to_host(accumulator[rows], part, stream, add=True)
+                return
+            with torch.cuda.stream(stream):
+                accumulator[rows] += part.cpu().to(accumulator.dtype)
 
         start = 0
         with torch.cuda.device(self.device), self._pair() as pair:
-            for i, block in enumerate(b for b in torch.split(features, step, dim=0) if b.shape[0]):
+            for i, block in enumerate(self._blocks(features, step)):
                 rows = slice(start, start + block.shape[0])
                 start += block.shape[0]
                 with pair.stream(i):
@@ -277,27 +299,15 @@ class B200ScoreComputer:
                         else:
                             accumulator[rows] += part.to(accumulator.dtype).to(accumulator.device)
                         continue
-                    # buffer i % 2 was last read by the flush of block i - 2, which has returned; the copy runs
-                    # on this block's stream, so the GEMM of the next block (other stream) overlaps it
-                    buf = stage[i % 2][:blk.shape[0]]
-                    buf.copy_(part, non_blocking=True)
-                    event = torch.cuda.Event()
-                    event.record(cur)
+                # the copy runs on this block's stream, under the GEMM of the next block on the other one
                 if pending is not None:
                     flush(pending)
-                pending = (rows, buf, event)
+                pending = (rows, part, cur)
         if pending is not None:
             flush(pending)
         _lib.device_status(self.device.index)
 
-    HOST_STAGE_BYTES = 256 << 20  # each of the two pinned buffers get_scores copies through
-
-    def _host_stage(self, rows: int, m: int):
-        """Two pinned fp32 buffers [rows, m], kept between calls (pinning is slow) and regrown when too small."""
-        stage = getattr(self, "_stage", None)
-        if stage is None or stage[0].shape[0] < rows or stage[0].shape[1] != m:
-            self._stage = stage = [torch.empty(rows, m, dtype=torch.float32).pin_memory() for _ in range(2)]
-        return stage
+    HOST_STAGE_BYTES = 128 << 20  # most bytes of scores that leave for a host accumulator at a time
 
 
 def reduce_gram(local_gram: torch.Tensor, process_group=None) -> torch.Tensor:
