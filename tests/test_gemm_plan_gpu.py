@@ -1,0 +1,52 @@
+"""Products and inverses at the sizes where the tile, the slices of the contraction and the block columns change."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float((a.double() - b).norm() / b.norm())
+
+
+# one 128-wide tile and its neighbours, few tiles and a long contraction (sliced), a ragged last slice, rows longer
+# than a warp, two, four, eight warps hold in registers and than one span of the packing kernel
+@pytest.mark.parametrize("M,N,K", [(1, 1, 40), (127, 129, 32), (128, 128, 64), (257, 255, 4096), (100, 300, 8192),
+                                   (513, 100, 1025), (64, 64, 2049), (40, 500, 4100), (33, 65, 9000), (1000, 512, 512)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_gemm_nt(cuda, M, N, K, dtype):
+    from trak_b200 import score_computers as sc
+    g = torch.Generator(device=cuda).manual_seed(M + N + K)
+    a = torch.randn(M, K, device=cuda, generator=g).to(dtype)
+    b = torch.randn(N, K, device=cuda, generator=g).to(dtype)
+    w = torch.rand(M, device=cuda, generator=g)
+    want = w.double()[:, None] * (a.double() @ b.double().T)
+    got = sc.gemm_nt(a, b, row_scale=w)
+    assert rel(got, want) <= 3e-5
+    assert rel(sc.gemm_nt(a, b, out=got.clone(), row_scale=w, accumulate=True), 2 * want) <= 3e-5
+
+
+@pytest.mark.parametrize("n,k", [(5000, 40), (4097, 129), (3001, 512), (20000, 300), (100, 700), (1, 5)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_gram(cuda, n, k, dtype):
+    from trak_b200 import score_computers as sc
+    x = torch.randn(n, k, device=cuda, generator=torch.Generator(device=cuda).manual_seed(n)).to(dtype)
+    want = x.double().T @ x.double()
+    got = sc.gram(x)
+    assert torch.equal(got, got.T)
+    assert rel(got, want) <= (2e-6 if dtype == torch.float32 else 3e-5)
+    got = sc.gram(x, out=got, accumulate=True)
+    assert torch.equal(got, got.T) and rel(got, 2 * want) <= (2e-6 if dtype == torch.float32 else 3e-5)
+
+
+@pytest.mark.parametrize("k", [1, 3, 4, 63, 65, 127, 130, 448, 449, 512, 575, 640, 1088])
+def test_inverse_at_tile_edges(cuda, k):
+    from trak_b200 import score_computers as sc
+    y = torch.randn(3 * k, k, device=cuda, dtype=torch.float64, generator=torch.Generator(device=cuda).manual_seed(k))
+    a = (y.T @ y / k).float()
+    want = torch.linalg.inv(a.double() + 1e-3 * torch.eye(k, device=cuda, dtype=torch.float64))
+    got = sc.spd_inverse_(a.clone(), 1e-3, rescale=False)
+    assert rel(got, want) <= 2e-5
+    wide = torch.zeros(k, k + 3, device=cuda)      # rows that are not 16-byte aligned
+    wide[:, :k] = a
+    assert rel(sc.spd_inverse_(wide[:, :k], 1e-3, rescale=False), want) <= 2e-5

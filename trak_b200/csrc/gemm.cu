@@ -56,12 +56,15 @@ struct GemmParams {
     int64_t ldc;
     uint32_t M, N;
     uint32_t kblocks;        // K / 32 (padded)
+    uint32_t kb_per_split;   // k blocks of one slice of the grid's z dimension (kblocks when there is one slice)
+    uint64_t split_stride;   // floats between the partial products of two slices
     uint32_t stages;
     uint32_t idesc;
     float alpha;
     int accumulate;
     int symmetric;           // A and B are the same packed operand; only tiles on/above the
                              // diagonal are computed and every result is stored twice
+    int mirror;              // symmetric: whether this launch stores the second copy (not for partial products)
 };
 
 // Power-of-two scale of a packed fp32 operand row whose largest magnitude has the bit pattern
@@ -88,70 +91,72 @@ __device__ __forceinline__ void gemm_fail(uint32_t* status, volatile uint32_t* a
 }
 
 
-// Epilogue store of one warp's 32 x 128 block of results, which sits in the warp's shared-memory
-// slab as slab[row][column] (row length SLAB_LD floats: odd, so rows and columns are both
-// conflict-free).  C[m_first + row, n0 + column] is written as rows of 128 consecutive floats
+// Epilogue store of one warp's 32 x COLS block of results, which sits in the warp's shared-memory
+// slab as slab[row][column] (row length COLS + 1 floats: odd, so rows and columns are both
+// conflict-free).  C[m_first + row, n0 + column] is written as rows of COLS consecutive floats
 // (a lane holding one row in registers would touch 32 rows per store instruction).  When
 // accumulating, the loads of a group are all issued before its first store: a load behind a store
 // to a possibly aliasing address would wait for it.  Symmetric products store only n >= m that way
 // and write the same bits to C[n, m] for n > m (for a fixed column the lanes run along m: coalesced).
-constexpr uint32_t SLAB_LD = 129;
-constexpr uint32_t SLAB_FLOATS = 32u * SLAB_LD;
-__device__ __forceinline__ void store_block_from_slab(const GemmParams& p, const float* slab, uint32_t m_first,
+template <uint32_t COLS>
+__device__ __forceinline__ void store_block_from_slab(const GemmParams& p, float* C, const float* slab, uint32_t m_first,
                                                       uint32_t n0, uint32_t lane) {
+    constexpr uint32_t LD = COLS + 1u, CH = COLS / 32u;
     const bool sym = p.symmetric != 0;
 #pragma unroll 1
     for (uint32_t r0 = 0; r0 < 32u && m_first + r0 < p.M; r0 += 4u) {
-        float v[4][4];
-        bool on[4][4];
+        float v[4][CH];
+        bool on[4][CH];
 #pragma unroll
         for (uint32_t u = 0; u < 4; ++u)
 #pragma unroll
-            for (uint32_t ch = 0; ch < 4; ++ch) {
+            for (uint32_t ch = 0; ch < CH; ++ch) {
                 const uint32_t mr = m_first + r0 + u, n = n0 + ch * 32u + lane;
                 on[u][ch] = mr < p.M && n < p.N && (!sym || n >= mr);
-                v[u][ch] = (p.accumulate && on[u][ch]) ? p.C[(int64_t)mr * p.ldc + n] : 0.0f;
+                v[u][ch] = (p.accumulate && on[u][ch]) ? C[(int64_t)mr * p.ldc + n] : 0.0f;
             }
 #pragma unroll
         for (uint32_t u = 0; u < 4; ++u)
 #pragma unroll
-            for (uint32_t ch = 0; ch < 4; ++ch)
+            for (uint32_t ch = 0; ch < CH; ++ch)
                 if (on[u][ch])
-                    p.C[(int64_t)(m_first + r0 + u) * p.ldc + n0 + ch * 32u + lane] =
-                        v[u][ch] + slab[(r0 + u) * SLAB_LD + ch * 32u + lane];
+                    C[(int64_t)(m_first + r0 + u) * p.ldc + n0 + ch * 32u + lane] =
+                        v[u][ch] + slab[(r0 + u) * LD + ch * 32u + lane];
     }
     const uint32_t m = m_first + lane;
-    if (sym && m < p.N) {
+    if (sym && p.mirror && m < p.N) {
 #pragma unroll 1
-        for (uint32_t i0 = 0; i0 < 128u; i0 += 16u) {
+        for (uint32_t i0 = 0; i0 < COLS; i0 += 16u) {
             float old[16];
 #pragma unroll
             for (uint32_t u = 0; u < 16; ++u) {
                 const bool on = n0 + i0 + u < p.M && n0 + i0 + u > m;
-                old[u] = (p.accumulate && on) ? p.C[(int64_t)(n0 + i0 + u) * p.ldc + m] : 0.0f;
+                old[u] = (p.accumulate && on) ? C[(int64_t)(n0 + i0 + u) * p.ldc + m] : 0.0f;
             }
 #pragma unroll
             for (uint32_t u = 0; u < 16; ++u)
                 if (n0 + i0 + u < p.M && n0 + i0 + u > m)
-                    p.C[(int64_t)(n0 + i0 + u) * p.ldc + m] = slab[lane * SLAB_LD + i0 + u] + old[u];
+                    C[(int64_t)(n0 + i0 + u) * p.ldc + m] = slab[lane * LD + i0 + u] + old[u];
         }
     }
 }
 
-template <int NPL>
-__global__ void __launch_bounds__(384, 1)
+// A CTA owns a tile of T x 128 rows by T x 128 columns; T = 1 is for products of few tiles (launch_gemm).
+template <int NPL, int T>
+__global__ void __launch_bounds__(384, 3 - T)
 gemm_nt_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const GemmParams p) {
     constexpr uint32_t MAXS = 8;
-    constexpr uint32_t A_BYTES = 2 * NPL * GTILE_BYTES;  // two row blocks x planes
+    constexpr uint32_t A_BYTES = T * NPL * GTILE_BYTES;  // row blocks x planes
     constexpr uint32_t STAGE_BYTES = 2 * A_BYTES;
+    constexpr uint32_t TILE = 128u * T, TMEM_COLS = 128u * T * T;
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t bar_full[MAXS];
     __shared__ uint64_t bar_empty[MAXS];
     __shared__ uint64_t bar_acc;
     __shared__ uint32_t tmem_slot;
     __shared__ uint32_t abort_word;
-    __shared__ float col_factor[256];  // inverse scale of every column of this tile (1 when unscaled)
+    __shared__ float col_factor[TILE];  // inverse scale of every column of this tile (1 when unscaled)
     volatile uint32_t* abort_flag = &abort_word;
 
     // Tile order: CTAs are numbered so that the ~148 that run together cover a block of about
@@ -164,6 +169,7 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const uint32_t gsize = min(tiles_m - first_m, GROUP_M);
     const uint32_t tile_m = first_m + (id % width) % gsize, tile_n = (id % width) / gsize;
     if (p.symmetric && tile_n < tile_m) return;  // whole CTA leaves before any barrier or TMEM use
+    const uint32_t kb_first = blockIdx.z * p.kb_per_split, kb_end = min(p.kblocks, kb_first + p.kb_per_split);
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t S = p.stages;
@@ -179,7 +185,7 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         fence_mbar_init();
     }
     if (warp == 1) {
-        tmem_alloc(smem_u32(&tmem_slot), 512);
+        tmem_alloc(smem_u32(&tmem_slot), TMEM_COLS);
         tmem_relinquish();
     }
     tc_fence_before();
@@ -192,7 +198,7 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         prefetch_tmap(&map_a);
         prefetch_tmap(&map_b);
         uint32_t slot = 0, ph = 0;
-        for (uint32_t kb = 0; kb < p.kblocks; ++kb) {
+        for (uint32_t kb = kb_first; kb < kb_end; ++kb) {
             if (!mbar_wait(smem_u32(&bar_empty[slot]), ph ^ 1u, abort_flag)) {
                 gemm_fail(p.status, abort_flag, ST_TIMEOUT_EMPTY, kb);
                 break;
@@ -202,14 +208,14 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             mbar_expect_tx(bar, STAGE_BYTES);
             // packed row index of (row block rb, k block kb, plane pl): ((rb*kblocks + kb)*NPL + pl)*128
 #pragma unroll
-            for (uint32_t h = 0; h < 2; ++h) {
-                const uint32_t rb_a = tile_m * 2u + h, rb_b = tile_n * 2u + h;
+            for (uint32_t h = 0; h < T; ++h) {
+                const uint32_t rb_a = tile_m * T + h, rb_b = tile_n * T + h;
 #pragma unroll
                 for (uint32_t pl = 0; pl < (uint32_t)NPL; ++pl) {
                     // A: [block h][plane]; B: [plane][block h] so that 256 rows of one plane are adjacent
                     tma_load_2d(sa + (h * NPL + pl) * GTILE_BYTES, &map_a, 0,
                                 (int)(((rb_a * p.kblocks + kb) * NPL + pl) * 128u), bar);
-                    tma_load_2d(sb + (pl * 2u + h) * GTILE_BYTES, &map_b, 0,
+                    tma_load_2d(sb + (pl * T + h) * GTILE_BYTES, &map_b, 0,
                                 (int)(((rb_b * p.kblocks + kb) * NPL + pl) * 128u), bar);
                 }
             }
@@ -224,7 +230,7 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const bool leader = elect_one();
         uint32_t slot = 0, ph = 0;
         bool ok = true;
-        for (uint32_t kb = 0; kb < p.kblocks; ++kb) {
+        for (uint32_t kb = kb_first; kb < kb_end; ++kb) {
             const bool got = mbar_wait(smem_u32(&bar_full[slot]), ph, abort_flag);
             if (!__all_sync(0xffffffffu, got)) {
                 if (leader) gemm_fail(p.status, abort_flag, ST_TIMEOUT_FULL_B, kb);
@@ -233,16 +239,16 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
             tc_fence_after();
             const uint32_t sa = smem_base + slot * STAGE_BYTES, sb = sa + A_BYTES;
-            const uint64_t b_hi = smem_desc_k_sw64(sb), b_lo = smem_desc_k_sw64(sb + 2u * GTILE_BYTES);
+            const uint64_t b_hi = smem_desc_k_sw64(sb), b_lo = smem_desc_k_sw64(sb + T * GTILE_BYTES);
 #pragma unroll
-            for (uint32_t mb = 0; mb < 2; ++mb) {
-                const uint32_t d = tmem_base + mb * 256u;
+            for (uint32_t mb = 0; mb < T; ++mb) {
+                const uint32_t d = tmem_base + mb * TILE;
                 const uint64_t a_hi = smem_desc_k_sw64(sa + (mb * NPL) * GTILE_BYTES);
                 const uint64_t a_lo = smem_desc_k_sw64(sa + (mb * NPL + (NPL - 1)) * GTILE_BYTES);
                 if (leader) {
 #pragma unroll
                     for (uint32_t kk = 0; kk < 2; ++kk) {
-                        const uint32_t acc = (kb > 0 || kk > 0) ? 1u : 0u;
+                        const uint32_t acc = (kb > kb_first || kk > 0) ? 1u : 0u;
                         umma_f16_ss(d, a_hi + 2u * kk, b_hi + 2u * kk, p.idesc, acc);
                         if (NPL == 2) {
                             umma_f16_ss(d, a_hi + 2u * kk, b_lo + 2u * kk, p.idesc, 1u);
@@ -262,8 +268,8 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // --------------------------------- epilogue ---------------------------------
         const uint32_t q = warp & 3u, chalf = (warp - 4u) >> 2;  // TMEM lane quarter, column half
         {
-            const uint32_t t = threadIdx.x - 128u, n = tile_n * 256u + t;
-            col_factor[t] = (p.amax_b && n < p.N) ? row_scale_down(p.amax_b[n]) : 1.0f;
+            const uint32_t t = threadIdx.x - 128u, n = tile_n * TILE + t;
+            if (t < TILE) col_factor[t] = (p.amax_b && n < p.N) ? row_scale_down(p.amax_b[n]) : 1.0f;
             asm volatile("bar.sync 1, 256;" ::: "memory");  // the eight epilogue warps only
         }
         bool got = mbar_wait(smem_u32(&bar_acc), 0u, abort_flag);
@@ -275,29 +281,31 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const uint32_t lane_base = (q * 32u) << 16;
             // The pipeline buffers are idle by now (the commit behind bar_acc covered every MMA and
             // every load has been consumed): each warp turns its 32 x 128 blocks around in its own slab.
+            constexpr uint32_t COLS = 64u * T, LD = COLS + 1u;  // columns of one epilogue warp
             float* slab = reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw))) +
-                          (size_t)(warp - 4u) * SLAB_FLOATS;
+                          (size_t)(warp - 4u) * (32u * LD);
+            float* C = p.C + blockIdx.z * p.split_stride;
 #pragma unroll 1
-            for (uint32_t mb = 0; mb < 2; ++mb) {
-                const uint32_t m_first = tile_m * 256u + mb * 128u + q * 32u, m = m_first + lane;
+            for (uint32_t mb = 0; mb < T; ++mb) {
+                const uint32_t m_first = tile_m * TILE + mb * 128u + q * 32u, m = m_first + lane;
                 const float rs = p.alpha * ((p.row_scale && m < p.M) ? p.row_scale[m] : 1.0f);
                 const float fa = (p.amax_a && m < p.M) ? row_scale_down(p.amax_a[m]) : 1.0f;
 #pragma unroll 1
-                for (uint32_t cb = 0; cb < 8; cb += 2) {
-                    const uint32_t c0 = chalf * 128u + cb * 16u;
+                for (uint32_t cb = 0; cb < COLS / 16u; cb += 2) {
+                    const uint32_t c0 = chalf * COLS + cb * 16u;
                     uint32_t r0[16], r1[16];
-                    tmem_ld_x16(tmem_base + lane_base + mb * 256u + c0, r0);
-                    tmem_ld_x16(tmem_base + lane_base + mb * 256u + c0 + 16u, r1);
+                    tmem_ld_x16(tmem_base + lane_base + mb * TILE + c0, r0);
+                    tmem_ld_x16(tmem_base + lane_base + mb * TILE + c0 + 16u, r1);
                     tmem_wait_ld();
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                        slab[lane * SLAB_LD + cb * 16u + j] = ((__uint_as_float(r0[j]) * fa) * col_factor[c0 + j]) * rs;
-                        slab[lane * SLAB_LD + cb * 16u + 16u + j] =
+                        slab[lane * LD + cb * 16u + j] = ((__uint_as_float(r0[j]) * fa) * col_factor[c0 + j]) * rs;
+                        slab[lane * LD + cb * 16u + 16u + j] =
                             ((__uint_as_float(r1[j]) * fa) * col_factor[c0 + 16u + j]) * rs;
                     }
                 }
                 __syncwarp();
-                store_block_from_slab(p, slab, m_first, tile_n * 256u + chalf * 128u, lane);
+                store_block_from_slab<COLS>(p, C, slab, m_first, tile_n * TILE + chalf * COLS, lane);
                 __syncwarp();  // the slab is rewritten for the second row block
             }
         }
@@ -308,7 +316,7 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (*abort_flag) __nanosleep(200000);
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, 512);
+        tmem_dealloc(tmem_base, TMEM_COLS);
     }
 }
 
@@ -354,7 +362,9 @@ gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t nchunks = (p.kblocks + 1u) >> 1;
+    // kb_per_split is even: a slice holds whole chunks
+    const uint32_t kb_first = blockIdx.z * p.kb_per_split, kb_end = min(p.kblocks, kb_first + p.kb_per_split);
+    const uint32_t nchunks = (kb_end - kb_first + 1u) >> 1;
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < CK_SLOTS; ++s) {
@@ -388,7 +398,7 @@ gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             prefetch_tmap(&map_a);
             prefetch_tmap(&map_b);
             uint32_t slot = 0, ph = 0;
-            for (uint32_t kb = 0; kb < p.kblocks; ++kb) {
+            for (uint32_t kb = kb_first; kb < kb_end; ++kb) {
                 if (!mbar_wait(smem_u32(&bar_empty[slot]), ph ^ 1u, abort_flag)) {
                     gemm_fail(p.status, abort_flag, ST_TIMEOUT_EMPTY, kb);
                     break;
@@ -426,7 +436,7 @@ gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 }
                 tc_fence_after();
                 const uint32_t d = tmem_base + set * 256u;
-                const uint32_t nkb = min(2u, p.kblocks - 2u * c);
+                const uint32_t nkb = min(2u, kb_end - kb_first - 2u * c);
                 // per 32-k slot: its small terms first, then its large ones, and the slot is released
                 for (uint32_t j = 0; j < nkb; ++j) {
                     got = mbar_wait(smem_u32(&bar_full[slot + j]), ph, abort_flag);
@@ -510,11 +520,11 @@ gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             // The pipeline buffers are idle by now (the last commit covered every MMA and every load
             // has been consumed), so each warp turns its 32 x 128 block around in its own slab of them.
             float* slab = reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw))) +
-                          (size_t)(warp - 4u) * SLAB_FLOATS;
+                          (size_t)(warp - 4u) * (32u * 129u);
 #pragma unroll
-            for (int i = 0; i < 128; ++i) slab[lane * SLAB_LD + i] = sum[i];
+            for (int i = 0; i < 128; ++i) slab[lane * 129u + i] = sum[i];
             __syncwarp();
-            store_block_from_slab(p, slab, tile_m * 128u + q * 32u, n0, lane);
+            store_block_from_slab<128>(p, p.C + blockIdx.z * p.split_stride, slab, tile_m * 128u + q * 32u, n0, lane);
         }
     }
 
@@ -527,23 +537,92 @@ gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     }
 }
 
-// ---- row maxima of fp32 operands (the scales of the packing pass) -------------------------
-// amax[R] = bit pattern of max_k |operand[R][k]|  (non-negative floats order like their bits).
-// Operand rows are source rows: one warp per row, lanes along k.
-__global__ void amax_rows_kernel(const float* __restrict__ src, uint32_t* __restrict__ amax, uint64_t rows,
-                                 uint64_t K, uint64_t ld) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t R = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; R < rows; R += warps) {
-        const uint32_t* row = reinterpret_cast<const uint32_t*>(src + R * ld);
-        uint32_t m = 0;
-#pragma unroll 8
-        for (uint64_t k = lane; k < K; k += 32u) m = max(m, row[k] & 0x7fffffffu);
+// ---- fp32 operands whose rows are source rows: row maxima and packing in one pass ---------------
+// packed[((rb*kblocks + kb)*2 + pl)*128 + r][kk] as below; amax[R] = bit pattern of max_k |operand[R][k]|
+// (non-negative floats order like their bits).  W warps share a row and keep it in registers (32 floats a lane,
+// W * 1024 k) between the maximum and the packing, so the source is read once -- two kernels, the second reading it
+// again, moved 12 bytes per element instead of 8.  Longer rows are walked twice in steps of that length.
+// One launch packs both operands of a product: rows beyond the first operand's belong to the second.
+struct PackRows {
+    const float* src;
+    uint16_t* packed;
+    uint32_t* amax;
+    uint64_t rows, K, ld;
+    uint32_t rowblocks, kblocks;
+};
+template <int W>
+__global__ void __launch_bounds__(256) pack_rows_f32_kernel(const PackRows a, const PackRows b) {
+    __shared__ uint32_t row_max[8];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, part = warp % W;
+    constexpr uint32_t SPAN = W * 1024u;
+    const uint64_t rows_a = (uint64_t)a.rowblocks * 128u, total = rows_a + (uint64_t)b.rowblocks * 128u;
+    for (uint64_t row0 = (uint64_t)blockIdx.x * (8u / W); row0 < total; row0 += (uint64_t)gridDim.x * (8u / W)) {
+        const uint64_t i = row0 + warp / W;  // 8 / W divides 128: a CTA's rows belong to one operand
+        const bool first = i < rows_a;
+        const PackRows& o = first ? a : b;
+        const uint64_t R = first ? i : i - rows_a, span_k = (uint64_t)o.kblocks * 32u;
+        const float* src = o.src + R * o.ld;
+        const bool live = R < o.rows, vec = (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
+        float x[4][8];
+        auto load = [&](uint64_t base) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (lane == 0) amax[R] = m;
+            for (uint32_t j = 0; j < 4; ++j) {
+                const uint64_t k = base + (part * 4u + j) * 256u + lane * 8u;
+                if (live && vec && k + 8u <= o.K) {
+                    const float4 lo = __ldg(reinterpret_cast<const float4*>(src + k));
+                    const float4 hi = __ldg(reinterpret_cast<const float4*>(src + k) + 1);
+                    x[j][0] = lo.x; x[j][1] = lo.y; x[j][2] = lo.z; x[j][3] = lo.w;
+                    x[j][4] = hi.x; x[j][5] = hi.y; x[j][6] = hi.z; x[j][7] = hi.w;
+                } else {
+#pragma unroll
+                    for (uint32_t e = 0; e < 8; ++e) x[j][e] = (live && k + e < o.K) ? __ldg(src + k + e) : 0.0f;
+                }
+            }
+        };
+        uint32_t m = 0;
+        for (uint64_t base = 0; base < o.K; base += SPAN) {
+            load(base);
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j)
+#pragma unroll
+                for (uint32_t e = 0; e < 8; ++e) m = max(m, __float_as_uint(x[j][e]) & 0x7fffffffu);
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
+        if (W > 1) {
+            if (lane == 0) row_max[warp] = m;
+            __syncthreads();
+#pragma unroll
+            for (uint32_t w = 0; w < W; ++w) m = max(m, row_max[warp / W * W + w]);
+            __syncthreads();
+        }
+        if (live && part == 0 && lane == 0) o.amax[R] = m;
+        const float up = row_scale_up(m);
+        uint16_t* out = o.packed + ((R >> 7) * o.kblocks * 256u + (R & 127u)) * 32u;
+        for (uint64_t base = 0; base < span_k; base += SPAN) {
+            if (o.K > SPAN) load(base);
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+                const uint64_t k = base + (part * 4u + j) * 256u + lane * 8u;
+                if (k >= span_k) continue;
+                uint32_t hi[4], lo[4];
+#pragma unroll
+                for (uint32_t e = 0; e < 4; ++e) {
+                    const float u = x[j][2 * e] * up, v = x[j][2 * e + 1] * up;  // exact: a power of two, below 2^15
+                    const __half2 h = __floats2half2_rn(u, v);
+                    const __half2 l = __floats2half2_rn(u - __low2float(h), v - __high2float(h));  // exact differences
+                    hi[e] = *reinterpret_cast<const uint32_t*>(&h);
+                    lo[e] = *reinterpret_cast<const uint32_t*>(&l);
+                }
+                uint16_t* dst = out + (k >> 5) * (256u * 32u) + (k & 31u);
+                *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4*>(dst + 128u * 32u) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            }
+        }
     }
 }
+
+// ---- transposed fp32 operands -------------------------------------------------------------------
 // Operand rows are source columns (the operand is the transpose): threads along the columns,
 // blockIdx.y walks chunks of source rows; amax must be zero before the launch.
 __global__ void amax_cols_kernel(const float* __restrict__ src, uint32_t* __restrict__ amax, uint64_t rows,
@@ -559,17 +638,15 @@ __global__ void amax_cols_kernel(const float* __restrict__ src, uint32_t* __rest
 }
 
 // ---- packing ---------------------------------------------------------------------------
-// packed[((rb*kblocks + kb)*NPL + pl)*128 + r][kk]  (16-bit), r < 128, kk < 32:
+// packed[((rb*kblocks + kb)*planes + pl)*128 + r][kk]  (16-bit), r < 128, kk < 32:
 //   operand row  R = rb*128 + r,  k = kb*32 + kk;
 //   value = src[R*ld + k]  (TRANS = false)  or  src[k*ld + R]  (TRANS = true: the operand is the
 //   transpose of the row-major source), zero outside [rows x K].
-// In: float (NPL = 2: the value times its row's power-of-two scale, as fp16 hi / lo planes) or a
-// 16-bit type copied as is (NPL = 1).
-template <typename In, int NPL, bool TRANS>
-__global__ void pack_kernel(const In* __restrict__ src, uint16_t* __restrict__ packed,
-                            const uint32_t* __restrict__ amax, uint64_t rows,
+// 16-bit types, copied as they are.
+template <bool TRANS>
+__global__ void pack_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ packed, uint64_t rows,
                             uint64_t K, uint64_t ld, uint32_t rowblocks, uint32_t kblocks) {
-    // one thread = 8 consecutive k of one operand row (a 16-byte store per plane)
+    // one thread = 8 consecutive k of one operand row (a 16-byte store)
     const uint64_t total = (uint64_t)rowblocks * kblocks * 128u * 4u;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total;
          i += (uint64_t)gridDim.x * blockDim.x) {
@@ -596,40 +673,21 @@ __global__ void pack_kernel(const In* __restrict__ src, uint16_t* __restrict__ p
             rb = TRANS ? rest % rowblocks : rest / kblocks;
         }
         const uint64_t R = rb * 128u + r, k0 = (uint64_t)kb * 32u + oct * 8u;
-        uint16_t hi[8], lo[8];
-        float up = 1.0f;
-        if constexpr (sizeof(In) == 4) up = R < rows ? row_scale_up(amax[R]) : 1.0f;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            hi[e] = 0;
-            lo[e] = 0;
-            if (R < rows && k0 + e < K) {
-                const In x = TRANS ? src[(k0 + e) * ld + R] : src[R * ld + k0 + e];
-                if constexpr (sizeof(In) == 4) {
-                    const float xs = x * up;  // exact: a power of two, |xs| < 2^15
-                    const __half h = __float2half_rn(xs);
-                    const __half l = __float2half_rn(xs - __half2float(h));  // the difference is exact
-                    hi[e] = __half_as_ushort(h);
-                    lo[e] = __half_as_ushort(l);
-                } else {
-                    hi[e] = *reinterpret_cast<const uint16_t*>(&x);
-                }
-            }
-        }
-        uint16_t* dst = packed + ((((rb * kblocks + kb) * NPL) * 128u + r) * 32u + oct * 8u);
         uint4 o;
-        o.x = hi[0] | ((uint32_t)hi[1] << 16);
-        o.y = hi[2] | ((uint32_t)hi[3] << 16);
-        o.z = hi[4] | ((uint32_t)hi[5] << 16);
-        o.w = hi[6] | ((uint32_t)hi[7] << 16);
-        *reinterpret_cast<uint4*>(dst) = o;
-        if (NPL == 2) {
-            o.x = lo[0] | ((uint32_t)lo[1] << 16);
-            o.y = lo[2] | ((uint32_t)lo[3] << 16);
-            o.z = lo[4] | ((uint32_t)lo[5] << 16);
-            o.w = lo[6] | ((uint32_t)lo[7] << 16);
-            *reinterpret_cast<uint4*>(dst + 128u * 32u) = o;
+        const uint16_t* from = src + R * ld + k0;
+        if (!TRANS && R < rows && k0 + 8u <= K && (reinterpret_cast<uintptr_t>(from) & 15u) == 0) {
+            o = __ldg(reinterpret_cast<const uint4*>(from));
+        } else {
+            uint16_t v[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                v[e] = (R < rows && k0 + e < K) ? (TRANS ? src[(k0 + e) * ld + R] : from[e]) : (uint16_t)0;
+            o.x = v[0] | ((uint32_t)v[1] << 16);
+            o.y = v[2] | ((uint32_t)v[3] << 16);
+            o.z = v[4] | ((uint32_t)v[5] << 16);
+            o.w = v[6] | ((uint32_t)v[7] << 16);
         }
+        *reinterpret_cast<uint4*>(packed + (((rb * kblocks + kb) * 128u + r) * 32u + oct * 8u)) = o;
     }
 }
 
@@ -678,6 +736,47 @@ __global__ void __launch_bounds__(256) pack_trans_f32_kernel(const float* __rest
     }
 }
 
+// ---- sum of the partial products of a split contraction ------------------------------------------
+// C (+)= ((sum_z partial[z]) * scale_a[m] * scale_b[n]) * alpha * row_scale[m], slices added in their order.  One CTA
+// per 32 x 32 block; symmetric products hold (and write) the blocks on or above the diagonal and turn each around in
+// shared memory for its second copy.
+__global__ void __launch_bounds__(256) reduce_splits_kernel(const float* __restrict__ partial, uint32_t splits,
+                                                            const GemmParams p) {
+    __shared__ float turn[32][33];
+    const uint32_t bm = blockIdx.y, bn = blockIdx.x, tx = threadIdx.x & 31u, ty = threadIdx.x >> 5;
+    if (p.symmetric && bn < bm) return;
+    const uint32_t n = bn * 32u + tx;
+    float v[4];
+#pragma unroll
+    for (uint32_t u = 0; u < 4; ++u) {
+        const uint32_t m = bm * 32u + ty + 8u * u;
+        v[u] = 0.0f;
+        if (m >= p.M || n >= p.N || (p.symmetric && n < m)) continue;
+        const float* src = partial + (uint64_t)m * p.N + n;
+        float sum = src[0];
+        for (uint32_t z = 1; z < splits; ++z) sum += src[z * p.split_stride];
+        const float rs = p.alpha * (p.row_scale ? p.row_scale[m] : 1.0f);
+        const float fa = p.amax_a ? row_scale_down(p.amax_a[m]) : 1.0f;
+        const float fb = p.amax_b ? row_scale_down(p.amax_b[n]) : 1.0f;
+        v[u] = ((sum * fa) * fb) * rs;
+        float* dst = p.C + (int64_t)m * p.ldc + n;
+        *dst = p.accumulate ? *dst + v[u] : v[u];
+    }
+    if (!p.symmetric) return;
+#pragma unroll
+    for (uint32_t u = 0; u < 4; ++u) turn[ty + 8u * u][tx] = v[u];
+    __syncthreads();
+    const uint32_t m2 = bm * 32u + tx;
+#pragma unroll
+    for (uint32_t u = 0; u < 4; ++u) {
+        const uint32_t n2 = bn * 32u + ty + 8u * u;
+        if (n2 >= p.N || m2 >= n2) continue;  // strictly below the diagonal of C
+        float* dst = p.C + (int64_t)n2 * p.ldc + m2;
+        const float w = turn[tx][ty + 8u * u];
+        *dst = p.accumulate ? *dst + w : w;
+    }
+}
+
 // ---- host side -----------------------------------------------------------------------------
 Packed packed_geometry(int dtype, int64_t rows, int64_t K) {
     Packed g;
@@ -691,39 +790,55 @@ Packed packed_geometry(int dtype, int64_t rows, int64_t K) {
     return g;
 }
 
-int launch_pack(const void* src, int dtype, bool trans, uint64_t rows, uint64_t K, uint64_t ld,
-                       uint16_t* packed, const Packed& g, int sm_count, cudaStream_t stream) {
-    const uint64_t total = (uint64_t)g.rowblocks * g.kblocks * 512u;
-    uint64_t blocks = (total + 255) / 256;
+static PackRows pack_rows_args(const void* src, uint64_t rows, uint64_t K, uint64_t ld, uint16_t* packed, const Packed& g) {
+    return PackRows{static_cast<const float*>(src), packed, packed_amax(packed, g), rows, K, ld, g.rowblocks, g.kblocks};
+}
+
+// One or two fp32 operands (b.rowblocks = 0: one) whose rows are source rows.
+static int launch_pack_rows(const PackRows& a, const PackRows& b, int sm_count, cudaStream_t stream) {
+    const uint64_t K = a.K > b.K ? a.K : b.K, rows = ((uint64_t)a.rowblocks + b.rowblocks) * 128u;
+    // warps per row: enough to hold it in registers, but not so many that most of their lanes idle
+    const int w = K <= 1024u ? 1 : K <= 2048u ? 2 : K <= 4096u ? 4 : 8;
+    uint64_t blocks = (rows * w + 7) / 8;
     const uint64_t cap = (uint64_t)sm_count * 32;
     if (blocks > cap) blocks = cap;
     const uint32_t nb = (uint32_t)blocks;
+    if (w == 1) pack_rows_f32_kernel<1><<<nb, 256, 0, stream>>>(a, b);
+    else if (w == 2) pack_rows_f32_kernel<2><<<nb, 256, 0, stream>>>(a, b);
+    else if (w == 4) pack_rows_f32_kernel<4><<<nb, 256, 0, stream>>>(a, b);
+    else pack_rows_f32_kernel<8><<<nb, 256, 0, stream>>>(a, b);
+    TB_CUDA(cudaGetLastError());
+    return TB_OK;
+}
+
+int launch_pack(const void* src, int dtype, bool trans, uint64_t rows, uint64_t K, uint64_t ld,
+                uint16_t* packed, const Packed& g, int sm_count, cudaStream_t stream) {
+    if (dtype == TB_F32 && !trans)
+        return launch_pack_rows(pack_rows_args(src, rows, K, ld, packed, g), PackRows{}, sm_count, stream);
     if (dtype == TB_F32) {
         const float* s = static_cast<const float*>(src);
         uint32_t* amax = packed_amax(packed, g);
-        if (trans) {
-            TB_CUDA(cudaMemsetAsync(amax, 0, (size_t)g.rowblocks * 128u * sizeof(uint32_t), stream));
-            const uint32_t bx = (uint32_t)((rows + 255) / 256);
-            uint64_t by = ((uint64_t)sm_count * 16 + bx - 1) / bx;  // about 16 CTAs per SM in all
-            if (by > (K + 63) / 64) by = (K + 63) / 64;
-            if (by > 65535) by = 65535;
-            const uint64_t chunk = (K + by - 1) / by;
-            amax_cols_kernel<<<dim3(bx, (uint32_t)((K + chunk - 1) / chunk)), 256, 0, stream>>>(s, amax, rows, K, ld, chunk);
-            uint64_t tb = (uint64_t)g.rowblocks * g.kblocks;
-            if (tb > (uint64_t)sm_count * 16) tb = (uint64_t)sm_count * 16;
-            pack_trans_f32_kernel<<<(uint32_t)tb, 256, 0, stream>>>(s, packed, amax, rows, K, ld, g.rowblocks, g.kblocks);
-        } else {
-            uint64_t ab = (rows + 7) / 8;  // eight warps (rows) per CTA
-            if (ab > cap) ab = cap;
-            amax_rows_kernel<<<(uint32_t)ab, 256, 0, stream>>>(s, amax, rows, K, ld);
-            pack_kernel<float, 2, false><<<nb, 256, 0, stream>>>(s, packed, amax, rows, K, ld, g.rowblocks, g.kblocks);
-        }
+        TB_CUDA(cudaMemsetAsync(amax, 0, (size_t)g.rowblocks * 128u * sizeof(uint32_t), stream));
+        const uint32_t bx = (uint32_t)((rows + 255) / 256);
+        uint64_t by = ((uint64_t)sm_count * 16 + bx - 1) / bx;  // about 16 CTAs per SM in all
+        if (by > (K + 63) / 64) by = (K + 63) / 64;
+        if (by > 65535) by = 65535;
+        const uint64_t chunk = (K + by - 1) / by;
+        amax_cols_kernel<<<dim3(bx, (uint32_t)((K + chunk - 1) / chunk)), 256, 0, stream>>>(s, amax, rows, K, ld, chunk);
+        uint64_t tb = (uint64_t)g.rowblocks * g.kblocks;
+        if (tb > (uint64_t)sm_count * 16) tb = (uint64_t)sm_count * 16;
+        pack_trans_f32_kernel<<<(uint32_t)tb, 256, 0, stream>>>(s, packed, amax, rows, K, ld, g.rowblocks, g.kblocks);
     } else {
+        const uint64_t total = (uint64_t)g.rowblocks * g.kblocks * 512u;
+        uint64_t blocks = (total + 255) / 256;
+        const uint64_t cap = (uint64_t)sm_count * 32;
+        if (blocks > cap) blocks = cap;
+        const uint32_t nb = (uint32_t)blocks;
         const uint16_t* s = static_cast<const uint16_t*>(src);
         if (trans)
-            pack_kernel<uint16_t, 1, true><<<nb, 256, 0, stream>>>(s, packed, nullptr, rows, K, ld, g.rowblocks, g.kblocks);
+            pack_kernel<true><<<nb, 256, 0, stream>>>(s, packed, rows, K, ld, g.rowblocks, g.kblocks);
         else
-            pack_kernel<uint16_t, 1, false><<<nb, 256, 0, stream>>>(s, packed, nullptr, rows, K, ld, g.rowblocks, g.kblocks);
+            pack_kernel<false><<<nb, 256, 0, stream>>>(s, packed, rows, K, ld, g.rowblocks, g.kblocks);
     }
     TB_CUDA(cudaGetLastError());
     return TB_OK;
@@ -740,20 +855,74 @@ static int packed_tmap(CUtensorMap* map, const uint16_t* packed, const Packed& g
                        2, packed, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
+// Tile and number of slices of the contraction.  A 256 x 256 (or 128 x 256) tile per CTA leaves most of the 148 SMs
+// idle when the product is small: the Gram of 2048 columns is 36 such tiles however many rows it sums over.  The
+// choice minimises an estimate in microseconds: per wave of CTAs a fixed part (launch, first loads, epilogue) plus the
+// tensor-core time of its k blocks; slicing adds the kernel that sums the slices, which is bound by memory.  The
+// 128 x 128 tile reads twice the operand bytes per flop and is for products of less than about a wave.
+GemmPlan plan_gemm(uint32_t npl, bool chunked, bool symmetric, int64_t M, int64_t N, uint32_t kblocks) {
+    constexpr double SMS = 148.0, SUM_FIXED = 4.0, SUM_BYTES_PER_US = 3.0e6;
+    constexpr uint32_t MAX_SPLITS = 64;
+    constexpr size_t MAX_PARTIAL = 256u << 20;
+    const double tm = (double)((M + 127) / 128), tn2 = (double)((N + 255) / 256), tm2 = (double)((M + 255) / 256);
+    GemmPlan best{2, 1, kblocks, 0};
+    double best_t = 1e300;
+    if (!chunked) {
+        const double tn = (double)((N + 127) / 128), tiles = symmetric ? tm * (tm + 1) / 2 : tm * tn;
+        const double waves = (double)(uint64_t)((tiles + SMS - 1) / SMS);
+        best_t = 5.0 + waves * kblocks * (npl == 2 ? 0.34 : 0.12);
+        best.tile = 1;
+    }
+    const double tiles = chunked ? (symmetric ? tm2 * (tm2 + 1) : tm * tn2) : symmetric ? tm2 * (tm2 + 1) / 2 : tm2 * tn2;
+    const double per_kb = chunked ? 0.48 : npl == 2 ? 0.9 : 0.3;
+    for (uint32_t s = 1; s <= MAX_SPLITS && s <= kblocks; ++s) {
+        const uint32_t per = ((kblocks + s - 1) / s + 1u) & ~1u;  // whole 64-wide chunks
+        const uint32_t used = (kblocks + per - 1) / per;
+        const size_t bytes = used > 1 ? (size_t)used * M * N * sizeof(float) : 0;
+        if (used != s || bytes > MAX_PARTIAL) continue;
+        const double waves = (double)(uint64_t)((tiles * s + SMS - 1) / SMS);
+        double t = waves * (8.0 + per * per_kb);
+        if (s > 1) t += SUM_FIXED + ((double)s * (symmetric ? 0.5 : 1.0) + 1.0) * M * N * 4.0 / SUM_BYTES_PER_US;
+        if (t < best_t) {
+            best_t = t;
+            best = GemmPlan{2, s, s > 1 ? per : kblocks, align_up(bytes, 1024)};
+        }
+    }
+    return best;
+}
+
+template <int NPL, int T>
+static int launch_gemm_nt(const CUtensorMap& map_a, const CUtensorMap& map_b, GemmParams& p, uint32_t splits,
+                          cudaStream_t stream) {
+    constexpr uint32_t stage_bytes = 2u * T * NPL * GTILE_BYTES;
+    // two CTAs of the small tile share an SM
+    p.stages = ((T == 2 ? 200u : 100u) * 1024u) / stage_bytes;
+    if (p.stages > 8) p.stages = 8;
+    const size_t smem = (size_t)p.stages * stage_bytes + 1024u;
+    p.idesc = (p.idesc & 1u) ? idesc_f16(1u, 128u * T) : idesc_f16(0u, 128u * T);
+    auto kern = gemm_nt_kernel<NPL, T>;
+    TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const dim3 grid((p.N + 128u * T - 1) / (128u * T), (p.M + 128u * T - 1) / (128u * T), splits);
+    kern<<<grid, 384, smem, stream>>>(map_a, map_b, p);
+    TB_CUDA(cudaGetLastError());
+    return TB_OK;
+}
+
 // C[M x N] (+)= alpha * row_scale[m] * Apacked . Bpacked^T
 int launch_gemm(int device, cudaStream_t stream, const uint16_t* pa, const Packed& ga,
-                       const uint16_t* pb, const Packed& gb, int dtype, int64_t M, int64_t N, float* C,
-                       int64_t ldc, const float* row_scale, float alpha, int accumulate, int symmetric,
-                       int chunked) {
+                const uint16_t* pb, const Packed& gb, int dtype, int64_t M, int64_t N, float* C,
+                int64_t ldc, const float* row_scale, float alpha, int accumulate, int symmetric,
+                int chunked, float* partial) {
     CUtensorMap map_a, map_b;
     int rc = packed_tmap(&map_a, pa, ga, dtype);
     if (rc != TB_OK) return rc;
     rc = packed_tmap(&map_b, pb, gb, dtype);
     if (rc != TB_OK) return rc;
+    if (ga.scaled != gb.scaled || (chunked && !ga.scaled)) return TB_ERR_BAD_ARG;
+    const GemmPlan pl = plan_gemm(ga.npl, chunked != 0, symmetric != 0, M, N, ga.kblocks);
     GemmParams p;
     p.C = C;
     p.row_scale = row_scale;
-    if (ga.scaled != gb.scaled || (chunked && !ga.scaled)) return TB_ERR_BAD_ARG;
     p.amax_a = ga.scaled ? packed_amax(pa, ga) : nullptr;
     p.amax_b = gb.scaled ? packed_amax(pb, gb) : nullptr;
     p.status = status_ptr(device);
@@ -761,33 +930,46 @@ int launch_gemm(int device, cudaStream_t stream, const uint16_t* pa, const Packe
     p.M = (uint32_t)M;
     p.N = (uint32_t)N;
     p.kblocks = ga.kblocks;
-    p.idesc = idesc_f16(planes_are_fp16(ga, dtype) ? 0u : 1u, 256);
+    p.kb_per_split = pl.kb_per_split;
+    p.split_stride = (uint64_t)M * N;
+    p.idesc = planes_are_fp16(ga, dtype) ? 0u : 1u;  // the element format; the shape is filled in below
     p.alpha = alpha;
     p.accumulate = accumulate;
     p.symmetric = symmetric;
-    if (chunked && ga.npl == 2) {
+    p.mirror = 1;
+    const GemmParams whole = p;
+    if (pl.splits > 1) {  // raw partial sums; the scales and the destination are the last kernel's
+        p.C = partial;
+        p.ldc = N;
+        p.row_scale = nullptr;
+        p.amax_a = p.amax_b = nullptr;
+        p.alpha = 1.0f;
+        p.accumulate = 0;
+        p.mirror = 0;
+    } else {
+        p.split_stride = 0;
+    }
+    if (chunked) {
+        p.idesc = idesc_f16(p.idesc, 256);
+        p.stages = CK_SLOTS;
         const size_t smem = (size_t)CK_SLOTS * CK_SLOT_BYTES + 1024u;
-        dim3 grid((uint32_t)((N + 255) / 256), (uint32_t)((M + 127) / 128), 1);
+        const dim3 grid((uint32_t)((N + 255) / 256), (uint32_t)((M + 127) / 128), pl.splits);
         TB_CUDA(cudaFuncSetAttribute(gemm_nt_chunked_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         gemm_nt_chunked_kernel<<<grid, 384, smem, stream>>>(map_a, map_b, p);
         TB_CUDA(cudaGetLastError());
-        return TB_OK;
-    }
-    const uint32_t stage_bytes = 4u * ga.npl * GTILE_BYTES;
-    p.stages = (200u * 1024u) / stage_bytes;
-    if (p.stages > 8) p.stages = 8;
-    const size_t smem = (size_t)p.stages * stage_bytes + 1024u;
-    dim3 grid((uint32_t)((N + 255) / 256), (uint32_t)((M + 255) / 256), 1);
-    if (ga.npl == 2) {
-        auto kern = gemm_nt_kernel<2>;
-        TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<grid, 384, smem, stream>>>(map_a, map_b, p);
+    } else if (pl.tile == 2) {
+        rc = ga.npl == 2 ? launch_gemm_nt<2, 2>(map_a, map_b, p, pl.splits, stream)
+                         : launch_gemm_nt<1, 2>(map_a, map_b, p, pl.splits, stream);
+        if (rc != TB_OK) return rc;
     } else {
-        auto kern = gemm_nt_kernel<1>;
-        TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<grid, 384, smem, stream>>>(map_a, map_b, p);
+        rc = ga.npl == 2 ? launch_gemm_nt<2, 1>(map_a, map_b, p, 1, stream) : launch_gemm_nt<1, 1>(map_a, map_b, p, 1, stream);
+        if (rc != TB_OK) return rc;
     }
-    TB_CUDA(cudaGetLastError());
+    if (pl.splits > 1) {
+        const dim3 grid((uint32_t)((N + 31) / 32), (uint32_t)((M + 31) / 32), 1);
+        reduce_splits_kernel<<<grid, 256, 0, stream>>>(partial, pl.splits, whole);
+        TB_CUDA(cudaGetLastError());
+    }
     return TB_OK;
 }
 
@@ -797,7 +979,8 @@ extern "C" {
 
 size_t tb_gemm_nt_workspace_bytes(int dtype, int64_t M, int64_t N, int64_t K) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
-    return tb::packed_geometry(dtype, M, K).bytes + tb::packed_geometry(dtype, N, K).bytes + 1024;
+    const tb::Packed a = tb::packed_geometry(dtype, M, K), b = tb::packed_geometry(dtype, N, K);
+    return a.bytes + b.bytes + tb::plan_gemm(a.npl, false, false, M, N, a.kblocks).partial_bytes + 1024;
 }
 
 int tb_gemm_nt(int device, void* stream_, const void* A, int64_t lda, const void* B, int64_t ldb, int dtype,
@@ -820,16 +1003,23 @@ int tb_gemm_nt(int device, void* stream_, const void* A, int64_t lda, const void
         return TB_ERR_UNSUPPORTED;
     uint16_t* pa = static_cast<uint16_t*>(ws);
     uint16_t* pb = reinterpret_cast<uint16_t*>(static_cast<uint8_t*>(ws) + ga.bytes);
-    rc = launch_pack(A, dtype, false, M, K, lda, pa, ga, sm_count, stream);
-    if (rc != TB_OK) return rc;
-    rc = launch_pack(B, dtype, false, N, K, ldb, pb, gb, sm_count, stream);
-    if (rc != TB_OK) return rc;
-    return launch_gemm(device, stream, pa, ga, pb, gb, dtype, M, N, C, ldc, row_scale, alpha, accumulate, 0, 0);
+    float* partial = reinterpret_cast<float*>(static_cast<uint8_t*>(ws) + ga.bytes + gb.bytes);
+    if (dtype == TB_F32) {
+        rc = launch_pack_rows(pack_rows_args(A, M, K, lda, pa, ga), pack_rows_args(B, N, K, ldb, pb, gb), sm_count, stream);
+        if (rc != TB_OK) return rc;
+    } else {
+        rc = launch_pack(A, dtype, false, M, K, lda, pa, ga, sm_count, stream);
+        if (rc != TB_OK) return rc;
+        rc = launch_pack(B, dtype, false, N, K, ldb, pb, gb, sm_count, stream);
+        if (rc != TB_OK) return rc;
+    }
+    return launch_gemm(device, stream, pa, ga, pb, gb, dtype, M, N, C, ldc, row_scale, alpha, accumulate, 0, 0, partial);
 }
 
 size_t tb_gram_workspace_bytes(int dtype, int64_t n, int64_t k) {
     if (n <= 0 || k <= 0) return 0;
-    return tb::packed_geometry(dtype, k, n).bytes + 1024;
+    const tb::Packed g = tb::packed_geometry(dtype, k, n);
+    return g.bytes + tb::plan_gemm(g.npl, dtype == TB_F32, true, k, k, g.kblocks).partial_bytes + 1024;
 }
 
 int tb_gram(int device, void* stream_, const void* X, int dtype, int64_t n, int64_t k, int64_t ld, float* G,
@@ -852,7 +1042,7 @@ int tb_gram(int device, void* stream_, const void* X, int dtype, int64_t n, int6
     if (rc != TB_OK) return rc;
     // the Gram feeds an inverse, which amplifies its error by the condition number: chunked accumulation
     return launch_gemm(device, stream, px, g, px, g, dtype, k, k, G, ldg, nullptr, 1.0f, accumulate, 1,
-                       dtype == TB_F32 ? 1 : 0);
+                       dtype == TB_F32 ? 1 : 0, reinterpret_cast<float*>(static_cast<uint8_t*>(ws) + g.bytes));
 }
 
 }  // extern "C"

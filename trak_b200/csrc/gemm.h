@@ -25,11 +25,20 @@ Packed packed_geometry(int dtype, int64_t rows, int64_t K);
 int launch_pack(const void* src, int dtype, bool trans, uint64_t rows, uint64_t K, uint64_t ld,
                 uint16_t* packed, const Packed& g, int sm_count, cudaStream_t stream);
 
+// How launch_gemm computes a product: CTA tile (2: 256 wide, 1: 128 wide), slices of the contraction, and the bytes
+// of the slices' partial products, which the caller provides as `partial`.
+struct GemmPlan {
+    int tile;
+    uint32_t splits, kb_per_split;
+    size_t partial_bytes;
+};
+GemmPlan plan_gemm(uint32_t npl, bool chunked, bool symmetric, int64_t M, int64_t N, uint32_t kblocks);
+
 // C[M x N] (+)= alpha * row_scale[m] * Apacked . Bpacked^T  (symmetric: A == B, mirrored stores;
 // chunked: scaled fp32 operands only -- the tensor core accumulates 64 k at a time and the chunks are
 // summed with rounded fp32 adds, for products whose error an inverse will amplify)
 int launch_gemm(int device, cudaStream_t stream, const uint16_t* pa, const Packed& ga, const uint16_t* pb,
                 const Packed& gb, int dtype, int64_t M, int64_t N, float* C, int64_t ldc,
-                const float* row_scale, float alpha, int accumulate, int symmetric, int chunked);
+                const float* row_scale, float alpha, int accumulate, int symmetric, int chunked, float* partial);
 
 }  // namespace tb

@@ -2,18 +2,16 @@
 // the mean absolute entry (the reference's rescale, trak/score_computers.py:160-168).
 //
 // The reference calls torch.linalg.inv (LU).  A + lambda*I is symmetric positive definite, so this
-// goes through Cholesky, all in fp32:
-//   1. two-level right-looking Cholesky A = L L^T: 64-wide steps (panel solve and update as tiled
-//      fp32 kernels) stay inside a 512-wide block column, and everything to the right of it gets
-//      one rank-512 update per block column from the tensor cores (gemm.cu, symmetric, chunked
-//      accumulation); the CTA that updates the first tile of the trailing block factors and inverts
-//      it right away (it is the next diagonal block) while the other CTAs finish the update;
-//   2. W = L^-1 bottom-up: the 64-wide diagonal blocks are inverted with the factorisation, then
-//      neighbouring blocks of size s = 64, 128, ... are merged, W21 = -W22 (L21 W11): all pairs of
-//      one size in two batched fp32 launches up to s = 512, tensor-core GEMMs (gemm.cu, chunked
-//      accumulation) from s = 1024 on;
-//   3. A^-1 = W^T W with the tensor-core GEMM of gemm.cu (symmetric mode, chunked accumulation);
-//   4. mean |entry| with a fixed-order two-pass reduction, then the rescale.
+// goes through Cholesky A = L L^T and W = L^-1, all in fp32, over 512-wide block columns:
+//   1. the diagonal block is factored and inverted at once, in eight 64-wide steps of one cooperative
+//      launch (block_kernel): one step finishes 64 rows of the block's W and updates everything below
+//      them; the CTA that updates the next 64 x 64 diagonal tile factors and inverts it on the spot;
+//   2. below it L21 = A21 W11^T, and to its right A22 -= L21 L21^T: tensor-core GEMMs (gemm.cu, chunked
+//      accumulation), so the long chain of small steps never touches more than 512 x 512;
+//   3. the inverted blocks are merged bottom-up, W21 = -W22 (L21 W11) for block sizes 512, 1024, ...,
+//      with the same GEMMs;
+//   4. A^-1 = W^T W (symmetric mode, chunked accumulation);
+//   5. mean |entry| with a fixed-order two-pass reduction, then the rescale.
 // A non-positive pivot is recorded in the device status word (ST_NOT_SPD).
 #include <algorithm>
 
@@ -23,10 +21,10 @@
 
 namespace tb {
 
-constexpr int NB = 64;      // panel width
-constexpr int OUTER = 512;    // block column of the two-level Cholesky
-constexpr int MERGE_TC_FROM = 1024;  // block size from which the merge products go to the tensor cores
+constexpr int NB = 64;      // tile of the steps inside a block column
+constexpr int OUTER = 512;  // block column
 constexpr int TS = 68;      // padded row length of a shared-memory tile (floats)
+typedef float Tile[NB][TS];
 
 // acc[4][4] += sum_t At[t][ty*4 + i] * Bt[t][tx*4 + j]   (both tiles stored t-major)
 __device__ __forceinline__ void tile_mma(const float (*At)[TS], const float (*Bt)[TS], int ty, int tx,
@@ -43,74 +41,91 @@ __device__ __forceinline__ void tile_mma(const float (*At)[TS], const float (*Bt
     }
 }
 
-// dst[t][i] = src[i*ld + t]  (operand element (i, t) is row-major in global memory), zero outside
-__device__ __forceinline__ void load_tile_T(float (*dst)[TS], const float* src, int64_t ld, int rows, int cols) {
-    for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
-        const int i = e >> 6, t = e & 63;
-        dst[t][i] = (i < rows && t < cols) ? src[(int64_t)i * ld + t] : 0.0f;
-    }
-}
-// dst[t][c] = src[t*ld + c]
-__device__ __forceinline__ void load_tile_N(float (*dst)[TS], const float* src, int64_t ld, int rows, int cols) {
-    for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
-        const int t = e >> 6, c = e & 63;
-        dst[t][c] = (t < rows && c < cols) ? src[(int64_t)t * ld + c] : 0.0f;
+// dst[t][i] = src[i*ld + t] (transposed) or dst[i][t] = src[i*ld + t], zero outside rows x cols.  The first 256 threads; four
+// consecutive elements of a row each where the rows are 16-byte aligned.  A warp covers eight rows x 16 columns, so
+// the transposed stores meet two to a bank.
+template <bool TRANS>
+__device__ __forceinline__ void load_tile(Tile& dst, const float* src, int64_t ld, int rows, int cols) {
+    if (threadIdx.x >= 256u) return;
+    const bool vec = (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+        const int e = it * 256 + (int)threadIdx.x, warp = e >> 5, lane = e & 31;
+        const int i = (warp >> 2) * 8 + (lane & 7), t = (warp & 3) * 16 + (lane >> 3) * 4;
+        float v[4];
+        if (vec && i < rows && t + 4 <= cols) {
+            const float4 x = *reinterpret_cast<const float4*>(src + (int64_t)i * ld + t);
+            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = (i < rows && t + u < cols) ? src[(int64_t)i * ld + t + u] : 0.0f;
+        }
+        if (TRANS) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) dst[t + u][i] = v[u];
+        } else {
+            *reinterpret_cast<float4*>(&dst[i][t]) = make_float4(v[0], v[1], v[2], v[3]);
+        }
     }
 }
 
-__global__ void add_diag_kernel(float* A, int64_t lda, int k, float lambda) {
+// A += lambda I, and zero for the counters that the block columns' CTAs meet at.
+__global__ void prepare_kernel(float* A, int64_t lda, int k, float lambda, uint32_t* counters, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < k) A[(int64_t)i * lda + i] += lambda;
+    if (i < k && lambda != 0.0f) A[(int64_t)i * lda + i] += lambda;
+    if (i < n) counters[i] = 0;
 }
 
-// Factors the jb x jb diagonal block A = L L^T and inverts L in the same sweep; writes L back over the
-// lower triangle and inv(L) (lower, zero above, zero-padded to 64 x 64) to dinv.  256 threads as a
-// 16 x 16 grid, thread (ty, tx) keeping the 4 x 4 piece S[4 ty.., 4 tx..] of the block and the same piece
-// of W (which starts as the identity and ends as inv(L): forward elimination of [L | I]) in registers.
-// The block is walked four columns at a time, two barriers per step instead of two per column (a
-// column-by-column sweep spent 1000 cycles per column, almost all of it waiting: 33 us per block):
-//   1. the thread on the diagonal publishes its 4 x 4 piece D;
-//   2. every thread of piece column q factors D = Ld Ld^T itself (a few dozen operations), turns its
-//      piece into the matching rows of L (B Ld^-T) and publishes them; every thread of piece row q
-//      applies Ld^-1 to its four rows of W, which makes them final, and publishes them;
-//   3. the threads below apply the rank-four updates  S -= L_q L_q^T  (pieces right of column q)
-//      and  W -= L_q W_q  (pieces up to column q; W_q is zero beyond).
-// Rows and columns beyond jb are an identity block.  `buf` is 16 + 2 * 256 floats of shared memory.
-struct Chol4 {
+// Factors the jb x jb diagonal tile S = L L^T (lower triangle used) and inverts L in the same sweep (forward
+// elimination of [L | I]); writes inv(L) (lower, zero above, zero-padded to 64 x 64) to dinv.  STEP_THREADS threads:
+// 256 as a 16 x 16 grid of 4 x 4 pieces in registers, and one more warp, the pivot warp, whose lane l keeps the
+// diagonal piece (l, l).  The tile is walked four columns at a time, piece column q in step q.  Thread (ty, tx) holds
+// a piece of S until step tx and a piece of W = inv(L) from then on (it is zero, or the identity, until its column has
+// been reached), so a step is one rank-four update whichever it is:
+//   1. the pivot warp has factored the diagonal piece q, D = Ld Ld^T, and published Ld;
+//   2. the threads of piece column q turn their pieces into rows of L (B Ld^-T), those of piece row q apply Ld^-1 to
+//      their four rows of W, which makes them final; both publish, one vector per column respectively row of q;
+//   3. the threads below update their pieces, S -= L_q L_q^T and W -= L_q W_q.
+// Beside 2 and 3 the pivot warp applies L_{q-1} to the diagonal pieces, computes the one piece of L_q that the next
+// one needs from what its owner published, updates it and factors it: the chain of four reciprocal square roots is
+// off the other warps' path.  (With S and W pieces updated one after the other in every thread, and the next piece
+// factored after its update by the grid's own diagonal thread, a tile took 9 us.)
+// Rows and columns beyond jb are an identity block.  `buf` is CHOL_FLOATS floats of shared memory outside S.
+constexpr int CHOL_FLOATS = 64 + 3 * 256;
+constexpr int STEP_THREADS = 288;
+struct __align__(16) Chol4 {
     float l10, l20, l30, l21, l31, l32;  // strictly lower part of Ld
     float r0, r1, r2, r3;                // reciprocals of its diagonal
-    float d0, d1, d2, d3;                // its diagonal
-    bool ok;
+    float ok, pad;
 };
+// 1 / sqrt(d) for a normal d; a subnormal one counts as not positive (the inverse would overflow)
 __device__ __forceinline__ float rsqrt_newton(float d) {
-    float r = rsqrtf(d);
-    return r * (1.5f - 0.5f * d * r * r);
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return fmaf(r, fmaf(-(0.5f * d) * r, r, 0.5f), r);
 }
-__device__ __forceinline__ Chol4 chol4(const float* D) {  // D: 4 x 4 row-major, lower part used
+__device__ __forceinline__ Chol4 chol4(const float (&D)[4][4]) {  // lower part used
     Chol4 c;
-    c.ok = true;
-    float p = D[0];
-    c.ok = c.ok && p > 0.0f;
+    float p = D[0][0];
+    bool ok = p >= 1.17549435e-38f;
     c.r0 = rsqrt_newton(p);
-    c.d0 = p * c.r0;
-    c.l10 = D[4] * c.r0;
-    c.l20 = D[8] * c.r0;
-    c.l30 = D[12] * c.r0;
-    p = fmaf(-c.l10, c.l10, D[5]);
-    c.ok = c.ok && p > 0.0f;
+    c.l10 = D[1][0] * c.r0;
+    c.l20 = D[2][0] * c.r0;
+    c.l30 = D[3][0] * c.r0;
+    p = fmaf(-c.l10, c.l10, D[1][1]);
+    ok = ok && p >= 1.17549435e-38f;
     c.r1 = rsqrt_newton(p);
-    c.d1 = p * c.r1;
-    c.l21 = fmaf(-c.l20, c.l10, D[9]) * c.r1;
-    c.l31 = fmaf(-c.l30, c.l10, D[13]) * c.r1;
-    p = fmaf(-c.l21, c.l21, fmaf(-c.l20, c.l20, D[10]));
-    c.ok = c.ok && p > 0.0f;
+    c.l21 = fmaf(-c.l20, c.l10, D[2][1]) * c.r1;
+    c.l31 = fmaf(-c.l30, c.l10, D[3][1]) * c.r1;
+    p = fmaf(-c.l21, c.l21, fmaf(-c.l20, c.l20, D[2][2]));
+    ok = ok && p >= 1.17549435e-38f;
     c.r2 = rsqrt_newton(p);
-    c.d2 = p * c.r2;
-    c.l32 = fmaf(-c.l31, c.l21, fmaf(-c.l30, c.l20, D[14])) * c.r2;
-    p = fmaf(-c.l32, c.l32, fmaf(-c.l31, c.l31, fmaf(-c.l30, c.l30, D[15])));
-    c.ok = c.ok && p > 0.0f;
+    c.l32 = fmaf(-c.l31, c.l21, fmaf(-c.l30, c.l20, D[3][2])) * c.r2;
+    p = fmaf(-c.l32, c.l32, fmaf(-c.l31, c.l31, fmaf(-c.l30, c.l30, D[3][3])));
+    ok = ok && p >= 1.17549435e-38f;
     c.r3 = rsqrt_newton(p);
-    c.d3 = p * c.r3;
+    c.ok = ok ? 1.0f : 0.0f;
+    c.pad = 0.0f;
     return c;
 }
 // x <- Ld^-1 x for one column of four values (forward substitution)
@@ -120,238 +135,299 @@ __device__ __forceinline__ void solve4(const Chol4& c, float& x0, float& x1, flo
     x2 = fmaf(-c.l21, x1, fmaf(-c.l20, x0, x2)) * c.r2;
     x3 = fmaf(-c.l32, x2, fmaf(-c.l31, x1, fmaf(-c.l30, x0, x3))) * c.r3;
 }
-__device__ void chol_block(float* A, int64_t lda, int jb, float* dinv, uint32_t* status, float* buf, int* bad) {
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-    float* diagbuf = buf;                                                  // [4][4]
-    float (*colbuf)[4] = reinterpret_cast<float(*)[4]>(buf + 16);          // [64][4]: rows of L_q
-    float (*rowbuf)[NB] = reinterpret_cast<float(*)[NB]>(buf + 16 + 256);  // [4][64]: rows of W_q
-    float sblk[4][4], wblk[4][4];
-    if (tid == 0) *bad = 0;
+__device__ __forceinline__ float4 row4(const float (&m)[4][4], int a) { return make_float4(m[a][0], m[a][1], m[a][2], m[a][3]); }
+__device__ __forceinline__ Chol4 load_factor(const Chol4* factor) {
+    const float4* f = reinterpret_cast<const float4*>(factor);
+    const float4 f0 = f[0], f1 = f[1], f2 = f[2];
+    return Chol4{f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w, f2.x, f2.y, f2.z, 0.0f};
+}
+__device__ void chol_block(const Tile& S, int jb, float* dinv, uint32_t* status, float* buf) {
+    const int tid = threadIdx.x;
+    Chol4* factor = reinterpret_cast<Chol4*>(buf);                         // [2]: of pieces q and q + 1
+    float4* raw = reinterpret_cast<float4*>(buf + 32);                     // [2][4]: piece (q + 1, q) of S before step q
+    float (*colbufs)[NB] = reinterpret_cast<float(*)[NB]>(buf + 64);       // [2][4][64]: columns of L_q and L_{q-1}
+    float (*rowbuf)[NB] = reinterpret_cast<float(*)[NB]>(buf + 64 + 512);  // [4][64]: rows of W_q
+    static_assert(sizeof(Chol4) <= 16 * sizeof(float), "two factors fit in front of raw");
+    const bool pivot = tid >= 256;
+    // the pivot warp's lane l stands at (l, l); lanes 16 to 31 repeat lane 15 and publish nothing
+    const int ty = pivot ? min(tid - 256, 15) : tid >> 4, tx = pivot ? ty : tid & 15;
+    float x[4][4];
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
             const int i = ty * 4 + a, j = tx * 4 + b;
-            // the diagonal pieces hold both triangles (symmetric), the others only what lies below
-            const bool in = i < jb && j < jb && (j <= i || tx == ty);
-            sblk[a][b] = in ? A[(int64_t)(j <= i ? i : j) * lda + (j <= i ? j : i)] : (i == j ? 1.0f : 0.0f);
-            wblk[a][b] = i == j ? 1.0f : 0.0f;
+            const float unit = i == j ? 1.0f : 0.0f;
+            // the grid's diagonal threads have no piece of S to keep (the pivot warp has): they start with W's identity
+            x[a][b] = (i < jb && j < jb && j <= i && (pivot || tx != ty)) ? S[i][j] : unit;
         }
     const int steps = (jb + 3) >> 2;
-    for (int q = 0; q < steps; ++q) {
-        if (ty == q && tx == q) {
+    bool bad = false;
+    if (tid == 256) {
+        const Chol4 c = chol4(x);
+        bad = c.ok == 0.0f;
+        factor[0] = c;
+    }
+    if (!pivot && ty == 1 && tx == 0) {
+#pragma unroll
+        for (int a = 0; a < 4; ++a) raw[a] = row4(x, a);
+    }
+    // x -= L[ty] . O[tx] with four columns of L and of O
+    auto update = [&](const float (*lcol)[NB], const float (*ocol)[NB]) {
+#pragma unroll
+        for (int cc = 0; cc < 4; ++cc) {
+            const float4 l = *reinterpret_cast<const float4*>(&lcol[cc][ty * 4]);
+            const float4 o = *reinterpret_cast<const float4*>(&ocol[cc][tx * 4]);
+            const float lv[4] = {l.x, l.y, l.z, l.w}, ov[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
             for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) diagbuf[a * 4 + b] = sblk[a][b];
+                for (int b = 0; b < 4; ++b) x[a][b] = fmaf(-lv[a], ov[b], x[a][b]);
         }
+    };
+    for (int q = 0; q < steps; ++q) {
         __syncthreads();
-        if (tx == q || ty == q) {
-            const Chol4 c = chol4(diagbuf);
-            if (ty == q && tx == q && !c.ok) *bad = 1;
-            if (tx == q && ty >= q) {
-                if (ty == q) {  // the diagonal piece becomes Ld
-                    sblk[0][0] = c.d0;
-                    sblk[1][0] = c.l10; sblk[1][1] = c.d1;
-                    sblk[2][0] = c.l20; sblk[2][1] = c.l21; sblk[2][2] = c.d2;
-                    sblk[3][0] = c.l30; sblk[3][1] = c.l31; sblk[3][2] = c.l32; sblk[3][3] = c.d3;
-                    sblk[0][1] = sblk[0][2] = sblk[0][3] = sblk[1][2] = sblk[1][3] = sblk[2][3] = 0.0f;
-                } else {        // rows of L below it: B Ld^-T, i.e. Ld^-1 applied along each row
+        float (*colbuf)[NB] = colbufs + 4 * (q & 1);
+        if (pivot) {
+            if (q + 1 < steps) {  // every lane computes lane q + 1's part; that lane keeps it
+                const Chol4 c = load_factor(factor + (q & 1));
+                const float (*before)[NB] = colbufs + 4 * ((q & 1) ^ 1);
+                float l[4][4], z[4][4];
 #pragma unroll
-                    for (int a = 0; a < 4; ++a) solve4(c, sblk[a][0], sblk[a][1], sblk[a][2], sblk[a][3]);
+                for (int a = 0; a < 4; ++a) {
+                    const float4 v = raw[4 * (q & 1) + a];
+                    l[a][0] = v.x; l[a][1] = v.y; l[a][2] = v.z; l[a][3] = v.w;
+                    solve4(c, l[a][0], l[a][1], l[a][2], l[a][3]);
                 }
+                if (q > 0) update(before, before);
 #pragma unroll
                 for (int a = 0; a < 4; ++a)
-                    *reinterpret_cast<float4*>(colbuf[ty * 4 + a]) =
-                        make_float4(sblk[a][0], sblk[a][1], sblk[a][2], sblk[a][3]);
+#pragma unroll
+                    for (int b = 0; b <= a; ++b)
+                        z[a][b] = fmaf(-l[a][3], l[b][3], fmaf(-l[a][2], l[b][2], fmaf(-l[a][1], l[b][1],
+                                       fmaf(-l[a][0], l[b][0], x[a][b]))));
+                const Chol4 n = chol4(z);
+                if (tid - 256 == q + 1) {
+                    bad = bad || n.ok == 0.0f;
+                    factor[(q + 1) & 1] = n;
+                }
             }
-            if (ty == q) {      // four rows of W become final: Ld^-1 applied down each column
+            continue;
+        }
+        if ((tx == q && ty > q) || (ty == q && tx <= q)) {
+            // rows of L: B Ld^-T, i.e. Ld^-1 applied along each row of the piece; rows of W: along each column
+            const Chol4 c = load_factor(factor + (q & 1));
+            const bool of_l = ty > q;
+            float y[4][4];
 #pragma unroll
-                for (int b = 0; b < 4; ++b) solve4(c, wblk[0][b], wblk[1][b], wblk[2][b], wblk[3][b]);
+            for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int a = 0; a < 4; ++a)
-                    *reinterpret_cast<float4*>(&rowbuf[a][tx * 4]) =
-                        make_float4(wblk[a][0], wblk[a][1], wblk[a][2], wblk[a][3]);
+                for (int b = 0; b < 4; ++b) y[a][b] = of_l ? x[a][b] : x[b][a];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) solve4(c, y[a][0], y[a][1], y[a][2], y[a][3]);
+            float (*dst)[NB] = of_l ? colbuf : rowbuf;
+            const int at = of_l ? ty * 4 : tx * 4;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                *reinterpret_cast<float4*>(&dst[b][at]) = make_float4(y[0][b], y[1][b], y[2][b], y[3][b]);
+#pragma unroll
+                for (int a = 0; a < 4; ++a) x[b][a] = of_l ? 0.0f : y[a][b];  // a piece of W (zero so far) from here on
             }
         }
-        __syncthreads();
-        if (ty > q) {
-            float li[4][4];
+        asm volatile("barrier.cta.sync 1, 256;" ::: "memory");  // the grid only
+        if (ty > q && tx < ty) {
+            update(colbuf, tx > q ? colbuf : rowbuf);
+            if (ty == q + 2 && tx == q + 1) {
 #pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                const float4 v = *reinterpret_cast<const float4*>(colbuf[ty * 4 + a]);
-                li[a][0] = v.x; li[a][1] = v.y; li[a][2] = v.z; li[a][3] = v.w;
-            }
-            if (tx > q && tx <= ty) {
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    const float4 v = *reinterpret_cast<const float4*>(colbuf[tx * 4 + b]);
-#pragma unroll
-                    for (int a = 0; a < 4; ++a)
-                        sblk[a][b] = fmaf(-li[a][3], v.w, fmaf(-li[a][2], v.z, fmaf(-li[a][1], v.y,
-                                          fmaf(-li[a][0], v.x, sblk[a][b]))));
-                }
-            }
-            if (tx <= q) {
-#pragma unroll
-                for (int cc = 0; cc < 4; ++cc) {
-                    const float4 v = *reinterpret_cast<const float4*>(&rowbuf[cc][tx * 4]);
-#pragma unroll
-                    for (int a = 0; a < 4; ++a) {
-                        wblk[a][0] = fmaf(-li[a][cc], v.x, wblk[a][0]);
-                        wblk[a][1] = fmaf(-li[a][cc], v.y, wblk[a][1]);
-                        wblk[a][2] = fmaf(-li[a][cc], v.z, wblk[a][2]);
-                        wblk[a][3] = fmaf(-li[a][cc], v.w, wblk[a][3]);
-                    }
-                }
+                for (int a = 0; a < 4; ++a) raw[4 * ((q + 1) & 1) + a] = row4(x, a);
             }
         }
     }
+    if (!pivot) {
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const int i = ty * 4 + a;
+            float w[4];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) w[b] = (i < jb && tx * 4 + b <= i) ? x[a][b] : 0.0f;
+            *reinterpret_cast<float4*>(dinv + i * NB + tx * 4) = make_float4(w[0], w[1], w[2], w[3]);
+        }
+    }
+    if (bad) atomicCAS(status, 0u, (uint32_t)ST_NOT_SPD);
+}
+
+// Step j of a block column's diagonal block (kb x kb, kb <= 512), in tiles of 64.  Before the step, rows i >= j hold
+// R[i, c] for c < j (what is left of the identity's elimination, W's future rows) and S[i, l] for l >= j (what is
+// left of A), and D = inv(chol(S[j, j])) is known.  The step makes row j of W final,
+//     W[j, c] = D R[j, c],   W[j, j] = D,
+// and with P_i = S[i, j] D^T (the rows of L) updates every row i > j:
+//     S[i, l] -= P_i P_l^T (j < l <= i),   R[i, c] -= P_i W[j, c] (c < j),   R[i, j] = -P_i D.
+// One CTA per tile, each computing the P and W tiles it needs itself (three 64^3 products, 1.1 us each on one SM,
+// instead of another meeting point and a trip through memory).  Rows i > j go from X to Y (tiles are read by many
+// CTAs, so they are not updated in place); W's rows go to `block`, the matrix itself, with zeros right of the diagonal.
+__device__ void block_tile(float* step_smem, const float* X, int64_t ldx, float* Y, int64_t ldy, float* block,
+                           int64_t lda, int kb, int j, int i, int c, const float* D, float* D_next, uint32_t* status) {
+    Tile& Dt = *reinterpret_cast<Tile*>(step_smem);                // Dt[t][c] = D[c][t]
+    Tile& T0 = *reinterpret_cast<Tile*>(step_smem + NB * TS);
+    Tile& T1 = *reinterpret_cast<Tile*>(step_smem + 2 * NB * TS);
+    Tile& T2 = *reinterpret_cast<Tile*>(step_smem + 3 * NB * TS);
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    const bool grid16 = tid < 256;  // the ninth warp is the factorisation's pivot warp
+    const int rows = min(NB, kb - i * NB), jw = min(NB, kb - j * NB), cols = min(NB, kb - c * NB);
+    float acc[4][4] = {};
+    if (i == j) {  // row j of W
+        if (c < j) {
+            load_tile<true>(Dt, D, NB, NB, NB);
+            load_tile<false>(T0, X + (int64_t)j * NB * ldx + c * NB, ldx, rows, NB);
+            __syncthreads();
+            if (grid16) tile_mma(Dt, T0, ty, tx, acc);
+        }
+        if (!grid16) return;
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const int r = ty * 4 + a, q = tx * 4 + b;
+                if (r < rows && q < cols)
+                    block[(int64_t)(j * NB + r) * lda + c * NB + q] = c < j ? acc[a][b] : c == j ? D[r * NB + q] : 0.0f;
+            }
+        return;
+    }
+    // P_i, t-major, into T0
+    load_tile<true>(Dt, D, NB, NB, NB);
+    load_tile<true>(T1, X + (int64_t)i * NB * ldx + j * NB, ldx, rows, jw);
+    if (c > j && c != i)
+        load_tile<true>(T2, X + (int64_t)c * NB * ldx + j * NB, ldx, cols, jw);
+    else if (c < j)
+        load_tile<false>(T2, X + (int64_t)j * NB * ldx + c * NB, ldx, jw, NB);
+    else if (c == j)
+        load_tile<false>(T2, D, NB, NB, NB);
+    // this CTA's own tile, in flight during the products
+    float own[4][4];
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-            const int i = ty * 4 + a, j = tx * 4 + b;
-            const bool in = i < jb && j <= i;
-            if (in) A[(int64_t)i * lda + j] = sblk[a][b];
-            dinv[i * NB + j] = in ? wblk[a][b] : 0.0f;
+            const int r = ty * 4 + a, q = tx * 4 + b;
+            own[a][b] = (grid16 && c != j && r < rows && q < cols) ? X[(int64_t)(i * NB + r) * ldx + c * NB + q] : 0.0f;
         }
     __syncthreads();
-    if (tid == 0 && *bad) atomicCAS(status, 0u, (uint32_t)ST_NOT_SPD);
-}
-
-__global__ void __launch_bounds__(256) chol_diag_kernel(float* A, int64_t lda, int jb, float* dinv,
-                                                        uint32_t* status) {
-    __shared__ __align__(16) float buf[16 + 2 * 256];
-    __shared__ int bad;
-    chol_block(A, lda, jb, dinv, status, buf, &bad);
-}
-
-// MODE 0 (Cholesky panel):  X[i, c] <- sum_t X[i, t] * D[c, t]      (X * D^T, in place)
-// MODE 1 (inverse, step 1): T[i, c] <- sum_t X[i, t] * D[t, c]      (X * D, to a separate buffer)
-// X is r x jb (leading dimension ldx), D is the zero-padded 64 x 64 block; one CTA per 64 rows.
-template <int MODE>
-__global__ void __launch_bounds__(256) panel_kernel(float* X, int64_t ldx, int r, int jb, const float* D,
-                                                    float* T, int64_t ldt) {
-    __shared__ __align__(16) float At[NB][TS];
-    __shared__ __align__(16) float Bt[NB][TS];
-    const int i0 = blockIdx.x * NB;
-    const int rows = min(NB, r - i0);
-    load_tile_T(At, X + (int64_t)i0 * ldx, ldx, rows, jb);
-    if (MODE == 0)
-        load_tile_T(Bt, D, NB, NB, NB);  // Bt[t][c] = D[c][t]
-    else
-        load_tile_N(Bt, D, NB, NB, NB);  // Bt[t][c] = D[t][c]
-    __syncthreads();
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    float acc[4][4] = {};
-    tile_mma(At, Bt, ty, tx, acc);
-    __syncthreads();  // everyone has read X before anyone overwrites it (MODE 0 is in place)
-    float* out = MODE == 0 ? X : T;
-    const int64_t ldo = MODE == 0 ? ldx : ldt;
+    if (grid16) {
+        tile_mma(T1, Dt, ty, tx, acc);
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+        for (int b = 0; b < 4; ++b)
+            *reinterpret_cast<float4*>(&T0[tx * 4 + b][ty * 4]) = make_float4(acc[0][b], acc[1][b], acc[2][b], acc[3][b]);
+    }
+    if (c != i && c != j) {  // the other operand: P_c (t-major) or W[j, c], over T1
+        float other[4][4] = {};
+        if (!grid16) {
+        } else if (c > j)
+            tile_mma(T2, Dt, ty, tx, other);
+        else
+            tile_mma(Dt, T2, ty, tx, other);
+        __syncthreads();
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int ii = ty * 4 + i, c = tx * 4 + j;
-            if (ii < rows && c < jb) out[(int64_t)(i0 + ii) * ldo + c] = acc[i][j];
+        for (int b = 0; b < 4 && grid16; ++b) {
+            if (c > j)
+                *reinterpret_cast<float4*>(&T1[tx * 4 + b][ty * 4]) =
+                    make_float4(other[0][b], other[1][b], other[2][b], other[3][b]);
+            else
+                *reinterpret_cast<float4*>(&T1[ty * 4 + b][tx * 4]) =
+                    make_float4(other[b][0], other[b][1], other[b][2], other[b][3]);
         }
-}
-
-// Trailing update of a Cholesky step:  C[i, j] -= sum_t P[i, t] * P[j, t]  for the tiles on or below
-// the diagonal in the first gridDim.x tile columns of the r x r trailing block; P is the r x jb panel
-// (same leading dimension as C).  The CTA of tile (0, 0) then holds the next diagonal block in its
-// final state and factors it on the spot (dinv_next = where its inverse goes), overlapping with the
-// other CTAs' updates.
-__global__ void __launch_bounds__(256) syrk_update_kernel(float* C, const float* P, int64_t ld, int r, int jb,
-                                                          float* dinv_next, uint32_t* status) {
-    if (blockIdx.x > blockIdx.y) return;  // tile column > tile row: upper part, not needed
-    __shared__ __align__(16) float At[NB][TS];
-    __shared__ __align__(16) float Bt[NB][TS];
-    __shared__ int bad;
-    const int i0 = blockIdx.y * NB, j0 = blockIdx.x * NB;
-    const int rows = min(NB, r - i0), cols = min(NB, r - j0);
-    load_tile_T(At, P + (int64_t)i0 * ld, ld, rows, jb);
-    load_tile_T(Bt, P + (int64_t)j0 * ld, ld, cols, jb);
+    }
     __syncthreads();
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    float acc[4][4] = {};
-    tile_mma(At, Bt, ty, tx, acc);
+    if (grid16) {
+        float upd[4][4] = {};
+        tile_mma(T0, c == i ? T0 : c == j ? T2 : T1, ty, tx, upd);
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+        for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int ii = ty * 4 + i, jj = tx * 4 + j;
-            if (ii < rows && jj < cols) C[(int64_t)(i0 + ii) * ld + j0 + jj] -= acc[i][j];
+            for (int b = 0; b < 4; ++b) {
+                const int r = ty * 4 + a, q = tx * 4 + b;
+                own[a][b] -= upd[a][b];
+                if (r < rows && q < cols) Y[(int64_t)(i * NB + r) * ldy + c * NB + q] = own[a][b];
+            }
+    }
+    if (D_next) {
+        if (grid16) {
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+                *reinterpret_cast<float4*>(&Dt[ty * 4 + a][tx * 4]) =
+                    make_float4(own[a][0], own[a][1], own[a][2], own[a][3]);
         }
-    if (blockIdx.x == 0 && blockIdx.y == 0 && dinv_next != nullptr) {
-        __syncthreads();  // the tile is complete in global memory and the operand tiles are free
-        chol_block(C, ld, rows, dinv_next, status, &At[0][0], &bad);
+        __syncthreads();
+        chol_block(Dt, rows, D_next, status, &T1[0][0]);
     }
 }
 
-// Inverse of the triangular factor, bottom-up.  At block size s the matrix holds, in every aligned
-// diagonal block of size s, the finished inverse W of that block of L (upper triangle zero).  Pair p
-// joins the blocks at base = 2 s p:  W11 = [base, base + s),  W22 = the s2 = min(s, k - base - s)
-// rows after it, and the block below W11 still holds L21.  The inverse of the joined block needs
-//     W21 = - W22 (L21 W11),
-// computed as T = L21 W11 (STEP 0, into Tbuf[row][0..s)) and W21 = -W22 T (STEP 1, over L21).
-// One CTA per 64 x 64 tile of the result, blockIdx.z = pair; the triangles skip their zero tiles.
-template <int STEP>
-__global__ void __launch_bounds__(256) tri_merge_kernel(float* A, int64_t lda, int k, int s, float* Tbuf) {
-    __shared__ __align__(16) float At[NB][TS];
-    __shared__ __align__(16) float Bt[NB][TS];
-    const int base = (int)blockIdx.z * 2 * s;
-    const int s2 = min(s, k - base - s);
-    const int i0 = blockIdx.y * NB, j0 = blockIdx.x * NB;
-    if (s2 <= 0 || i0 >= s2) return;
-    const int rows = min(NB, s2 - i0), cols = min(NB, s - j0);
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    float acc[4][4] = {};
-    const float* L21 = A + (int64_t)(base + s) * lda + base;
-    const float* W11 = A + (int64_t)base * lda + base;
-    const float* W22 = A + (int64_t)(base + s) * lda + base + s;
-    const float* T = Tbuf + (int64_t)(base + s) * s;
-    // STEP 0: t runs over the columns of L21 / rows of W11, and W11[t, j] = 0 for t < j
-    // STEP 1: t runs over the columns of W22 / rows of T,   and W22[i, t] = 0 for t > i
-    const int t_first = STEP == 0 ? j0 : 0;
-    const int t_end = STEP == 0 ? s : min(s2, i0 + NB);
-    for (int t0 = t_first; t0 < t_end; t0 += NB) {
-        const int tc = min(NB, t_end - t0);
-        if (STEP == 0) {
-            load_tile_T(At, L21 + (int64_t)i0 * lda + t0, lda, rows, tc);
-            load_tile_N(Bt, W11 + (int64_t)t0 * lda + j0, lda, tc, cols);
-        } else {
-            load_tile_T(At, W22 + (int64_t)i0 * lda + t0, lda, rows, tc);
-            load_tile_N(Bt, T + (int64_t)t0 * s + j0, s, tc, cols);
-        }
-        __syncthreads();
-        tile_mma(At, Bt, ty, tx, acc);
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int ii = ty * 4 + i, jj = tx * 4 + j;
-            if (ii < rows && jj < cols) {
-                if (STEP == 0)
-                    Tbuf[(int64_t)(base + s + i0 + ii) * s + j0 + jj] = acc[i][j];
-                else
-                    A[(int64_t)(base + s + i0 + ii) * lda + base + j0 + jj] = -acc[i][j];
+// All CTAs of a cooperative launch meet: true when they have all arrived `round` times (1, 2, ...).  Bounded.
+__device__ bool meet(uint32_t* counter, uint32_t round, uint32_t* status) {
+    __shared__ uint32_t met;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const uint32_t target = round * gridDim.x;
+        uint32_t seen;
+        __threadfence();
+        atomicAdd(counter, 1u);
+        const uint64_t t0 = globaltimer_ns();
+        bool late = false;
+        for (uint32_t n = 1;; ++n) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
+            if (seen >= target) break;
+            if ((n & 255u) == 0 && globaltimer_ns() - t0 > WAIT_LIMIT_NS) {
+                late = true;
+                break;
             }
         }
+        __threadfence();
+        if (late && atomicCAS(status, 0u, (uint32_t)ST_TIMEOUT_ACC) == 0u) status[1] = blockIdx.x;
+        met = late ? 0u : 1u;
+    }
+    __syncthreads();
+    return met != 0;
 }
 
-// Every 64-wide diagonal block <- its inverse from the factorisation (lower, zero above); one CTA each.
-__global__ void write_diag_inverse_kernel(float* A, int64_t lda, int k, const float* dinv) {
-    const int j0 = blockIdx.x * NB, jb = min(NB, k - j0);
-    const float* D = dinv + (size_t)blockIdx.x * NB * NB;
-    for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
-        const int i = e >> 6, j = e & 63;
-        if (i < jb && j < jb) A[(int64_t)(j0 + i) * lda + j0 + j] = D[e];
+// Factors and inverts a diagonal block (kb x kb): CTA 0 takes the first tile and then every step's next diagonal tile,
+// the others share the rest.  A cooperative launch of about as many CTAs as the largest step has tiles; meeting through
+// a counter in the L2 between steps instead of one launch per step took the 512-wide block from 155 to 125 us.
+__global__ void __launch_bounds__(STEP_THREADS) block_kernel(float* block, int64_t lda, int kb, float* blocks, float* dinv,
+                                                             uint32_t* counter, uint32_t* status) {
+    extern __shared__ __align__(16) float step_smem[];
+    const int nt = (kb + NB - 1) / NB;
+    if (blockIdx.x == 0) {
+        Tile& S = *reinterpret_cast<Tile*>(step_smem);
+        load_tile<false>(S, block, lda, min(NB, kb), min(NB, kb));
+        __syncthreads();
+        chol_block(S, min(NB, kb), dinv, status, step_smem + NB * TS);
+    }
+    for (int j = 0; j < nt; ++j) {
+        if (!meet(counter, j + 1, status)) return;
+        const float* X = j == 0 ? block : blocks + (size_t)((j - 1) & 1) * OUTER * OUTER;
+        float* Y = blocks + (size_t)(j & 1) * OUTER * OUTER;
+        const int64_t ldx = j == 0 ? lda : OUTER;
+        const float* D = dinv + (size_t)j * NB * NB;
+        if (blockIdx.x == 0) {
+            if (j + 1 < nt)
+                block_tile(step_smem, X, ldx, Y, OUTER, block, lda, kb, j, j + 1, j + 1, D,
+                           dinv + (size_t)(j + 1) * NB * NB, status);
+            continue;
+        }
+        int tiles = nt;  // row j of W, and the tiles (i, c), c <= i, of the rows below
+        for (int i = j + 1; i < nt; ++i) tiles += i + 1;
+        for (int t = (int)blockIdx.x - 1; t < tiles; t += (int)gridDim.x - 1) {
+            int i = j, c = t;
+            if (t >= nt) {
+                c = t - nt;
+                for (i = j + 1; c > i; ++i) c -= i + 1;
+                if (i == j + 1 && c == j + 1) continue;  // CTA 0's
+            }
+            block_tile(step_smem, X, ldx, Y, OUTER, block, lda, kb, j, i, c, D, nullptr, status);
+            __syncthreads();
+        }
     }
 }
+
 // The three whole-matrix passes below walk rows per CTA and columns per thread (no index division), four
 // columns at a time where the rows are 16-byte aligned.
 __device__ __forceinline__ bool rows_are_vec4(const float* A, int64_t lda, int k) {
@@ -418,36 +494,51 @@ __global__ void scale_by_inverse_kernel(float* A, int64_t lda, int k, const floa
     }
 }
 
-struct InvLayout {
-    size_t dinv, partial, mean, scratch, total;
+// C[m x n] = alpha * A[m x kk] . B[n x kk]^T (+ C) with chunked accumulation, operands packed first: the bytes of the
+// packed operands (0 rows: B is A, symmetric) and of the partial products behind them.
+struct Product {
+    Packed a, b;
+    size_t partial;
+    size_t bytes() const { return a.bytes + b.bytes + partial; }
 };
-// Scratch of the merge at block size s (first block s rows, second block s2 rows): both packed
-// operands of the larger product and T; all of it is free again before W^T W is packed.
-static size_t merge_scratch_bytes(int64_t s, int64_t s2) {
-    const size_t pa = std::max(packed_geometry(TB_F32, s2, s).bytes, packed_geometry(TB_F32, s2, s2).bytes);
-    const size_t pb = packed_geometry(TB_F32, s, std::max(s, s2)).bytes;
-    return pa + pb + align_up((size_t)s2 * s * sizeof(float), 1024);
+static Product product(int64_t m, int64_t n, int64_t kk, bool symmetric) {
+    Product p;
+    p.a = packed_geometry(TB_F32, m, kk);
+    p.b = symmetric ? Packed{} : packed_geometry(TB_F32, n, kk);
+    p.partial = plan_gemm(2, true, symmetric, m, n, p.a.kblocks).partial_bytes;
+    return p;
 }
+
+struct InvLayout {
+    size_t dinv, blocks, partial, mean, counters, scratch, total;
+};
 static InvLayout inv_layout(int64_t k) {
     InvLayout l;
-    const size_t nblk = (size_t)((k + NB - 1) / NB);
     size_t off = 0;
     l.dinv = off;
-    off += align_up(nblk * NB * NB * sizeof(float), 256);
+    off += (OUTER / NB) * NB * NB * sizeof(float);
+    l.blocks = off;  // the two copies of a diagonal block that its steps alternate between
+    off += 2u * OUTER * OUTER * sizeof(float);
     l.partial = off;
     off += align_up(RED_BLOCKS * sizeof(double), 256);
     l.mean = off;
     off += 256;
-    l.scratch = off;
-    size_t need = packed_geometry(TB_F32, k, k).bytes;  // also covers the r x OUTER panels of the Cholesky
-    for (int64_t s = NB; s < k; s *= 2) {
-        if (s < MERGE_TC_FROM)
-            need = std::max(need, align_up((size_t)k * s * sizeof(float), 1024));  // T of every pair
-        else
-            need = std::max(need, merge_scratch_bytes(s, std::min<int64_t>(s, k - s)));
+    l.counters = off;
+    off += align_up((size_t)((k + OUTER - 1) / OUTER) * sizeof(uint32_t), 256);
+    l.scratch = off = align_up(off, 1024);
+    size_t need = product(k, k, k, true).bytes();  // W^T W
+    for (int64_t o = 0; o + OUTER < k; o += OUTER) {
+        need = std::max(need, product(k - o - OUTER, OUTER, OUTER, false).bytes());
+        need = std::max(need, product(k - o - OUTER, k - o - OUTER, OUTER, true).bytes());
     }
-    off += need;
-    l.total = off + 1024;
+    for (int64_t s = OUTER; s < k; s *= 2)
+        for (int64_t b0 = 0; b0 + s < k; b0 += 2 * s) {
+            const int64_t s2 = std::min<int64_t>(s, k - b0 - s);
+            // L21 W11 and its fp32 result, then W22 times that
+            const size_t t = align_up((size_t)s2 * s * sizeof(float), 1024);
+            need = std::max(need, t + std::max(product(s2, s, s, false).bytes(), product(s2, s, s2, false).bytes()));
+        }
+    l.total = off + need + 1024;
     return l;
 }
 
@@ -473,103 +564,85 @@ int tb_spd_inverse(int device, void* stream_, float* A, int64_t k, int64_t lda, 
     const InvLayout l = inv_layout(k);
     uint8_t* base = static_cast<uint8_t*>(ws);
     float* dinv = reinterpret_cast<float*>(base + l.dinv);
+    float* blocks = reinterpret_cast<float*>(base + l.blocks);
     double* partial = reinterpret_cast<double*>(base + l.partial);
     float* mean = reinterpret_cast<float*>(base + l.mean);
     uint8_t* scratch = base + l.scratch;
     const int K = (int)k;
-    const int nblk = (K + NB - 1) / NB;
 
-    if (lambda != 0.0f) add_diag_kernel<<<(K + 255) / 256, 256, 0, stream>>>(A, lda, K, lambda);
-
-    // 1. Cholesky (lower triangle of A becomes L); dinv[b] = inverse of the b-th diagonal block of L.
-    //    Two levels: inside a block column of OUTER columns the 64-wide steps update only that block
-    //    column (fp32 tiles); what lies to its right gets one rank-OUTER update per block column from
-    //    the tensor cores (symmetric chunked GEMM, alpha = -1, accumulating).  The first diagonal block
-    //    of a block column is factored by its own launch, every other one inside the update that
-    //    completes it.
-    for (int o0 = 0; o0 < K; o0 += OUTER) {
-        const int o1 = o0 + OUTER < K ? o0 + OUTER : K;  // end of this block column
-        chol_diag_kernel<<<1, 256, 0, stream>>>(A + (int64_t)o0 * lda + o0, lda, o1 - o0 < NB ? o1 - o0 : NB,
-                                                dinv + (size_t)(o0 / NB) * NB * NB, status_ptr(device));
-        for (int j0 = o0; j0 < o1; j0 += NB) {
-            const int b = j0 / NB, jb = K - j0 < NB ? K - j0 : NB, r = K - j0 - jb;
-            if (r <= 0) break;
-            float* A21 = A + (int64_t)(j0 + jb) * lda + j0;
-            const int rt = (r + NB - 1) / NB;
-            panel_kernel<0><<<rt, 256, 0, stream>>>(A21, lda, r, jb, dinv + (size_t)b * NB * NB, nullptr, 0);
-            const int wt = (o1 - j0 - jb + NB - 1) / NB;  // tile columns left in the block column
-            if (wt > 0)
-                syrk_update_kernel<<<dim3(wt, rt), 256, 0, stream>>>(A + (int64_t)(j0 + jb) * lda + j0 + jb, A21, lda, r, jb,
-                                                                      dinv + (size_t)(b + 1) * NB * NB, status_ptr(device));
+    // operands of one product at `at`, then the product itself
+    auto multiply = [&](const Product& pr, uint8_t* at, const float* a, int64_t ld_a, bool trans_a, const float* b,
+                        int64_t ld_b, bool trans_b, int64_t m, int64_t n, int64_t kk, float* c, int64_t ld_c, float alpha,
+                        int accumulate) -> int {
+        const bool symmetric = b == nullptr;
+        uint16_t* pa = reinterpret_cast<uint16_t*>(at);
+        uint16_t* pb = symmetric ? pa : reinterpret_cast<uint16_t*>(at + pr.a.bytes);
+        int r = launch_pack(a, TB_F32, trans_a, (uint64_t)m, (uint64_t)kk, (uint64_t)ld_a, pa, pr.a, sm_count, stream);
+        if (r != TB_OK) return r;
+        if (!symmetric) {
+            r = launch_pack(b, TB_F32, trans_b, (uint64_t)n, (uint64_t)kk, (uint64_t)ld_b, pb, pr.b, sm_count, stream);
+            if (r != TB_OK) return r;
         }
-        const int64_t r = K - o1;
+        return launch_gemm(device, stream, pa, pr.a, pb, symmetric ? pr.a : pr.b, TB_F32, m, n, c, ld_c, nullptr, alpha,
+                           accumulate, symmetric ? 1 : 0, 1, reinterpret_cast<float*>(at + pr.a.bytes + pr.b.bytes));
+    };
+
+    uint32_t* counters = reinterpret_cast<uint32_t*>(base + l.counters);
+    prepare_kernel<<<(K + 255) / 256, 256, 0, stream>>>(A, lda, K, lambda, counters, (K + OUTER - 1) / OUTER);
+
+    // 1. Block columns: the diagonal block becomes its W, the block below it L21, what is right of both is updated.
+    constexpr size_t step_smem = 4u * NB * TS * sizeof(float);
+    TB_CUDA(cudaFuncSetAttribute(block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)step_smem));
+    for (int64_t o = 0; o < k; o += OUTER) {
+        const int kb = (int)std::min<int64_t>(OUTER, k - o), nt = (kb + NB - 1) / NB;
+        float* block = A + o * lda + o;
+        int tiles = nt;  // of the first step, the largest
+        for (int i = 1; i < nt; ++i) tiles += i + 1;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeCooperative;
+        attr.val.cooperative = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)std::min(tiles + 1, sm_count));
+        cfg.blockDim = dim3(STEP_THREADS);
+        cfg.dynamicSmemBytes = step_smem;
+        cfg.stream = stream;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        TB_CUDA(cudaLaunchKernelEx(&cfg, block_kernel, block, lda, kb, blocks, dinv, counters + o / OUTER,
+                                   status_ptr(device)));
+        const int64_t r = k - o - kb;
         if (r > 0) {
-            // A22 -= L21 L21^T with L21 = the r x (o1 - o0) block below this block column's diagonal block
-            const int64_t w = o1 - o0;
-            uint16_t* packed = reinterpret_cast<uint16_t*>(scratch);
-            const Packed g = packed_geometry(TB_F32, r, w);
-            rc = launch_pack(A + (int64_t)o1 * lda + o0, TB_F32, false, (uint64_t)r, (uint64_t)w, (uint64_t)lda, packed, g,
-                             sm_count, stream);
+            float* A21 = A + (o + kb) * lda + o;
+            float* A22 = A + (o + kb) * lda + o + kb;
+            rc = multiply(product(r, kb, kb, false), scratch, A21, lda, false, block, lda, false, r, kb, kb, A21, lda, 1.0f, 0);
             if (rc != TB_OK) return rc;
-            rc = launch_gemm(device, stream, packed, g, packed, g, TB_F32, r, r, A + (int64_t)o1 * lda + o1, lda, nullptr,
-                             -1.0f, 1, 1, 1);
+            rc = multiply(product(r, r, kb, true), scratch, A21, lda, false, nullptr, 0, false, r, r, kb, A22, lda, -1.0f, 1);
             if (rc != TB_OK) return rc;
         }
     }
     TB_CUDA(cudaGetLastError());
 
-    // 2. W = L^-1: clear the upper triangle, put the inverted diagonal blocks in place, then merge
-    //    neighbouring blocks of size 64, 128, ...
-    zero_upper_kernel<<<sm_count * 8, 256, 0, stream>>>(A, lda, K);
-    write_diag_inverse_kernel<<<nblk, 256, 0, stream>>>(A, lda, K, dinv);
-    for (int64_t s = NB; s < k; s *= 2) {
-        const int pairs = (int)((k + 2 * s - 1) / (2 * s));
-        if (s < MERGE_TC_FROM) {
-            float* Tbuf = reinterpret_cast<float*>(scratch);
-            const dim3 grid((unsigned)(s / NB), (unsigned)(s / NB), (unsigned)pairs);
-            tri_merge_kernel<0><<<grid, 256, 0, stream>>>(A, lda, K, (int)s, Tbuf);
-            tri_merge_kernel<1><<<grid, 256, 0, stream>>>(A, lda, K, (int)s, Tbuf);
-            continue;
-        }
-        for (int pr = 0; pr < pairs; ++pr) {
-            const int64_t b0 = (int64_t)pr * 2 * s, s2 = std::min<int64_t>(s, k - b0 - s);
-            if (s2 <= 0) continue;
+    // 2. W = L^-1: blocks of OUTER are inverted and clear above the diagonal; clear the rest, then merge neighbours.
+    if (k > OUTER) zero_upper_kernel<<<sm_count * 8, 256, 0, stream>>>(A, lda, K);
+    for (int64_t s = OUTER; s < k; s *= 2)
+        for (int64_t b0 = 0; b0 + s < k; b0 += 2 * s) {
+            const int64_t s2 = std::min<int64_t>(s, k - b0 - s);
             float* W11 = A + b0 * lda + b0;
             float* L21 = A + (b0 + s) * lda + b0;
             float* W22 = A + (b0 + s) * lda + b0 + s;
-            const Packed g_l21 = packed_geometry(TB_F32, s2, s), g_w22 = packed_geometry(TB_F32, s2, s2);
-            const Packed g_w11t = packed_geometry(TB_F32, s, s), g_tt = packed_geometry(TB_F32, s, s2);
-            const size_t pa_bytes = std::max(g_l21.bytes, g_w22.bytes), pb_bytes = std::max(g_w11t.bytes, g_tt.bytes);
-            uint16_t* pa = reinterpret_cast<uint16_t*>(scratch);
-            uint16_t* pb = reinterpret_cast<uint16_t*>(scratch + pa_bytes);
-            float* T = reinterpret_cast<float*>(scratch + pa_bytes + pb_bytes);
-            // T[s2 x s] = L21 . W11 = L21 . (W11^T)^T
-            rc = launch_pack(L21, TB_F32, false, (uint64_t)s2, (uint64_t)s, (uint64_t)lda, pa, g_l21, sm_count, stream);
+            float* T = reinterpret_cast<float*>(scratch);
+            uint8_t* at = scratch + align_up((size_t)s2 * s * sizeof(float), 1024);
+            // T[s2 x s] = L21 . W11 = L21 . (W11^T)^T;  W21 = - W22 . (T^T)^T, written over L21
+            rc = multiply(product(s2, s, s, false), at, L21, lda, false, W11, lda, true, s2, s, s, T, s, 1.0f, 0);
             if (rc != TB_OK) return rc;
-            rc = launch_pack(W11, TB_F32, true, (uint64_t)s, (uint64_t)s, (uint64_t)lda, pb, g_w11t, sm_count, stream);
-            if (rc != TB_OK) return rc;
-            rc = launch_gemm(device, stream, pa, g_l21, pb, g_w11t, TB_F32, s2, s, T, s, nullptr, 1.0f, 0, 0, 1);
-            if (rc != TB_OK) return rc;
-            // W21[s2 x s] = - W22 . T = - W22 . (T^T)^T, written over L21
-            rc = launch_pack(W22, TB_F32, false, (uint64_t)s2, (uint64_t)s2, (uint64_t)lda, pa, g_w22, sm_count, stream);
-            if (rc != TB_OK) return rc;
-            rc = launch_pack(T, TB_F32, true, (uint64_t)s, (uint64_t)s2, (uint64_t)s, pb, g_tt, sm_count, stream);
-            if (rc != TB_OK) return rc;
-            rc = launch_gemm(device, stream, pa, g_w22, pb, g_tt, TB_F32, s2, s, L21, lda, nullptr, -1.0f, 0, 0, 1);
+            rc = multiply(product(s2, s, s2, false), at, W22, lda, false, T, s, true, s2, s, s2, L21, lda, -1.0f, 0);
             if (rc != TB_OK) return rc;
         }
-    }
     TB_CUDA(cudaGetLastError());
 
-    // 3. A^-1 = W^T W (full symmetric result written over A; the operand was packed first)
-    {
-        uint16_t* packed = reinterpret_cast<uint16_t*>(scratch);
-        const Packed g = packed_geometry(TB_F32, k, k);
-        rc = launch_pack(A, TB_F32, true, (uint64_t)k, (uint64_t)k, (uint64_t)lda, packed, g, sm_count, stream);
-        if (rc != TB_OK) return rc;
-        rc = launch_gemm(device, stream, packed, g, packed, g, TB_F32, k, k, A, lda, nullptr, 1.0f, 0, 1, 1);
-        if (rc != TB_OK) return rc;
-    }
+    // 3. A^-1 = W^T W (full symmetric result written over A; the operand is packed first)
+    rc = multiply(product(k, k, k, true), scratch, A, lda, true, nullptr, 0, false, k, k, k, A, lda, 1.0f, 0);
+    if (rc != TB_OK) return rc;
 
     // 4. mean |entry| and the reference's rescale
     if (rescale_by_mean_abs || mean_abs_out) {
