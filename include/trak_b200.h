@@ -58,6 +58,9 @@ const char *tb_last_cuda_error(void);
  * *detail, if not null, receives the raw status word. */
 int tb_device_status(int device, uint32_t *detail);
 
+/* The same after waiting for the work queued on `stream` only. */
+int tb_stream_status(int device, void *stream, uint32_t *detail);
+
 /* Failure-path self-test (no counterpart in the reference): launches one CTA that waits, with the
  * same bounded wait the pipelines use, on a barrier nothing arrives at.  After `limit_ms`
  * (1..2000) the wait gives up and records the time-out; the next tb_device_status returns

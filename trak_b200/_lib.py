@@ -7,6 +7,8 @@ import ctypes
 import os
 import threading
 
+import torch
+
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libtrakb200.so")
 
@@ -36,6 +38,7 @@ SIGNATURES = {
     "tb_strerror": (ctypes.c_char_p, [_i]),
     "tb_last_cuda_error": (ctypes.c_char_p, []),
     "tb_device_status": (_i, [_i, ctypes.POINTER(_u32)]),
+    "tb_stream_status": (_i, [_i, _vp, ctypes.POINTER(_u32)]),
     "tb_selftest_wait_timeout": (_i, [_i, _vp, _u32]),
     "tb_selftest_sqrt": (_i, [_i, _vp, ctypes.c_uint64, ctypes.c_uint64, _vp]),
     "tb_project_workspace_bytes": (_sz, [_i, _i64, _i64, _u32, _u32]),
@@ -67,6 +70,8 @@ SIGNATURES = {
 def lib():
     """The loaded library.  Raises ImportError (with the build hint) when absent."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is None:
             if not os.path.exists(LIB_PATH):
@@ -117,3 +122,35 @@ def device_status(device: int) -> None:
     if rc == TB_ERR_DEVICE_TIMEOUT:
         raise DeviceTimeout(f"trak_b200: a bounded wait inside a kernel ran out (status {detail.value})")
     check(rc)
+
+
+def stream_status(device: int, stream: int) -> None:
+    """Waits for the work queued on ``stream`` and raises what ``device_status`` would raise for it."""
+    detail = _u32(0)
+    rc = lib().tb_stream_status(device, stream, ctypes.byref(detail))
+    if rc == TB_ERR_DEVICE_TIMEOUT:
+        raise DeviceTimeout(f"trak_b200: a bounded wait inside a kernel ran out (status {detail.value})")
+    check(rc)
+
+
+def current_stream(device: torch.device) -> int:
+    """The handle of torch's current stream on ``device``."""
+    return torch._C._cuda_getCurrentRawStream(device.index)
+
+
+class on_device:
+    """``torch.cuda.device(device)`` that costs next to nothing where ``device`` is the current one already."""
+
+    __slots__ = ("guard",)
+
+    def __init__(self, device: torch.device):
+        self.guard = None if torch.cuda.current_device() == device.index else torch.cuda.device(device)
+
+    def __enter__(self):
+        if self.guard is not None:
+            self.guard.__enter__()
+
+    def __exit__(self, *exc):
+        if self.guard is not None:
+            self.guard.__exit__(*exc)
+        return False

@@ -1,7 +1,10 @@
 // Library-wide pieces of the C ABI: version, error text, device selection,
 // the per-device status word and tensor-map encoding.
+#include <algorithm>
 #include <cstring>
 #include <mutex>
+#include <utility>
+#include <vector>
 
 #include "host_util.h"
 #include "ptx.cuh"
@@ -77,6 +80,43 @@ __global__ void selftest_wait_kernel(uint32_t* status, uint64_t limit_ns) {
         }
     }
     __syncthreads();
+}
+
+// Pinned words that status reads land in: taken for the length of a read, made as they are needed, at most as many as
+// threads ever read at once.
+static std::mutex g_words_mu;
+static std::vector<uint32_t*> g_words;
+
+static int take_word(uint32_t** word) {
+    {
+        std::lock_guard<std::mutex> lk(g_words_mu);
+        if (!g_words.empty()) {
+            *word = g_words.back();
+            g_words.pop_back();
+            return TB_OK;
+        }
+    }
+    TB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(word), 4 * sizeof(uint32_t), cudaHostAllocPortable));
+    return TB_OK;
+}
+static void give_word(uint32_t* word) {
+    std::lock_guard<std::mutex> lk(g_words_mu);
+    g_words.push_back(word);
+}
+
+int set_smem_limit(const void* kernel, int device) {
+    static std::mutex mu;
+    static std::vector<std::pair<const void*, uint64_t>> done;  // devices on which the kernel's limit has been raised
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = std::find_if(done.begin(), done.end(), [&](const auto& d) { return d.first == kernel; });
+    if (it != done.end() && (it->second >> device & 1u)) return TB_OK;
+    cudaFuncAttributes attr;
+    TB_CUDA(cudaFuncGetAttributes(&attr, kernel));
+    TB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(SMEM_PER_CTA - attr.sharedSizeBytes)));
+    if (it == done.end()) it = done.insert(done.end(), {kernel, 0});
+    it->second |= 1ull << device;
+    return TB_OK;
 }
 
 typedef CUresult (*encode_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -175,6 +215,24 @@ int tb_device_status(int device, uint32_t* detail) {
         TB_CUDA(cudaMemset(tb::status_ptr(device), 0, sizeof(host)));
         return host[0] == 6u ? TB_ERR_NOT_SPD : TB_ERR_DEVICE_TIMEOUT;
     }
+    return TB_OK;
+}
+
+int tb_stream_status(int device, void* stream_, uint32_t* detail) {
+    int rc = tb::select_device(device, nullptr);
+    if (rc != TB_OK) return rc;
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    uint32_t* word = nullptr;
+    rc = tb::take_word(&word);
+    if (rc != TB_OK) return rc;
+    // the read is queued behind the stream's work, so one wait serves both
+    cudaError_t e = cudaMemcpyAsync(word, tb::status_ptr(device), sizeof(uint32_t), cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    const uint32_t code = *word;
+    if (e != cudaSuccess) TB_CUDA(e);  // the word may still be written to: it is not handed out again
+    tb::give_word(word);
+    if (code != 0) return tb_device_status(device, detail);
+    if (detail) *detail = 0;
     return TB_OK;
 }
 

@@ -892,7 +892,7 @@ GemmPlan plan_gemm(uint32_t npl, bool chunked, bool symmetric, int64_t M, int64_
 }
 
 template <int NPL, int T>
-static int launch_gemm_nt(const CUtensorMap& map_a, const CUtensorMap& map_b, GemmParams& p, uint32_t splits,
+static int launch_gemm_nt(int device, const CUtensorMap& map_a, const CUtensorMap& map_b, GemmParams& p, uint32_t splits,
                           cudaStream_t stream) {
     constexpr uint32_t stage_bytes = 2u * T * NPL * GTILE_BYTES;
     // two CTAs of the small tile share an SM
@@ -901,7 +901,7 @@ static int launch_gemm_nt(const CUtensorMap& map_a, const CUtensorMap& map_b, Ge
     const size_t smem = (size_t)p.stages * stage_bytes + 1024u;
     p.idesc = (p.idesc & 1u) ? idesc_f16(1u, 128u * T) : idesc_f16(0u, 128u * T);
     auto kern = gemm_nt_kernel<NPL, T>;
-    TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (const int e = set_smem_limit((const void*)kern, device)) return e;
     const dim3 grid((p.N + 128u * T - 1) / (128u * T), (p.M + 128u * T - 1) / (128u * T), splits);
     kern<<<grid, 384, smem, stream>>>(map_a, map_b, p);
     TB_CUDA(cudaGetLastError());
@@ -954,15 +954,15 @@ int launch_gemm(int device, cudaStream_t stream, const uint16_t* pa, const Packe
         p.stages = CK_SLOTS;
         const size_t smem = (size_t)CK_SLOTS * CK_SLOT_BYTES + 1024u;
         const dim3 grid((uint32_t)((N + 255) / 256), (uint32_t)((M + 127) / 128), pl.splits);
-        TB_CUDA(cudaFuncSetAttribute(gemm_nt_chunked_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (const int e = set_smem_limit((const void*)gemm_nt_chunked_kernel, device)) return e;
         gemm_nt_chunked_kernel<<<grid, 384, smem, stream>>>(map_a, map_b, p);
         TB_CUDA(cudaGetLastError());
     } else if (pl.tile == 2) {
-        rc = ga.npl == 2 ? launch_gemm_nt<2, 2>(map_a, map_b, p, pl.splits, stream)
-                         : launch_gemm_nt<1, 2>(map_a, map_b, p, pl.splits, stream);
+        rc = ga.npl == 2 ? launch_gemm_nt<2, 2>(device, map_a, map_b, p, pl.splits, stream)
+                         : launch_gemm_nt<1, 2>(device, map_a, map_b, p, pl.splits, stream);
         if (rc != TB_OK) return rc;
     } else {
-        rc = ga.npl == 2 ? launch_gemm_nt<2, 1>(map_a, map_b, p, 1, stream) : launch_gemm_nt<1, 1>(map_a, map_b, p, 1, stream);
+        rc = ga.npl == 2 ? launch_gemm_nt<2, 1>(device, map_a, map_b, p, 1, stream) : launch_gemm_nt<1, 1>(device, map_a, map_b, p, 1, stream);
         if (rc != TB_OK) return rc;
     }
     if (pl.splits > 1) {

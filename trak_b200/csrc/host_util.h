@@ -39,6 +39,10 @@ int encode_tmap(CUtensorMap* map, CUtensorMapDataType dt, uint32_t rank, const v
                 const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box,
                 CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B);
 
+// Lets `kernel` use all of an SM's shared memory on `device` (the current one); once per kernel and device.
+constexpr int SMEM_PER_CTA = 227 * 1024;
+int set_smem_limit(const void* kernel, int device);
+
 // Events armed by tb_profile_events for this thread (null when not armed); taking clears them.
 void take_profile_events(cudaEvent_t* before, cudaEvent_t* after);
 

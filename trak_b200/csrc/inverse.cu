@@ -592,7 +592,7 @@ int tb_spd_inverse(int device, void* stream_, float* A, int64_t k, int64_t lda, 
 
     // 1. Block columns: the diagonal block becomes its W, the block below it L21, what is right of both is updated.
     constexpr size_t step_smem = 4u * NB * TS * sizeof(float);
-    TB_CUDA(cudaFuncSetAttribute(block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)step_smem));
+    if (const int e = set_smem_limit((const void*)block_kernel, device)) return e;
     for (int64_t o = 0; o < k; o += OUTER) {
         const int kb = (int)std::min<int64_t>(OUTER, k - o), nt = (kb + NB - 1) / NB;
         float* block = A + o * lda + o;

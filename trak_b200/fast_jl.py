@@ -25,6 +25,8 @@ _MAX_CACHED_WORKSPACES = 8  # per process; streams come and go, their workspaces
 
 
 def _u32(name, v):
+    if type(v) is int and 0 <= v <= 0xFFFFFFFF:
+        return v
     if isinstance(v, bool) or not isinstance(v, int):
         try:
             v = v.__index__()
@@ -128,8 +130,8 @@ def project(input, N, seed, num_feature_tiles, proj_type, *, alpha=1.0, out=None
                 or out.shape[1] != N or out.stride(1) != 1:
             raise RuntimeError("out must be a float32 [B, N] tensor on the input's device")
     dt = _DTYPES[input.dtype]
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
+    with _lib.on_device(dev):
+        stream = _lib.current_stream(dev)
         nbytes = l.tb_project_workspace_bytes(dt, B, F, N, max(num_feature_tiles, 1))
         ws = _workspace(dev, stream, max(nbytes, 256))
         if matrix is not None:
@@ -146,7 +148,7 @@ def project(input, N, seed, num_feature_tiles, proj_type, *, alpha=1.0, out=None
                               ws.numel())
         _lib.check(rc)
         if _STRICT if strict is None else strict:
-            _lib.device_status(dev.index)
+            _lib.stream_status(dev.index, stream)
     return out
 
 
@@ -189,8 +191,8 @@ def project_segments(tensors, N, seed, num_feature_tiles, proj_type, *, alpha=1.
     elif out.device != dev or out.dtype != torch.float32 or tuple(out.shape) != (B, N) or out.stride(1) != 1:
         raise RuntimeError("out must be a float32 [B, N] tensor on the gradients' device")
     dt = _DTYPES[dtype]
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
+    with _lib.on_device(dev):
+        stream = _lib.current_stream(dev)
         nbytes = l.tb_project_segments_workspace_bytes(dt, B, F, N, max(num_feature_tiles, 1), len(tensors))
         ws = _workspace(dev, stream, max(nbytes, 256))
         if matrix is not None:
@@ -207,7 +209,7 @@ def project_segments(tensors, N, seed, num_feature_tiles, proj_type, *, alpha=1.
                                        ws.data_ptr(), ws.numel())
         _lib.check(rc)
         if _STRICT if strict is None else strict:
-            _lib.device_status(dev.index)
+            _lib.stream_status(dev.index, stream)
     return out
 
 

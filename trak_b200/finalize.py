@@ -166,7 +166,7 @@ class ScoreFinalizer:
                 pending = (r0, block, event)
             if pending is not None:
                 flush(pending)
-            _lib.device_status(dev.index)
+            _lib.stream_status(dev.index, _lib.current_stream(dev))
         if not is_tensor and hasattr(scores_store, "flush"):
             scores_store.flush()
         return scores_store

@@ -53,6 +53,8 @@ def _segmentable(vals, device) -> bool:
     if not vals:
         return False
     d = torch.device(device)
+    if d.type == "cuda" and d.index is None:
+        d = torch.device("cuda", torch.cuda.current_device())
     return all(v.is_cuda and v.device == d and v.dtype == vals[0].dtype for v in vals) and \
         vals[0].dtype in (torch.float16, torch.bfloat16, torch.float32)
 

@@ -73,6 +73,50 @@ class StreamPair:
     def stream(self, i: int):
         return torch.cuda.stream(self.streams[i % 2])
 
+    def current(self, i: int):
+        return self.streams[i % 2]
+
+    def uses(self, t: torch.Tensor):
+        """``t`` is used on the current stream, which may not be the one it was allocated on."""
+        t.record_stream(torch.cuda.current_stream(self.device))
+
+    def mark(self):
+        """The point the current stream has reached, for ``after``."""
+        event = torch.cuda.Event()
+        event.record(torch.cuda.current_stream(self.device))
+        return event
+
+    def after(self, event):
+        torch.cuda.current_stream(self.device).wait_event(event)
+
+
+class OneStream:
+    """Stands in for a ``StreamPair`` where there is one block only: everything stays on the caller's stream."""
+
+    def __init__(self, device):
+        self.device = device
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        return False
+
+    def stream(self, i: int):
+        return self
+
+    def current(self, i: int):
+        return torch.cuda.current_stream(self.device)
+
+    def uses(self, t):
+        pass
+
+    def mark(self):
+        pass
+
+    def after(self, event):
+        pass
+
 
 def _as_device_matrix(t: torch.Tensor, device) -> torch.Tensor:
     if not t.is_cuda and t.dtype in _DTYPES and t.is_contiguous() and torch.device(device).type == "cuda" \
@@ -97,8 +141,8 @@ def gram(x: torch.Tensor, out: torch.Tensor = None, accumulate: bool = False) ->
         out = torch.empty((k, k), dtype=torch.float32, device=dev)
         accumulate = False
     lib = _lib.lib()
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
+    with _lib.on_device(dev):
+        stream = _lib.current_stream(dev)
         dt = _DTYPES[x.dtype]
         ws = _workspace(dev, stream, lib.tb_gram_workspace_bytes(dt, n, k))
         _lib.check(lib.tb_gram(dev.index, stream, x.data_ptr(), dt, n, k, x.stride(0), out.data_ptr(),
@@ -109,7 +153,7 @@ def gram(x: torch.Tensor, out: torch.Tensor = None, accumulate: bool = False) ->
 def spd_inverse_(a: torch.Tensor, lambda_reg: float = 0.0, rescale: bool = True) -> torch.Tensor:
     """In place: a <- inv(a + lambda I) [/ mean |entry|] for a CUDA fp32 [k, k] matrix."""
     _launch_spd_inverse(a, lambda_reg, rescale)
-    _lib.device_status(a.device.index)  # raises NotPositiveDefinite / DeviceTimeout
+    _lib.stream_status(a.device.index, _lib.current_stream(a.device))  # raises NotPositiveDefinite / DeviceTimeout
     return a
 
 
@@ -119,8 +163,8 @@ def _launch_spd_inverse(a: torch.Tensor, lambda_reg: float, rescale: bool) -> No
         raise RuntimeError("expected a square fp32 matrix with unit column stride")
     dev = a.device
     lib = _lib.lib()
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
+    with _lib.on_device(dev):
+        stream = _lib.current_stream(dev)
         ws = _workspace(dev, stream, lib.tb_spd_inverse_workspace_bytes(a.shape[0]))
         _lib.check(lib.tb_spd_inverse(dev.index, stream, a.data_ptr(), a.shape[0], a.stride(0),
                                       float(lambda_reg), int(rescale), None, ws.data_ptr(), ws.numel()))
@@ -144,8 +188,8 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, row_scal
         if row_scale.numel() != M:
             raise RuntimeError("row_scale must have one entry per row of a")
     lib = _lib.lib()
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
+    with _lib.on_device(dev):
+        stream = _lib.current_stream(dev)
         dt = _DTYPES[a.dtype]
         ws = _workspace(dev, stream, lib.tb_gemm_nt_workspace_bytes(dt, M, N, K))
         _lib.check(lib.tb_gemm_nt(dev.index, stream, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), dt,
@@ -178,16 +222,16 @@ class B200ScoreComputer:
     def get_xtx(self, grads: torch.Tensor) -> torch.Tensor:
         self.proj_dim = grads.shape[1]
         accs = [None, None]   # one partial Gram per stream of the pair (blocks alternate between them)
-        with torch.cuda.device(self.device), self._pair() as pair:
-            for i, block in enumerate(self._blocks(grads)):
+        blocks = self._blocks(grads)
+        with _lib.on_device(self.device), self._pair(len(blocks) > 1) as pair:
+            for i, block in enumerate(blocks):
                 with pair.stream(i):
                     blk = _as_device_matrix(block, self.device)
-                    blk.record_stream(torch.cuda.current_stream(self.device))
+                    pair.uses(blk)
                     accs[i % 2] = gram(blk, out=accs[i % 2], accumulate=accs[i % 2] is not None)
-        main = torch.cuda.current_stream(self.device)
         for a in accs:   # allocated on a side stream, used on the caller's from here on
             if a is not None:
-                a.record_stream(main)
+                pair.uses(a)
         acc = accs[0]
         if acc is None:
             # a rank whose shard holds no rows still has to reach the all-reduce: it contributes zeros
@@ -195,14 +239,15 @@ class B200ScoreComputer:
         elif accs[1] is not None:
             acc.add_(accs[1])
         acc = reduce_gram(acc, self.process_group)
-        _lib.device_status(self.device.index)
+        _lib.stream_status(self.device.index, _lib.current_stream(self.device))
         return acc.to(self.dtype)
 
     # -- trak/score_computers.py:157-177
     def get_x_xtx_inv(self, grads: torch.Tensor, xtx: torch.Tensor) -> torch.Tensor:
         result = torch.empty(grads.shape[0], xtx.shape[1], dtype=self.dtype, device=self.device)
         start = 0
-        with torch.cuda.device(self.device), self._pair() as pair:
+        blocks = self._blocks(grads)
+        with _lib.on_device(self.device), self._pair(len(blocks) > 1 or not grads.is_cuda) as pair:
             # the pair's streams do not wait for the inverse: the blocks are copied and converted meanwhile
             inv = xtx.to(self.device, torch.float32, copy=True)
             _launch_spd_inverse(inv, self.lambda_reg, rescale=True)
@@ -210,21 +255,20 @@ class B200ScoreComputer:
             in_dtype = grads.dtype if grads.dtype in _DTYPES else torch.float32
             if in_dtype != inv.dtype:  # the narrower operand is promoted, never the inverse demoted
                 inv = inv.to(torch.promote_types(in_dtype, inv.dtype))
-            inverted = torch.cuda.Event()
-            inverted.record(torch.cuda.current_stream(self.device))
-            for i, block in enumerate(self._blocks(grads)):
+            inverted = pair.mark()
+            for i, block in enumerate(blocks):
                 rows = slice(start, start + block.shape[0])
                 start += block.shape[0]
                 with pair.stream(i):
                     blk = _as_device_matrix(block, self.device).to(inv.dtype)
-                    blk.record_stream(torch.cuda.current_stream(self.device))
-                    torch.cuda.current_stream(self.device).wait_event(inverted)
+                    pair.uses(blk)
+                    pair.after(inverted)
                     # the inverse is symmetric, so block @ inv == block @ inv.T
                     if result.dtype == torch.float32:
                         gemm_nt(blk, inv, out=result[rows])
                     else:
                         result[rows] = gemm_nt(blk, inv).to(self.dtype)
-        _lib.device_status(self.device.index)  # raises NotPositiveDefinite / DeviceTimeout
+        _lib.stream_status(self.device.index, _lib.current_stream(self.device))  # raises NotPositiveDefinite / DeviceTimeout
         return result
 
     UPLOAD_BYTES = 96 << 20  # about so many bytes of a host matrix are uploaded at a time, under the work on the last
@@ -234,9 +278,11 @@ class B200ScoreComputer:
         rows = self.CUDA_MAX_DIM_SIZE if rows is None else rows
         if not t.is_cuda:
             rows = min(rows, max(8192, self.UPLOAD_BYTES // max(1, t.shape[1] * t.element_size()) // 256 * 256))
-        return (b for b in torch.split(t, rows, dim=0) if b.shape[0])
+        return [b for b in torch.split(t, rows, dim=0) if b.shape[0]] if t.shape[0] > rows else [t] if t.shape[0] else []
 
-    def _pair(self) -> StreamPair:
+    def _pair(self, wanted: bool):
+        if not wanted:
+            return OneStream(self.device)
         pair = getattr(self, "_stream_pair", None)
         if pair is None:
             self._stream_pair = pair = StreamPair(self.device)
@@ -283,14 +329,14 @@ class B200ScoreComputer:
                 accumulator[rows] += part.cpu().to(accumulator.dtype)
 
         start = 0
-        with torch.cuda.device(self.device), self._pair() as pair:
-            for i, block in enumerate(self._blocks(features, step)):
+        blocks = self._blocks(features, step)
+        with _lib.on_device(self.device), self._pair(len(blocks) > 1) as pair:
+            for i, block in enumerate(blocks):
                 rows = slice(start, start + block.shape[0])
                 start += block.shape[0]
                 with pair.stream(i):
-                    cur = torch.cuda.current_stream(self.device)
                     blk = _as_device_matrix(block, self.device)
-                    blk.record_stream(cur)
+                    pair.uses(blk)
                     rs = None if row_scale is None else row_scale.reshape(-1)[rows]
                     part = gemm_nt(blk, targets, row_scale=rs)
                     if not on_host:
@@ -302,10 +348,10 @@ class B200ScoreComputer:
                 # the copy runs on this block's stream, under the GEMM of the next block on the other one
                 if pending is not None:
                     flush(pending)
-                pending = (rows, part, cur)
+                pending = (rows, part, pair.current(i))
         if pending is not None:
             flush(pending)
-        _lib.device_status(self.device.index)
+        _lib.stream_status(self.device.index, _lib.current_stream(self.device))
 
     HOST_STAGE_BYTES = 128 << 20  # most bytes of scores that leave for a host accumulator at a time
 
