@@ -821,7 +821,7 @@ int launch_pack(const void* src, int dtype, bool trans, uint64_t rows, uint64_t 
         TB_CUDA(cudaMemsetAsync(amax, 0, (size_t)g.rowblocks * 128u * sizeof(uint32_t), stream));
         const uint32_t bx = (uint32_t)((rows + 255) / 256);
         uint64_t by = ((uint64_t)sm_count * 16 + bx - 1) / bx;  // about 16 CTAs per SM in all
-        if (by > (K + 63) / 64) by = (K + 63) / 64;
+        if (by > (K + 15) / 16) by = (K + 15) / 16;
         if (by > 65535) by = 65535;
         const uint64_t chunk = (K + by - 1) / by;
         amax_cols_kernel<<<dim3(bx, (uint32_t)((K + chunk - 1) / chunk)), 256, 0, stream>>>(s, amax, rows, K, ld, chunk);

@@ -39,6 +39,10 @@ int encode_tmap(CUtensorMap* map, CUtensorMapDataType dt, uint32_t rank, const v
                 const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box,
                 CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B);
 
+// A word in mapped host memory that the last launch of this call on `stream` stores the status word to: the thread's
+// next tb_stream_status on that stream then needs no launch of its own.
+int arm_status(int device, cudaStream_t stream, uint32_t** word);
+
 // Lets `kernel` use all of an SM's shared memory on `device` (the current one); once per kernel and device.
 constexpr int SMEM_PER_CTA = 227 * 1024;
 int set_smem_limit(const void* kernel, int device);

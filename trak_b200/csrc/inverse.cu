@@ -92,6 +92,7 @@ __global__ void prepare_kernel(float* A, int64_t lda, int k, float lambda, uint3
 // factored after its update by the grid's own diagonal thread, a tile took 9 us.)
 // Rows and columns beyond jb are an identity block.  `buf` is CHOL_FLOATS floats of shared memory outside S.
 constexpr int CHOL_FLOATS = 64 + 3 * 256;
+static_assert(CHOL_FLOATS <= NB * TS, "a tile's worth of shared memory holds chol_block's buffers");
 constexpr int STEP_THREADS = 288;
 struct __align__(16) Chol4 {
     float l10, l20, l30, l21, l31, l32;  // strictly lower part of Ld

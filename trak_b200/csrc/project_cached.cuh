@@ -69,6 +69,7 @@ project_cached_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     __shared__ uint32_t abort_word;
     volatile uint32_t* abort_flag = &abort_word;
 
+    cudaTriggerProgrammaticLaunchCompletion();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t S = p.stages;
     const uint32_t b_bytes = p.Bpad * 128u, stage_bytes = CACHED_A_BYTES + b_bytes;
@@ -106,6 +107,7 @@ project_cached_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             prefetch_tmap(&tmap_a);
             prefetch_tmap(&tmap_b);
         }
+        cudaGridDependencySynchronize();  // the restaged gradients
         uint32_t slot = 0, ph = 0;
         for (uint32_t it = 0; it < nblocks; ++it) {
             bool got = mbar_wait(smem_u32(&bar_empty[slot]), ph ^ 1u, abort_flag);

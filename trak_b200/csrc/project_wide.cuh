@@ -45,6 +45,7 @@ project_wide_kernel(const __grid_constant__ CUtensorMap tmap, const ProjParams p
     __shared__ uint32_t abort_word;
     volatile uint32_t* abort_flag = &abort_word;
 
+    cudaTriggerProgrammaticLaunchCompletion();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t SB = p.stages;
     const uint32_t half_rows = p.Bpad / 2u;            // rows per MMA (N of the instruction)
@@ -159,6 +160,7 @@ project_wide_kernel(const __grid_constant__ CUtensorMap tmap, const ProjParams p
             // ------------------------------ TMA producer ------------------------------
             const bool leader = elect_one();
             if (leader) prefetch_tmap(&tmap);
+            cudaGridDependencySynchronize();  // the restaged gradients
             bool ok = true;
             uint32_t slot = 0, ph = 0, s = 0, trow = 0;
             for (uint32_t it = 0; it < maxcnt && ok; ++it) {
