@@ -12,7 +12,9 @@ To make an unmodified ``trak`` pick this module up::
     import sys, trak_b200.fast_jl
     sys.modules["fast_jl"] = trak_b200.fast_jl
 """
+import ctypes
 import os
+from array import array
 
 import torch
 
@@ -168,22 +170,25 @@ def project_segments(tensors, N, seed, num_feature_tiles, proj_type, *, alpha=1.
     N = _u32("N", N)
     seed = _u32("seed", seed)
     num_feature_tiles = _u32("num_feature_tiles", num_feature_tiles)
-    segs = (_lib.Segment * len(tensors))()
-    keep = []
-    F = 0
-    for i, t in enumerate(tensors):
+    if B == 0:
+        raise RuntimeError("input must not be empty")
+    table, keep, F = array("Q"), [], 0   # (ptr, numel, row_stride) of every parameter: tb_segment
+    for t in tensors:
         if t.device != dev or t.dtype != dtype or t.shape[0] != B:
             raise RuntimeError("all gradient tensors must share device, dtype and batch size")
-        flat = t.reshape(B, 1) if t.dim() < 2 else t.flatten(start_dim=1)
-        if flat.shape[1] == 0:
+        numel = t.numel() // B
+        if numel == 0:
             raise RuntimeError("empty parameter")
-        if flat.stride(1) != 1 or (B > 1 and flat.stride(0) < flat.shape[1]):
-            flat = flat.contiguous()
-        keep.append(flat)
-        segs[i].ptr = flat.data_ptr()
-        segs[i].numel = flat.shape[1]
-        segs[i].row_stride = flat.stride(0) if B > 1 else flat.shape[1]
-        F += flat.shape[1]
+        if t.is_contiguous():
+            table.extend((t.data_ptr(), numel, numel))
+        else:
+            flat = t.reshape(B, 1) if t.dim() < 2 else t.flatten(start_dim=1)
+            if flat.stride(1) != 1 or (B > 1 and flat.stride(0) < numel):
+                flat = flat.contiguous()
+            keep.append(flat)
+            table.extend((flat.data_ptr(), numel, flat.stride(0) if B > 1 else numel))
+        F += numel
+    segs = ctypes.cast(table.buffer_info()[0], ctypes.POINTER(_lib.Segment))
     l = _lib.lib()
     if out is None:
         out = torch.empty((B, N), dtype=torch.float32, device=dev)

@@ -104,7 +104,7 @@ class CudaProjector:
             vals = list(grads.values())
             if _segmentable(vals, self.device):
                 # straight from the per-parameter tensors: no [B, D] copy (trak/utils.py:80-110)
-                width = sum(1 if v.dim() < 2 else v[0].numel() for v in vals)
+                width = sum(v.numel() // v.shape[0] for v in vals) if self.store_matrix else 0
                 return _fast_jl.project_segments(vals, self.proj_dim, seed, self.num_sms, self._ptype,
                                                  alpha=alpha, out=out, accumulate=accumulate,
                                                  matrix=self._stored(seed, width, vals[0].dtype))
@@ -173,13 +173,13 @@ class ChunkedCudaProjector:
         (no packing into ch_input) and accumulated into `out` by the kernel."""
         chunk, width, index = [], 0, 0
         for p in vals:
-            w = 1 if p.dim() < 2 else p[0].numel()
+            w = 1 if p.dim() < 2 else p.numel() // max(p.shape[0], 1)
             if width + w > self.max_chunk_size:
                 self._check_chunk(index, width)
                 self.projector_per_chunk[index].project(dict(enumerate(chunk)), model_id, out=out,
                                                         accumulate=index > 0)
                 chunk, width, index = [], 0, index + 1
-            chunk.append(p[:rows])
+            chunk.append(p if p.shape[0] == rows else p[:rows])
             width += w
         self._check_chunk(index, width)
         self.projector_per_chunk[index].project(dict(enumerate(chunk)), model_id, out=out, accumulate=index > 0)

@@ -21,6 +21,7 @@ passed to an unmodified ``TRAKer(score_computer=B200ScoreComputer)``
 There is no CPU path: tensors are moved to ``device`` and the CUDA library must load.
 """
 import logging
+import threading
 
 import torch
 
@@ -28,6 +29,7 @@ from . import _lib, mmap_io
 
 _DTYPES = {torch.float16: _lib.TB_F16, torch.bfloat16: _lib.TB_BF16, torch.float32: _lib.TB_F32}
 _workspaces = {}
+_pairs = threading.local()
 _MAX_CACHED_WORKSPACES = 8  # per process; streams come and go, their workspaces should not pile up
 
 
@@ -283,9 +285,11 @@ class B200ScoreComputer:
     def _pair(self, wanted: bool):
         if not wanted:
             return OneStream(self.device)
-        pair = getattr(self, "_stream_pair", None)
+        # one pair per thread and device, for all its computers: the workspaces are kept by stream
+        pairs = _pairs.__dict__
+        pair = pairs.get(self.device.index)
         if pair is None:
-            self._stream_pair = pair = StreamPair(self.device)
+            pairs[self.device.index] = pair = StreamPair(self.device)
         return pair
 
     # -- trak/score_computers.py:179-189
