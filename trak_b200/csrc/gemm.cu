@@ -861,7 +861,7 @@ static int packed_tmap(CUtensorMap* map, const uint16_t* packed, const Packed& g
 // tensor-core time of its k blocks; slicing adds the kernel that sums the slices, which is bound by memory.  The
 // 128 x 128 tile reads twice the operand bytes per flop and is for products of less than about a wave.
 GemmPlan plan_gemm(uint32_t npl, bool chunked, bool symmetric, int64_t M, int64_t N, uint32_t kblocks) {
-    constexpr double SMS = 148.0, SUM_FIXED = 4.0, SUM_BYTES_PER_US = 3.0e6;
+    constexpr double SMS = 148.0, SUM_FIXED = 7.0, SUM_BYTES_PER_US = 3.0e6;
     constexpr uint32_t MAX_SPLITS = 64;
     constexpr size_t MAX_PARTIAL = 256u << 20;
     const double tm = (double)((M + 127) / 128), tn2 = (double)((N + 255) / 256), tm2 = (double)((M + 255) / 256);

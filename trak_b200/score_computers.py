@@ -342,6 +342,11 @@ class B200ScoreComputer:
                     blk = _as_device_matrix(block, self.device)
                     pair.uses(blk)
                     rs = None if row_scale is None else row_scale.reshape(-1)[rows]
+                    into = accumulator[rows]
+                    if into.device == blk.device and into.dtype == torch.float32 and into.stride(1) == 1 \
+                            and into.stride(0) >= m:
+                        gemm_nt(blk, targets, out=into, row_scale=rs, accumulate=True)  # the epilogue's += is the same
+                        continue
                     part = gemm_nt(blk, targets, row_scale=rs)
                     if not on_host:
                         if accumulator.device == part.device:
