@@ -10,9 +10,9 @@
 // every element within 2^-18 of its row's maximum, an absolute floor of 2^-40 of that maximum
 // below), the kernels accumulate  hi*hi + hi*lo + lo*hi  in fp32 -- three MMAs per k-step at the
 // 16-bit rate, the dropped lo*lo term is under 2^-22 -- and the epilogue multiplies the two
-// inverse scales back in (powers of two: exact).  The scales cost one more read of the operand
-// (row maxima) before the packing pass.  What is left is the tensor core's own accumulation,
-// which truncates instead of rounding: every MMA whose addends reach below the accumulator's
+// inverse scales back in (powers of two: exact).  The row maxima and the planes come out of one
+// read of the operand where a row fits in a block's registers (pack_rows_f32_kernel).
+// What is left is the tensor core's own accumulation, which truncates instead of rounding: every MMA whose addends reach below the accumulator's
 // last place pulls the sum towards zero, and a K-long contraction is a chain of 3K/16 such steps.
 //  * X . inv and features . targets^T (gemm_nt_kernel) keep one accumulation over all of K:
 //    about 1e-5 relative at K = 3000 ... 8192 (one TF32 pass would give 5e-4).  With bf16
@@ -30,10 +30,11 @@
 // [128-row block][32-wide k block][plane][128 rows][32 k], so every TMA box is one
 // contiguous 8 KB run, and it can transpose (for X^T X the operand is X^T).
 //
-// Kernel: one CTA per 256 x 256 tile of C.  Warp 0 issues TMA (64-byte swizzle boxes,
-// never multicast), warp 1 issues tcgen05.mma (both operands from shared memory,
-// M = 128, N = 256, two accumulators fill the 512 TMEM columns), warps 4-11 run the
-// epilogue (tcgen05.ld, scale, optional accumulate, optional mirrored store for the
+// Kernel: one CTA per 256 x 256 tile of C, or per 128 x 128 tile (two CTAs per SM), with the
+// contraction split over several CTAs, where the large tile leaves SMs idle (plan_gemm).
+// Warp 0 issues TMA (64-byte swizzle boxes, never multicast), warp 1 issues tcgen05.mma (both
+// operands from shared memory; M = 128, N = 256, two accumulators fill the 512 TMEM columns of
+// the large tile), the warps from the fifth on run the epilogue (tcgen05.ld, scale, optional accumulate, optional mirrored store for the
 // symmetric product).  Every mbarrier wait is bounded.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>

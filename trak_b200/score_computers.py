@@ -46,6 +46,7 @@ def _workspace(device, stream, nbytes):
 
 def free_workspaces():
     _workspaces.clear()
+    _lib.check(_lib.lib().tb_host_staging_release())
 
 
 class StreamPair:
