@@ -50,3 +50,25 @@ def test_inverse_at_tile_edges(cuda, k):
     wide = torch.zeros(k, k + 3, device=cuda)      # rows that are not 16-byte aligned
     wide[:, :k] = a
     assert rel(sc.spd_inverse_(wide[:, :k], 1e-3, rescale=False), want) <= 2e-5
+
+
+@pytest.mark.parametrize("k", [1025, 1536, 1537, 2100, 2560, 3111])
+def test_inverse_of_several_block_columns(cuda, k):
+    """Columns, updates and merges run on three streams: the same bits from call to call and from several threads."""
+    from concurrent.futures import ThreadPoolExecutor
+    from trak_b200 import score_computers as sc
+    y = torch.randn(2 * k, k, device=cuda, dtype=torch.float64, generator=torch.Generator(device=cuda).manual_seed(k))
+    a = (y.T @ y / k).float()
+    want = torch.linalg.inv(a.double() + 1e-2 * torch.eye(k, device=cuda, dtype=torch.float64))
+    got = sc.spd_inverse_(a.clone(), 1e-2, rescale=False)
+    assert rel(got, want) <= 2e-5
+    assert torch.equal(got, got.T)
+    torch.cuda.synchronize()
+
+    def again(_):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            out = [sc.spd_inverse_(a.clone(), 1e-2, rescale=False) for _ in range(3)]
+            torch.cuda.current_stream().synchronize()
+        return all(torch.equal(o, got) for o in out)
+    with ThreadPoolExecutor(3) as pool:
+        assert all(pool.map(again, range(3)))

@@ -812,6 +812,23 @@ static int launch_pack_rows(const PackRows& a, const PackRows& b, int sm_count, 
     return TB_OK;
 }
 
+int launch_pack_pair(const float* a, uint64_t rows_a, uint64_t K_a, uint64_t ld_a, uint16_t* packed_a, const Packed& ga,
+                     const float* b, uint64_t rows_b, uint64_t K_b, uint64_t ld_b, uint16_t* packed_b, const Packed& gb,
+                     int sm_count, cudaStream_t stream) {
+    return launch_pack_rows(pack_rows_args(a, rows_a, K_a, ld_a, packed_a, ga),
+                            pack_rows_args(b, rows_b, K_b, ld_b, packed_b, gb), sm_count, stream);
+}
+
+Packed packed_tail(const uint16_t** packed, const Packed& g, uint32_t skip) {
+    const size_t skipped = (size_t)skip * g.kblocks * g.npl * GTILE_BYTES;
+    Packed t = g;
+    t.rowblocks -= skip;
+    t.data_bytes = g.data_bytes - skipped + (size_t)skip * 128u * sizeof(uint32_t);  // the row maxima stay where they are
+    t.bytes = g.bytes - skipped;
+    *packed += skipped / sizeof(uint16_t);
+    return t;
+}
+
 int launch_pack(const void* src, int dtype, bool trans, uint64_t rows, uint64_t K, uint64_t ld,
                 uint16_t* packed, const Packed& g, int sm_count, cudaStream_t stream) {
     if (dtype == TB_F32 && !trans)

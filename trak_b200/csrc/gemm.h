@@ -25,6 +25,14 @@ Packed packed_geometry(int dtype, int64_t rows, int64_t K);
 int launch_pack(const void* src, int dtype, bool trans, uint64_t rows, uint64_t K, uint64_t ld,
                 uint16_t* packed, const Packed& g, int sm_count, cudaStream_t stream);
 
+// The same for two fp32 operands in one launch (neither transposed).
+int launch_pack_pair(const float* a, uint64_t rows_a, uint64_t K_a, uint64_t ld_a, uint16_t* packed_a, const Packed& ga,
+                     const float* b, uint64_t rows_b, uint64_t K_b, uint64_t ld_b, uint16_t* packed_b, const Packed& gb,
+                     int sm_count, cudaStream_t stream);
+
+// The packed operand without its first `skip` row blocks: moves `packed` and returns the geometry of what is left.
+Packed packed_tail(const uint16_t** packed, const Packed& g, uint32_t skip);
+
 // How launch_gemm computes a product: CTA tile (2: 256 wide, 1: 128 wide), slices of the contraction, and the bytes
 // of the slices' partial products, which the caller provides as `partial`.
 struct GemmPlan {

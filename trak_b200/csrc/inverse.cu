@@ -14,6 +14,9 @@
 //   5. mean |entry| with a fixed-order two-pass reduction, then the rescale.
 // A non-positive pivot is recorded in the device status word (ST_NOT_SPD).
 #include <algorithm>
+#include <map>
+#include <mutex>
+#include <vector>
 
 #include "gemm.h"
 #include "host_util.h"
@@ -435,13 +438,6 @@ __device__ __forceinline__ bool rows_are_vec4(const float* A, int64_t lda, int k
     return (k & 3) == 0 && (lda & 3) == 0 && (reinterpret_cast<uintptr_t>(A) & 15u) == 0;
 }
 
-__global__ void zero_upper_kernel(float* A, int64_t lda, int k) {
-    for (int i = blockIdx.x; i < k; i += gridDim.x) {
-        float* row = A + (int64_t)i * lda;
-        for (int j = i + 1 + threadIdx.x; j < k; j += blockDim.x) row[j] = 0.0f;
-    }
-}
-
 constexpr int RED_BLOCKS = 1024;
 __global__ void __launch_bounds__(256) abs_partial_kernel(const float* A, int64_t lda, int k, double* partial) {
     __shared__ double sh[256];
@@ -511,7 +507,7 @@ static Product product(int64_t m, int64_t n, int64_t kk, bool symmetric) {
 }
 
 struct InvLayout {
-    size_t dinv, blocks, partial, mean, counters, scratch, total;
+    size_t dinv, blocks, partial, mean, counters, chain, rest, merge, total;
 };
 static InvLayout inv_layout(int64_t k) {
     InvLayout l;
@@ -526,22 +522,90 @@ static InvLayout inv_layout(int64_t k) {
     off += 256;
     l.counters = off;
     off += align_up((size_t)((k + OUTER - 1) / OUTER) * sizeof(uint32_t), 256);
-    l.scratch = off = align_up(off, 1024);
-    size_t need = product(k, k, k, true).bytes();  // W^T W
+    // what the block columns, the rest of their updates and the merges use at the same time
+    size_t chain = 0, rest = 0, merge = product(k, k, k, true).bytes();  // W^T W
     for (int64_t o = 0; o + OUTER < k; o += OUTER) {
-        need = std::max(need, product(k - o - OUTER, OUTER, OUTER, false).bytes());
-        need = std::max(need, product(k - o - OUTER, k - o - OUTER, OUTER, true).bytes());
+        const int64_t r = k - o - OUTER, d = std::min<int64_t>(OUTER, r);
+        chain = std::max(chain, product(r, OUTER, OUTER, false).bytes());
+        chain = std::max(chain, product(r, OUTER, OUTER, true).a.bytes + product(d, d, OUTER, true).partial);
+        if (r > d) rest = std::max(rest, std::max(product(r - d, d, OUTER, false).partial, product(r - d, r - d, OUTER, true).partial));
     }
     for (int64_t s = OUTER; s < k; s *= 2)
         for (int64_t b0 = 0; b0 + s < k; b0 += 2 * s) {
             const int64_t s2 = std::min<int64_t>(s, k - b0 - s);
-            // L21 W11 and its fp32 result, then W22 times that
+            // (L21 W11)^T in fp32, the operands of that product, then those of W22 times it
             const size_t t = align_up((size_t)s2 * s * sizeof(float), 1024);
-            need = std::max(need, t + std::max(product(s2, s, s, false).bytes(), product(s2, s, s2, false).bytes()));
+            merge = std::max(merge, t + std::max(product(s, s2, s, false).bytes(), product(s2, s, s2, false).bytes()));
         }
-    l.total = off + need + 1024;
+    l.chain = off = align_up(off, 1024);
+    l.rest = off = align_up(off + chain, 1024);
+    l.merge = off = align_up(off + rest, 1024);
+    l.total = off + merge + 1024;
     return l;
 }
+
+// Two streams beside the caller's: `chain` (high priority) factors the block columns one after the other, `rest` applies
+// the part of their updates that the next column does not wait for.  A call borrows a set and gives it back when
+// everything is queued and the caller's stream waits for it (a later borrower at most waits for that work too); at most
+// MAX_KEPT idle sets are kept per device.
+struct SideStreams {
+    cudaStream_t chain = nullptr, rest = nullptr;
+    cudaEvent_t forked = nullptr, block = nullptr, packed = nullptr, updated = nullptr;
+    int make() {
+        int least = 0, greatest = 0;
+        TB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        TB_CUDA(cudaStreamCreateWithPriority(&chain, cudaStreamNonBlocking, greatest));
+        TB_CUDA(cudaStreamCreateWithPriority(&rest, cudaStreamNonBlocking, least));
+        for (cudaEvent_t* e : {&forked, &block, &packed, &updated})
+            TB_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+        return TB_OK;
+    }
+    void destroy() {
+        for (cudaEvent_t e : {forked, block, packed, updated})
+            if (e) cudaEventDestroy(e);
+        if (rest) cudaStreamDestroy(rest);
+        if (chain) cudaStreamDestroy(chain);
+    }
+};
+constexpr size_t MAX_KEPT = 4;
+static std::mutex g_side_mu;
+static std::map<int, std::vector<SideStreams>> g_side;
+
+class BorrowedStreams {
+   public:
+    int take(int device) {
+        device_ = device;
+        {
+            std::lock_guard<std::mutex> lk(g_side_mu);
+            std::vector<SideStreams>& idle = g_side[device];
+            if (!idle.empty()) {
+                s = idle.back();
+                idle.pop_back();
+                return TB_OK;
+            }
+        }
+        return s.make();
+    }
+    ~BorrowedStreams() {
+        if (!s.updated) {  // not taken, or not made completely
+            s.destroy();
+            return;
+        }
+        if (!joined) {  // the call gave up half way: the workspace is the caller's again
+            cudaStreamSynchronize(s.chain);
+            cudaStreamSynchronize(s.rest);
+        }
+        std::lock_guard<std::mutex> lk(g_side_mu);
+        std::vector<SideStreams>& idle = g_side[device_];
+        if (idle.size() < MAX_KEPT) idle.push_back(s);
+        else s.destroy();
+    }
+    SideStreams s;
+    bool joined = false;  // everything on them is waited for by the caller's stream
+
+   private:
+    int device_ = 0;
+};
 
 }  // namespace tb
 
@@ -568,33 +632,71 @@ int tb_spd_inverse(int device, void* stream_, float* A, int64_t k, int64_t lda, 
     float* blocks = reinterpret_cast<float*>(base + l.blocks);
     double* partial = reinterpret_cast<double*>(base + l.partial);
     float* mean = reinterpret_cast<float*>(base + l.mean);
-    uint8_t* scratch = base + l.scratch;
     const int K = (int)k;
 
+    // The block columns, the rest of their updates and the merges run on three streams where there is more than one
+    // column.  A capture stays on the caller's stream: borrowed streams must not be part of a graph under construction.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    TB_CUDA(cudaStreamIsCapturing(stream, &capture));
+    BorrowedStreams side;
+    const bool apart = k > OUTER && capture == cudaStreamCaptureStatusNone;
+    if (apart && (rc = side.take(device)) != TB_OK) return rc;
+    const cudaStream_t chain = apart ? side.s.chain : stream, rest = apart ? side.s.rest : stream;
+    auto record = [&](cudaEvent_t event, cudaStream_t on) -> int {
+        if (apart) TB_CUDA(cudaEventRecord(event, on));
+        return TB_OK;
+    };
+    auto wait = [&](cudaStream_t on, cudaEvent_t event) -> int {
+        if (apart) TB_CUDA(cudaStreamWaitEvent(on, event, 0));
+        return TB_OK;
+    };
+
     // operands of one product at `at`, then the product itself
-    auto multiply = [&](const Product& pr, uint8_t* at, const float* a, int64_t ld_a, bool trans_a, const float* b,
-                        int64_t ld_b, bool trans_b, int64_t m, int64_t n, int64_t kk, float* c, int64_t ld_c, float alpha,
-                        int accumulate) -> int {
+    auto multiply = [&](cudaStream_t on, const Product& pr, uint8_t* at, const float* a, int64_t ld_a, bool trans_a,
+                        const float* b, int64_t ld_b, int64_t m, int64_t n, int64_t kk, float* c, int64_t ld_c,
+                        float alpha) -> int {
         const bool symmetric = b == nullptr;
         uint16_t* pa = reinterpret_cast<uint16_t*>(at);
         uint16_t* pb = symmetric ? pa : reinterpret_cast<uint16_t*>(at + pr.a.bytes);
-        int r = launch_pack(a, TB_F32, trans_a, (uint64_t)m, (uint64_t)kk, (uint64_t)ld_a, pa, pr.a, sm_count, stream);
-        if (r != TB_OK) return r;
-        if (!symmetric) {
-            r = launch_pack(b, TB_F32, trans_b, (uint64_t)n, (uint64_t)kk, (uint64_t)ld_b, pb, pr.b, sm_count, stream);
+        int r;
+        if (!symmetric && !trans_a) {
+            r = launch_pack_pair(a, m, kk, ld_a, pa, pr.a, b, n, kk, ld_b, pb, pr.b, sm_count, on);
+            if (r != TB_OK) return r;
+        } else {
+            r = launch_pack(a, TB_F32, trans_a, (uint64_t)m, (uint64_t)kk, (uint64_t)ld_a, pa, pr.a, sm_count, on);
+            if (r != TB_OK) return r;
+            if (!symmetric) r = launch_pack(b, TB_F32, false, (uint64_t)n, (uint64_t)kk, (uint64_t)ld_b, pb, pr.b, sm_count, on);
             if (r != TB_OK) return r;
         }
-        return launch_gemm(device, stream, pa, pr.a, pb, symmetric ? pr.a : pr.b, TB_F32, m, n, c, ld_c, nullptr, alpha,
-                           accumulate, symmetric ? 1 : 0, 1, reinterpret_cast<float*>(at + pr.a.bytes + pr.b.bytes));
+        return launch_gemm(device, on, pa, pr.a, pb, symmetric ? pr.a : pr.b, TB_F32, m, n, c, ld_c, nullptr, alpha, 0,
+                           symmetric ? 1 : 0, 1, reinterpret_cast<float*>(at + pr.a.bytes + pr.b.bytes));
+    };
+
+    // W21 = -W22 (L21 W11), written over L21, and zeros in L's place above the diagonal
+    auto merge = [&](int64_t b0, int64_t s, int64_t s2) -> int {
+        float* W11 = A + b0 * lda + b0;
+        float* L21 = A + (b0 + s) * lda + b0;
+        float* W22 = A + (b0 + s) * lda + b0 + s;
+        float* T = reinterpret_cast<float*>(base + l.merge);
+        uint8_t* at = base + l.merge + align_up((size_t)s2 * s * sizeof(float), 1024);
+        // T[s x s2] = (L21 W11)^T = W11^T . L21^T;  W21 = - W22 . T^T
+        int r = multiply(stream, product(s, s2, s, false), at, W11, lda, true, L21, lda, s, s2, s, T, s2, 1.0f);
+        if (r != TB_OK) return r;
+        r = multiply(stream, product(s2, s, s2, false), at, W22, lda, false, T, s2, s2, s, s2, L21, lda, -1.0f);
+        if (r != TB_OK) return r;
+        TB_CUDA(cudaMemset2DAsync(W11 + s, (size_t)lda * sizeof(float), 0, (size_t)s2 * sizeof(float), (size_t)s, stream));
+        return TB_OK;
     };
 
     uint32_t* counters = reinterpret_cast<uint32_t*>(base + l.counters);
     prepare_kernel<<<(K + 255) / 256, 256, 0, stream>>>(A, lda, K, lambda, counters, (K + OUTER - 1) / OUTER);
+    if ((rc = record(side.s.forked, stream)) != TB_OK || (rc = wait(chain, side.s.forked)) != TB_OK) return rc;
 
-    // 1. Block columns: the diagonal block becomes its W, the block below it L21, what is right of both is updated.
     constexpr size_t step_smem = 4u * NB * TS * sizeof(float);
     if (const int e = set_smem_limit((const void*)block_kernel, device)) return e;
+    uint8_t* const chain_at = base + l.chain;
     for (int64_t o = 0; o < k; o += OUTER) {
+        // 1. The diagonal block becomes its W.
         const int kb = (int)std::min<int64_t>(OUTER, k - o), nt = (kb + NB - 1) / NB;
         float* block = A + o * lda + o;
         int tiles = nt;  // of the first step, the largest
@@ -606,46 +708,58 @@ int tb_spd_inverse(int device, void* stream_, float* A, int64_t k, int64_t lda, 
         cfg.gridDim = dim3((unsigned)std::min(tiles + 1, sm_count));
         cfg.blockDim = dim3(STEP_THREADS);
         cfg.dynamicSmemBytes = step_smem;
-        cfg.stream = stream;
+        cfg.stream = chain;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         TB_CUDA(cudaLaunchKernelEx(&cfg, block_kernel, block, lda, kb, blocks, dinv, counters + o / OUTER,
                                    status_ptr(device)));
-        const int64_t r = k - o - kb;
+        if ((rc = record(side.s.block, chain)) != TB_OK || (rc = wait(stream, side.s.block)) != TB_OK) return rc;
+
+        // 2. Below it L21; of what is right of both, first the next diagonal block, then the rest beside the chain.
+        const int64_t r = k - o - kb, d = std::min<int64_t>(OUTER, r);
         if (r > 0) {
             float* A21 = A + (o + kb) * lda + o;
             float* A22 = A + (o + kb) * lda + o + kb;
-            rc = multiply(product(r, kb, kb, false), scratch, A21, lda, false, block, lda, false, r, kb, kb, A21, lda, 1.0f, 0);
+            if (o > 0 && (rc = wait(chain, side.s.updated)) != TB_OK) return rc;
+            rc = multiply(chain, product(r, kb, kb, false), chain_at, A21, lda, false, block, lda, r, kb, kb, A21, lda, 1.0f);
             if (rc != TB_OK) return rc;
-            rc = multiply(product(r, r, kb, true), scratch, A21, lda, false, nullptr, 0, false, r, r, kb, A22, lda, -1.0f, 1);
+            const Packed g = packed_geometry(TB_F32, r, kb);
+            const uint16_t *L = reinterpret_cast<uint16_t*>(chain_at), *tail = L;
+            rc = launch_pack(A21, TB_F32, false, r, kb, lda, const_cast<uint16_t*>(L), g, sm_count, chain);
             if (rc != TB_OK) return rc;
+            if ((rc = record(side.s.packed, chain)) != TB_OK || (rc = wait(rest, side.s.packed)) != TB_OK) return rc;
+            rc = launch_gemm(device, chain, L, g, L, g, TB_F32, d, d, A22, lda, nullptr, -1.0f, 1, 1, 1,
+                             reinterpret_cast<float*>(chain_at + g.bytes));
+            if (rc != TB_OK) return rc;
+            if (r > d) {
+                const Packed gt = packed_tail(&tail, g, OUTER / 128);
+                float* partial_sums = reinterpret_cast<float*>(base + l.rest);
+                rc = launch_gemm(device, rest, tail, gt, L, g, TB_F32, r - d, d, A22 + d * lda, lda, nullptr, -1.0f, 1, 0, 1,
+                                 partial_sums);
+                if (rc != TB_OK) return rc;
+                rc = launch_gemm(device, rest, tail, gt, tail, gt, TB_F32, r - d, r - d, A22 + d * lda + d, lda, nullptr,
+                                 -1.0f, 1, 1, 1, partial_sums);
+                if (rc != TB_OK) return rc;
+                if ((rc = record(side.s.updated, rest)) != TB_OK) return rc;
+            }
+        }
+
+        // 3. The inverted blocks so far that complete a pair, and the pairs of pairs.
+        const int64_t done = o + kb;
+        for (int64_t s = OUTER; s < done; s *= 2) {
+            if (done < k && done % (2 * s) != 0) break;
+            const int64_t b0 = (done - 1) / (2 * s) * (2 * s);
+            if (b0 + s < done && (rc = merge(b0, s, done - b0 - s)) != TB_OK) return rc;
         }
     }
     TB_CUDA(cudaGetLastError());
+    side.joined = true;  // the last block waited for the last update, the caller's stream for the last block
 
-    // 2. W = L^-1: blocks of OUTER are inverted and clear above the diagonal; clear the rest, then merge neighbours.
-    if (k > OUTER) zero_upper_kernel<<<sm_count * 8, 256, 0, stream>>>(A, lda, K);
-    for (int64_t s = OUTER; s < k; s *= 2)
-        for (int64_t b0 = 0; b0 + s < k; b0 += 2 * s) {
-            const int64_t s2 = std::min<int64_t>(s, k - b0 - s);
-            float* W11 = A + b0 * lda + b0;
-            float* L21 = A + (b0 + s) * lda + b0;
-            float* W22 = A + (b0 + s) * lda + b0 + s;
-            float* T = reinterpret_cast<float*>(scratch);
-            uint8_t* at = scratch + align_up((size_t)s2 * s * sizeof(float), 1024);
-            // T[s2 x s] = L21 . W11 = L21 . (W11^T)^T;  W21 = - W22 . (T^T)^T, written over L21
-            rc = multiply(product(s2, s, s, false), at, L21, lda, false, W11, lda, true, s2, s, s, T, s, 1.0f, 0);
-            if (rc != TB_OK) return rc;
-            rc = multiply(product(s2, s, s2, false), at, W22, lda, false, T, s, true, s2, s, s2, L21, lda, -1.0f, 0);
-            if (rc != TB_OK) return rc;
-        }
-    TB_CUDA(cudaGetLastError());
-
-    // 3. A^-1 = W^T W (full symmetric result written over A; the operand is packed first)
-    rc = multiply(product(k, k, k, true), scratch, A, lda, true, nullptr, 0, false, k, k, k, A, lda, 1.0f, 0);
+    // A^-1 = W^T W (full symmetric result written over A; the operand is packed first)
+    rc = multiply(stream, product(k, k, k, true), base + l.merge, A, lda, true, nullptr, 0, k, k, k, A, lda, 1.0f);
     if (rc != TB_OK) return rc;
 
-    // 4. mean |entry| and the reference's rescale
+    // mean |entry| and the reference's rescale
     if (rescale_by_mean_abs || mean_abs_out) {
         abs_partial_kernel<<<RED_BLOCKS, 256, 0, stream>>>(A, lda, K, partial);
         abs_final_kernel<<<1, 256, 0, stream>>>(partial, K, mean);
