@@ -65,6 +65,7 @@ struct GemmParams {
     int accumulate;
     int symmetric;           // A and B are the same packed operand; only tiles on/above the
                              // diagonal are computed and every result is stored twice
+    int range;               // KRange, chunked kernel only
     int mirror;              // symmetric: whether this launch stores the second copy (not for partial products)
 };
 
@@ -357,14 +358,22 @@ gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     const uint32_t width = GROUP_M * tiles_n;
     const uint32_t first_m = (id / width) * GROUP_M;
     const uint32_t gsize = min(tiles_m - first_m, GROUP_M);
-    const uint32_t tile_m = first_m + (id % width) % gsize, tile_n = (id % width) / gsize;
+    uint32_t tile_m = first_m + (id % width) % gsize;
+    const uint32_t tile_n = (id % width) / gsize;
+    if (p.range == K_TO_ROW) tile_m = tiles_m - 1u - tile_m;  // the longest contractions first
     // symmetric: a tile is needed when it holds some entry with n >= m
     if (p.symmetric && tile_n < (tile_m >> 1)) return;
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    // kb_per_split is even: a slice holds whole chunks
-    const uint32_t kb_first = blockIdx.z * p.kb_per_split, kb_end = min(p.kblocks, kb_first + p.kb_per_split);
+    // The k blocks of this tile, less those where an operand is zero (a triangular factor: a third of W^T W and half of
+    // a merge is left), and of them this slice's.  Starts are multiples of 128 and slices even: whole chunks.
+    uint32_t kb_lo = 0, kb_hi = p.kblocks;
+    if (p.range == K_FROM_ROW) kb_lo = min(p.kblocks, max(tile_m * 4u, p.symmetric ? tile_n * 8u : 0u));
+    if (p.range == K_TO_ROW) kb_hi = min(p.kblocks, tile_m * 4u + 4u);
+    if (p.range == K_TO_COL) kb_hi = min(p.kblocks, tile_n * 8u + 8u);
+    const uint32_t slice = ((kb_hi - kb_lo + gridDim.z - 1u) / gridDim.z + 1u) & ~1u;
+    const uint32_t kb_first = min(kb_hi, kb_lo + blockIdx.z * slice), kb_end = min(kb_hi, kb_first + slice);
     const uint32_t nchunks = (kb_end - kb_first + 1u) >> 1;
 
     if (threadIdx.x == 0) {
@@ -930,7 +939,7 @@ static int launch_gemm_nt(int device, const CUtensorMap& map_a, const CUtensorMa
 int launch_gemm(int device, cudaStream_t stream, const uint16_t* pa, const Packed& ga,
                 const uint16_t* pb, const Packed& gb, int dtype, int64_t M, int64_t N, float* C,
                 int64_t ldc, const float* row_scale, float alpha, int accumulate, int symmetric,
-                int chunked, float* partial) {
+                int chunked, float* partial, KRange range) {
     CUtensorMap map_a, map_b;
     int rc = packed_tmap(&map_a, pa, ga, dtype);
     if (rc != TB_OK) return rc;
@@ -954,6 +963,7 @@ int launch_gemm(int device, cudaStream_t stream, const uint16_t* pa, const Packe
     p.alpha = alpha;
     p.accumulate = accumulate;
     p.symmetric = symmetric;
+    p.range = range;
     p.mirror = 1;
     const GemmParams whole = p;
     if (pl.splits > 1) {  // raw partial sums; the scales and the destination are the last kernel's

@@ -42,11 +42,21 @@ struct GemmPlan {
 };
 GemmPlan plan_gemm(uint32_t npl, bool chunked, bool symmetric, int64_t M, int64_t N, uint32_t kblocks);
 
+// Which k of a product are known to be zero in one of its operands, so that a tile's contraction leaves them out
+// (chunked products only).  m and n are rows of A and of B.
+enum KRange : int {
+    K_ALL,
+    K_FROM_ROW,  // A[m][k] = 0 for k < m; symmetric: also for k < n
+    K_TO_ROW,    // A[m][k] = 0 for k > m
+    K_TO_COL,    // B[n][k] = 0 for k > n
+};
+
 // C[M x N] (+)= alpha * row_scale[m] * Apacked . Bpacked^T  (symmetric: A == B, mirrored stores;
 // chunked: scaled fp32 operands only -- the tensor core accumulates 64 k at a time and the chunks are
 // summed with rounded fp32 adds, for products whose error an inverse will amplify)
 int launch_gemm(int device, cudaStream_t stream, const uint16_t* pa, const Packed& ga, const uint16_t* pb,
                 const Packed& gb, int dtype, int64_t M, int64_t N, float* C, int64_t ldc,
-                const float* row_scale, float alpha, int accumulate, int symmetric, int chunked, float* partial);
+                const float* row_scale, float alpha, int accumulate, int symmetric, int chunked, float* partial,
+                KRange range = K_ALL);
 
 }  // namespace tb

@@ -654,7 +654,7 @@ int tb_spd_inverse(int device, void* stream_, float* A, int64_t k, int64_t lda, 
     // operands of one product at `at`, then the product itself
     auto multiply = [&](cudaStream_t on, const Product& pr, uint8_t* at, const float* a, int64_t ld_a, bool trans_a,
                         const float* b, int64_t ld_b, int64_t m, int64_t n, int64_t kk, float* c, int64_t ld_c,
-                        float alpha) -> int {
+                        float alpha, KRange range) -> int {
         const bool symmetric = b == nullptr;
         uint16_t* pa = reinterpret_cast<uint16_t*>(at);
         uint16_t* pb = symmetric ? pa : reinterpret_cast<uint16_t*>(at + pr.a.bytes);
@@ -669,7 +669,7 @@ int tb_spd_inverse(int device, void* stream_, float* A, int64_t k, int64_t lda, 
             if (r != TB_OK) return r;
         }
         return launch_gemm(device, on, pa, pr.a, pb, symmetric ? pr.a : pr.b, TB_F32, m, n, c, ld_c, nullptr, alpha, 0,
-                           symmetric ? 1 : 0, 1, reinterpret_cast<float*>(at + pr.a.bytes + pr.b.bytes));
+                           symmetric ? 1 : 0, 1, reinterpret_cast<float*>(at + pr.a.bytes + pr.b.bytes), range);
     };
 
     // W21 = -W22 (L21 W11), written over L21, and zeros in L's place above the diagonal
@@ -680,9 +680,11 @@ int tb_spd_inverse(int device, void* stream_, float* A, int64_t k, int64_t lda, 
         float* T = reinterpret_cast<float*>(base + l.merge);
         uint8_t* at = base + l.merge + align_up((size_t)s2 * s * sizeof(float), 1024);
         // T[s x s2] = (L21 W11)^T = W11^T . L21^T;  W21 = - W22 . T^T
-        int r = multiply(stream, product(s, s2, s, false), at, W11, lda, true, L21, lda, s, s2, s, T, s2, 1.0f);
+        int r = multiply(stream, product(s, s2, s, false), at, W11, lda, true, L21, lda, s, s2, s, T, s2, 1.0f,
+                         K_FROM_ROW);
         if (r != TB_OK) return r;
-        r = multiply(stream, product(s2, s, s2, false), at, W22, lda, false, T, s2, s2, s, s2, L21, lda, -1.0f);
+        r = multiply(stream, product(s2, s, s2, false), at, W22, lda, false, T, s2, s2, s, s2, L21, lda, -1.0f,
+                     K_TO_ROW);
         if (r != TB_OK) return r;
         TB_CUDA(cudaMemset2DAsync(W11 + s, (size_t)lda * sizeof(float), 0, (size_t)s2 * sizeof(float), (size_t)s, stream));
         return TB_OK;
@@ -721,7 +723,8 @@ int tb_spd_inverse(int device, void* stream_, float* A, int64_t k, int64_t lda, 
             float* A21 = A + (o + kb) * lda + o;
             float* A22 = A + (o + kb) * lda + o + kb;
             if (o > 0 && (rc = wait(chain, side.s.updated)) != TB_OK) return rc;
-            rc = multiply(chain, product(r, kb, kb, false), chain_at, A21, lda, false, block, lda, r, kb, kb, A21, lda, 1.0f);
+            rc = multiply(chain, product(r, kb, kb, false), chain_at, A21, lda, false, block, lda, r, kb, kb, A21, lda, 1.0f,
+                          K_TO_COL);
             if (rc != TB_OK) return rc;
             const Packed g = packed_geometry(TB_F32, r, kb);
             const uint16_t *L = reinterpret_cast<uint16_t*>(chain_at), *tail = L;
@@ -756,7 +759,7 @@ int tb_spd_inverse(int device, void* stream_, float* A, int64_t k, int64_t lda, 
     side.joined = true;  // the last block waited for the last update, the caller's stream for the last block
 
     // A^-1 = W^T W (full symmetric result written over A; the operand is packed first)
-    rc = multiply(stream, product(k, k, k, true), base + l.merge, A, lda, true, nullptr, 0, k, k, k, A, lda, 1.0f);
+    rc = multiply(stream, product(k, k, k, true), base + l.merge, A, lda, true, nullptr, 0, k, k, k, A, lda, 1.0f, K_FROM_ROW);
     if (rc != TB_OK) return rc;
 
     // mean |entry| and the reference's rescale
