@@ -507,7 +507,13 @@ static Product product(int64_t m, int64_t n, int64_t kk, bool symmetric) {
 }
 
 struct InvLayout {
-    size_t dinv, blocks, partial, mean, counters, chain, rest, merge, total;
+    size_t dinv, blocks, partial, mean, counters, chain, rest, left, merge, total;
+    // the merges' first products: one per level is waiting for its second at a time
+    size_t left_at(int64_t s) const {
+        size_t at = left;
+        for (int64_t t = OUTER; t < s; t *= 2) at += (size_t)t * t * sizeof(float);
+        return at;
+    }
 };
 static InvLayout inv_layout(int64_t k) {
     InvLayout l;
@@ -533,13 +539,14 @@ static InvLayout inv_layout(int64_t k) {
     for (int64_t s = OUTER; s < k; s *= 2)
         for (int64_t b0 = 0; b0 + s < k; b0 += 2 * s) {
             const int64_t s2 = std::min<int64_t>(s, k - b0 - s);
-            // (L21 W11)^T in fp32, the operands of that product, then those of W22 times it
-            const size_t t = align_up((size_t)s2 * s * sizeof(float), 1024);
-            merge = std::max(merge, t + std::max(product(s, s2, s, false).bytes(), product(s2, s, s2, false).bytes()));
+            merge = std::max(merge, std::max(product(s, s2, s, false).bytes(), product(s2, s, s2, false).bytes()));
         }
     l.chain = off = align_up(off, 1024);
     l.rest = off = align_up(off + chain, 1024);
-    l.merge = off = align_up(off + rest, 1024);
+    l.left = off = align_up(off + rest, 1024);
+    int64_t levels = OUTER;
+    while (levels < k) levels *= 2;
+    l.merge = off = l.left_at(levels);
     l.total = off + merge + 1024;
     return l;
 }
@@ -672,21 +679,20 @@ int tb_spd_inverse(int device, void* stream_, float* A, int64_t k, int64_t lda, 
                            symmetric ? 1 : 0, 1, reinterpret_cast<float*>(at + pr.a.bytes + pr.b.bytes), range);
     };
 
-    // W21 = -W22 (L21 W11), written over L21, and zeros in L's place above the diagonal
+    // W21 = -W22 (L21 W11), written over L21, in two products: the first as soon as W11 is there, in transposed form
+    // (T[s x s2] = W11^T . L21^T), the second when W22 is.  Then zeros in L's place above the diagonal.
+    auto merge_left = [&](int64_t b0, int64_t s, int64_t s2) -> int {
+        const float *W11 = A + b0 * lda + b0, *L21 = A + (b0 + s) * lda + b0;
+        return multiply(stream, product(s, s2, s, false), base + l.merge, W11, lda, true, L21, lda, s, s2, s,
+                        reinterpret_cast<float*>(base + l.left_at(s)), s2, 1.0f, K_FROM_ROW);
+    };
     auto merge = [&](int64_t b0, int64_t s, int64_t s2) -> int {
-        float* W11 = A + b0 * lda + b0;
-        float* L21 = A + (b0 + s) * lda + b0;
-        float* W22 = A + (b0 + s) * lda + b0 + s;
-        float* T = reinterpret_cast<float*>(base + l.merge);
-        uint8_t* at = base + l.merge + align_up((size_t)s2 * s * sizeof(float), 1024);
-        // T[s x s2] = (L21 W11)^T = W11^T . L21^T;  W21 = - W22 . T^T
-        int r = multiply(stream, product(s, s2, s, false), at, W11, lda, true, L21, lda, s, s2, s, T, s2, 1.0f,
-                         K_FROM_ROW);
+        float *L21 = A + (b0 + s) * lda + b0, *W22 = A + (b0 + s) * lda + b0 + s;
+        const int r = multiply(stream, product(s2, s, s2, false), base + l.merge, W22, lda, false,
+                               reinterpret_cast<float*>(base + l.left_at(s)), s2, s2, s, s2, L21, lda, -1.0f, K_TO_ROW);
         if (r != TB_OK) return r;
-        r = multiply(stream, product(s2, s, s2, false), at, W22, lda, false, T, s2, s2, s, s2, L21, lda, -1.0f,
-                     K_TO_ROW);
-        if (r != TB_OK) return r;
-        TB_CUDA(cudaMemset2DAsync(W11 + s, (size_t)lda * sizeof(float), 0, (size_t)s2 * sizeof(float), (size_t)s, stream));
+        TB_CUDA(cudaMemset2DAsync(A + b0 * lda + b0 + s, (size_t)lda * sizeof(float), 0, (size_t)s2 * sizeof(float), (size_t)s,
+                                  stream));
         return TB_OK;
     };
 
@@ -747,12 +753,18 @@ int tb_spd_inverse(int device, void* stream_, float* A, int64_t k, int64_t lda, 
             }
         }
 
-        // 3. The inverted blocks so far that complete a pair, and the pairs of pairs.
+        // 3. The inverted blocks so far that complete a pair, and the pairs of pairs; then the first product of the
+        // pair whose left half is now complete.
         const int64_t done = o + kb;
-        for (int64_t s = OUTER; s < done; s *= 2) {
+        int64_t s = OUTER;
+        for (; s < done; s *= 2) {
             if (done < k && done % (2 * s) != 0) break;
             const int64_t b0 = (done - 1) / (2 * s) * (2 * s);
             if (b0 + s < done && (rc = merge(b0, s, done - b0 - s)) != TB_OK) return rc;
+        }
+        if (done < k) {  // s is now the largest level that divides `done`
+            if ((rc = wait(stream, side.s.packed)) != TB_OK) return rc;
+            if ((rc = merge_left(done - s, s, std::min<int64_t>(s, k - done))) != TB_OK) return rc;
         }
     }
     TB_CUDA(cudaGetLastError());
