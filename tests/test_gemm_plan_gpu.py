@@ -72,3 +72,25 @@ def test_inverse_of_several_block_columns(cuda, k):
         return all(torch.equal(o, got) for o in out)
     with ThreadPoolExecutor(3) as pool:
         assert all(pool.map(again, range(3)))
+
+
+@pytest.mark.parametrize("m, n, k", [(1, 1, 1), (129, 257, 33), (3000, 512, 1100)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_product_in_two_steps(cuda, m, n, k, dtype):
+    from trak_b200 import score_computers as sc
+    gen = torch.Generator(device=cuda).manual_seed(m + n)
+    a = torch.randn(m, k, device=cuda, generator=gen).to(dtype)
+    b = torch.zeros(n, k, device=cuda, dtype=dtype)
+    values = torch.randn(n, k, device=cuda, generator=gen).to(dtype)
+    scale = torch.rand(m, device=cuda, generator=gen)
+    got = sc.gemm_nt(a, b, row_scale=scale, b_ready=lambda: b.copy_(values))
+    assert torch.equal(got, sc.gemm_nt(a, values, row_scale=scale))
+
+
+def test_features_of_a_matrix_packed_beside_the_inverse(cuda, monkeypatch):
+    from trak_b200 import score_computers as sc
+    x = torch.randn(5000, 1100, device=cuda, generator=torch.Generator(device=cuda).manual_seed(3))
+    one = sc.B200ScoreComputer(torch.float32, cuda, 1100)
+    want = one.get_x_xtx_inv(x, one.get_xtx(x))
+    monkeypatch.setattr(sc.B200ScoreComputer, "APART_BYTES", 0)
+    assert torch.equal(one.get_x_xtx_inv(x, one.get_xtx(x)), want)

@@ -1011,14 +1011,15 @@ size_t tb_gemm_nt_workspace_bytes(int dtype, int64_t M, int64_t N, int64_t K) {
     return a.bytes + b.bytes + tb::plan_gemm(a.npl, false, false, M, N, a.kblocks).partial_bytes + 1024;
 }
 
-int tb_gemm_nt(int device, void* stream_, const void* A, int64_t lda, const void* B, int64_t ldb, int dtype,
-               int64_t M, int64_t N, int64_t K, float* C, int64_t ldc, const float* row_scale, float alpha,
-               int accumulate, void* ws, size_t ws_bytes) {
+// The parts of tb_gemm_nt: A packed at the workspace's start, B packed behind it and the product.
+static int gemm_nt_parts(int device, void* stream_, const void* A, int64_t lda, const void* B, int64_t ldb, int dtype,
+                         int64_t M, int64_t N, int64_t K, float* C, int64_t ldc, const float* row_scale, float alpha,
+                         int accumulate, void* ws, size_t ws_bytes) {
     using namespace tb;
     if (dtype != TB_F16 && dtype != TB_BF16 && dtype != TB_F32) return TB_ERR_BAD_DTYPE;
     if (M <= 0 || N <= 0 || K <= 0 || lda < K || ldb < K || ldc < N || M > 0x7fffffff || N > 0x7fffffff)
         return TB_ERR_BAD_SHAPE;
-    if (!A || !B || !C) return TB_ERR_BAD_ARG;
+    if (!A && !B) return TB_ERR_BAD_ARG;
     if (!ws || ((uintptr_t)ws & 255u) != 0 || ws_bytes < tb_gemm_nt_workspace_bytes(dtype, M, N, K))
         return TB_ERR_WORKSPACE;
     int sm_count = 0;
@@ -1032,16 +1033,34 @@ int tb_gemm_nt(int device, void* stream_, const void* A, int64_t lda, const void
     uint16_t* pa = static_cast<uint16_t*>(ws);
     uint16_t* pb = reinterpret_cast<uint16_t*>(static_cast<uint8_t*>(ws) + ga.bytes);
     float* partial = reinterpret_cast<float*>(static_cast<uint8_t*>(ws) + ga.bytes + gb.bytes);
-    if (dtype == TB_F32) {
+    if (A && B && dtype == TB_F32) {
         rc = launch_pack_rows(pack_rows_args(A, M, K, lda, pa, ga), pack_rows_args(B, N, K, ldb, pb, gb), sm_count, stream);
         if (rc != TB_OK) return rc;
     } else {
-        rc = launch_pack(A, dtype, false, M, K, lda, pa, ga, sm_count, stream);
-        if (rc != TB_OK) return rc;
-        rc = launch_pack(B, dtype, false, N, K, ldb, pb, gb, sm_count, stream);
-        if (rc != TB_OK) return rc;
+        if (A && (rc = launch_pack(A, dtype, false, M, K, lda, pa, ga, sm_count, stream)) != TB_OK) return rc;
+        if (B && (rc = launch_pack(B, dtype, false, N, K, ldb, pb, gb, sm_count, stream)) != TB_OK) return rc;
     }
+    if (!B) return TB_OK;
     return launch_gemm(device, stream, pa, ga, pb, gb, dtype, M, N, C, ldc, row_scale, alpha, accumulate, 0, 0, partial);
+}
+
+int tb_gemm_nt(int device, void* stream, const void* A, int64_t lda, const void* B, int64_t ldb, int dtype, int64_t M,
+               int64_t N, int64_t K, float* C, int64_t ldc, const float* row_scale, float alpha, int accumulate, void* ws,
+               size_t ws_bytes) {
+    const bool all = A && B && C;  // none of them: a bad type or shape is still reported before a missing matrix
+    return gemm_nt_parts(device, stream, all ? A : nullptr, lda, all ? B : nullptr, ldb, dtype, M, N, K, C, ldc, row_scale,
+                         alpha, accumulate, ws, ws_bytes);
+}
+
+int tb_gemm_nt_pack(int device, void* stream, const void* A, int64_t lda, int dtype, int64_t M, int64_t N, int64_t K,
+                    void* ws, size_t ws_bytes) {
+    return gemm_nt_parts(device, stream, A, lda, nullptr, K, dtype, M, N, K, nullptr, N, nullptr, 1.0f, 0, ws, ws_bytes);
+}
+
+int tb_gemm_nt_packed(int device, void* stream, const void* B, int64_t ldb, int dtype, int64_t M, int64_t N, int64_t K,
+                      float* C, int64_t ldc, const float* row_scale, float alpha, int accumulate, void* ws, size_t ws_bytes) {
+    return gemm_nt_parts(device, stream, nullptr, K, C ? B : nullptr, ldb, dtype, M, N, K, C, ldc, row_scale, alpha,
+                         accumulate, ws, ws_bytes);
 }
 
 size_t tb_gram_workspace_bytes(int dtype, int64_t n, int64_t k) {

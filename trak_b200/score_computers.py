@@ -54,27 +54,34 @@ class StreamPair:
     (row maxima, fp16 hi / lo planes) followed by a tensor-core GEMM; on one stream the packing of block i + 1
     waits for the GEMM of block i although the two use different parts of the SM.  With blocks alternating
     between two streams the packing (and any host-to-device copy) of one block runs under the GEMM of the other.
-    Inside ``with pair:`` the side streams first wait for the caller's stream, and the caller's stream waits for
-    both on exit; ``with pair.stream(i):`` makes stream ``i % 2`` current.  Work that touches the same memory
+    Inside ``with pair:`` a side stream waits for what the caller's stream had been given on entry, and the caller's
+    stream waits on exit for the side streams that were used; ``with pair.stream(i):`` makes stream ``i % 2`` current.  Work that touches the same memory
     from consecutive blocks (an accumulator, a reused buffer) must be given one buffer per stream."""
 
     def __init__(self, device):
         self.device = torch.device(device)
         self.streams = [torch.cuda.Stream(self.device), torch.cuda.Stream(self.device)]
+        self.entered, self.done = torch.cuda.Event(), [torch.cuda.Event(), torch.cuda.Event()]
 
     def __enter__(self):
         self.main = torch.cuda.current_stream(self.device)
-        for s in self.streams:
-            s.wait_stream(self.main)
+        self.entered.record(self.main)
+        self.used = [False, False]
         return self
 
     def __exit__(self, *exc):
-        for s in self.streams:
-            self.main.wait_stream(s)
+        for s, done, used in zip(self.streams, self.done, self.used):
+            if used:
+                done.record(s)
+                self.main.wait_event(done)
         return False
 
     def stream(self, i: int):
-        return torch.cuda.stream(self.streams[i % 2])
+        s = self.streams[i % 2]
+        if not self.used[i % 2]:
+            self.used[i % 2] = True
+            s.wait_event(self.entered)
+        return torch.cuda.stream(s)
 
     def current(self, i: int):
         return self.streams[i % 2]
@@ -174,9 +181,14 @@ def _launch_spd_inverse(a: torch.Tensor, lambda_reg: float, rescale: bool) -> No
 
 
 def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, row_scale: torch.Tensor = None,
-            alpha: float = 1.0, accumulate: bool = False) -> torch.Tensor:
-    """fp32 [M, N] = alpha * row_scale[:, None] * a @ b.T (+ out) for CUDA a [M, K], b [N, K]."""
+            alpha: float = 1.0, accumulate: bool = False, b_ready=None) -> torch.Tensor:
+    """fp32 [M, N] = alpha * row_scale[:, None] * a @ b.T (+ out) for CUDA a [M, K], b [N, K].
+
+    ``b_ready`` makes the current stream wait for ``b``; it is called when ``a`` has been laid out for the product."""
     if a.dtype != b.dtype:
+        if b_ready is not None:
+            b_ready()
+            b_ready = None
         a, b = a.float(), b.float()
     M, K = a.shape
     N = b.shape[0]
@@ -195,10 +207,18 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, row_scal
         stream = _lib.current_stream(dev)
         dt = _DTYPES[a.dtype]
         ws = _workspace(dev, stream, lib.tb_gemm_nt_workspace_bytes(dt, M, N, K))
-        _lib.check(lib.tb_gemm_nt(dev.index, stream, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), dt,
-                                  M, N, K, out.data_ptr(), out.stride(0),
-                                  row_scale.data_ptr() if row_scale is not None else None, float(alpha),
-                                  int(accumulate), ws.data_ptr(), ws.numel()))
+        scale = row_scale.data_ptr() if row_scale is not None else None
+        if b_ready is not None:
+            _lib.check(lib.tb_gemm_nt_pack(dev.index, stream, a.data_ptr(), a.stride(0), dt, M, N, K, ws.data_ptr(),
+                                           ws.numel()))
+            b_ready()
+            _lib.check(lib.tb_gemm_nt_packed(dev.index, stream, b.data_ptr(), b.stride(0), dt, M, N, K, out.data_ptr(),
+                                             out.stride(0), scale, float(alpha), int(accumulate), ws.data_ptr(),
+                                             ws.numel()))
+        else:
+            _lib.check(lib.tb_gemm_nt(dev.index, stream, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), dt, M, N,
+                                      K, out.data_ptr(), out.stride(0), scale, float(alpha), int(accumulate),
+                                      ws.data_ptr(), ws.numel()))
     return out
 
 
@@ -250,8 +270,9 @@ class B200ScoreComputer:
         result = torch.empty(grads.shape[0], xtx.shape[1], dtype=self.dtype, device=self.device)
         start = 0
         blocks = self._blocks(grads)
-        with _lib.on_device(self.device), self._pair(len(blocks) > 1 or not grads.is_cuda) as pair:
-            # the pair's streams do not wait for the inverse: the blocks are copied and converted meanwhile
+        apart = len(blocks) > 1 or not grads.is_cuda or grads.numel() * grads.element_size() >= self.APART_BYTES
+        with _lib.on_device(self.device), self._pair(apart) as pair:
+            # the pair's streams do not wait for the inverse: the blocks are copied, converted and packed meanwhile
             inv = xtx.to(self.device, torch.float32, copy=True)
             _launch_spd_inverse(inv, self.lambda_reg, rescale=True)
             inv = inv.to(self.dtype)
@@ -265,15 +286,18 @@ class B200ScoreComputer:
                 with pair.stream(i):
                     blk = _as_device_matrix(block, self.device).to(inv.dtype)
                     pair.uses(blk)
-                    pair.after(inverted)
+                    ready = (lambda: pair.after(inverted)) if apart else None
                     # the inverse is symmetric, so block @ inv == block @ inv.T
                     if result.dtype == torch.float32:
-                        gemm_nt(blk, inv, out=result[rows])
+                        gemm_nt(blk, inv, out=result[rows], b_ready=ready)
                     else:
-                        result[rows] = gemm_nt(blk, inv).to(self.dtype)
+                        result[rows] = gemm_nt(blk, inv, b_ready=ready).to(self.dtype)
         _lib.stream_status(self.device.index, _lib.current_stream(self.device))  # raises NotPositiveDefinite / DeviceTimeout
         return result
 
+    # A device matrix from this size on is packed on a stream of its own while the inverse, which leaves most of the device
+    # idle, is computed: that hides 40 us and more (126 us at 50,000 x 2048 fp32) for about 20 us of host time.
+    APART_BYTES = 128 << 20
     UPLOAD_BYTES = 96 << 20  # about so many bytes of a host matrix are uploaded at a time, under the work on the last
 
     def _blocks(self, t: torch.Tensor, rows: int = None):
