@@ -26,7 +26,8 @@ def test_gemm_nt(cuda, M, N, K, dtype):
     assert rel(sc.gemm_nt(a, b, out=got.clone(), row_scale=w, accumulate=True), 2 * want) <= 3e-5
 
 
-@pytest.mark.parametrize("n,k", [(5000, 40), (4097, 129), (3001, 512), (20000, 300), (100, 700), (1, 5)])
+@pytest.mark.parametrize("n,k", [(5000, 40), (4097, 129), (3001, 512), (20000, 300), (100, 700), (1, 5), (513, 17), (1030, 145),
+                                 (2048, 300), (2049, 31)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
 def test_gram(cuda, n, k, dtype):
     from trak_b200 import score_computers as sc

@@ -647,6 +647,58 @@ __global__ void amax_cols_kernel(const float* __restrict__ src, uint32_t* __rest
     atomicMax(&amax[R], m);
 }
 
+// The same and the packing in one launch for up to J * 256 source rows: a CTA keeps 16 source columns in registers, 8
+// consecutive k at a time per thread, finds their maxima and writes both planes.  Bound by latency: a memset, the maxima
+// and the packing were three launches of 1 to 8 us with gaps as long (Gram of 2048 x 2048: 70 -> 60 us in all, 2000 x 8192: 430 -> 408).  Longer columns do
+// not fit and go through the two kernels, which stream them.
+template <int J>
+__global__ void __launch_bounds__(512) pack_cols_f32_kernel(const float* __restrict__ src, uint16_t* __restrict__ packed,
+                                                            uint32_t* __restrict__ amax, uint64_t rows, uint64_t K,
+                                                            uint64_t ld, uint32_t kblocks) {
+    __shared__ uint32_t warp_max[16][16];
+    const uint32_t c = threadIdx.x & 15u, group = threadIdx.x >> 4, warp = threadIdx.x >> 5;
+    const uint64_t R = (uint64_t)blockIdx.x * 16u + c, span_k = (uint64_t)kblocks * 32u;
+    const bool live = R < rows;
+    float x[J][8];
+    uint32_t m = 0;
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const uint64_t k = (uint32_t)(j * 256 + e) + group * 8u;
+            x[j][e] = (live && k < K) ? __ldg(src + k * ld + R) : 0.0f;
+        }
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) m = max(m, __float_as_uint(x[j][e]) & 0x7fffffffu);
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
+    if ((threadIdx.x & 16u) == 0) warp_max[warp][c] = m;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 16; ++w) m = max(m, warp_max[w][c]);
+    if (live && group == 0) amax[R] = m;
+    const float up = row_scale_up(m);
+    uint16_t* out = packed + ((R >> 7) * kblocks * 256u + (R & 127u)) * 32u;
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+        const uint32_t k = (uint32_t)j * 256u + group * 8u;
+        if (k >= span_k) continue;
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float u = x[j][2 * e] * up, v = x[j][2 * e + 1] * up;
+            const __half2 h = __floats2half2_rn(u, v);
+            const __half2 l = __floats2half2_rn(u - __low2float(h), v - __high2float(h));
+            hi[e] = *reinterpret_cast<const uint32_t*>(&h);
+            lo[e] = *reinterpret_cast<const uint32_t*>(&l);
+        }
+        uint16_t* dst = out + (k >> 5) * (256u * 32u) + (k & 31u);
+        *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(dst + 128u * 32u) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
+}
+
 // ---- packing ---------------------------------------------------------------------------
 // packed[((rb*kblocks + kb)*planes + pl)*128 + r][kk]  (16-bit), r < 128, kk < 32:
 //   operand row  R = rb*128 + r,  k = kb*32 + kk;
@@ -845,6 +897,14 @@ int launch_pack(const void* src, int dtype, bool trans, uint64_t rows, uint64_t 
     if (dtype == TB_F32) {
         const float* s = static_cast<const float*>(src);
         uint32_t* amax = packed_amax(packed, g);
+        if (K <= 2048u) {
+            const uint32_t nb = g.rowblocks * 8u;
+            if (K <= 512u) pack_cols_f32_kernel<2><<<nb, 512, 0, stream>>>(s, packed, amax, rows, K, ld, g.kblocks);
+            else if (K <= 1024u) pack_cols_f32_kernel<4><<<nb, 512, 0, stream>>>(s, packed, amax, rows, K, ld, g.kblocks);
+            else pack_cols_f32_kernel<8><<<nb, 512, 0, stream>>>(s, packed, amax, rows, K, ld, g.kblocks);
+            TB_CUDA(cudaGetLastError());
+            return TB_OK;
+        }
         TB_CUDA(cudaMemsetAsync(amax, 0, (size_t)g.rowblocks * 128u * sizeof(uint32_t), stream));
         const uint32_t bx = (uint32_t)((rows + 255) / 256);
         uint64_t by = ((uint64_t)sm_count * 16 + bx - 1) / bx;  // about 16 CTAs per SM in all
