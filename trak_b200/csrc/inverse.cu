@@ -462,7 +462,8 @@ __global__ void __launch_bounds__(256) abs_partial_kernel(const float* A, int64_
     }
     if (threadIdx.x == 0) partial[blockIdx.x] = sh[0];
 }
-__global__ void __launch_bounds__(256) abs_final_kernel(const double* partial, int k, float* mean_out) {
+// The mean of |entry| from the partial sums, the same in every CTA (256 threads).
+__device__ float mean_abs(const double* partial, int k) {
     __shared__ double sh[256];
     double s = 0.0;
     for (int e = threadIdx.x; e < RED_BLOCKS; e += 256) s += partial[e];
@@ -472,10 +473,17 @@ __global__ void __launch_bounds__(256) abs_final_kernel(const double* partial, i
         if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
         __syncthreads();
     }
-    if (threadIdx.x == 0) *mean_out = (float)(sh[0] / ((double)k * (double)k));
+    return (float)(sh[0] / ((double)k * (double)k));
 }
-__global__ void scale_by_inverse_kernel(float* A, int64_t lda, int k, const float* mean) {
-    const float inv = 1.0f / *mean;
+__global__ void __launch_bounds__(256) abs_final_kernel(const double* partial, int k, float* mean_out) {
+    const float mean = mean_abs(partial, k);
+    if (threadIdx.x == 0) *mean_out = mean;
+}
+// Every CTA sums the 8 KB of partial sums itself (about 1 us) instead of waiting for a launch that does.
+__global__ void __launch_bounds__(256) scale_by_inverse_kernel(float* A, int64_t lda, int k, const double* partial,
+                                                               float* mean_out) {
+    const float mean = mean_abs(partial, k), inv = 1.0f / mean;
+    if (mean_out && blockIdx.x == 0 && threadIdx.x == 0) *mean_out = mean;
     const bool vec = rows_are_vec4(A, lda, k);
     for (int i = blockIdx.x; i < k; i += gridDim.x) {
         float* row = A + (int64_t)i * lda;
@@ -507,7 +515,7 @@ static Product product(int64_t m, int64_t n, int64_t kk, bool symmetric) {
 }
 
 struct InvLayout {
-    size_t dinv, blocks, partial, mean, counters, chain, rest, left, merge, total;
+    size_t dinv, blocks, partial, counters, chain, rest, left, merge, total;
     // the merges' first products: one per level is waiting for its second at a time
     size_t left_at(int64_t s) const {
         size_t at = left;
@@ -524,8 +532,6 @@ static InvLayout inv_layout(int64_t k) {
     off += 2u * OUTER * OUTER * sizeof(float);
     l.partial = off;
     off += align_up(RED_BLOCKS * sizeof(double), 256);
-    l.mean = off;
-    off += 256;
     l.counters = off;
     off += align_up((size_t)((k + OUTER - 1) / OUTER) * sizeof(uint32_t), 256);
     // what the block columns, the rest of their updates and the merges use at the same time
@@ -638,7 +644,6 @@ int tb_spd_inverse(int device, void* stream_, float* A, int64_t k, int64_t lda, 
     float* dinv = reinterpret_cast<float*>(base + l.dinv);
     float* blocks = reinterpret_cast<float*>(base + l.blocks);
     double* partial = reinterpret_cast<double*>(base + l.partial);
-    float* mean = reinterpret_cast<float*>(base + l.mean);
     const int K = (int)k;
 
     // The block columns, the rest of their updates and the merges run on three streams where there is more than one
@@ -777,10 +782,10 @@ int tb_spd_inverse(int device, void* stream_, float* A, int64_t k, int64_t lda, 
     // mean |entry| and the reference's rescale
     if (rescale_by_mean_abs || mean_abs_out) {
         abs_partial_kernel<<<RED_BLOCKS, 256, 0, stream>>>(A, lda, K, partial);
-        abs_final_kernel<<<1, 256, 0, stream>>>(partial, K, mean);
-        if (mean_abs_out)
-            TB_CUDA(cudaMemcpyAsync(mean_abs_out, mean, sizeof(float), cudaMemcpyDeviceToDevice, stream));
-        if (rescale_by_mean_abs) scale_by_inverse_kernel<<<sm_count * 8, 256, 0, stream>>>(A, lda, K, mean);
+        if (rescale_by_mean_abs)
+            scale_by_inverse_kernel<<<std::min(K, sm_count * 8), 256, 0, stream>>>(A, lda, K, partial, mean_abs_out);
+        else
+            abs_final_kernel<<<1, 256, 0, stream>>>(partial, K, mean_abs_out);
     }
     TB_CUDA(cudaGetLastError());
     return TB_OK;
