@@ -649,8 +649,8 @@ __global__ void amax_cols_kernel(const float* __restrict__ src, uint32_t* __rest
 
 // The same and the packing in one launch for up to J * 256 source rows: a CTA keeps 16 source columns in registers, 8
 // consecutive k at a time per thread, finds their maxima and writes both planes.  Bound by latency: a memset, the maxima
-// and the packing were three launches of 1 to 8 us with gaps as long (Gram of 2048 x 2048: 70 -> 60 us in all, 2000 x 8192: 430 -> 408).  Longer columns do
-// not fit and go through the two kernels, which stream them.
+// and the packing were three launches of 1 to 8 us with gaps as long (Gram of 2048 x 2048: 70 -> 60 us in all,
+// 2000 x 8192: 430 -> 408).  Longer columns do not fit and go through the two kernels, which stream them.
 template <int J>
 __global__ void __launch_bounds__(512) pack_cols_f32_kernel(const float* __restrict__ src, uint16_t* __restrict__ packed,
                                                             uint32_t* __restrict__ amax, uint64_t rows, uint64_t K,
