@@ -45,6 +45,8 @@ def host_to_device(src, device) -> torch.Tensor:
     """A copy of a C-contiguous numpy array or CPU tensor on a CUDA device, ordered on its current stream; ``src``
     has been read when the call returns."""
     device = torch.device(device)
+    if not (src.flags.c_contiguous if isinstance(src, np.ndarray) else src.is_contiguous() and src.device.type == "cpu"):
+        raise ValueError("the source must be contiguous host memory")
     if isinstance(src, np.ndarray):
         dtype, ptr, nbytes = _TORCH[src.dtype], src.ctypes.data, src.nbytes
     else:
@@ -59,7 +61,16 @@ def host_to_device(src, device) -> torch.Tensor:
 def device_to_host(dst, src: torch.Tensor, stream=None, add: bool = False) -> None:
     """Copies a contiguous CUDA tensor over a C-contiguous host array or CPU tensor of the same size and dtype (or,
     fp32 only, adds it), ordered on ``stream`` (default: the device's current one); complete on return."""
-    ptr = dst.ctypes.data if isinstance(dst, np.ndarray) else dst.data_ptr()
+    array = isinstance(dst, np.ndarray)
+    # the library's threads write from the bare pointer on: nothing behind this call looks at shapes or types any more
+    if tuple(dst.shape) != tuple(src.shape):
+        raise ValueError(f"{list(src.shape)} values do not fit a host array of shape {list(dst.shape)}")
+    if (_TORCH.get(dst.dtype) if array else dst.dtype) != src.dtype or (add and src.dtype != torch.float32):
+        raise ValueError(f"cannot {'add' if add else 'copy'} {src.dtype} values to a host array of {dst.dtype}")
+    if not (dst.flags.c_contiguous if array else dst.is_contiguous() and dst.device.type == "cpu") \
+            or not src.is_contiguous():
+        raise ValueError("source and destination must be contiguous, the destination in host memory")
+    ptr = dst.ctypes.data if array else dst.data_ptr()
     with torch.cuda.device(src.device):
         stream = torch.cuda.current_stream(src.device) if stream is None else stream
         _lib.check(_lib.lib().tb_device_to_host(src.device.index, stream.cuda_stream, ptr, src.data_ptr(),

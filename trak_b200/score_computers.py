@@ -143,13 +143,38 @@ def _as_device_matrix(t: torch.Tensor, device) -> torch.Tensor:
     return t
 
 
+def _check_operand(t: torch.Tensor, device) -> None:
+    if t.dim() != 2 or t.device != device or not t.is_cuda or (t.shape[1] > 1 and t.stride(1) != 1):
+        raise RuntimeError("expected CUDA matrices with unit column stride on one device")
+
+
+def _check_out(out: torch.Tensor, rows: int, cols: int, device) -> None:
+    """The kernels write ``rows`` x ``cols`` floats from ``out``'s pointer on: anything else would be written past its
+    end, or not where the caller looks."""
+    if out.device != device or out.dtype != torch.float32 or tuple(out.shape) != (rows, cols) \
+            or (cols > 1 and out.stride(1) != 1):
+        raise RuntimeError(f"out must be a float32 [{rows}, {cols}] tensor with unit column stride on the operands' device")
+
+
+def _check_accumulator(n: int, m: int, accumulator: torch.Tensor, row_scale) -> None:
+    """Raises before anything is queued where ``accumulator += [n, m] scores`` is not defined.  Rows beyond ``n`` are
+    left as they are; a single column of scores is added to every column, as torch's broadcasting has it."""
+    if accumulator.dim() != 2 or accumulator.shape[0] < n or (accumulator.shape[1] != m and m != 1):
+        raise RuntimeError(f"accumulator of shape {list(accumulator.shape)} does not hold [{n}, {m}] scores")
+    if row_scale is not None and row_scale.numel() < n:
+        raise RuntimeError("row_scale must have one entry per row of the features")
+
+
 def gram(x: torch.Tensor, out: torch.Tensor = None, accumulate: bool = False) -> torch.Tensor:
     """fp32 [k, k] = x^T x (+ out) for a CUDA matrix x [n, k] (fp16 / bf16 / fp32)."""
     n, k = x.shape
     dev = x.device
+    _check_operand(x, dev)
     if out is None:
         out = torch.empty((k, k), dtype=torch.float32, device=dev)
         accumulate = False
+    else:
+        _check_out(out, k, k, dev)
     lib = _lib.lib()
     with _lib.on_device(dev):
         stream = _lib.current_stream(dev)
@@ -195,9 +220,13 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, row_scal
     if b.shape[1] != K:
         raise RuntimeError("inner dimensions differ")
     dev = a.device
+    _check_operand(a, dev)
+    _check_operand(b, dev)
     if out is None:
         out = torch.empty((M, N), dtype=torch.float32, device=dev)
         accumulate = False
+    else:
+        _check_out(out, M, N, dev)
     if row_scale is not None:
         row_scale = row_scale.to(dev, torch.float32).reshape(-1).contiguous()
         if row_scale.numel() != M:
@@ -325,6 +354,7 @@ class B200ScoreComputer:
         TRAKer keeps the accumulator on the host (trak/traker.py:632): the product then leaves the GPU in row
         blocks of at most ``HOST_STAGE_BYTES``, copied and added by several host threads while the GPU multiplies
         the next block, instead of one synchronous pageable copy per block."""
+        _check_accumulator(features.shape[0], target_grads.shape[0], accumulator, row_scale)
         self._accumulate_products(features, _as_device_matrix(target_grads, self.device), accumulator, row_scale)
 
     def get_scores_from_grads(self, grads: torch.Tensor, xtx: torch.Tensor, target_grads: torch.Tensor,
@@ -334,6 +364,7 @@ class B200ScoreComputer:
         ``xtx`` exactly as ``get_x_xtx_inv`` forms it (trak/score_computers.py:157-168).  One product over
         the train rows instead of two: ``2 k^2 m`` flop for ``inv @ target_grads.T`` replace the ``2 n k^2``
         of the features.  For callers that do not need the features themselves (TRAKer stores them)."""
+        _check_accumulator(grads.shape[0], target_grads.shape[0], accumulator, row_scale)
         inv = xtx.to(self.device, torch.float32, copy=True)
         spd_inverse_(inv, self.lambda_reg, rescale=True)   # raises before anything is added to the accumulator
         targets = _as_device_matrix(target_grads, self.device)
@@ -343,10 +374,11 @@ class B200ScoreComputer:
     def _accumulate_products(self, features, targets, accumulator, row_scale):
         m = targets.shape[0]
         on_host = accumulator.device.type == "cpu"
+        exact = accumulator.shape[1] == m and not accumulator.requires_grad  # else torch's own += decides
         step = self.CUDA_MAX_DIM_SIZE
         if on_host:
             step = max(256, min(step, self.HOST_STAGE_BYTES // (4 * m) // 256 * 256))
-            threaded = accumulator.dtype == torch.float32 and accumulator.is_contiguous()
+            threaded = exact and accumulator.dtype == torch.float32 and accumulator.is_contiguous()
         pending = None
 
         def flush(item):
@@ -368,7 +400,7 @@ class B200ScoreComputer:
                     pair.uses(blk)
                     rs = None if row_scale is None else row_scale.reshape(-1)[rows]
                     into = accumulator[rows]
-                    if into.device == blk.device and into.dtype == torch.float32 and into.stride(1) == 1 \
+                    if exact and into.device == blk.device and into.dtype == torch.float32 and into.stride(1) == 1 \
                             and into.stride(0) >= m:
                         gemm_nt(blk, targets, out=into, row_scale=rs, accumulate=True)  # the epilogue's += is the same
                         continue
