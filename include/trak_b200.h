@@ -231,7 +231,8 @@ int tb_finalize_scores(int device, void *stream, const float *score_sum, int64_t
  * process exits).  Meant for hosts that cannot allocate device memory themselves,
  * e.g. a plugin in a process whose device memory already belongs to another
  * component's pool, or a serving loop that must avoid the device-wide
- * synchronisation of cudaMalloc / cudaFree.  The call allocates nothing.
+ * synchronisation of cudaMalloc / cudaFree.  The call allocates neither device nor
+ * pinned host memory (a tb_stream_status after it may take a word of the latter).
  *
  *   - shapes with tb_project_workspace_bytes(...) > TB_PROJECT_STATIC_SCRATCH_BYTES
  *     are refused with TB_ERR_SCRATCH_LIMIT

@@ -1,0 +1,56 @@
+"""The status word on its way to the host: what a call takes from the driver for it, and whose status a read reports."""
+import threading
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+B, F, N, TILES = 16, 50021, 1024, 148
+
+
+def _call(lib, dev, name, g, out, ws=None, nbytes=None):
+    stream = torch.cuda.current_stream(dev).cuda_stream
+    args = [dev.index, stream, g.data_ptr(), 0, g.shape[0], g.shape[1], g.stride(0), out.data_ptr(), N, N, 17, TILES, 0,
+            1.0, 0]
+    if name == "tb_project":
+        args += [ws.data_ptr(), ws.numel() if nbytes is None else nbytes]
+    return getattr(lib, name)(*args)
+
+
+@pytest.fixture
+def job(cuda):
+    from trak_b200 import _lib
+    lib = _lib.lib()
+    g = (torch.randn(B, F, device=cuda) * 1e-2).half()
+    ws = torch.empty(lib.tb_project_workspace_bytes(0, B, F, N, TILES), dtype=torch.uint8, device=cuda)
+    out = torch.empty(B, N, device=cuda)
+    for name in ("tb_project", "tb_project_static"):   # the one-time set-up of this device, before any capture
+        assert _call(lib, cuda, name, g, out, ws) == 0
+    torch.cuda.synchronize()
+    return lib, g, out, ws
+
+
+@pytest.mark.parametrize("name", ["tb_project_static"])
+def test_first_call_of_a_thread_can_be_captured(cuda, job, name):
+    """A thread's first call allocates nothing: under a capture an allocation would be refused and end it."""
+    lib, g, want, ws = job
+    got, codes = torch.zeros_like(want), []
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream(cuda)
+    torch.cuda.synchronize()
+
+    def work():
+        with torch.cuda.stream(stream):
+            graph.capture_begin(capture_error_mode="global")
+            try:
+                codes.append(_call(lib, cuda, name, g, got, ws))
+            finally:
+                graph.capture_end()
+
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    assert codes == [0], lib.tb_last_cuda_error()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)

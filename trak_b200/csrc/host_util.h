@@ -29,6 +29,12 @@ int select_device(int device, int* sm_count);
 int validate_project_args(const void* grads, int dtype, int64_t B, int64_t F, int64_t ld, const float* out,
                           int64_t ld_out, uint32_t N, uint32_t num_feature_tiles, int proj_type);
 
+// tb_project; with `publish` its last launch stores the status word to pinned host memory (arm_status), without it the
+// call takes no memory of any kind from the driver.
+int project_dense(int device, void* stream, const void* grads, int dtype, int64_t B, int64_t F, int64_t ld, float* out,
+                  int64_t ld_out, uint32_t N, uint32_t seed, uint32_t num_feature_tiles, int proj_type, float alpha,
+                  int accumulate, void* ws, size_t ws_bytes, bool publish);
+
 // Device address of the status word of `device` (valid after select_device).
 uint32_t* status_ptr(int device);
 

@@ -7,8 +7,8 @@
 // handed out in full to another component's pool, or a latency-critical loop that must
 // not run into the device-wide synchronisation a cudaMalloc / cudaFree implies.  For them
 // this entry point keeps the scratch in a fixed array that is part of the loaded module.
-// Nothing is allocated here or anywhere below it: no cudaMalloc, no cudaFree, no library
-// routine that allocates.
+// No device memory and no pinned host memory is allocated here or anywhere below it: no
+// cudaMalloc, no cudaFree, no cudaHostAlloc, no library routine that does.
 #include <mutex>
 
 #include "host_util.h"
@@ -66,6 +66,8 @@ extern "C" int tb_project_static(int device, void* stream, const void* grads, in
     // Every scratch byte the kernels read (staged gradients including their zero padding,
     // partial sums) is written earlier in the same call, so nothing has to start at zero
     // and the previous call's leftovers are harmless.
-    return tb_project(device, stream, grads, dtype, B, F, ld, out, ld_out, N, seed, num_feature_tiles,
-                      proj_type, alpha, accumulate, scratch, tb::STATIC_SCRATCH_BYTES);
+    // No status word is published: that takes a word of pinned host memory, and this call allocates none.  A
+    // tb_stream_status after it reads the word with a launch of its own.
+    return tb::project_dense(device, stream, grads, dtype, B, F, ld, out, ld_out, N, seed, num_feature_tiles,
+                             proj_type, alpha, accumulate, scratch, tb::STATIC_SCRATCH_BYTES, false);
 }
