@@ -1,5 +1,6 @@
 """The status word on its way to the host: what a call takes from the driver for it, and whose status a read reports."""
 import threading
+from concurrent.futures import ThreadPoolExecutor
 
 import pytest
 import torch
@@ -31,9 +32,10 @@ def job(cuda):
     return lib, g, out, ws
 
 
-@pytest.mark.parametrize("name", ["tb_project_static"])
+@pytest.mark.parametrize("name", ["tb_project_static", "tb_project"])
 def test_first_call_of_a_thread_can_be_captured(cuda, job, name):
-    """A thread's first call allocates nothing: under a capture an allocation would be refused and end it."""
+    """A thread's first call allocates nothing: under a capture an allocation would be refused and end it.  (So no
+    memory is left behind by threads that end, either.)"""
     lib, g, want, ws = job
     got, codes = torch.zeros_like(want), []
     graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream(cuda)
@@ -54,3 +56,25 @@ def test_first_call_of_a_thread_can_be_captured(cuda, job, name):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(got, want)
+
+
+def test_a_word_that_was_handed_out_again_is_not_believed(cuda, job):
+    """More reads than there are words between a call and its status: the status comes from the device then."""
+    lib, g, out, ws = job
+    own, other = torch.cuda.Stream(cuda), torch.cuda.Stream(cuda)
+    torch.cuda.synchronize()
+    with ThreadPoolExecutor(1) as pool, torch.cuda.stream(own):
+        def call():
+            with torch.cuda.stream(own):
+                return _call(lib, cuda, "tb_project", g, out, ws)
+        assert pool.submit(call).result() == 0
+        for _ in range(1500):
+            assert lib.tb_stream_status(cuda.index, other.cuda_stream, None) == 0
+        assert pool.submit(lib.tb_stream_status, cuda.index, own.cuda_stream, None).result() == 0
+        assert pool.submit(call).result() == 0
+        for _ in range(1500):
+            assert lib.tb_stream_status(cuda.index, other.cuda_stream, None) == 0
+        assert lib.tb_selftest_wait_timeout(cuda.index, other.cuda_stream, 20) == 0
+        other.synchronize()
+        assert pool.submit(lib.tb_stream_status, cuda.index, own.cuda_stream, None).result() == 7
+    assert lib.tb_stream_status(cuda.index, own.cuda_stream, None) == 0

@@ -1,6 +1,7 @@
 // Library-wide pieces of the C ABI: version, error text, device selection,
 // the per-device status word and tensor-map encoding.
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <utility>
@@ -39,7 +40,7 @@ static uint32_t* g_dev_status_ptr[MAX_DEV];
 static thread_local struct {
     int device = -1;
     cudaStream_t stream = nullptr;
-    uint32_t* word = nullptr;
+    StatusNote note;
 } t_armed;
 
 int select_device(int device, int* sm_count) {
@@ -91,38 +92,52 @@ __global__ void selftest_wait_kernel(uint32_t* status, uint64_t limit_ns) {
     __syncthreads();
 }
 
-// Pinned words that status reads land in: taken for the length of a read, made as they are needed, at most as many as
-// threads ever read at once.
+// Where kernels store the status word for the host: one ring of pinned words per process, made on first use and never
+// given up, handed out in turn.  A word carries the number of the call it was handed out for beside the status, so it
+// needs no owner: when it has been handed out again and a kernel of either call stores to it late (a thread that ended
+// without waiting, the replay of a captured call), the reader sees a number that is not its own and asks the device.
+constexpr uint32_t STATUS_WORDS = 1024;
 static std::mutex g_words_mu;
-static std::vector<uint32_t*> g_words;
+static uint64_t* g_words = nullptr;
+static std::atomic<uint32_t> g_calls{0};
 
-static int take_word(uint32_t** word) {
+static int take_note(StatusNote* note) {
+    uint64_t* words;
     {
         std::lock_guard<std::mutex> lk(g_words_mu);
-        if (!g_words.empty()) {
-            *word = g_words.back();
-            g_words.pop_back();
-            return TB_OK;
+        if (!g_words) {
+            // a capture of any thread forbids allocations that are not told to be relaxed
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            TB_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+            void* p = nullptr;
+            const cudaError_t e = cudaHostAlloc(&p, STATUS_WORDS * sizeof(uint64_t), cudaHostAllocPortable | cudaHostAllocMapped);
+            TB_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+            TB_CUDA(e);
+            memset(p, 0, STATUS_WORDS * sizeof(uint64_t));
+            g_words = static_cast<uint64_t*>(p);
         }
+        words = g_words;
     }
-    TB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(word), sizeof(uint32_t), cudaHostAllocPortable | cudaHostAllocMapped));
+    do note->call = g_calls.fetch_add(1, std::memory_order_relaxed) + 1u;
+    while (note->call == 0);  // 0 is what a word holds that nothing has been stored to
+    note->word = words + note->call % STATUS_WORDS;
     return TB_OK;
 }
-// A store by the SM reaches the host some 8 us earlier than a copy engine that has to be set going.
-__global__ void publish_status_kernel(const uint32_t* status, uint32_t* word) { *word = *status; }
-static void give_word(uint32_t* word) {
-    std::lock_guard<std::mutex> lk(g_words_mu);
-    g_words.push_back(word);
+// After the kernel that stores it has ended: false where a later call has the word by now.
+static bool read_note(const StatusNote& note, uint32_t* status) {
+    const uint64_t v = *static_cast<volatile uint64_t*>(note.word);
+    *status = (uint32_t)v;
+    return (uint32_t)(v >> 32) == note.call;
 }
+// A store by the SM reaches the host some 8 us earlier than a copy engine that has to be set going.
+__global__ void publish_status_kernel(const uint32_t* status, StatusNote note) { publish_status(status, note); }
 
-int arm_status(int device, cudaStream_t stream, uint32_t** word) {
-    if (!t_armed.word) {  // one for the thread's life
-        const int rc = take_word(&t_armed.word);
-        if (rc != TB_OK) return rc;
-    }
+int arm_status(int device, cudaStream_t stream, StatusNote* note) {
+    const int rc = take_note(note);
+    if (rc != TB_OK) return rc;
     t_armed.device = device;
     t_armed.stream = stream;
-    *word = t_armed.word;
+    t_armed.note = *note;
     return TB_OK;
 }
 
@@ -245,23 +260,17 @@ int tb_stream_status(int device, void* stream_, uint32_t* detail) {
     const bool armed = tb::t_armed.device == device && tb::t_armed.stream == stream;
     int rc = tb::select_device(device, nullptr);
     if (rc != TB_OK) return rc;
-    if (armed) {
-        TB_CUDA(cudaStreamSynchronize(stream));
-        if (*static_cast<volatile uint32_t*>(tb::t_armed.word) != 0) return tb_device_status(device, detail);
-        if (detail) *detail = 0;
-        return TB_OK;
+    tb::StatusNote note = tb::t_armed.note;
+    if (!armed) {
+        rc = tb::take_note(&note);
+        if (rc != TB_OK) return rc;
+        // the read is queued behind the stream's work, so one wait serves both
+        tb::publish_status_kernel<<<1, 1, 0, stream>>>(tb::status_ptr(device), note);
+        TB_CUDA(cudaGetLastError());
     }
-    uint32_t* word = nullptr;
-    rc = tb::take_word(&word);
-    if (rc != TB_OK) return rc;
-    // the read is queued behind the stream's work, so one wait serves both
-    tb::publish_status_kernel<<<1, 1, 0, stream>>>(tb::status_ptr(device), word);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    const uint32_t code = *static_cast<volatile uint32_t*>(word);
-    if (e != cudaSuccess) TB_CUDA(e);  // the word may still be written to: it is not handed out again
-    tb::give_word(word);
-    if (code != 0) return tb_device_status(device, detail);
+    TB_CUDA(cudaStreamSynchronize(stream));
+    uint32_t code = 0;
+    if (!tb::read_note(note, &code) || code != 0) return tb_device_status(device, detail);
     if (detail) *detail = 0;
     return TB_OK;
 }

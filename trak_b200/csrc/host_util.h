@@ -45,9 +45,19 @@ int encode_tmap(CUtensorMap* map, CUtensorMapDataType dt, uint32_t rank, const v
                 const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box,
                 CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B);
 
-// A word in mapped host memory that the last launch of this call on `stream` stores the status word to: the thread's
-// next tb_stream_status on that stream then needs no launch of its own.
-int arm_status(int device, cudaStream_t stream, uint32_t** word);
+// A word in mapped host memory that the last launch of this call on `stream` stores the status word to
+// (publish_status): the thread's next tb_stream_status on that stream then needs no launch of its own.
+struct StatusNote {
+    uint64_t* word = nullptr;  // null: nothing is stored
+    uint32_t call = 0;
+};
+int arm_status(int device, cudaStream_t stream, StatusNote* note);
+#ifdef __CUDACC__
+__device__ __forceinline__ void publish_status(const uint32_t* status, const StatusNote& note) {
+    // one aligned store of eight bytes: the host sees both halves or neither
+    if (note.word) *static_cast<volatile uint64_t*>(note.word) = (uint64_t)note.call << 32 | *status;
+}
+#endif
 
 // Lets `kernel` use all of an SM's shared memory on `device` (the current one); once per kernel and device.
 constexpr int SMEM_PER_CTA = 227 * 1024;
