@@ -78,3 +78,20 @@ def test_a_word_that_was_handed_out_again_is_not_believed(cuda, job):
         other.synchronize()
         assert pool.submit(lib.tb_stream_status, cuda.index, own.cuda_stream, None).result() == 7
     assert lib.tb_stream_status(cuda.index, own.cuda_stream, None) == 0
+
+
+def test_a_call_that_was_refused_does_not_vouch_for_the_device(cuda, job):
+    """A wait runs out, then a projection is refused for its size: the status read after it reports the wait, and not
+    the word that the last accepted call left."""
+    lib, g, out, ws = job
+    stream = torch.cuda.current_stream(cuda)
+    assert _call(lib, cuda, "tb_project", g, out, ws) == 0
+    assert lib.tb_stream_status(cuda.index, stream.cuda_stream, None) == 0
+    assert lib.tb_selftest_wait_timeout(cuda.index, stream.cuda_stream, 20) == 0
+    # 2^31 rows of 64 features and more do not fit a tensor map; the sizes are looked at before any pointer is used
+    F, rows = 1 << 34, 16
+    rc = lib.tb_project(cuda.index, stream.cuda_stream, g.data_ptr(), 0, rows, F, F, out.data_ptr(), N, N, 17, TILES, 0,
+                        1.0, 0, ws.data_ptr(), 1 << 60)
+    assert rc == 8, lib.tb_strerror(rc)
+    assert lib.tb_stream_status(cuda.index, stream.cuda_stream, None) == 7
+    assert lib.tb_stream_status(cuda.index, stream.cuda_stream, None) == 0

@@ -101,7 +101,7 @@ static std::mutex g_words_mu;
 static uint64_t* g_words = nullptr;
 static std::atomic<uint32_t> g_calls{0};
 
-static int take_note(StatusNote* note) {
+int take_note(StatusNote* note) {
     uint64_t* words;
     {
         std::lock_guard<std::mutex> lk(g_words_mu);
@@ -132,13 +132,10 @@ static bool read_note(const StatusNote& note, uint32_t* status) {
 // A store by the SM reaches the host some 8 us earlier than a copy engine that has to be set going.
 __global__ void publish_status_kernel(const uint32_t* status, StatusNote note) { publish_status(status, note); }
 
-int arm_status(int device, cudaStream_t stream, StatusNote* note) {
-    const int rc = take_note(note);
-    if (rc != TB_OK) return rc;
+void arm_status(int device, cudaStream_t stream, const StatusNote& note) {
     t_armed.device = device;
     t_armed.stream = stream;
-    t_armed.note = *note;
-    return TB_OK;
+    t_armed.note = note;
 }
 
 int set_smem_limit(const void* kernel, int device) {

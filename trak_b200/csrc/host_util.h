@@ -29,7 +29,7 @@ int select_device(int device, int* sm_count);
 int validate_project_args(const void* grads, int dtype, int64_t B, int64_t F, int64_t ld, const float* out,
                           int64_t ld_out, uint32_t N, uint32_t num_feature_tiles, int proj_type);
 
-// tb_project; with `publish` its last launch stores the status word to pinned host memory (arm_status), without it the
+// tb_project; with `publish` its last launch stores the status word to pinned host memory (take_note), without it the
 // call takes no memory of any kind from the driver.
 int project_dense(int device, void* stream, const void* grads, int dtype, int64_t B, int64_t F, int64_t ld, float* out,
                   int64_t ld_out, uint32_t N, uint32_t seed, uint32_t num_feature_tiles, int proj_type, float alpha,
@@ -45,13 +45,15 @@ int encode_tmap(CUtensorMap* map, CUtensorMapDataType dt, uint32_t rank, const v
                 const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box,
                 CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B);
 
-// A word in mapped host memory that the last launch of this call on `stream` stores the status word to
-// (publish_status): the thread's next tb_stream_status on that stream then needs no launch of its own.
+// A word in mapped host memory that a kernel stores the status word to (publish_status).
 struct StatusNote {
     uint64_t* word = nullptr;  // null: nothing is stored
     uint32_t call = 0;
 };
-int arm_status(int device, cudaStream_t stream, StatusNote* note);
+int take_note(StatusNote* note);
+// To be called when the launch that stores `note` has been queued on `stream` as the last of its call: the thread's next
+// tb_stream_status on that stream then needs no launch of its own.
+void arm_status(int device, cudaStream_t stream, const StatusNote& note);
 #ifdef __CUDACC__
 __device__ __forceinline__ void publish_status(const uint32_t* status, const StatusNote& note) {
     // one aligned store of eight bytes: the host sees both halves or neither
