@@ -59,6 +59,12 @@ def test_only_floats_are_added():
         mmap_io.device_to_host(torch.zeros(4, 5).half(), torch.zeros(4, 5).half(), object(), add=True)
 
 
+def test_stores_opened_for_reading_are_not_written_to(tmp_path):
+    mmap_io.create_store(tmp_path / "scores.mmap", (4, 5), torch.float32).flush()
+    with pytest.raises(ValueError, match="read-only"):
+        mmap_io.device_to_host(mmap_io.open_store(tmp_path / "scores.mmap", mode="r"), torch.zeros(4, 5), object())
+
+
 @pytest.mark.parametrize("src", [np.zeros((4, 10), np.float32)[:, ::2], torch.zeros(5, 4).T])
 def test_strided_host_sources_are_refused(src):
     with pytest.raises(ValueError, match="contiguous"):

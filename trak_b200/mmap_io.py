@@ -70,6 +70,8 @@ def device_to_host(dst, src: torch.Tensor, stream=None, add: bool = False) -> No
     if not (dst.flags.c_contiguous if array else dst.is_contiguous() and dst.device.type == "cpu") \
             or not src.is_contiguous():
         raise ValueError("source and destination must be contiguous, the destination in host memory")
+    if array and not dst.flags.writeable:   # a store opened for reading: its pages would fault under the threads
+        raise ValueError("assignment destination is read-only")
     ptr = dst.ctypes.data if array else dst.data_ptr()
     with torch.cuda.device(src.device):
         stream = torch.cuda.current_stream(src.device) if stream is None else stream
