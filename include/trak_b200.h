@@ -264,13 +264,18 @@ int tb_selftest_sqrt(int device, void *stream, uint64_t first, uint64_t count, u
 
 /* ---- pageable host memory (no counterpart in the reference) ---------------------
  * Copies between pageable host memory (numpy memmaps, host accumulators) and the device through a small pinned
- * ring per device and direction; several host threads share the host side, which runs under the PCIe copies.
+ * ring per device and direction; several host threads share the host side, which runs under the PCIe copies: the
+ * process's OpenMP team where it has one (torch's; omp_set_num_threads, torch.set_num_threads and OMP_NUM_THREADS set
+ * its size), else threads of the library's own, OMP_NUM_THREADS of them or up to 12.
  * Both calls are ordered on `stream` and may be made from any thread.
  *   tb_host_to_device  returns when `src` has been read; the last device copies may still be in flight.
  *   tb_device_to_host  returns when `dst` is complete; with add_f32 the data are floats and `dst += data`.
+ *   tb_host_threads    how many threads that is for a call of this thread, itself included; *openmp (nullable): whether
+ *                      they are an OpenMP team
  *   tb_host_staging_release  frees the pinned rings (16 MB each; made again on the next use). */
 int tb_host_to_device(int device, void *stream, void *dst, const void *src, size_t bytes);
 int tb_device_to_host(int device, void *stream, void *dst, const void *src, size_t bytes, int add_f32);
+int tb_host_threads(int *openmp);
 int tb_host_staging_release(void);
 
 /* ---- measurement aid (no counterpart in the reference) -------------------------

@@ -63,6 +63,7 @@ SIGNATURES = {
     "tb_project_static": (_i, [_i, _vp, _vp, _i, _i64, _i64, _i64, _vp, _i64, _u32, _u32, _u32, _i, _f, _i]),
     "tb_host_to_device": (_i, [_i, _vp, _vp, _vp, _sz]),
     "tb_device_to_host": (_i, [_i, _vp, _vp, _vp, _sz, _i]),
+    "tb_host_threads": (_i, [ctypes.POINTER(_i)]),
     "tb_host_staging_release": (_i, []),
     "tb_project": (_i, [_i, _vp, _vp, _i, _i64, _i64, _i64, _vp, _i64, _u32, _u32, _u32, _i, _f, _i,
                         _vp, _sz]),

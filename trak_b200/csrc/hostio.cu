@@ -7,7 +7,8 @@
 // (a copy, or the fp32 accumulation `dst += chunk`) is done by several threads in pieces they take one after the
 // other; the calling thread starts the PCIe copies and hands out slots, and takes pieces in between, so host and PCIe
 // work run side by side with no meeting point per chunk (with one, waking and joining the threads took a third of
-// the time at 4 MB a chunk, half at 2 MB).  Measured on 16 cores: 627 MB of features go up at 44 GB/s, 100 MB of
+// the time at 4 MB a chunk, half at 2 MB).  Where a transfer stalls, as the first chunk does behind the stream's earlier
+// work, the threads sleep.  Measured on 16 cores: 627 MB of features go up at 44 GB/s, 100 MB of
 // scores come down at 37.
 //
 // The rings (16 MB per device and direction, made on first use: larger ones crowd the L3) and the threads outlive a
@@ -15,11 +16,14 @@
 // copy that last used it.  tb_host_staging_release gives the pinned memory back.
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <condition_variable>
+#include <cstdlib>
 #include <cstring>
 #include <functional>
 #include <memory>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -39,6 +43,7 @@ namespace tb {
 // Where the process has an OpenMP runtime (torch's), the helpers are its team: after any parallel region its threads
 // keep spinning for milliseconds, and threads of our own beside them would get half of the cores (a score block added
 // to a host accumulator that had just been cleared: 27 GB/s with our own, 40 with the team).  Else a few of our own.
+// Either way as many as the user asks for: the team's size, or OMP_NUM_THREADS (tb_host_threads tells).
 struct OpenMp {
     void (*parallel)(void (*)(void*), void*, unsigned, unsigned) = nullptr;
     int (*max_threads)() = nullptr;
@@ -46,8 +51,9 @@ struct OpenMp {
     int (*in_parallel)() = nullptr;
 
     OpenMp() {
-        void* lib = dlopen("libgomp.so.1", RTLD_LAZY | RTLD_NOLOAD);  // never loads one
-        if (!lib) return;
+        // what the process's own code would be linked to, under whatever file name, else a libgomp that some module
+        // has loaded for itself; never loads one
+        void* lib = dlsym(RTLD_DEFAULT, "GOMP_parallel") ? RTLD_DEFAULT : dlopen("libgomp.so.1", RTLD_LAZY | RTLD_NOLOAD);
         max_threads = reinterpret_cast<int (*)()>(dlsym(lib, "omp_get_max_threads"));
         thread_num = reinterpret_cast<int (*)()>(dlsym(lib, "omp_get_thread_num"));
         in_parallel = reinterpret_cast<int (*)()>(dlsym(lib, "omp_in_parallel"));
@@ -58,7 +64,8 @@ struct OpenMp {
         static const OpenMp omp;
         return omp;
     }
-    bool usable() const { return parallel && !in_parallel() && max_threads() > 1; }
+    // the calling thread's team; inside a parallel region the team is at work already
+    int threads() const { return in_parallel() ? 1 : max_threads(); }
 
     struct Region {
         const OpenMp* omp;
@@ -85,6 +92,15 @@ class HostThreads {
         std::lock_guard<std::mutex> lk(mu);
         if (!pool || pool->pid_ != getpid()) pool = new HostThreads();  // a forked child has none of the threads
         return *pool;
+    }
+
+    // Threads that share a job, the calling one included: OMP_NUM_THREADS where it is a number, else most of the cores.
+    static int wanted() {
+        if (const char* env = getenv("OMP_NUM_THREADS")) {
+            const long n = strtol(env, nullptr, 10);
+            if (n > 0) return (int)std::min<long>(n, 256);
+        }
+        return std::max(1, std::min(MAX_HELPERS + 1, (int)std::thread::hardware_concurrency() - 1));
     }
 
     // `body` on the helpers while `caller` runs here; returns when both have ended.
@@ -115,9 +131,13 @@ class HostThreads {
     };
 
     HostThreads() : pid_(getpid()) {
-        const int cores = (int)std::thread::hardware_concurrency();
-        const int helpers = std::max(0, std::min(MAX_HELPERS, cores - 2));
-        for (int i = 0; i < helpers; ++i) std::thread([this] { loop(); }).detach();
+        for (int i = 1; i < wanted(); ++i) {
+            try {
+                std::thread([this] { loop(); }).detach();
+            } catch (const std::system_error&) {  // no more threads to be had: those that are there do the work
+                break;
+            }
+        }
     }
     void loop() {
         uint64_t seen = 0;
@@ -141,6 +161,26 @@ class HostThreads {
     std::condition_variable wake_;
     std::shared_ptr<Job> job_;
     uint64_t generation_ = 0;
+};
+
+// Threads that share the host side of a transfer started by this thread.
+static int host_threads() { return OpenMp::get().parallel ? OpenMp::get().threads() : HostThreads::wanted(); }
+
+// Waits a moment: pauses at first, sleeps once it has taken longer than a transfer that gets on ever stalls (a chunk
+// crosses PCIe in 40 us; with sleeps from 20 us on, 2 MB came down in 300 us instead of 120).
+struct Patience {
+    int spins = 0;
+    std::chrono::steady_clock::time_point since;
+
+    void wait() {
+        _mm_pause();
+        if (++spins % 64) return;
+        const auto now = std::chrono::steady_clock::now();
+        if (spins == 64)
+            since = now;
+        else if (now - since > std::chrono::microseconds(400))
+            std::this_thread::sleep_for(std::chrono::microseconds(50));
+    }
 };
 
 // ---- pinned rings ------------------------------------------------------------------------------
@@ -222,10 +262,8 @@ struct Transfer {
     }
     void helper() {
         for (int p; (p = next.fetch_add(1, std::memory_order_relaxed)) < pieces;) {
-            while (opened.load(std::memory_order_acquire) <= p / pieces_per_chunk) {
+            for (Patience idle; opened.load(std::memory_order_acquire) <= p / pieces_per_chunk; idle.wait())
                 if (stop.load(std::memory_order_relaxed)) return;
-                _mm_pause();
-            }
             piece(p);
         }
     }
@@ -235,22 +273,31 @@ struct Transfer {
         int rc = TB_OK;
         const std::function<void()> body = [this] { helper(); }, caller = [&] {
             int held = -1;  // a piece taken whose chunk was not open yet
+            Patience idle;
             for (bool done = false; !done;) {
+                const int before = opened.load(std::memory_order_relaxed);
                 rc = advance(&done);
                 if (rc != TB_OK) break;
-                if (held < 0 && next.load(std::memory_order_relaxed) < pieces &&
-                    next.load(std::memory_order_relaxed) / pieces_per_chunk < opened.load(std::memory_order_relaxed)) {
+                const int open = opened.load(std::memory_order_relaxed), coming = next.load(std::memory_order_relaxed);
+                if (held < 0 && coming < pieces && coming / pieces_per_chunk < open) {
                     held = next.fetch_add(1, std::memory_order_relaxed);
                     if (held >= pieces) held = -1;
                 }
-                if (held >= 0 && held / pieces_per_chunk < opened.load(std::memory_order_relaxed)) {
+                if (held >= 0 && held / pieces_per_chunk < open) {
                     piece(held);
                     held = -1;
+                    idle = Patience();
+                } else if (open != before) {
+                    idle = Patience();
+                } else if (!done) {
+                    idle.wait();
                 }
             }
             stop.store(true, std::memory_order_relaxed);
         };
-        if (OpenMp::get().usable())
+        if (host_threads() < 2)
+            caller();
+        else if (OpenMp::get().parallel)
             OpenMp::get().run(body, caller);
         else
             HostThreads::get().help(body, caller);
@@ -273,6 +320,14 @@ static int slot_idle(Ring& ring, int slot, bool* idle) {
     return TB_OK;
 }
 
+// What one thread can do, the driver's own copy does better: up 10 to 20 GB/s against 7 to 15 through the ring, down 15
+// to 21 against 9 to 15 (2 to 400 MB).  Memory that turns out to be pinned is waited for like any other.
+static int copy_alone(void* dst, const void* src, size_t bytes, cudaMemcpyKind kind, cudaStream_t stream) {
+    TB_CUDA(cudaMemcpyAsync(dst, src, bytes, kind, stream));
+    TB_CUDA(cudaStreamSynchronize(stream));
+    return TB_OK;
+}
+
 }  // namespace tb
 
 extern "C" {
@@ -284,6 +339,7 @@ int tb_host_to_device(int device, void* stream_, void* dst, const void* src, siz
     int rc = select_device(device, nullptr);
     if (rc != TB_OK) return rc;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    if (host_threads() < 2) return copy_alone(dst, src, bytes, cudaMemcpyHostToDevice, stream);
     Ring& ring = g_up[device];
     std::lock_guard<std::mutex> lk(ring.mu);
     rc = ring.make();
@@ -320,6 +376,7 @@ int tb_device_to_host(int device, void* stream_, void* dst, const void* src, siz
     int rc = select_device(device, nullptr);
     if (rc != TB_OK) return rc;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    if (host_threads() < 2 && !add_f32) return copy_alone(dst, src, bytes, cudaMemcpyDeviceToHost, stream);
     Ring& ring = g_down[device];
     std::lock_guard<std::mutex> lk(ring.mu);
     rc = ring.make();
@@ -354,6 +411,11 @@ int tb_device_to_host(int device, void* stream_, void* dst, const void* src, siz
         *done = finished == t.chunks;
         return (int)TB_OK;
     });
+}
+
+int tb_host_threads(int* openmp) {
+    if (openmp) *openmp = tb::OpenMp::get().parallel ? 1 : 0;
+    return tb::host_threads();
 }
 
 int tb_host_staging_release(void) {
