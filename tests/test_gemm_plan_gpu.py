@@ -26,6 +26,15 @@ def test_gemm_nt(cuda, M, N, K, dtype):
     assert rel(sc.gemm_nt(a, b, out=got.clone(), row_scale=w, accumulate=True), 2 * want) <= 3e-5
 
 
+@pytest.mark.parametrize("M", [65535 * 128, 65535 * 128 + 1])
+def test_gemm_nt_of_more_rows_than_a_grid_of_small_tiles_has(cuda, M):
+    from trak_b200 import score_computers as sc
+    a = torch.randn(M, 8, device=cuda, generator=torch.Generator(device=cuda).manual_seed(M)).half()
+    b = torch.randn(3, 8, device=cuda, generator=torch.Generator(device=cuda).manual_seed(8)).half()
+    want = a.float() @ b.float().T
+    assert rel(sc.gemm_nt(a, b), want.double()) <= 1e-6   # eight products of 11-bit numbers: nearly exact either way
+
+
 @pytest.mark.parametrize("n,k", [(5000, 40), (4097, 129), (3001, 512), (20000, 300), (100, 700), (1, 5), (513, 17), (1030, 145),
                                  (2048, 300), (2049, 31)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])

@@ -991,10 +991,11 @@ GemmPlan plan_gemm(uint32_t npl, bool chunked, bool symmetric, int64_t M, int64_
     constexpr double SMS = 148.0, SUM_FIXED = 7.0, SUM_BYTES_PER_US = 3.0e6;
     constexpr uint32_t MAX_SPLITS = 64;
     constexpr size_t MAX_PARTIAL = 256u << 20;
+    constexpr double MAX_GRID_Y = 65535.0;  // tile rows of a launch, 32-row blocks of the sum
     const double tm = (double)((M + 127) / 128), tn2 = (double)((N + 255) / 256), tm2 = (double)((M + 255) / 256);
     GemmPlan best{2, 1, kblocks, 0};
     double best_t = 1e300;
-    if (!chunked) {
+    if (!chunked && tm <= MAX_GRID_Y) {
         const double tn = (double)((N + 127) / 128), tiles = symmetric ? tm * (tm + 1) / 2 : tm * tn;
         const double waves = (double)(uint64_t)((tiles + SMS - 1) / SMS);
         best_t = 5.0 + waves * kblocks * (npl == 2 ? 0.34 : 0.12);
@@ -1006,7 +1007,7 @@ GemmPlan plan_gemm(uint32_t npl, bool chunked, bool symmetric, int64_t M, int64_
         const uint32_t per = ((kblocks + s - 1) / s + 1u) & ~1u;  // whole 64-wide chunks
         const uint32_t used = (kblocks + per - 1) / per;
         const size_t bytes = used > 1 ? (size_t)used * M * N * sizeof(float) : 0;
-        if (used != s || bytes > MAX_PARTIAL) continue;
+        if (used != s || bytes > MAX_PARTIAL || (s > 1 && M > 32 * MAX_GRID_Y)) continue;
         const double waves = (double)(uint64_t)((tiles * s + SMS - 1) / SMS);
         double t = waves * (8.0 + per * per_kb);
         if (s > 1) t += SUM_FIXED + ((double)s * (symmetric ? 0.5 : 1.0) + 1.0) * M * N * 4.0 / SUM_BYTES_PER_US;
