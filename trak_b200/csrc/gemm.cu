@@ -985,8 +985,16 @@ static int packed_tmap(CUtensorMap* map, const uint16_t* packed, const Packed& g
 // Tile and number of slices of the contraction.  A 256 x 256 (or 128 x 256) tile per CTA leaves most of the 148 SMs
 // idle when the product is small: the Gram of 2048 columns is 36 such tiles however many rows it sums over.  The
 // choice minimises an estimate in microseconds: per wave of CTAs a fixed part (launch, first loads, epilogue) plus the
-// tensor-core time of its k blocks; slicing adds the kernel that sums the slices, which is bound by memory.  The
-// 128 x 128 tile reads twice the operand bytes per flop and is for products of less than about a wave.
+// tensor-core time of its k blocks; slicing adds the kernel that sums the slices, which is bound by memory.
+// The 128 x 128 tile, two CTAs to an SM, reads twice the operand bytes per flop, so it is the better one where the
+// large tile would compute padding (any number of rows by up to 128 columns) or leave SMs idle, and a contraction is too
+// short to slice; at equal fill it is 10 to 30 % slower.  Both tiles measured over 128 to 1,000,000 rows x 64 to 2048
+// columns x 512 to 8192, in us, small and large: fp32 1000 x 512 x 512 19 and 32, 20,000 x 300 x 2048 106 and 151,
+// 200,000 x 128 x 2048 370 and 517, 200,000 x 512 x 512 341 and 298, 50,000 x 2048 x 2048 1113 and 931; fp16
+// 50,000 x 2048 x 512 214 and 171, 1000 x 1024 x 8192 83 and 48 (sliced).  Over those 284 products the choice is 0.3 % (mean)
+// and 15 % (worst) slower than the better of the two; with one wave length for both tiles it was 3 % and 72 %.
+// The sizes alone decide, so that the workspace query, which names no device, agrees: every B200 has 148 SMs.  A product
+// that leaves out the k blocks where a triangular factor is zero (KRange) is planned like a whole one.
 GemmPlan plan_gemm(uint32_t npl, bool chunked, bool symmetric, int64_t M, int64_t N, uint32_t kblocks) {
     constexpr double SMS = 148.0, SUM_FIXED = 7.0, SUM_BYTES_PER_US = 3.0e6;
     constexpr uint32_t MAX_SPLITS = 64;
@@ -996,9 +1004,12 @@ GemmPlan plan_gemm(uint32_t npl, bool chunked, bool symmetric, int64_t M, int64_
     GemmPlan best{2, 1, kblocks, 0};
     double best_t = 1e300;
     if (!chunked && tm <= MAX_GRID_Y) {
+        // rounds of two CTAs on every SM; what is left over after the last whole one has the SMs to itself, or nearly
         const double tn = (double)((N + 127) / 128), tiles = symmetric ? tm * (tm + 1) / 2 : tm * tn;
-        const double waves = (double)(uint64_t)((tiles + SMS - 1) / SMS);
-        best_t = 5.0 + waves * kblocks * (npl == 2 ? 0.34 : 0.12);
+        const double rounds = (double)(uint64_t)(tiles / (2 * SMS)), rest = tiles - rounds * 2 * SMS;
+        const double pair = npl == 2 ? 2.0 + 0.68 * kblocks : 4.0 + 0.26 * kblocks;
+        const double single = 4.0 + (npl == 2 ? 0.5 : 0.18) * kblocks;
+        best_t = rounds * pair + (rest > SMS ? pair : rest > 0 ? single : 0.0);
         best.tile = 1;
     }
     const double tiles = chunked ? (symmetric ? tm2 * (tm2 + 1) : tm * tn2) : symmetric ? tm2 * (tm2 + 1) / 2 : tm2 * tn2;
