@@ -57,7 +57,8 @@ struct GemmParams {
     int64_t ldc;
     uint32_t M, N;
     uint32_t kblocks;        // K / 32 (padded)
-    uint32_t kb_per_split;   // k blocks of one slice of the grid's z dimension (kblocks when there is one slice)
+    uint32_t kb_per_split;   // k blocks of one slice of the grid's z dimension (kblocks when there is one slice);
+                             // the chunked kernel divides what `range` leaves of each tile instead
     uint64_t split_stride;   // floats between the partial products of two slices
     uint32_t stages;
     uint32_t idesc;
