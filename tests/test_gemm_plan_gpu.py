@@ -97,10 +97,30 @@ def test_product_in_two_steps(cuda, m, n, k, dtype):
     assert torch.equal(got, sc.gemm_nt(a, values, row_scale=scale))
 
 
-def test_features_of_a_matrix_packed_beside_the_inverse(cuda, monkeypatch):
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_features_of_a_matrix_packed_beside_the_inverse(cuda, monkeypatch, dtype):
+    """A single block, on the caller's stream and packed on a stream of its own while the inverse is computed."""
     from trak_b200 import score_computers as sc
-    x = torch.randn(5000, 1100, device=cuda, generator=torch.Generator(device=cuda).manual_seed(3))
-    one = sc.B200ScoreComputer(torch.float32, cuda, 1100)
-    want = one.get_x_xtx_inv(x, one.get_xtx(x))
+    asked, pair = [], sc.B200ScoreComputer._pair
+    monkeypatch.setattr(sc.B200ScoreComputer, "_pair", lambda self, wanted: asked.append(wanted) or pair(self, wanted))
+    x = torch.randn(5000, 1100, device=cuda, generator=torch.Generator(device=cuda).manual_seed(3)).to(dtype)
+    computer = sc.B200ScoreComputer(dtype, cuda)
+    xtx = computer.get_xtx(x)
+    want = computer.get_x_xtx_inv(x, xtx)
     monkeypatch.setattr(sc.B200ScoreComputer, "APART_BYTES", 0)
-    assert torch.equal(one.get_x_xtx_inv(x, one.get_xtx(x)), want)
+    got = computer.get_x_xtx_inv(x, xtx)
+    assert asked == [False, False, True]   # the Gram, then the features either way
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("where", ["cuda", "cpu"])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_one_plane_gram_of_many_rows(cuda, where, dtype):
+    """A chain of n / 16 steps, each of which truncates below the last of 24 places, loses at most n / 16 * 2^-23; blocks
+    of a host matrix, two partial sums and slices only shorten it."""
+    from trak_b200 import score_computers as sc
+    n, k = 50_000, 300
+    x = torch.randn(n, k, device=cuda, generator=torch.Generator(device=cuda).manual_seed(5)).to(dtype)
+    want = x.double().T @ x.double()
+    got = sc.B200ScoreComputer(torch.float32, cuda).get_xtx(x.to(where))
+    assert rel(got, want) <= n / 16 * 2.0 ** -23
