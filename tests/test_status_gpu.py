@@ -1,4 +1,7 @@
 """The status word on its way to the host: what a call takes from the driver for it, and whose status a read reports."""
+import os
+import subprocess
+import sys
 import threading
 from concurrent.futures import ThreadPoolExecutor
 
@@ -56,6 +59,35 @@ def test_first_call_of_a_thread_can_be_captured(cuda, job, name):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(got, want)
+
+
+FIRST_WORD = """
+import torch
+from trak_b200 import _lib
+lib, dev = _lib.lib(), torch.device("cuda", 0)
+g, out = (torch.randn(16, 50021, device=dev) * 1e-2).half(), torch.empty(16, 1024, device=dev)
+ws = torch.empty(lib.tb_project_workspace_bytes(0, 16, 50021, 1024, 148), dtype=torch.uint8, device=dev)
+def args():
+    return [0, torch.cuda.current_stream().cuda_stream, g.data_ptr(), 0, 16, 50021, 50021, out.data_ptr(), 1024, 1024, 17,
+            148, 0, 1.0, 0]
+assert lib.tb_project_static(*args()) == 0
+want = out.clone()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph, capture_error_mode="global"):
+    assert lib.tb_project(*args(), ws.data_ptr(), ws.numel()) == 0, lib.tb_last_cuda_error()
+out.zero_()
+graph.replay()
+torch.cuda.synchronize()
+assert torch.equal(out, want)
+assert lib.tb_stream_status(0, torch.cuda.current_stream().cuda_stream, None) == 0
+"""
+
+
+def test_the_process_makes_its_words_under_a_capture(cuda):
+    """tb_project_static makes no words, so the first ones may be wanted while a capture is going on."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    p = subprocess.run([sys.executable, "-c", FIRST_WORD], cwd=root, capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr
 
 
 def test_a_word_that_was_handed_out_again_is_not_believed(cuda, job):

@@ -143,17 +143,13 @@ def _as_device_matrix(t: torch.Tensor, device) -> torch.Tensor:
     return t
 
 
-def _check_operand(t: torch.Tensor, device) -> None:
-    if t.dim() != 2 or t.device != device or not t.is_cuda or (t.shape[1] > 1 and t.stride(1) != 1):
-        raise RuntimeError("expected CUDA matrices with unit column stride on one device")
-
-
-def _check_out(out: torch.Tensor, rows: int, cols: int, device) -> None:
+def _check_out(out: torch.Tensor, rows: int, cols: int, device) -> int:
     """The kernels write ``rows`` x ``cols`` floats from ``out``'s pointer on: anything else would be written past its
-    end, or not where the caller looks."""
-    if out.device != device or out.dtype != torch.float32 or tuple(out.shape) != (rows, cols) \
+    end, or not where the caller looks.  Returns the rows' distance."""
+    if out.shape != (rows, cols) or out.dtype != torch.float32 or out.device != device \
             or (cols > 1 and out.stride(1) != 1):
         raise RuntimeError(f"out must be a float32 [{rows}, {cols}] tensor with unit column stride on the operands' device")
+    return out.stride(0)
 
 
 def _check_accumulator(n: int, m: int, accumulator: torch.Tensor, row_scale) -> None:
@@ -169,19 +165,22 @@ def gram(x: torch.Tensor, out: torch.Tensor = None, accumulate: bool = False) ->
     """fp32 [k, k] = x^T x (+ out) for a CUDA matrix x [n, k] (fp16 / bf16 / fp32)."""
     n, k = x.shape
     dev = x.device
-    _check_operand(x, dev)
+    ld, step = x.stride()
+    if not x.is_cuda or (k > 1 and step != 1):
+        raise RuntimeError("expected a CUDA matrix with unit column stride")
     if out is None:
         out = torch.empty((k, k), dtype=torch.float32, device=dev)
         accumulate = False
+        ldg = k
     else:
-        _check_out(out, k, k, dev)
+        ldg = _check_out(out, k, k, dev)
     lib = _lib.lib()
     with _lib.on_device(dev):
         stream = _lib.current_stream(dev)
         dt = _DTYPES[x.dtype]
         ws = _workspace(dev, stream, lib.tb_gram_workspace_bytes(dt, n, k))
-        _lib.check(lib.tb_gram(dev.index, stream, x.data_ptr(), dt, n, k, x.stride(0), out.data_ptr(),
-                               out.stride(0), int(accumulate), ws.data_ptr(), ws.numel()))
+        _lib.check(lib.tb_gram(dev.index, stream, x.data_ptr(), dt, n, k, ld, out.data_ptr(), ldg, int(accumulate),
+                               ws.data_ptr(), ws.numel()))
     return out
 
 
@@ -215,18 +214,18 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, row_scal
             b_ready()
             b_ready = None
         a, b = a.float(), b.float()
-    M, K = a.shape
-    N = b.shape[0]
-    if b.shape[1] != K:
+    (M, K), (N, Kb), dev = a.shape, b.shape, a.device
+    (lda, step_a), (ldb, step_b) = a.stride(), b.stride()
+    if Kb != K:
         raise RuntimeError("inner dimensions differ")
-    dev = a.device
-    _check_operand(a, dev)
-    _check_operand(b, dev)
+    if not a.is_cuda or b.device != dev or (K > 1 and (step_a != 1 or step_b != 1)):
+        raise RuntimeError("expected CUDA matrices with unit column stride on one device")
     if out is None:
         out = torch.empty((M, N), dtype=torch.float32, device=dev)
         accumulate = False
+        ldc = N
     else:
-        _check_out(out, M, N, dev)
+        ldc = _check_out(out, M, N, dev)
     if row_scale is not None:
         row_scale = row_scale.to(dev, torch.float32).reshape(-1).contiguous()
         if row_scale.numel() != M:
@@ -238,16 +237,14 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, row_scal
         ws = _workspace(dev, stream, lib.tb_gemm_nt_workspace_bytes(dt, M, N, K))
         scale = row_scale.data_ptr() if row_scale is not None else None
         if b_ready is not None:
-            _lib.check(lib.tb_gemm_nt_pack(dev.index, stream, a.data_ptr(), a.stride(0), dt, M, N, K, ws.data_ptr(),
-                                           ws.numel()))
+            _lib.check(lib.tb_gemm_nt_pack(dev.index, stream, a.data_ptr(), lda, dt, M, N, K, ws.data_ptr(), ws.numel()))
             b_ready()
-            _lib.check(lib.tb_gemm_nt_packed(dev.index, stream, b.data_ptr(), b.stride(0), dt, M, N, K, out.data_ptr(),
-                                             out.stride(0), scale, float(alpha), int(accumulate), ws.data_ptr(),
-                                             ws.numel()))
+            _lib.check(lib.tb_gemm_nt_packed(dev.index, stream, b.data_ptr(), ldb, dt, M, N, K, out.data_ptr(), ldc,
+                                             scale, float(alpha), int(accumulate), ws.data_ptr(), ws.numel()))
         else:
-            _lib.check(lib.tb_gemm_nt(dev.index, stream, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), dt, M, N,
-                                      K, out.data_ptr(), out.stride(0), scale, float(alpha), int(accumulate),
-                                      ws.data_ptr(), ws.numel()))
+            _lib.check(lib.tb_gemm_nt(dev.index, stream, a.data_ptr(), lda, b.data_ptr(), ldb, dt, M, N, K,
+                                      out.data_ptr(), ldc, scale, float(alpha), int(accumulate), ws.data_ptr(),
+                                      ws.numel()))
     return out
 
 
@@ -263,7 +260,7 @@ class B200ScoreComputer:
         if device.index is None:
             device = torch.device("cuda", torch.cuda.current_device())
         self.device = device
-        self.CUDA_MAX_DIM_SIZE = CUDA_MAX_DIM_SIZE  # rows moved to the GPU and multiplied at a time
+        self.CUDA_MAX_DIM_SIZE = CUDA_MAX_DIM_SIZE  # most rows moved to the GPU and multiplied at a time (_blocks)
         self.logger = logging.getLogger("ScoreComputer")
         self.logger.setLevel(logging_level)
         self.lambda_reg = lambda_reg
