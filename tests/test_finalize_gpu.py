@@ -137,3 +137,14 @@ def test_half_precision_stores_as_traker_writes_them_by_default(cuda, tmp_path):
     want = (S / M) * (w / M)
     err = float((got - want).norm() / want.norm())
     assert err <= 1e-3, err        # fp16 rounding of the stored scores (2^-11 per entry)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.int64])
+def test_target_gradients_of_other_types_are_converted(cuda, dtype):
+    from trak_b200.finalize import ScoreFinalizer
+    feats, targs, o2l = _checkpoints(2, 300, 64, 9, 31)
+    targs = [(100 * t).numpy().astype(dtype) for t in targs]
+    out = torch.zeros(300, 9)
+    ScoreFinalizer(feats, targs, o2l, cuda).run(out)
+    want = _oracle_scores(feats, [torch.from_numpy(t).float() for t in targs], o2l)
+    assert float((out - want).norm() / want.norm()) <= 1e-4

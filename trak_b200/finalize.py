@@ -64,6 +64,8 @@ def _rows_to_device(src, lo, hi, device):
 def _whole_to_device(src, device):
     if isinstance(src, torch.Tensor):
         return sc._as_device_matrix(src, device)
+    if src.dtype not in mmap_io._TORCH:   # not a type of the stores: converted to fp32
+        return sc._as_device_matrix(torch.from_numpy(np.array(src)), device)
     return sc._as_device_matrix(mmap_io.read_rows(src, 0, src.shape[0], device), device)
 
 
