@@ -148,3 +148,10 @@ def test_target_gradients_of_other_types_are_converted(cuda, dtype):
     ScoreFinalizer(feats, targs, o2l, cuda).run(out)
     want = _oracle_scores(feats, [torch.from_numpy(t).float() for t in targs], o2l)
     assert float((out - want).norm() / want.norm()) <= 1e-4
+
+
+def test_a_store_that_autograd_watches_is_refused(cuda):
+    from trak_b200.finalize import ScoreFinalizer
+    feats, targs, o2l = _checkpoints(1, 300, 64, 9, 32)
+    with pytest.raises(RuntimeError, match="grad"):
+        ScoreFinalizer(feats, targs, o2l, cuda).run(torch.zeros(300, 9, requires_grad=True))

@@ -125,8 +125,9 @@ class ScoreFinalizer:
             row_bytes = max(f.shape[1] * (f.element_size() if isinstance(f, torch.Tensor) else f.itemsize) for f in host)
             step = min(step, max(4096, self.UPLOAD_BYTES // row_bytes // 256 * 256))
         step = min(step, max(1, hi - lo))
-        contiguous = scores_store.is_contiguous() and not scores_store.is_cuda if is_tensor \
-            else scores_store.flags.c_contiguous
+        # what the host threads may write to; any other store is assigned to, by its own rules
+        contiguous = scores_store.is_contiguous() and not scores_store.is_cuda and not scores_store.requires_grad \
+            if is_tensor else scores_store.flags.c_contiguous
         with torch.cuda.device(dev):
             acc = torch.empty(step, m, dtype=torch.float32, device=dev)
             done = [torch.empty(step, m, dtype=out_dtype, device=dev) for _ in range(2)]
