@@ -157,3 +157,26 @@ class on_device:
         if self.guard is not None:
             self.guard.__exit__(*exc)
         return False
+
+
+class Workspaces:
+    """Scratch buffers kept by device and stream.  A buffer is its taker's alone until everything that uses it has been
+    queued and it is given back; the stream orders the next user behind that.  (Were it left in the cache meanwhile, two
+    threads that queue work on one stream would write over each other's operands between their launches.)"""
+
+    def __init__(self, most_kept: int = 8):   # per process; streams come and go, their buffers should not pile up
+        self.most_kept, self.kept = most_kept, {}
+
+    def take(self, device: torch.device, stream: int, nbytes: int) -> torch.Tensor:
+        ws = self.kept.pop((device.index, stream), None)
+        if ws is None or ws.numel() < nbytes:
+            ws = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
+        return ws
+
+    def give(self, device: torch.device, stream: int, ws: torch.Tensor) -> None:
+        self.kept[(device.index, stream)] = ws  # most recently used last
+        while len(self.kept) > self.most_kept:
+            self.kept.pop(next(iter(list(self.kept))), None)
+
+    def clear(self) -> None:
+        self.kept.clear()

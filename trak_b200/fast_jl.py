@@ -22,8 +22,7 @@ from . import _lib
 
 _STRICT = os.environ.get("TRAK_B200_STRICT", "1") != "0"
 _DTYPES = {torch.float16: _lib.TB_F16, torch.bfloat16: _lib.TB_BF16, torch.float32: _lib.TB_F32}
-_workspaces = {}
-_MAX_CACHED_WORKSPACES = 8  # per process; streams come and go, their workspaces should not pile up
+_workspaces = _lib.Workspaces()
 
 
 def _u32(name, v):
@@ -37,17 +36,6 @@ def _u32(name, v):
     if v < 0 or v > 0xFFFFFFFF:
         raise TypeError(f"{name} must be an unsigned 32-bit integer, got {v}")
     return v
-
-
-def _workspace(device, stream, nbytes):
-    key = (device.index, stream)
-    ws = _workspaces.pop(key, None)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
-    _workspaces[key] = ws  # most recently used last
-    while len(_workspaces) > _MAX_CACHED_WORKSPACES:
-        _workspaces.pop(next(iter(_workspaces)))
-    return ws
 
 
 def free_workspaces():
@@ -135,7 +123,7 @@ def project(input, N, seed, num_feature_tiles, proj_type, *, alpha=1.0, out=None
     with _lib.on_device(dev):
         stream = _lib.current_stream(dev)
         nbytes = l.tb_project_workspace_bytes(dt, B, F, N, max(num_feature_tiles, 1))
-        ws = _workspace(dev, stream, max(nbytes, 256))
+        ws = _workspaces.take(dev, stream, nbytes)
         if matrix is not None:
             if not matrix.matches(input, N, num_feature_tiles) or matrix.seed != seed or \
                     matrix.proj_type != int(proj_type):
@@ -148,6 +136,7 @@ def project(input, N, seed, num_feature_tiles, proj_type, *, alpha=1.0, out=None
                               out.data_ptr(), out.stride(0), N, seed, num_feature_tiles,
                               int(proj_type), float(alpha), int(bool(accumulate)), ws.data_ptr(),
                               ws.numel())
+        _workspaces.give(dev, stream, ws)
         _lib.check(rc)
         if _STRICT if strict is None else strict:
             _lib.stream_status(dev.index, stream)
@@ -199,7 +188,7 @@ def project_segments(tensors, N, seed, num_feature_tiles, proj_type, *, alpha=1.
     with _lib.on_device(dev):
         stream = _lib.current_stream(dev)
         nbytes = l.tb_project_segments_workspace_bytes(dt, B, F, N, max(num_feature_tiles, 1), len(tensors))
-        ws = _workspace(dev, stream, max(nbytes, 256))
+        ws = _workspaces.take(dev, stream, nbytes)
         if matrix is not None:
             elem = _lib.TB_BF16 if dtype == torch.bfloat16 else _lib.TB_F16
             if (matrix.F, matrix.N, matrix.tiles, matrix.elem, matrix.device) != (F, N, num_feature_tiles, elem, dev) \
@@ -212,6 +201,7 @@ def project_segments(tensors, N, seed, num_feature_tiles, proj_type, *, alpha=1.
             rc = l.tb_project_segments(dev.index, stream, segs, len(tensors), dt, B, out.data_ptr(), out.stride(0), N,
                                        seed, num_feature_tiles, int(proj_type), float(alpha), int(bool(accumulate)),
                                        ws.data_ptr(), ws.numel())
+        _workspaces.give(dev, stream, ws)
         _lib.check(rc)
         if _STRICT if strict is None else strict:
             _lib.stream_status(dev.index, stream)

@@ -28,20 +28,8 @@ import torch
 from . import _lib, mmap_io
 
 _DTYPES = {torch.float16: _lib.TB_F16, torch.bfloat16: _lib.TB_BF16, torch.float32: _lib.TB_F32}
-_workspaces = {}
+_workspaces = _lib.Workspaces()
 _pairs = threading.local()
-_MAX_CACHED_WORKSPACES = 8  # per process; streams come and go, their workspaces should not pile up
-
-
-def _workspace(device, stream, nbytes):
-    key = (device.index, stream)
-    ws = _workspaces.pop(key, None)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
-    _workspaces[key] = ws  # most recently used last
-    while len(_workspaces) > _MAX_CACHED_WORKSPACES:
-        _workspaces.pop(next(iter(_workspaces)))
-    return ws
 
 
 def free_workspaces():
@@ -178,9 +166,10 @@ def gram(x: torch.Tensor, out: torch.Tensor = None, accumulate: bool = False) ->
     with _lib.on_device(dev):
         stream = _lib.current_stream(dev)
         dt = _DTYPES[x.dtype]
-        ws = _workspace(dev, stream, lib.tb_gram_workspace_bytes(dt, n, k))
+        ws = _workspaces.take(dev, stream, lib.tb_gram_workspace_bytes(dt, n, k))
         _lib.check(lib.tb_gram(dev.index, stream, x.data_ptr(), dt, n, k, ld, out.data_ptr(), ldg, int(accumulate),
                                ws.data_ptr(), ws.numel()))
+        _workspaces.give(dev, stream, ws)
     return out
 
 
@@ -199,9 +188,10 @@ def _launch_spd_inverse(a: torch.Tensor, lambda_reg: float, rescale: bool) -> No
     lib = _lib.lib()
     with _lib.on_device(dev):
         stream = _lib.current_stream(dev)
-        ws = _workspace(dev, stream, lib.tb_spd_inverse_workspace_bytes(a.shape[0]))
+        ws = _workspaces.take(dev, stream, lib.tb_spd_inverse_workspace_bytes(a.shape[0]))
         _lib.check(lib.tb_spd_inverse(dev.index, stream, a.data_ptr(), a.shape[0], a.stride(0),
                                       float(lambda_reg), int(rescale), None, ws.data_ptr(), ws.numel()))
+        _workspaces.give(dev, stream, ws)
 
 
 def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, row_scale: torch.Tensor = None,
@@ -234,7 +224,7 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, row_scal
     with _lib.on_device(dev):
         stream = _lib.current_stream(dev)
         dt = _DTYPES[a.dtype]
-        ws = _workspace(dev, stream, lib.tb_gemm_nt_workspace_bytes(dt, M, N, K))
+        ws = _workspaces.take(dev, stream, lib.tb_gemm_nt_workspace_bytes(dt, M, N, K))
         scale = row_scale.data_ptr() if row_scale is not None else None
         if b_ready is not None:
             _lib.check(lib.tb_gemm_nt_pack(dev.index, stream, a.data_ptr(), lda, dt, M, N, K, ws.data_ptr(), ws.numel()))
@@ -245,6 +235,7 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, row_scal
             _lib.check(lib.tb_gemm_nt(dev.index, stream, a.data_ptr(), lda, b.data_ptr(), ldb, dt, M, N, K,
                                       out.data_ptr(), ldc, scale, float(alpha), int(accumulate), ws.data_ptr(),
                                       ws.numel()))
+        _workspaces.give(dev, stream, ws)
     return out
 
 
