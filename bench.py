@@ -1152,8 +1152,8 @@ def run_ours(args, D):
             line["scaling_strong"] = strong
         if stored is not None:
             line["stored_matrix"] = stored
-        line["strict"] = ("timed with strict=False (no device synchronisation after each call); the drop-in default "
-                          "TRAK_B200_STRICT=1 adds a cudaDeviceSynchronize and a status read per call")
+        line["strict"] = ("timed with strict=False (no wait after each call); the drop-in default "
+                          "TRAK_B200_STRICT=1 adds a wait for the stream per call, after which it looks at the status word")
         if featurize is not None:
             line["featurize"] = featurize
         if featurize_job is not None:
