@@ -21,6 +21,17 @@ namespace tb {
 constexpr uint32_t CACHED_A_BYTES = 128u * STAGE_K * 2u;  // one stored tile: 16 KB
 constexpr uint32_t CACHED_MAX_STAGES = 8;
 
+// gen_normal's halves of the even and the odd column to all 16 features, in order, of the column 2 (lane & 15) + h
+__device__ __forceinline__ void meet_halves(const uint32_t (&even)[4], const uint32_t (&odd)[4], uint32_t h, uint32_t (&w)[8]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t keep = h ? odd[i] : even[i];
+        const uint32_t recv = __shfl_xor_sync(0xffffffffu, h ? even[i] : odd[i], 16);
+        w[2 * i] = __byte_perm(keep, recv, h ? 0x1054u : 0x5410u);
+        w[2 * i + 1] = __byte_perm(keep, recv, h ? 0x3276u : 0x7632u);
+    }
+}
+
 // grid (N / 128, feature tiles), 128 threads: thread = one output column = one XORWOW stream of that tile
 template <int PTYPE, bool BF16>
 __global__ void __launch_bounds__(128) materialize_kernel(uint16_t* __restrict__ matrix, uint32_t seed, uint32_t tiles,
@@ -28,8 +39,6 @@ __global__ void __launch_bounds__(128) materialize_kernel(uint16_t* __restrict__
     const uint32_t q = threadIdx.x >> 5, lane = threadIdx.x & 31u, h = lane >> 4;
     const uint32_t stream_col = blockIdx.x * 128u + q * 32u + lane;
     const uint32_t by = blockIdx.y;
-    const uint32_t sel_lo = h ? 0x1054u : 0x5410u;
-    const uint32_t sel_hi = h ? 0x3276u : 0x7632u;
     SignBases<BF16> bases;
     if (PTYPE == TB_RADEMACHER) bases.load();
     Xw st;
@@ -41,10 +50,13 @@ __global__ void __launch_bounds__(128) materialize_kernel(uint16_t* __restrict__
 #pragma unroll CHUNK_UNROLL
         for (uint32_t c = 0; c < 4; ++c) {
             uint32_t w[8];
-            if (PTYPE == TB_RADEMACHER)
-                gen_rademacher<BF16>(st, h, sel_lo, bases, w);
-            else
-                gen_normal<BF16>(st, h, sel_lo, sel_hi, w);
+            if constexpr (PTYPE == TB_RADEMACHER) {
+                gen_rademacher<BF16>(st, h, bases, w);
+            } else {
+                uint32_t even[4], odd[4];
+                gen_normal<BF16>(st, even, odd);
+                meet_halves(even, odd, h, w);
+            }
             row[2u * c] = make_uint4(w[0], w[1], w[2], w[3]);
             row[2u * c + 1u] = make_uint4(w[4], w[5], w[6], w[7]);
         }

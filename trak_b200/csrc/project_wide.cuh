@@ -6,7 +6,7 @@
 // accumulate.  All 512 TMEM columns are accumulators here (128 output columns x up to 512 rows,
 // two N = Bpad/2 MMAs per 16 features), which leaves no tensor memory for the generated operand:
 // the generator threads write their slice into shared memory in the K-major 64-byte-swizzle
-// layout (one thread = one output column = one 64-byte row of the operand) and hand it over with
+// layout (two threads = two output columns = two 64-byte rows of the operand) and hand it over with
 // fence.proxy.async + an mbarrier; both MMA operands then come from shared memory.
 //
 //   * WIDE_NG generator groups of four warps, one CTA per SM; group g walks feature tiles
@@ -30,7 +30,7 @@ constexpr uint32_t WIDE_A_RING = WIDE_NG * WIDE_SA * WIDE_A_BYTES;
 constexpr uint32_t WIDE_MAX_STAGES = 6;                // deepest gradient ring
 constexpr uint32_t WIDE_MAX_ROWS = 512;                // rows per launch (all 512 TMEM columns)
 
-template <int PTYPE, bool BF16>
+template <bool BF16>
 __global__ void __launch_bounds__((4 * WIDE_NG + 2) * 32, 1)
 project_wide_kernel(const __grid_constant__ CUtensorMap tmap, const ProjParams p) {
     constexpr uint32_t NG = WIDE_NG, SA = WIDE_SA;
@@ -46,7 +46,7 @@ project_wide_kernel(const __grid_constant__ CUtensorMap tmap, const ProjParams p
     volatile uint32_t* abort_flag = &abort_word;
 
     cudaTriggerProgrammaticLaunchCompletion();
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t SB = p.stages;
     const uint32_t half_rows = p.Bpad / 2u;            // rows per MMA (N of the instruction)
     const uint32_t stage_bytes = p.Bpad * (WIDE_K * 2u);
@@ -89,14 +89,11 @@ project_wide_kernel(const __grid_constant__ CUtensorMap tmap, const ProjParams p
         // ------------------------- generators, then epilogue -------------------------
         const uint32_t g = warp >> 2, q = warp & 3u;
         const uint32_t h = lane >> 4;
-        const uint32_t m = q * 32u + lane;                 // operand row = TMEM lane of the results
-        const uint32_t stream_col = col0 + m;
-        const uint32_t sel_lo = h ? 0x1054u : 0x5410u;
-        const uint32_t sel_hi = h ? 0x3276u : 0x7632u;
-        SignBases<BF16> bases;
-        if (PTYPE == TB_RADEMACHER) bases.load();
-        const uint32_t row_addr = smem_base + g * (SA * WIDE_A_BYTES) + m * 64u;
-        const uint32_t sw = (m >> 1) & 3u;                 // 64-byte swizzle of this row
+        const uint32_t stream_col = col0 + q * 32u + lane;
+        // even columns are operand rows 0 to 15 of the warp's 32, odd ones 16 to 31, as in project_kernel; this lane
+        // writes 16-byte piece 2c + h of both rows per 16 features c
+        const uint32_t row_addr = smem_base + g * (SA * WIDE_A_BYTES) + (q * 32u + (lane & 15u)) * 64u;
+        const uint32_t sw = (lane >> 1) & 3u;              // 64-byte swizzle of both rows
         bool ok = true;
         uint32_t slot = 0, ph = 0;
         for (uint32_t ti = g; ti < ntile && ok; ti += NG) {
@@ -116,17 +113,13 @@ project_wide_kernel(const __grid_constant__ CUtensorMap tmap, const ProjParams p
                     }
                     const uint32_t dst = row_addr + slot * WIDE_A_BYTES;
                     // one copy of the (long) Gaussian chunk body keeps the loop in the instruction cache
-                    constexpr int CHUNK_UNROLL = PTYPE == TB_NORMAL ? 1 : 2;
-#pragma unroll CHUNK_UNROLL
+#pragma unroll 1
                     for (uint32_t c = 0; c < 2; ++c) {
-                        uint32_t w[8];
-                        if (PTYPE == TB_RADEMACHER)
-                            gen_rademacher<BF16>(st, h, sel_lo, bases, w);
-                        else
-                            gen_normal<BF16>(st, h, sel_lo, sel_hi, w);
-                        // features 16c .. 16c+15 of this column: 16-byte pieces 2c and 2c + 1 of the row
-                        st_shared_v4(dst + (((2u * c) ^ sw) << 4), w[0], w[1], w[2], w[3]);
-                        st_shared_v4(dst + (((2u * c + 1u) ^ sw) << 4), w[4], w[5], w[6], w[7]);
+                        uint32_t even[4], odd[4];
+                        gen_normal<BF16>(st, even, odd);
+                        const uint32_t piece = dst + (((2u * c + h) ^ sw) << 4);
+                        st_shared_v4(piece, even[0], even[1], even[2], even[3]);
+                        st_shared_v4(piece + 16u * 64u, odd[0], odd[1], odd[2], odd[3]);
                     }
                     fence_proxy_async_smem();
                     mbar_arrive(smem_u32(&bar_full_a[g][slot]));
@@ -137,7 +130,7 @@ project_wide_kernel(const __grid_constant__ CUtensorMap tmap, const ProjParams p
                 }
                 if (!ok) break;
                 const uint32_t tl = (ti - g) / NG;  // tiles this group has finished
-                ok = drain_accumulators<NG, 4u>(p, smem_u32(&bar_acc), smem_u32(&bar_drained), &tmem_slot,
+                ok = drain_accumulators<NG, false>(p, smem_u32(&bar_acc), smem_u32(&bar_drained), &tmem_slot,
                                                 tl * p.drains_per_tile + s0 / p.epoch,
                                                 !(s1 == p.nst && tl + 1u == (ntile + NG - 1) / NG), abort_flag);
             }
@@ -147,7 +140,7 @@ project_wide_kernel(const __grid_constant__ CUtensorMap tmap, const ProjParams p
             const uint32_t drains = ((ntile + NG - 1) / NG) * p.drains_per_tile;
             uint32_t d = (ntile > g ? (ntile - g + NG - 1) / NG : 0u) * p.drains_per_tile;
             for (; ok && d < drains; ++d)
-                ok = drain_accumulators<NG, 4u>(p, smem_u32(&bar_acc), smem_u32(&bar_drained), &tmem_slot, d,
+                ok = drain_accumulators<NG, false>(p, smem_u32(&bar_acc), smem_u32(&bar_drained), &tmem_slot, d,
                                                 d + 1u < drains, abort_flag);
         }
     } else {

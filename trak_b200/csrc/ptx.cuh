@@ -142,6 +142,13 @@ __device__ __forceinline__ void tmem_st_x8(uint32_t taddr, const uint32_t (&r)[8
                  "r"(r[6]), "r"(r[7])
                  : "memory");
 }
+// One warp writes 8 consecutive 32-bit columns of 16 tensor-memory lanes: threads 0 to 15 the first four of lanes 0 to 15,
+// threads 16 to 31 the last four of the same lanes.
+__device__ __forceinline__ void tmem_st_halves_x4(uint32_t taddr, const uint32_t (&r)[4]) {
+    asm volatile("tcgen05.st.sync.aligned.16x32bx2.x4.b32 [%0], 4, {%1, %2, %3, %4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
+                 "r"(r[2]), "r"(r[3])
+                 : "memory");
+}
 // One warp reads 16 consecutive 32-bit columns of its own 32 lanes.
 __device__ __forceinline__ void tmem_ld_x16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
@@ -166,6 +173,10 @@ __device__ __forceinline__ void tmem_ld_x8(uint32_t taddr, uint32_t (&r)[8]) {
 // Fire-and-forget fp32 add (round to nearest) performed by the L2: no read comes back to the SM.
 __device__ __forceinline__ void red_add_f32(float* addr, float v) {
     asm volatile("red.global.add.f32 [%0], %1;" ::"l"(addr), "f"(v) : "memory");
+}
+
+__device__ __forceinline__ void red_add_f32x2(float2* addr, float2 v) {
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(addr), "f"(v.x), "f"(v.y) : "memory");
 }
 
 // ---- MMA issue ----------------------------------------------------------------
