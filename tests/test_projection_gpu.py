@@ -511,6 +511,25 @@ def test_wide_gaussian_batches(cuda, B, F, N, seed, T, dt):
     torch.testing.assert_close(out, 0.5 + 0.25 * wide, rtol=1e-6, atol=1e-5)
 
 
+@pytest.mark.parametrize("T,N", [(148, 512), (148, 1536), (147, 1024), (37, 1536), (13, 2048), (1, 512), (700, 512)])
+def test_wide_grid_splits(cuda, T, N):
+    """Bundles of one size, of two, more than seven tiles in one, a shorter last bundle, fewer tiles than generator groups:
+    every feature tile is walked exactly once.  One-hot rows in the first and last feature of tiles that lie in different
+    bundles give the narrow kernel's bits."""
+    F, B = 32 * T + 5, 272
+    fts = o.feature_tile_size(F, T)
+    tiles = -(-F // fts)
+    g = torch.randn(B, F, generator=torch.Generator().manual_seed(T)).half()
+    for r in range(128):
+        g[r].zero_()
+        t = r * (tiles - 1) // 127
+        g[r, min(F - 1, t * fts + (fts - 1) * (r & 1))] = 1.0
+    g = g.to(cuda)
+    wide, narrow = ours(g, N, 5, T, NOR), torch.cat([ours(g[i:i + 136], N, 5, T, NOR) for i in (0, 136)])
+    assert torch.equal(wide[:128], narrow[:128])
+    assert rel_rows(wide.cpu().numpy(), narrow.cpu().numpy()) <= 1e-4   # as above
+
+
 def test_randomised_wide_shapes_against_the_narrow_kernel(cuda):
     """Sixteen seeded random shapes for the 512-row Gaussian kernel (row counts on both sides of a pass, feature
     counts around tile and stage boundaries, tile counts that leave generator groups idle or give ragged last
