@@ -618,6 +618,8 @@ STORED_SHAPES = [  # B, F, N, seed, tiles, dtype
     (300, 4097, 512, 99, 37, "bf16"),     # two passes of the stored-matrix kernel
     (5, 16, 512, 9, 148, "f16"),          # fewer features than tiles
     (64, 4096, 1536, 4, 4, "f16"),        # tile size a multiple of 64
+    (65, 70_001, 2048, 3, 1, "f16"),      # two column tiles a CTA with two sets of accumulators, three chains
+    (129, 3001, 512, 3, 5, "f16"),        # two column tiles a CTA, one set
 ]
 
 

@@ -20,6 +20,7 @@ namespace tb {
 
 constexpr uint32_t CACHED_A_BYTES = 128u * STAGE_K * 2u;  // one stored tile: 16 KB
 constexpr uint32_t CACHED_MAX_STAGES = 8;
+constexpr uint32_t cached_threads(uint32_t nacc) { return (2u + 4u * nacc) * 32u; }
 
 // gen_normal's halves of the even and the odd column to all 16 features, in order, of the column 2 (lane & 15) + h
 __device__ __forceinline__ void meet_halves(const uint32_t (&even)[4], const uint32_t (&odd)[4], uint32_t h, uint32_t (&w)[8]) {
@@ -64,12 +65,16 @@ __global__ void __launch_bounds__(128) materialize_kernel(uint16_t* __restrict__
     }
 }
 
-// One CTA = 128 output columns x up to 256 rows x a bundle of feature tiles.  Warp 0 issues TMA (a stored matrix
-// tile and the matching gradient box per 64 features, never multicast), warp 1 the MMAs, warps 2-5 read the
-// accumulators out.  Both operands come from shared memory; the kernel is bound by the HBM stream of the matrix.
-// The accumulation chains (ProjParams::epoch) alternate between two accumulators of 256 TMEM columns, so the MMA
-// warp starts the next chain while the epilogue warps add the finished one to the partial.
-__global__ void __launch_bounds__(192, 1)
+// One CTA = NACC x 128 output columns x up to 256 rows x a bundle of feature tiles.  Warp 0 issues TMA (NACC stored matrix
+// tiles and the matching gradient box per 64 features, never multicast), warp 1 the MMAs, four warps per accumulator of
+// 128 columns read the results out.  Both operands come from shared memory.  The accumulation chains
+// (ProjParams::epoch) alternate between two sets of accumulators, so the MMA warp starts the next chain while the
+// epilogue warps add the finished one to the partial; two accumulators of more than 128 rows leave room for one set only.
+// Bound by the power limit at 256 rows (SM clock 0.9 GHz in a row of calls) and by the HBM stream of the matrix below.
+// With one column tile per CTA every gradient box crossed from the L2 twice as often (34 GB instead of 17 for 256 rows x
+// 2,097,169 features -> 4096, beside the 17 GB of the matrix): 4.98 -> 4.71 ms a call.
+template <uint32_t NACC>
+__global__ void __launch_bounds__(cached_threads(NACC), 1)
 project_cached_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                       const ProjParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -82,14 +87,15 @@ project_cached_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     volatile uint32_t* abort_flag = &abort_word;
 
     cudaTriggerProgrammaticLaunchCompletion();
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t S = p.stages;
-    const uint32_t b_bytes = p.Bpad * 128u, stage_bytes = CACHED_A_BYTES + b_bytes;
+    const uint32_t b_bytes = p.Bpad * 128u, stage_bytes = NACC * CACHED_A_BYTES + b_bytes;
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t ct = blockIdx.x;
+    const uint32_t ct = blockIdx.x * NACC;  // first of this CTA's column tiles
     const uint32_t tile0 = blockIdx.y * p.tiles_per_bundle;
     const uint32_t ntile = min(p.tiles_per_bundle, p.tiles - tile0);
     const uint32_t nblocks = ntile * p.nst;
+    const uint32_t set_cols = NACC * p.Bpad, sets = set_cols <= 256u ? 2u : 1u;
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < S; ++s) {
@@ -98,7 +104,7 @@ project_cached_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         }
         for (uint32_t a = 0; a < 2; ++a) {
             mbar_init(smem_u32(&bar_acc[a]), 1);
-            mbar_init(smem_u32(&bar_drained[a]), 128u);
+            mbar_init(smem_u32(&bar_drained[a]), 4u * NACC * 32u);
         }
         abort_word = 0;
         fence_mbar_init();
@@ -133,8 +139,10 @@ project_cached_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 const uint32_t bar = smem_u32(&bar_full[slot]);
                 const uint32_t dst = smem_base + slot * stage_bytes;
                 mbar_expect_tx(bar, stage_bytes);
-                tma_load_3d(dst, &tmap_a, 0, 0, (int)(ct * p.tiles * p.nst + z), bar);
-                tma_load_2d(dst + CACHED_A_BYTES, &tmap_b, 0, (int)(z * p.Bpad), bar);
+#pragma unroll
+                for (uint32_t a = 0; a < NACC; ++a)
+                    tma_load_3d(dst + a * CACHED_A_BYTES, &tmap_a, 0, 0, (int)((ct + a) * p.tiles * p.nst + z), bar);
+                tma_load_2d(dst + NACC * CACHED_A_BYTES, &tmap_b, 0, (int)(z * p.Bpad), bar);
             }
             if (++slot == S) {
                 slot = 0;
@@ -145,7 +153,8 @@ project_cached_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         // ------------------------------- MMA issuer -------------------------------
         const bool leader = elect_one();
         bool ok = true;
-        uint32_t slot = 0, ph = 0, started = 0, epoch_no = 0, until = p.epoch;
+        uint32_t slot = 0, ph = 0, started = 0, until = p.epoch;
+        uint32_t set = 0, set_ph = 1u;  // the chain's accumulators; parity of the wait for their last read-out
         for (uint32_t it = 0; it < nblocks; ++it) {
             bool got = mbar_wait(smem_u32(&bar_full[slot]), ph, abort_flag);
             if (!__all_sync(0xffffffffu, got)) {
@@ -155,12 +164,16 @@ project_cached_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             }
             tc_fence_after();
             const uint32_t sa = smem_base + slot * stage_bytes;
-            const uint64_t a_desc = smem_desc_k_sw128(sa), b_desc = smem_desc_k_sw128(sa + CACHED_A_BYTES);
+            const uint64_t a_desc = smem_desc_k_sw128(sa), a1_desc = smem_desc_k_sw128(sa + CACHED_A_BYTES);
+            const uint64_t b_desc = smem_desc_k_sw128(sa + NACC * CACHED_A_BYTES);
             if (leader) {
+                const uint32_t d = tmem_base + set * set_cols;
 #pragma unroll
-                for (uint32_t k = 0; k < 4; ++k)  // 16 features further: 32 bytes inside the swizzle row
-                    umma_f16_ss(tmem_base + (epoch_no & 1u) * 256u, a_desc + 2u * k, b_desc + 2u * k, p.idesc,
-                                started | (k > 0 ? 1u : 0u));
+                for (uint32_t k = 0; k < 4; ++k) {  // 16 features further: 32 bytes inside the swizzle row
+                    const uint32_t acc = started | (k > 0 ? 1u : 0u);
+                    umma_f16_ss(d, a_desc + 2u * k, b_desc + 2u * k, p.idesc, acc);
+                    if (NACC == 2) umma_f16_ss(d + p.Bpad, a1_desc + 2u * k, b_desc + 2u * k, p.idesc, acc);
+                }
                 tc_commit(smem_u32(&bar_empty[slot]));
             }
             started = 1u;
@@ -169,33 +182,37 @@ project_cached_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 ph ^= 1u;
             }
             if (--until == 0 && it + 1 < nblocks) {
-                // end of an accumulation chain (see ProjParams::epoch): hand this accumulator to the epilogue warps
-                // and go on in the other one, once its chain before last has been read out
+                // end of an accumulation chain (see ProjParams::epoch): hand these accumulators to the epilogue warps and
+                // go on in the other set, or the same one, once its last chain has been read out
                 until = p.epoch;
-                if (leader) tc_commit(smem_u32(&bar_acc[epoch_no & 1u]));
+                if (leader) tc_commit(smem_u32(&bar_acc[set]));
                 started = 0;
-                ++epoch_no;
-                if (epoch_no >= 2u) {
-                    got = mbar_wait(smem_u32(&bar_drained[epoch_no & 1u]), ((epoch_no >> 1) - 1u) & 1u, abort_flag);
-                    if (!__all_sync(0xffffffffu, got)) {
-                        if (leader) fail(p.status, abort_flag, ST_TIMEOUT_ACC, 0x8000u | it);
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
+                if (++set == sets) {
+                    set = 0;
+                    set_ph ^= 1u;
                 }
+                // (the first wait for the second set returns at once)
+                got = mbar_wait(smem_u32(&bar_drained[set]), set_ph, abort_flag);
+                if (!__all_sync(0xffffffffu, got)) {
+                    if (leader) fail(p.status, abort_flag, ST_TIMEOUT_ACC, 0x8000u | it);
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
             }
         }
-        if (ok && leader) tc_commit(smem_u32(&bar_acc[epoch_no & 1u]));
+        if (ok && leader) tc_commit(smem_u32(&bar_acc[set]));
     } else {
         // --------------------------------- epilogue ---------------------------------
         const uint32_t q = warp & 3u, h = lane >> 4;   // a warp reaches the TMEM lanes 32 (warp % 4) ...
-        const uint32_t n_out = ct * 128u + q * 32u + 2u * (lane & 15u) + h;  // lane order of the generator
+        const uint32_t acc = (warp - 2u) >> 2;
+        const uint32_t n_out = (ct + acc) * 128u + q * 32u + 2u * (lane & 15u) + h;  // lane order of the generator
         float* dst = p.partials + (size_t)blockIdx.y * p.B * p.N + n_out;
-        const uint32_t lane_base = (q * 32u) << 16;
+        const uint32_t src = tmem_base + ((q * 32u) << 16) + acc * p.Bpad;
         const uint32_t drains = (nblocks + p.epoch - 1u) / p.epoch;
+        uint32_t set = 0, ph = 0;
         for (uint32_t e = 0; e < drains; ++e) {
-            bool got = mbar_wait(smem_u32(&bar_acc[e & 1u]), (e >> 1) & 1u, abort_flag);
+            bool got = mbar_wait(smem_u32(&bar_acc[set]), ph, abort_flag);
             got = __all_sync(0xffffffffu, got);
             if (!got) {
                 if (lane == 0) fail(p.status, abort_flag, ST_TIMEOUT_ACC, warp);
@@ -203,13 +220,13 @@ project_cached_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             }
             tc_fence_after();
             // chain 0 stores, the later chains add in the L2 (see drain_accumulators)
-            for (uint32_t cb = 0; cb < p.Bpad / 8u; ++cb) {
-                uint32_t r[8];
-                tmem_ld_x8(tmem_base + lane_base + (e & 1u) * 256u + cb * 8u, r);
+            for (uint32_t cb = 0; cb < p.Bpad / 16u; ++cb) {
+                uint32_t r[16];
+                tmem_ld_x16(src + set * set_cols + cb * 16u, r);
                 tmem_wait_ld();
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const uint32_t b = cb * 8u + j;
+                for (int j = 0; j < 16; ++j) {
+                    const uint32_t b = cb * 16u + j;
                     if (b < p.B) {
                         if (e == 0)
                             __stcg(dst + (size_t)b * p.N, __uint_as_float(r[j]));
@@ -218,9 +235,13 @@ project_cached_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                     }
                 }
             }
-            if (e + 2 < drains) {  // the chain after next accumulates here again
+            if (e + sets < drains) {  // a later chain accumulates here again
                 tc_fence_before();
-                mbar_arrive(smem_u32(&bar_drained[e & 1u]));
+                mbar_arrive(smem_u32(&bar_drained[set]));
+            }
+            if (++set == sets) {
+                set = 0;
+                ph ^= 1u;
             }
         }
     }
