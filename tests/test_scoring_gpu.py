@@ -206,6 +206,26 @@ def test_inverse_at_sizes_around_the_block_boundaries(cuda, k):
     assert rel(inv2, ref / ref.abs().mean()) <= 2e-5
 
 
+@pytest.mark.parametrize("k,ld", [(1, 1), (3, 7), (4, 4), (8, 9), (9, 12), (63, 64), (64, 64), (65, 65), (72, 73), (100, 128),
+                                  (129, 131), (450, 450), (512, 515)])
+def test_inverse_inside_a_diagonal_block(cuda, k, ld):
+    """Sizes around the factorisation's pieces of 4, steps of 8 and tiles of 64, rows that are 16-byte aligned and rows that
+    are not; the last pivot alone not positive."""
+    from trak_b200 import _lib, score_computers as sc
+    y = torch.randn(3 * k + 5, k, device=cuda, generator=torch.Generator(device=cuda).manual_seed(k), dtype=torch.float64)
+    A = torch.full((k, ld), float("nan"), device=cuda)[:, :k]
+    A.copy_(y.T @ y / k)
+    ref = torch.linalg.inv(A.double() + 1e-2 * torch.eye(k, device=cuda, dtype=torch.float64))
+    inv = sc.spd_inverse_(A, 1e-2, rescale=False)
+    assert torch.equal(inv, inv.T)
+    assert rel(inv, ref) <= 2e-5   # as at the sizes above
+    bad = torch.eye(k, device=cuda)
+    bad[-1, -1] = -1.0
+    with pytest.raises(_lib.NotPositiveDefinite):
+        sc.spd_inverse_(bad, 0.0)
+    _lib.device_status(cuda.index)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 1, 1), (129, 257, 33), (300, 700, 95), (128, 256, 64), (513, 100, 4097)])
 def test_gram_and_gemm_at_ragged_sizes(cuda, M, N, K):
     """Tile, chunk (64 k) and slot (32 k) boundaries of both GEMM kernels, with accumulation into existing output."""

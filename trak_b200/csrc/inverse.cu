@@ -29,48 +29,127 @@ constexpr int OUTER = 512;  // block column
 constexpr int TS = 68;      // padded row length of a shared-memory tile (floats)
 typedef float Tile[NB][TS];
 
-// acc[4][4] += sum_t At[t][ty*4 + i] * Bt[t][tx*4 + j]   (both tiles stored t-major)
-__device__ __forceinline__ void tile_mma(const float (*At)[TS], const float (*Bt)[TS], int ty, int tx,
-                                         float (&acc)[4][4]) {
-#pragma unroll 8
-    for (int t = 0; t < NB; ++t) {
-        const float4 a = *reinterpret_cast<const float4*>(&At[t][ty * 4]);
-        const float4 b = *reinterpret_cast<const float4*>(&Bt[t][tx * 4]);
-        const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+// The 256 threads of a CTA share the products of 64 x 64 tiles: a thread of the k group g = tid / 64 accumulates
+// four 4 x 4 pieces, 32 rows and 32 columns apart, over a quarter of k, and ends with the piece (ty, tx) of the result.
+__device__ __forceinline__ int piece_row(int tid) { return 8 * (tid >> 7) + ((tid & 63) >> 3); }
+__device__ __forceinline__ int piece_col(int tid) { return 8 * ((tid >> 6) & 1) + (tid & 7); }
+constexpr int EXCHANGE_FLOATS = 4 * 3 * 16 * 64;  // what a product's k groups hand to one another
+
+// acc[4][4] = sum_t At[t][ty*4 + i] * Bt[t][tx*4 + j]   (both tiles stored t-major; 256 threads)
+// Shared memory bounds it: a 16-byte load takes the SM four cycles whatever its lanes share.  With one piece a thread
+// and all of k that is 1024 loads a product and 4450 cycles; four pieces over a quarter of k each and the exchange of three
+// quarters of the partial sums are 704 and 4000, with the next loads issued before a step's multiplications.
+__device__ __forceinline__ void tile_mma(const float (*At)[TS], const float (*Bt)[TS], float* exchange, float (&acc)[4][4]) {
+    const int tid = threadIdx.x, g = tid >> 6, u = tid & 63, r0 = (u >> 3) * 4, c0 = (u & 7) * 4;
+    uint64_t s2[8][4] = {};
+    float4 a0, a1, a0n, a1n;
+    ulonglong2 b0, b1, b0n, b1n;
+    auto load = [&](int t) {
+        a0n = *reinterpret_cast<const float4*>(&At[t][r0]);
+        a1n = *reinterpret_cast<const float4*>(&At[t][r0 + 32]);
+        b0n = *reinterpret_cast<const ulonglong2*>(&Bt[t][c0]);
+        b1n = *reinterpret_cast<const ulonglong2*>(&Bt[t][c0 + 32]);
+    };
+    load(g * 16);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+    for (int t = 0; t < 16; ++t) {
+        a0 = a0n; a1 = a1n; b0 = b0n; b1 = b1n;
+        if (t < 15) load(g * 16 + t + 1);
+        const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        const uint64_t bv[4] = {b0.x, b0.y, b1.x, b1.y};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+        for (int i = 0; i < 8; ++i) {
+            const uint64_t a = pack_f32x2(av[i], av[i]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s2[i][j] = fma_f32x2(a, bv[j], s2[i][j]);
+        }
     }
+    float s[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) unpack_f32x2(s2[i][j], s[i][2 * j], s[i][2 * j + 1]);
+    // group g keeps its threads' piece in the rows 32 (g >> 1) .. and the columns 32 (g & 1) ..
+    float4* ex = reinterpret_cast<float4*>(exchange);
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+        if (d == g) continue;
+        float4* to = ex + ((d * 3 + (g - (g > d))) * 4) * 64 + u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float* row = &s[4 * (d >> 1) + i][4 * (d & 1)];
+            to[i * 64] = make_float4(row[0], row[1], row[2], row[3]);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int d = 0; d < 4; ++d)
+        if (d == g) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = s[4 * (d >> 1) + i][4 * (d & 1) + j];
+        }
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+        const float4* from = ex + ((g * 3 + e) * 4) * 64 + u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 v = from[i * 64];
+            acc[i][0] += v.x; acc[i][1] += v.y; acc[i][2] += v.z; acc[i][3] += v.w;
+        }
+    }
+    __syncthreads();  // the next product writes there again
 }
 
-// dst[t][i] = src[i*ld + t] (transposed) or dst[i][t] = src[i*ld + t], zero outside rows x cols.  The first 256 threads; four
-// consecutive elements of a row each where the rows are 16-byte aligned.  A warp covers eight rows x 16 columns, so
-// the transposed stores meet two to a bank.
-template <bool TRANS>
-__device__ __forceinline__ void load_tile(Tile& dst, const float* src, int64_t ld, int rows, int cols) {
-    if (threadIdx.x >= 256u) return;
-    const bool vec = (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
+__device__ __forceinline__ void put_piece(Tile& T, int ty, int tx, const float (&acc)[4][4]) {
 #pragma unroll
-    for (int it = 0; it < 4; ++it) {
-        const int e = it * 256 + (int)threadIdx.x, warp = e >> 5, lane = e & 31;
-        const int i = (warp >> 2) * 8 + (lane & 7), t = (warp & 3) * 16 + (lane >> 3) * 4;
-        float v[4];
-        if (vec && i < rows && t + 4 <= cols) {
-            const float4 x = *reinterpret_cast<const float4*>(src + (int64_t)i * ld + t);
-            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-        } else {
+    for (int a = 0; a < 4; ++a)
+        *reinterpret_cast<float4*>(&T[ty * 4 + a][tx * 4]) = make_float4(acc[a][0], acc[a][1], acc[a][2], acc[a][3]);
+}
+
+// Rows and columns [0, rows) x [0, cols) of a 64 x 64 tile at src, zero outside, in the registers of N threads (this one is
+// number `id`); four consecutive elements of a row each where the rows are 16-byte aligned.  Past the L1: other CTAs write
+// the tiles between a CTA's reads.
+template <int N>
+struct TileRegs {
+    float v[4096 / (4 * N)][4];
+    static __device__ __forceinline__ void place(int id, int it, int& i, int& t) {  // eight rows x 16 columns a warp
+        const int e = it * N + id, warp = e >> 5, lane = e & 31;
+        i = (warp >> 2) * 8 + (lane & 7);
+        t = (warp & 3) * 16 + (lane >> 3) * 4;
+    }
+    __device__ __forceinline__ void fetch(int id, const float* src, int64_t ld, int rows, int cols) {
+        const bool vec = (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] = (i < rows && t + u < cols) ? src[(int64_t)i * ld + t + u] : 0.0f;
-        }
-        if (TRANS) {
+        for (int it = 0; it < 4096 / (4 * N); ++it) {
+            int i, t;
+            place(id, it, i, t);
+            if (vec && i < rows && t + 4 <= cols) {
+                const float4 x = __ldcg(reinterpret_cast<const float4*>(src + (int64_t)i * ld + t));
+                v[it][0] = x.x; v[it][1] = x.y; v[it][2] = x.z; v[it][3] = x.w;
+            } else {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) dst[t + u][i] = v[u];
-        } else {
-            *reinterpret_cast<float4*>(&dst[i][t]) = make_float4(v[0], v[1], v[2], v[3]);
+                for (int u = 0; u < 4; ++u) v[it][u] = (i < rows && t + u < cols) ? __ldcg(src + (int64_t)i * ld + t + u) : 0.0f;
+            }
         }
     }
-}
+    // dst[t][i] (TRANS; the stores meet two to a bank) or dst[i][t]
+    template <bool TRANS>
+    __device__ __forceinline__ void put(int id, Tile& dst) const {
+#pragma unroll
+        for (int it = 0; it < 4096 / (4 * N); ++it) {
+            int i, t;
+            place(id, it, i, t);
+            if (TRANS) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) dst[t + u][i] = v[it][u];
+            } else {
+                *reinterpret_cast<float4*>(&dst[i][t]) = make_float4(v[it][0], v[it][1], v[it][2], v[it][3]);
+            }
+        }
+    }
+};
 
 // A += lambda I, and zero for the counters that the block columns' CTAs meet at.
 __global__ void prepare_kernel(float* A, int64_t lda, int k, float lambda, uint32_t* counters, int n) {
@@ -80,184 +159,223 @@ __global__ void prepare_kernel(float* A, int64_t lda, int k, float lambda, uint3
 }
 
 // Factors the jb x jb diagonal tile S = L L^T (lower triangle used) and inverts L in the same sweep (forward
-// elimination of [L | I]); writes inv(L) (lower, zero above, zero-padded to 64 x 64) to dinv.  STEP_THREADS threads:
-// 256 as a 16 x 16 grid of 4 x 4 pieces in registers, and one more warp, the pivot warp, whose lane l keeps the
-// diagonal piece (l, l).  The tile is walked four columns at a time, piece column q in step q.  Thread (ty, tx) holds
-// a piece of S until step tx and a piece of W = inv(L) from then on (it is zero, or the identity, until its column has
-// been reached), so a step is one rank-four update whichever it is:
-//   1. the pivot warp has factored the diagonal piece q, D = Ld Ld^T, and published Ld;
-//   2. the threads of piece column q turn their pieces into rows of L (B Ld^-T), those of piece row q apply Ld^-1 to
-//      their four rows of W, which makes them final; both publish, one vector per column respectively row of q;
-//   3. the threads below update their pieces, S -= L_q L_q^T and W -= L_q W_q.
-// Beside 2 and 3 the pivot warp applies L_{q-1} to the diagonal pieces, computes the one piece of L_q that the next
-// one needs from what its owner published, updates it and factors it: the chain of four reciprocal square roots is
-// off the other warps' path.  (With S and W pieces updated one after the other in every thread, and the next piece
-// factored after its update by the grid's own diagonal thread, a tile took 9 us.)
+// elimination of [L | I]); writes inv(L) (lower, zero above, zero-padded to 64 x 64) to dinv and, t-major, to Dt.
+// CHOL_THREADS threads: 136 hold the lower triangle's 4 x 4 pieces in registers, warp 0 is the pivot warp.  The tile is
+// walked eight columns at a time.  The thread of piece (ty, tx) holds it of S until the step of its columns and of
+// W = inv(L) from then on (it is zero until its column has been reached, final from the step of its rows on), so that a
+// step is one small product and one rank-eight update whichever it is.  With Ld Ld^T the diagonal block of step q and
+//     P[d][i] = S[i, 8q + d] below the block, the identity in it, W[8q + d, i] left of it,
+//   1. the pivot warp has factored the block and published Ld^-1;
+//   2. O = Ld^-1 P: below the block the columns of L, in it and left of it the block's rows of W, final;
+//   3. the threads below update their pieces, x[i, j] -= sum_c O[c][i] O[c][j], and publish P of the next step.
+// Beside 3 the pivot warp takes the next diagonal block as it was before this step, updates it from O and factors it,
+// every lane for itself in registers (a lane then solves for one column of the inverse): a chain of eight reciprocal
+// square roots, 50 cycles each.
+// With four columns a step, a factor published instead of its inverse and substitutions by the threads of its pieces, a
+// tile took 12,500 cycles, 9,700 now (with 8 x 4 pieces in three warps 12,400:
+// half of it is stores and loads of shared memory, of which a warp gets one of 16 bytes every 14 cycles).
 // Rows and columns beyond jb are an identity block.  `buf` is CHOL_FLOATS floats of shared memory outside S.
-constexpr int CHOL_FLOATS = 64 + 3 * 256;
+constexpr int CW = 8;                                             // columns of a step
+constexpr int CHOL_FLOATS = 2 * CW * NB + 4 * CW * CW;
 static_assert(CHOL_FLOATS <= NB * TS, "a tile's worth of shared memory holds chol_block's buffers");
-constexpr int STEP_THREADS = 288;
-struct __align__(16) Chol4 {
-    float l10, l20, l30, l21, l31, l32;  // strictly lower part of Ld
-    float r0, r1, r2, r3;                // reciprocals of its diagonal
-    float ok, pad;
-};
+constexpr int CHOL_THREADS = 192;  // warps 0 (pivot), 1, 2, 3, 5 and 6
 // 1 / sqrt(d) for a normal d; a subnormal one counts as not positive (the inverse would overflow)
 __device__ __forceinline__ float rsqrt_newton(float d) {
     float r;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     return fmaf(r, fmaf(-(0.5f * d) * r, r, 0.5f), r);
 }
-__device__ __forceinline__ Chol4 chol4(const float (&D)[4][4]) {  // lower part used
-    Chol4 c;
-    float p = D[0][0];
-    bool ok = p >= 1.17549435e-38f;
-    c.r0 = rsqrt_newton(p);
-    c.l10 = D[1][0] * c.r0;
-    c.l20 = D[2][0] * c.r0;
-    c.l30 = D[3][0] * c.r0;
-    p = fmaf(-c.l10, c.l10, D[1][1]);
-    ok = ok && p >= 1.17549435e-38f;
-    c.r1 = rsqrt_newton(p);
-    c.l21 = fmaf(-c.l20, c.l10, D[2][1]) * c.r1;
-    c.l31 = fmaf(-c.l30, c.l10, D[3][1]) * c.r1;
-    p = fmaf(-c.l21, c.l21, fmaf(-c.l20, c.l20, D[2][2]));
-    ok = ok && p >= 1.17549435e-38f;
-    c.r2 = rsqrt_newton(p);
-    c.l32 = fmaf(-c.l31, c.l21, fmaf(-c.l30, c.l20, D[3][2])) * c.r2;
-    p = fmaf(-c.l32, c.l32, fmaf(-c.l31, c.l31, fmaf(-c.l30, c.l30, D[3][3])));
-    ok = ok && p >= 1.17549435e-38f;
-    c.r3 = rsqrt_newton(p);
-    c.ok = ok ? 1.0f : 0.0f;
-    c.pad = 0.0f;
-    return c;
+// Column `col` of inv(chol(z)) (rows of z, lower part used) in y; false when a pivot is not positive.
+__device__ __forceinline__ bool invert_block(float (&z)[CW][CW], int col, float (&y)[CW]) {
+    bool ok = true;
+#pragma unroll
+    for (int j = 0; j < CW; ++j) {
+        ok = ok && z[j][j] >= 1.17549435e-38f;
+        const float r = rsqrt_newton(z[j][j]);
+#pragma unroll
+        for (int i = j + 1; i < CW; ++i) z[i][j] *= r;
+#pragma unroll
+        for (int l = j + 1; l < CW; ++l)
+#pragma unroll
+            for (int i = l; i < CW; ++i) z[i][l] = fmaf(-z[i][j], z[l][j], z[i][l]);
+        float t = j == col ? 1.0f : 0.0f;
+#pragma unroll
+        for (int k = 0; k < j; ++k) t = fmaf(-z[j][k], y[k], t);
+        y[j] = t * r;
+    }
+    return ok;
 }
-// x <- Ld^-1 x for one column of four values (forward substitution)
-__device__ __forceinline__ void solve4(const Chol4& c, float& x0, float& x1, float& x2, float& x3) {
-    x0 = x0 * c.r0;
-    x1 = fmaf(-c.l10, x0, x1) * c.r1;
-    x2 = fmaf(-c.l21, x1, fmaf(-c.l20, x0, x2)) * c.r2;
-    x3 = fmaf(-c.l32, x2, fmaf(-c.l31, x1, fmaf(-c.l30, x0, x3))) * c.r3;
-}
-__device__ __forceinline__ float4 row4(const float (&m)[4][4], int a) { return make_float4(m[a][0], m[a][1], m[a][2], m[a][3]); }
-__device__ __forceinline__ Chol4 load_factor(const Chol4* factor) {
-    const float4* f = reinterpret_cast<const float4*>(factor);
-    const float4 f0 = f[0], f1 = f[1], f2 = f[2];
-    return Chol4{f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w, f2.x, f2.y, f2.z, 0.0f};
-}
-__device__ void chol_block(const Tile& S, int jb, float* dinv, uint32_t* status, float* buf) {
-    const int tid = threadIdx.x;
-    Chol4* factor = reinterpret_cast<Chol4*>(buf);                         // [2]: of pieces q and q + 1
-    float4* raw = reinterpret_cast<float4*>(buf + 32);                     // [2][4]: piece (q + 1, q) of S before step q
-    float (*colbufs)[NB] = reinterpret_cast<float(*)[NB]>(buf + 64);       // [2][4][64]: columns of L_q and L_{q-1}
-    float (*rowbuf)[NB] = reinterpret_cast<float(*)[NB]>(buf + 64 + 512);  // [4][64]: rows of W_q
-    static_assert(sizeof(Chol4) <= 16 * sizeof(float), "two factors fit in front of raw");
-    const bool pivot = tid >= 256;
-    // the pivot warp's lane l stands at (l, l); lanes 16 to 31 repeat lane 15 and publish nothing
-    const int ty = pivot ? min(tid - 256, 15) : tid >> 4, tx = pivot ? ty : tid & 15;
+__device__ void chol_block(const Tile& S, int jb, float* dinv, Tile& Dt, uint32_t* status, float* buf) {
+    auto sync = [] { asm volatile("barrier.cta.sync 1, %0;" ::"n"(CHOL_THREADS) : "memory"); };
+    const int tid = threadIdx.x, lane = tid & 31;
+    float (*P)[NB] = reinterpret_cast<float(*)[NB]>(buf);
+    float (*O)[NB] = reinterpret_cast<float(*)[NB]>(buf + CW * NB);
+    float (*inv)[CW] = reinterpret_cast<float(*)[CW]>(buf + 2 * CW * NB);  // Ld^-1 of the step
+    float* const before = buf + 2 * CW * NB + CW * CW;   // [2][CW][CW]: diagonal blocks as they were a step earlier
+    float (*now)[CW] = reinterpret_cast<float(*)[CW]>(before + 2 * CW * CW);
+    const int warp = tid >> 5;
+    const bool pivot = warp == 0;
+    // piece (ty, tx) of the grid's threads, row by row: the first rows' warp, done early, shares a scheduler
+    const int n = (warp == 5 ? 0 : warp == 6 ? 4 : warp) * 32 + lane;
+    const int ty = (int)((sqrtf(8.0f * n + 1.0f) - 1.0f) * 0.5f), tx = n - ty * (ty + 1) / 2;
+    const bool owner = !pivot && n < 136;
+    const int panel = warp == 5 ? lane : warp >= 1 && warp <= 3 ? warp * 32 + lane : -1;  // of the 128 threads that compute O
+    const int steps = (jb + CW - 1) / CW;
+    auto entry = [&](int i, int j) { return i < jb && j < jb ? S[i][j] : i == j ? 1.0f : 0.0f; };
     float x[4][4];
+    if (owner) {
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+        for (int a = 0; a < 4; ++a) {
+            if (ty * 4 + 4 <= jb) {  // (what is above the diagonal of a diagonal piece is never used)
+                const float4 v = *reinterpret_cast<const float4*>(&S[ty * 4 + a][tx * 4]);
+                x[a][0] = v.x; x[a][1] = v.y; x[a][2] = v.z; x[a][3] = v.w;
+            } else {
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int i = ty * 4 + a, j = tx * 4 + b;
-            const float unit = i == j ? 1.0f : 0.0f;
-            // the grid's diagonal threads have no piece of S to keep (the pivot warp has): they start with W's identity
-            x[a][b] = (i < jb && j < jb && j <= i && (pivot || tx != ty)) ? S[i][j] : unit;
+                for (int b = 0; b < 4; ++b) x[a][b] = entry(ty * 4 + a, tx * 4 + b);
+            }
         }
-    const int steps = (jb + 3) >> 2;
-    bool bad = false;
-    if (tid == 256) {
-        const Chol4 c = chol4(x);
-        bad = c.ok == 0.0f;
-        factor[0] = c;
     }
-    if (!pivot && ty == 1 && tx == 0) {
+    // P of step q, and the diagonal block of step q + 1 for the pivot warp
+    auto publish = [&](int q) {
+        const int r = ty - 2 * q, c = tx - 2 * q;  // piece row and column relative to the step's block
+        if (c >= 0 && c < 2 && r >= 2) {
 #pragma unroll
-        for (int a = 0; a < 4; ++a) raw[a] = row4(x, a);
-    }
-    // x -= L[ty] . O[tx] with four columns of L and of O
-    auto update = [&](const float (*lcol)[NB], const float (*ocol)[NB]) {
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-            const float4 l = *reinterpret_cast<const float4*>(&lcol[cc][ty * 4]);
-            const float4 o = *reinterpret_cast<const float4*>(&ocol[cc][tx * 4]);
-            const float lv[4] = {l.x, l.y, l.z, l.w}, ov[4] = {o.x, o.y, o.z, o.w};
+            for (int b = 0; b < 4; ++b)
+                *reinterpret_cast<float4*>(&P[c * 4 + b][ty * 4]) = make_float4(x[0][b], x[1][b], x[2][b], x[3][b]);
+        }
+        if (r >= 0 && r < 2) {
 #pragma unroll
             for (int a = 0; a < 4; ++a)
+                *reinterpret_cast<float4*>(&P[r * 4 + a][tx * 4]) =
+                    c < 0 ? make_float4(x[a][0], x[a][1], x[a][2], x[a][3])
+                          : make_float4(r == c && a == 0, r == c && a == 1, r == c && a == 2, r == c && a == 3);
+            if (r == 0 && c == 0) {  // nobody's piece right of it
 #pragma unroll
-                for (int b = 0; b < 4; ++b) x[a][b] = fmaf(-lv[a], ov[b], x[a][b]);
+                for (int a = 0; a < 4; ++a) *reinterpret_cast<float4*>(&P[a][tx * 4 + 4]) = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+        if (r >= 2 && r < 4 && c >= 2) {
+            float (*d)[CW] = reinterpret_cast<float(*)[CW]>(before + ((q + 1) & 1) * CW * CW);
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+                *reinterpret_cast<float4*>(&d[(r - 2) * 4 + a][(c - 2) * 4]) = make_float4(x[a][0], x[a][1], x[a][2], x[a][3]);
         }
     };
+    bool ok = true;
+    float z[CW][CW], y[CW];
+    // factors z and publishes the inverse, one column per lane
+    auto factor = [&] {
+        ok = invert_block(z, lane & (CW - 1), y) && ok;
+        if (lane < CW) {
+#pragma unroll
+            for (int r = 0; r < CW; ++r) inv[r][lane] = r >= lane ? y[r] : 0.0f;
+        }
+    };
+    if (pivot) {
+#pragma unroll
+        for (int i = 0; i < CW; ++i)
+#pragma unroll
+            for (int j = 0; j < CW; ++j) z[i][j] = j <= i ? entry(i, j) : 0.0f;
+        factor();
+    } else if (owner) {
+        publish(0);
+    }
     for (int q = 0; q < steps; ++q) {
-        __syncthreads();
-        float (*colbuf)[NB] = colbufs + 4 * (q & 1);
+        sync();
+        if (panel >= 0) {  // four entries of O each
+            const int at = panel & 63, c = (panel >> 6) * 4;
+            float o[4] = {}, v[4][CW];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                *reinterpret_cast<float4*>(&v[k][0]) = *reinterpret_cast<const float4*>(&inv[c + k][0]);
+                *reinterpret_cast<float4*>(&v[k][4]) = *reinterpret_cast<const float4*>(&inv[c + k][4]);
+            }
+#pragma unroll
+            for (int d = 0; d < CW; ++d) {
+                const float p = P[d][at];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) o[k] = fmaf(v[k][d], p, o[k]);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) O[c + k][at] = o[k];
+        }
+        sync();
         if (pivot) {
-            if (q + 1 < steps) {  // every lane computes lane q + 1's part; that lane keeps it
-                const Chol4 c = load_factor(factor + (q & 1));
-                const float (*before)[NB] = colbufs + 4 * ((q & 1) ^ 1);
-                float l[4][4], z[4][4];
+            if (q + 1 < steps) {
+                const float (*d)[CW] = reinterpret_cast<const float(*)[CW]>(before + ((q + 1) & 1) * CW * CW);
+                const int r = lane >> 2, c = (lane & 3) * 2, at = (q + 1) * CW;
+                float2 v = *reinterpret_cast<const float2*>(&d[r][c]), m[CW];
+                float l[CW];
 #pragma unroll
-                for (int a = 0; a < 4; ++a) {
-                    const float4 v = raw[4 * (q & 1) + a];
-                    l[a][0] = v.x; l[a][1] = v.y; l[a][2] = v.z; l[a][3] = v.w;
-                    solve4(c, l[a][0], l[a][1], l[a][2], l[a][3]);
+                for (int k = 0; k < CW; ++k) {
+                    l[k] = O[k][at + r];
+                    m[k] = *reinterpret_cast<const float2*>(&O[k][at + c]);
                 }
-                if (q > 0) update(before, before);
 #pragma unroll
-                for (int a = 0; a < 4; ++a)
-#pragma unroll
-                    for (int b = 0; b <= a; ++b)
-                        z[a][b] = fmaf(-l[a][3], l[b][3], fmaf(-l[a][2], l[b][2], fmaf(-l[a][1], l[b][1],
-                                       fmaf(-l[a][0], l[b][0], x[a][b]))));
-                const Chol4 n = chol4(z);
-                if (tid - 256 == q + 1) {
-                    bad = bad || n.ok == 0.0f;
-                    factor[(q + 1) & 1] = n;
+                for (int k = 0; k < CW; ++k) {
+                    v.x = fmaf(-l[k], m[k].x, v.x);
+                    v.y = fmaf(-l[k], m[k].y, v.y);
                 }
+                *reinterpret_cast<float2*>(&now[r][c]) = v;
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < CW; ++i)
+#pragma unroll
+                    for (int j = 0; j < CW; j += 4) {
+                        if (j > i) continue;
+                        const float4 w = *reinterpret_cast<const float4*>(&now[i][j]);
+                        z[i][j] = w.x; z[i][j + 1] = w.y; z[i][j + 2] = w.z; z[i][j + 3] = w.w;
+                    }
+                factor();
             }
             continue;
         }
-        if ((tx == q && ty > q) || (ty == q && tx <= q)) {
-            // rows of L: B Ld^-T, i.e. Ld^-1 applied along each row of the piece; rows of W: along each column
-            const Chol4 c = load_factor(factor + (q & 1));
-            const bool of_l = ty > q;
-            float y[4][4];
+        if (!owner) continue;
+        const int r = ty - 2 * q, c = tx - 2 * q;
+        if (r >= 0 && r < 2) {  // the step's rows of W
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+            for (int a = 0; a < 4; ++a) {
+                const float4 w = *reinterpret_cast<const float4*>(&O[r * 4 + a][tx * 4]);
+                x[a][0] = w.x; x[a][1] = w.y; x[a][2] = w.z; x[a][3] = w.w;
+            }
+        } else if (r >= 2) {
+            if (c >= 0 && c < 2) {  // from S, which has become L, to W
 #pragma unroll
-                for (int b = 0; b < 4; ++b) y[a][b] = of_l ? x[a][b] : x[b][a];
+                for (int a = 0; a < 4; ++a)
 #pragma unroll
-            for (int a = 0; a < 4; ++a) solve4(c, y[a][0], y[a][1], y[a][2], y[a][3]);
-            float (*dst)[NB] = of_l ? colbuf : rowbuf;
-            const int at = of_l ? ty * 4 : tx * 4;
+                    for (int b = 0; b < 4; ++b) x[a][b] = 0.0f;
+            }
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                *reinterpret_cast<float4*>(&dst[b][at]) = make_float4(y[0][b], y[1][b], y[2][b], y[3][b]);
+            for (int k = 0; k < CW; ++k) {
+                const float4 l = *reinterpret_cast<const float4*>(&O[k][ty * 4]);
+                const float4 o = *reinterpret_cast<const float4*>(&O[k][tx * 4]);
+                const float lv[4] = {l.x, l.y, l.z, l.w}, ov[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
-                for (int a = 0; a < 4; ++a) x[b][a] = of_l ? 0.0f : y[a][b];  // a piece of W (zero so far) from here on
+                for (int a = 0; a < 4; ++a)
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) x[a][b] = fmaf(-lv[a], ov[b], x[a][b]);
             }
         }
-        asm volatile("barrier.cta.sync 1, 256;" ::: "memory");  // the grid only
-        if (ty > q && tx < ty) {
-            update(colbuf, tx > q ? colbuf : rowbuf);
-            if (ty == q + 2 && tx == q + 1) {
-#pragma unroll
-                for (int a = 0; a < 4; ++a) raw[4 * ((q + 1) & 1) + a] = row4(x, a);
-            }
-        }
+        if (q + 1 < steps) publish(q + 1);
     }
-    if (!pivot) {
+    if (owner) {
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
             const int i = ty * 4 + a;
-            float w[4];
 #pragma unroll
-            for (int b = 0; b < 4; ++b) w[b] = (i < jb && tx * 4 + b <= i) ? x[a][b] : 0.0f;
-            *reinterpret_cast<float4*>(dinv + i * NB + tx * 4) = make_float4(w[0], w[1], w[2], w[3]);
+            for (int b = 0; b < 4; ++b) x[a][b] = (i < jb && tx * 4 + b <= i) ? x[a][b] : 0.0f;
+            *reinterpret_cast<float4*>(dinv + i * NB + tx * 4) = make_float4(x[a][0], x[a][1], x[a][2], x[a][3]);
+            if (tx < ty) {  // the piece across the diagonal
+                *reinterpret_cast<float4*>(dinv + (tx * 4 + a) * NB + ty * 4) = zero;
+                *reinterpret_cast<float4*>(&Dt[i][tx * 4]) = zero;
+            }
         }
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+            *reinterpret_cast<float4*>(&Dt[tx * 4 + b][ty * 4]) = make_float4(x[0][b], x[1][b], x[2][b], x[3][b]);
     }
-    if (bad) atomicCAS(status, 0u, (uint32_t)ST_NOT_SPD);
+    if (!ok) atomicCAS(status, 0u, (uint32_t)ST_NOT_SPD);
 }
 
 // Step j of a block column's diagonal block (kb x kb, kb <= 512), in tiles of 64.  Before the step, rows i >= j hold
@@ -266,169 +384,195 @@ __device__ void chol_block(const Tile& S, int jb, float* dinv, uint32_t* status,
 //     W[j, c] = D R[j, c],   W[j, j] = D,
 // and with P_i = S[i, j] D^T (the rows of L) updates every row i > j:
 //     S[i, l] -= P_i P_l^T (j < l <= i),   R[i, c] -= P_i W[j, c] (c < j),   R[i, j] = -P_i D.
-// One CTA per tile, each computing the P and W tiles it needs itself (three 64^3 products, 1.1 us each on one SM,
-// instead of another meeting point and a trip through memory).  Rows i > j go from X to Y (tiles are read by many
-// CTAs, so they are not updated in place); W's rows go to `block`, the matrix itself, with zeros right of the diagonal.
-__device__ void block_tile(float* step_smem, const float* X, int64_t ldx, float* Y, int64_t ldy, float* block,
-                           int64_t lda, int kb, int j, int i, int c, const float* D, float* D_next, uint32_t* status) {
-    Tile& Dt = *reinterpret_cast<Tile*>(step_smem);                // Dt[t][c] = D[c][t]
-    Tile& T0 = *reinterpret_cast<Tile*>(step_smem + NB * TS);
-    Tile& T1 = *reinterpret_cast<Tile*>(step_smem + 2 * NB * TS);
-    Tile& T2 = *reinterpret_cast<Tile*>(step_smem + 3 * NB * TS);
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-    const bool grid16 = tid < 256;  // the ninth warp is the factorisation's pivot warp
+// One CTA per tile, each computing the P and W tiles it needs itself (three 64^3 products instead of another meeting point
+// and a trip through memory).  Rows i > j go from X to Y (tiles are read by many CTAs, so they are not updated in place);
+// W's rows go to `block`, the matrix itself, with zeros right of the diagonal.
+__device__ void block_tile(float* smem, const float* X, int64_t ldx, float* Y, float* block, int64_t lda, int kb,
+                           int j, int i, int c, const float* D) {
+    Tile& Dt = *reinterpret_cast<Tile*>(smem);                // Dt[t][c] = D[c][t]
+    Tile& T0 = *reinterpret_cast<Tile*>(smem + NB * TS);
+    Tile& T1 = *reinterpret_cast<Tile*>(smem + 2 * NB * TS);
+    Tile& T2 = *reinterpret_cast<Tile*>(smem + 3 * NB * TS);
+    float* const exchange = smem + 4 * NB * TS;
+    const int tid = threadIdx.x, ty = piece_row(tid), tx = piece_col(tid);
     const int rows = min(NB, kb - i * NB), jw = min(NB, kb - j * NB), cols = min(NB, kb - c * NB);
-    float acc[4][4] = {};
+    float acc[4][4];
+    TileRegs<256> d, t1, t2;
     if (i == j) {  // row j of W
         if (c < j) {
-            load_tile<true>(Dt, D, NB, NB, NB);
-            load_tile<false>(T0, X + (int64_t)j * NB * ldx + c * NB, ldx, rows, NB);
+            d.fetch(tid, D, NB, NB, NB);
+            t1.fetch(tid, X + (int64_t)j * NB * ldx + c * NB, ldx, rows, NB);
+            d.put<true>(tid, Dt);
+            t1.put<false>(tid, T0);
             __syncthreads();
-            if (grid16) tile_mma(Dt, T0, ty, tx, acc);
+            tile_mma(Dt, T0, exchange, acc);
         }
-        if (!grid16) return;
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
                 const int r = ty * 4 + a, q = tx * 4 + b;
                 if (r < rows && q < cols)
-                    block[(int64_t)(j * NB + r) * lda + c * NB + q] = c < j ? acc[a][b] : c == j ? D[r * NB + q] : 0.0f;
+                    block[(int64_t)(j * NB + r) * lda + c * NB + q] = c < j ? acc[a][b] : c == j ? __ldcg(D + r * NB + q) : 0.0f;
             }
         return;
     }
-    // P_i, t-major, into T0
-    load_tile<true>(Dt, D, NB, NB, NB);
-    load_tile<true>(T1, X + (int64_t)i * NB * ldx + j * NB, ldx, rows, jw);
+    d.fetch(tid, D, NB, NB, NB);
+    t1.fetch(tid, X + (int64_t)i * NB * ldx + j * NB, ldx, rows, jw);
     if (c > j && c != i)
-        load_tile<true>(T2, X + (int64_t)c * NB * ldx + j * NB, ldx, cols, jw);
+        t2.fetch(tid, X + (int64_t)c * NB * ldx + j * NB, ldx, cols, jw);
     else if (c < j)
-        load_tile<false>(T2, X + (int64_t)j * NB * ldx + c * NB, ldx, jw, NB);
-    else if (c == j)
-        load_tile<false>(T2, D, NB, NB, NB);
+        t2.fetch(tid, X + (int64_t)j * NB * ldx + c * NB, ldx, jw, NB);
     // this CTA's own tile, in flight during the products
     float own[4][4];
+    const float* mine = X + (int64_t)(i * NB + ty * 4) * ldx + c * NB + tx * 4;
+    const bool vec = (ldx & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15u) == 0 && tx * 4 + 4 <= cols;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const bool live = c != j && ty * 4 + a < rows;
+        if (vec && live) {
+            *reinterpret_cast<float4*>(own[a]) = __ldcg(reinterpret_cast<const float4*>(mine + a * ldx));
+        } else {
+#pragma unroll
+            for (int b = 0; b < 4; ++b) own[a][b] = (live && tx * 4 + b < cols) ? __ldcg(mine + a * ldx + b) : 0.0f;
+        }
+    }
+    d.put<true>(tid, Dt);
+    t1.put<true>(tid, T1);  // P_i^T = D S[i, j]^T, i.e. t-major, goes to T0
+    if (c > j && c != i)
+        t2.put<true>(tid, T2);
+    else if (c < j)
+        t2.put<false>(tid, T2);
+    else if (c == j)
+        d.put<false>(tid, T2);
+    __syncthreads();
+    tile_mma(Dt, T1, exchange, acc);
+    put_piece(T0, ty, tx, acc);
+    if (c != i && c != j) {  // the other operand, P_c^T or W[j, c], over T1 (the product above is done with it)
+        tile_mma(Dt, T2, exchange, acc);
+        put_piece(T1, ty, tx, acc);
+    }
+    __syncthreads();
+    tile_mma(T0, c == i ? T0 : c == j ? T2 : T1, exchange, acc);
 #pragma unroll
     for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int r = ty * 4 + a, q = tx * 4 + b;
-            own[a][b] = (grid16 && c != j && r < rows && q < cols) ? X[(int64_t)(i * NB + r) * ldx + c * NB + q] : 0.0f;
-        }
-    __syncthreads();
-    if (grid16) {
-        tile_mma(T1, Dt, ty, tx, acc);
-#pragma unroll
-        for (int b = 0; b < 4; ++b)
-            *reinterpret_cast<float4*>(&T0[tx * 4 + b][ty * 4]) = make_float4(acc[0][b], acc[1][b], acc[2][b], acc[3][b]);
-    }
-    if (c != i && c != j) {  // the other operand: P_c (t-major) or W[j, c], over T1
-        float other[4][4] = {};
-        if (!grid16) {
-        } else if (c > j)
-            tile_mma(T2, Dt, ty, tx, other);
-        else
-            tile_mma(Dt, T2, ty, tx, other);
-        __syncthreads();
-#pragma unroll
-        for (int b = 0; b < 4 && grid16; ++b) {
-            if (c > j)
-                *reinterpret_cast<float4*>(&T1[tx * 4 + b][ty * 4]) =
-                    make_float4(other[0][b], other[1][b], other[2][b], other[3][b]);
-            else
-                *reinterpret_cast<float4*>(&T1[ty * 4 + b][tx * 4]) =
-                    make_float4(other[b][0], other[b][1], other[b][2], other[b][3]);
-        }
-    }
-    __syncthreads();
-    if (grid16) {
-        float upd[4][4] = {};
-        tile_mma(T0, c == i ? T0 : c == j ? T2 : T1, ty, tx, upd);
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const int r = ty * 4 + a, q = tx * 4 + b;
-                own[a][b] -= upd[a][b];
-                if (r < rows && q < cols) Y[(int64_t)(i * NB + r) * ldy + c * NB + q] = own[a][b];
-            }
-    }
-    if (D_next) {
-        if (grid16) {
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-                *reinterpret_cast<float4*>(&Dt[ty * 4 + a][tx * 4]) =
-                    make_float4(own[a][0], own[a][1], own[a][2], own[a][3]);
-        }
-        __syncthreads();
-        chol_block(Dt, rows, D_next, status, &T1[0][0]);
-    }
+        *reinterpret_cast<float4*>(Y + (int64_t)(i * NB + ty * 4 + a) * OUTER + c * NB + tx * 4) =
+            make_float4(own[a][0] - acc[a][0], own[a][1] - acc[a][1], own[a][2] - acc[a][2], own[a][3] - acc[a][3]);
 }
 
-// All CTAs of a cooperative launch meet: true when they have all arrived `round` times (1, 2, ...).  Bounded.
-__device__ bool meet(uint32_t* counter, uint32_t round, uint32_t* status) {
-    __shared__ uint32_t met;
+// Counters of a block column: `factored` tiles of the diagonal (CTA 0), and steps x CTAs finished by the others.
+struct BlockCounters {
+    uint32_t factored, finished;
+};
+// Waits until *counter has reached `target`; one thread.  Bounded.
+__device__ bool reached(const uint32_t* counter, uint32_t target, uint32_t* status) {
+    const uint64_t t0 = globaltimer_ns();
+    for (uint32_t n = 1;; ++n) {
+        uint32_t seen;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
+        if (seen >= target) return true;
+        if ((n & 255u) == 0 && globaltimer_ns() - t0 > WAIT_LIMIT_NS) {
+            if (atomicCAS(status, 0u, (uint32_t)ST_TIMEOUT_ACC) == 0u) status[1] = blockIdx.x;
+            return false;
+        }
+    }
+}
+// What this CTA's threads have written, then the counter.  All threads; the next use of what they read needs no further
+// barrier.
+__device__ __forceinline__ void announce(uint32_t* counter) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        const uint32_t target = round * gridDim.x;
-        uint32_t seen;
         __threadfence();
         atomicAdd(counter, 1u);
-        const uint64_t t0 = globaltimer_ns();
-        bool late = false;
-        for (uint32_t n = 1;; ++n) {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
-            if (seen >= target) break;
-            if ((n & 255u) == 0 && globaltimer_ns() - t0 > WAIT_LIMIT_NS) {
-                late = true;
-                break;
-            }
-        }
-        __threadfence();
-        if (late && atomicCAS(status, 0u, (uint32_t)ST_TIMEOUT_ACC) == 0u) status[1] = blockIdx.x;
-        met = late ? 0u : 1u;
     }
-    __syncthreads();
-    return met != 0;
 }
 
-// Factors and inverts a diagonal block (kb x kb): CTA 0 takes the first tile and then every step's next diagonal tile,
-// the others share the rest.  A cooperative launch of about as many CTAs as the largest step has tiles; meeting through
-// a counter in the L2 between steps instead of one launch per step took the 512-wide block from 155 to 125 us.
-__global__ void __launch_bounds__(STEP_THREADS) block_kernel(float* block, int64_t lda, int kb, float* blocks, float* dinv,
-                                                             uint32_t* counter, uint32_t* status) {
-    extern __shared__ __align__(16) float step_smem[];
-    const int nt = (kb + NB - 1) / NB;
+// Factors and inverts a diagonal block (kb x kb).  CTA 0 walks down the diagonal: it factors a tile, updates the next one
+// with it from what the two warps left over have fetched meanwhile (the column's tile beside it and the tile itself, as the others
+// left them a step earlier) and goes on, without waiting for anyone unless the others fall behind.  They wait for a tile's
+// inverse, share the step's tiles and wait for one another.  A cooperative launch of about as many CTAs as the largest step
+// has tiles.  With one meeting point of all CTAs per step, CTA 0's tiles fetched behind it and the slower products and
+// factorisation of before, the 512-wide block took 126 us, 97 now.
+constexpr int STEP_THREADS = 256;
+constexpr size_t STEP_SMEM = (5 * NB * TS + EXCHANGE_FLOATS + CHOL_FLOATS) * sizeof(float);
+__global__ void __launch_bounds__(STEP_THREADS, 1) block_kernel(float* block, int64_t lda, int kb, float* blocks, float* dinv,
+                                                                BlockCounters* counters, uint32_t* status) {
+    extern __shared__ __align__(16) float smem[];
+    __shared__ uint32_t proceed;
+    const int nt = (kb + NB - 1) / NB, tid = threadIdx.x;
+    const uint32_t others = gridDim.x - 1;
+    auto source = [&](int j) { return j == 0 ? block : blocks + (size_t)((j - 1) & 1) * OUTER * OUTER; };
+    auto source_ld = [&](int j) { return j == 0 ? lda : (int64_t)OUTER; };
     if (blockIdx.x == 0) {
-        Tile& S = *reinterpret_cast<Tile*>(step_smem);
-        load_tile<false>(S, block, lda, min(NB, kb), min(NB, kb));
-        __syncthreads();
-        chol_block(S, min(NB, kb), dinv, status, step_smem + NB * TS);
+        Tile& Dt = *reinterpret_cast<Tile*>(smem);
+        Tile& T0 = *reinterpret_cast<Tile*>(smem + NB * TS);
+        Tile& T1 = *reinterpret_cast<Tile*>(smem + 2 * NB * TS);
+        Tile& S = *reinterpret_cast<Tile*>(smem + 3 * NB * TS);
+        Tile& next = *reinterpret_cast<Tile*>(smem + 4 * NB * TS);
+        float* const exchange = smem + 5 * NB * TS;
+        float* const buf = exchange + EXCHANGE_FLOATS;
+        const int warp = tid >> 5, ty = piece_row(tid), tx = piece_col(tid);
+        TileRegs<256> first;
+        first.fetch(tid, block, lda, min(NB, kb), min(NB, kb));
+        first.put<false>(tid, S);
+        if (tid == 0) proceed = 1;
+        for (int j = 0;; ++j) {
+            __syncthreads();
+            // the tiles (j + 1, j) and (j + 1, j + 1) of step j, beside the factorisation
+            const int rows = min(NB, kb - (j + 1) * NB);
+            if (warp != 4 && warp != 7) {
+                chol_block(S, min(NB, kb - j * NB), dinv + (size_t)j * NB * NB, Dt, status, buf);
+            } else if (j + 1 < nt) {
+                const int lane = tid & 31, id = (warp == 7 ? 32 : 0) + lane;
+                bool ok = lane != 0 || reached(&counters->finished, (uint32_t)j * others, status);
+                ok = __all_sync(0xffffffffu, ok);
+                const float* at = source(j) + (int64_t)(j + 1) * NB * source_ld(j) + j * NB;
+                if (ok) {
+                    TileRegs<64> t, u;
+                    t.fetch(id, at, source_ld(j), rows, NB);
+                    u.fetch(id, at + NB, source_ld(j), rows, rows);
+                    t.put<true>(id, T1);
+                    u.put<false>(id, next);
+                } else if (lane == 0) {
+                    proceed = 0;
+                }
+            }
+            announce(&counters->factored);
+            if (j + 1 == nt || !*const_cast<volatile uint32_t*>(&proceed)) return;
+            float acc[4][4];
+            tile_mma(Dt, T1, exchange, acc);  // P^T
+            put_piece(T0, ty, tx, acc);
+            __syncthreads();
+            tile_mma(T0, T0, exchange, acc);
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                const float4 v = *reinterpret_cast<const float4*>(&next[ty * 4 + a][tx * 4]);
+                *reinterpret_cast<float4*>(&S[ty * 4 + a][tx * 4]) =
+                    make_float4(v.x - acc[a][0], v.y - acc[a][1], v.z - acc[a][2], v.w - acc[a][3]);
+            }
+        }
     }
     for (int j = 0; j < nt; ++j) {
-        if (!meet(counter, j + 1, status)) return;
-        const float* X = j == 0 ? block : blocks + (size_t)((j - 1) & 1) * OUTER * OUTER;
+        if (tid == 0)
+            proceed = reached(&counters->factored, (uint32_t)j + 1u, status) &&
+                      reached(&counters->finished, (uint32_t)j * others, status);
+        __syncthreads();
+        if (!proceed) return;
         float* Y = blocks + (size_t)(j & 1) * OUTER * OUTER;
-        const int64_t ldx = j == 0 ? lda : OUTER;
         const float* D = dinv + (size_t)j * NB * NB;
-        if (blockIdx.x == 0) {
-            if (j + 1 < nt)
-                block_tile(step_smem, X, ldx, Y, OUTER, block, lda, kb, j, j + 1, j + 1, D,
-                           dinv + (size_t)(j + 1) * NB * NB, status);
-            continue;
-        }
         int tiles = nt;  // row j of W, and the tiles (i, c), c <= i, of the rows below
         for (int i = j + 1; i < nt; ++i) tiles += i + 1;
-        for (int t = (int)blockIdx.x - 1; t < tiles; t += (int)gridDim.x - 1) {
+        for (int t = (int)blockIdx.x - 1; t < tiles; t += (int)others) {
             int i = j, c = t;
             if (t >= nt) {
                 c = t - nt;
                 for (i = j + 1; c > i; ++i) c -= i + 1;
                 if (i == j + 1 && c == j + 1) continue;  // CTA 0's
             }
-            block_tile(step_smem, X, ldx, Y, OUTER, block, lda, kb, j, i, c, D, nullptr, status);
+            block_tile(smem, source(j), source_ld(j), Y, block, lda, kb, j, i, c, D);
             __syncthreads();
         }
+        announce(&counters->finished);
     }
 }
 
@@ -533,7 +677,7 @@ static InvLayout inv_layout(int64_t k) {
     l.partial = off;
     off += align_up(RED_BLOCKS * sizeof(double), 256);
     l.counters = off;
-    off += align_up((size_t)((k + OUTER - 1) / OUTER) * sizeof(uint32_t), 256);
+    off += align_up((size_t)((k + OUTER - 1) / OUTER) * sizeof(BlockCounters), 256);
     // what the block columns, the rest of their updates and the merges use at the same time
     size_t chain = 0, rest = 0, merge = product(k, k, k, true).bytes();  // W^T W
     for (int64_t o = 0; o + OUTER < k; o += OUTER) {
@@ -701,11 +845,11 @@ int tb_spd_inverse(int device, void* stream_, float* A, int64_t k, int64_t lda, 
         return TB_OK;
     };
 
-    uint32_t* counters = reinterpret_cast<uint32_t*>(base + l.counters);
-    prepare_kernel<<<(K + 255) / 256, 256, 0, stream>>>(A, lda, K, lambda, counters, (K + OUTER - 1) / OUTER);
+    BlockCounters* counters = reinterpret_cast<BlockCounters*>(base + l.counters);
+    prepare_kernel<<<(K + 255) / 256, 256, 0, stream>>>(A, lda, K, lambda, reinterpret_cast<uint32_t*>(counters),
+                                                        2 * ((K + OUTER - 1) / OUTER));
     if ((rc = record(side.s.forked, stream)) != TB_OK || (rc = wait(chain, side.s.forked)) != TB_OK) return rc;
 
-    constexpr size_t step_smem = 4u * NB * TS * sizeof(float);
     if (const int e = set_smem_limit((const void*)block_kernel, device)) return e;
     uint8_t* const chain_at = base + l.chain;
     for (int64_t o = 0; o < k; o += OUTER) {
@@ -720,7 +864,7 @@ int tb_spd_inverse(int device, void* stream_, float* A, int64_t k, int64_t lda, 
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)std::min(tiles + 1, sm_count));
         cfg.blockDim = dim3(STEP_THREADS);
-        cfg.dynamicSmemBytes = step_smem;
+        cfg.dynamicSmemBytes = STEP_SMEM;
         cfg.stream = chain;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
