@@ -226,6 +226,41 @@ def test_inverse_inside_a_diagonal_block(cuda, k, ld):
     _lib.device_status(cuda.index)
 
 
+@pytest.mark.parametrize("n,k,m", [(300, 100, 7), (3000, 1100, 40)])
+def test_chained_launches_give_the_same_under_capture(cuda, n, k, m):
+    """The launches of Gram, inverse and products begin before the ones in front of them have ended: replayed from a graph,
+    and repeated back to back over one workspace, they give the bits of the first call."""
+    from trak_b200 import score_computers as sc
+    g = torch.Generator(device=cuda).manual_seed(k)
+    x, t = torch.randn(n, k, device=cuda, generator=g), torch.randn(m, k, device=cuda, generator=g)
+    out = [torch.empty(k, k, device=cuda), torch.empty(n, k, device=cuda), torch.empty(n, m, device=cuda)]
+
+    def chain():
+        sc.gram(x, out=out[0])
+        sc._launch_spd_inverse(out[0], 1e-2, True)
+        sc.gemm_nt(x, out[0], out=out[1])
+        sc.gemm_nt(out[1], t, out=out[2])
+
+    stream = torch.cuda.Stream(cuda)
+    stream.wait_stream(torch.cuda.current_stream(cuda))
+    with torch.cuda.stream(stream):
+        chain()
+        first = [o.clone() for o in out]
+        for _ in range(5):
+            chain()
+        assert all(torch.equal(a, b) for a, b in zip(first, out))
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            chain()
+        for o in out:
+            o.zero_()
+        graph.replay()
+        graph.replay()
+        stream.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(first, out))
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 1, 1), (129, 257, 33), (300, 700, 95), (128, 256, 64), (513, 100, 4097)])
 def test_gram_and_gemm_at_ragged_sizes(cuda, M, N, K):
     """Tile, chunk (64 k) and slot (32 k) boundaries of both GEMM kernels, with accumulation into existing output."""

@@ -130,7 +130,10 @@ static bool read_note(const StatusNote& note, uint32_t* status) {
     return (uint32_t)(v >> 32) == note.call;
 }
 // A store by the SM reaches the host some 8 us earlier than a copy engine that has to be set going.
-__global__ void publish_status_kernel(const uint32_t* status, StatusNote note) { publish_status(status, note); }
+__global__ void publish_status_kernel(const uint32_t* status, StatusNote note) {
+    after_earlier_launch();
+    publish_status(status, note);
+}
 
 void arm_status(int device, cudaStream_t stream, const StatusNote& note) {
     t_armed.device = device;
@@ -262,8 +265,8 @@ int tb_stream_status(int device, void* stream_, uint32_t* detail) {
         rc = tb::take_note(&note);
         if (rc != TB_OK) return rc;
         // the read is queued behind the stream's work, so one wait serves both
-        tb::publish_status_kernel<<<1, 1, 0, stream>>>(tb::status_ptr(device), note);
-        TB_CUDA(cudaGetLastError());
+        rc = tb::launch_after(tb::publish_status_kernel, 1, 1, 0, stream, true, tb::status_ptr(device), note);
+        if (rc != TB_OK) return rc;
     }
     TB_CUDA(cudaStreamSynchronize(stream));
     uint32_t code = 0;

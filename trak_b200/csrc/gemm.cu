@@ -227,6 +227,7 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_slot;
+    after_earlier_launch();
 
     if (warp == 0 && lane == 0) {
         // ------------------------------- TMA producer -------------------------------
@@ -435,6 +436,7 @@ gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_slot;
+    after_earlier_launch();
 
     // Registers follow the work: the warpgroup of the two single-thread roles gives most of its
     // allocation back (168 -> 56 per thread), the two epilogue warpgroups take it (168 -> 224:
@@ -603,6 +605,7 @@ struct PackRows {
 };
 template <int W>
 __global__ void __launch_bounds__(256) pack_rows_f32_kernel(const PackRows a, const PackRows b) {
+    after_earlier_launch();
     __shared__ uint32_t row_max[8];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, part = warp % W;
     constexpr uint32_t SPAN = W * 1024u;
@@ -678,6 +681,7 @@ __global__ void __launch_bounds__(256) pack_rows_f32_kernel(const PackRows a, co
 // blockIdx.y walks chunks of source rows; amax must be zero before the launch.
 __global__ void amax_cols_kernel(const float* __restrict__ src, uint32_t* __restrict__ amax, uint64_t rows,
                                  uint64_t K, uint64_t ld, uint64_t chunk) {
+    after_earlier_launch();
     const uint64_t R = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (R >= rows) return;
     const uint64_t k0 = (uint64_t)blockIdx.y * chunk, k1 = min(K, k0 + chunk);
@@ -696,6 +700,7 @@ template <int J>
 __global__ void __launch_bounds__(512) pack_cols_f32_kernel(const float* __restrict__ src, uint16_t* __restrict__ packed,
                                                             uint32_t* __restrict__ amax, uint64_t rows, uint64_t K,
                                                             uint64_t ld, uint32_t kblocks) {
+    after_earlier_launch();
     __shared__ uint32_t warp_max[16][16];
     const uint32_t c = threadIdx.x & 15u, group = threadIdx.x >> 4, warp = threadIdx.x >> 5;
     const uint64_t R = (uint64_t)blockIdx.x * 16u + c, span_k = (uint64_t)kblocks * 32u;
@@ -749,6 +754,7 @@ __global__ void __launch_bounds__(512) pack_cols_f32_kernel(const float* __restr
 template <bool TRANS>
 __global__ void pack_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ packed, uint64_t rows,
                             uint64_t K, uint64_t ld, uint32_t rowblocks, uint32_t kblocks) {
+    after_earlier_launch();
     // one thread = 8 consecutive k of one operand row (a 16-byte store)
     const uint64_t total = (uint64_t)rowblocks * kblocks * 128u * 4u;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total;
@@ -801,6 +807,7 @@ __global__ void pack_kernel(const uint16_t* __restrict__ src, uint16_t* __restri
 __global__ void __launch_bounds__(256) pack_trans_f32_kernel(const float* __restrict__ src, uint16_t* __restrict__ packed,
                                                              const uint32_t* __restrict__ amax, uint64_t rows, uint64_t K,
                                                              uint64_t ld, uint32_t rowblocks, uint32_t kblocks) {
+    after_earlier_launch();
     constexpr int LDS = 34;  // padded row of a plane tile, in 16-bit elements (17 words: conflict-free)
     __shared__ __align__(16) uint16_t tile[2][128][LDS];
     const uint32_t c = threadIdx.x & 127u, half = threadIdx.x >> 7;
@@ -845,6 +852,7 @@ __global__ void __launch_bounds__(256) pack_trans_f32_kernel(const float* __rest
 // shared memory for its second copy.
 __global__ void __launch_bounds__(256) reduce_splits_kernel(const float* __restrict__ partial, uint32_t splits,
                                                             const GemmParams p) {
+    after_earlier_launch();
     __shared__ float turn[32][33];
     const uint32_t bm = blockIdx.y, bn = blockIdx.x, tx = threadIdx.x & 31u, ty = threadIdx.x >> 5;
     if (p.symmetric && bn < bm) return;
@@ -906,12 +914,10 @@ static int launch_pack_rows(const PackRows& a, const PackRows& b, int sm_count, 
     const uint64_t cap = (uint64_t)sm_count * 32;
     if (blocks > cap) blocks = cap;
     const uint32_t nb = (uint32_t)blocks;
-    if (w == 1) pack_rows_f32_kernel<1><<<nb, 256, 0, stream>>>(a, b);
-    else if (w == 2) pack_rows_f32_kernel<2><<<nb, 256, 0, stream>>>(a, b);
-    else if (w == 4) pack_rows_f32_kernel<4><<<nb, 256, 0, stream>>>(a, b);
-    else pack_rows_f32_kernel<8><<<nb, 256, 0, stream>>>(a, b);
-    TB_CUDA(cudaGetLastError());
-    return TB_OK;
+    if (w == 1) return launch_after(pack_rows_f32_kernel<1>, nb, 256, 0, stream, true, a, b);
+    if (w == 2) return launch_after(pack_rows_f32_kernel<2>, nb, 256, 0, stream, true, a, b);
+    if (w == 4) return launch_after(pack_rows_f32_kernel<4>, nb, 256, 0, stream, true, a, b);
+    return launch_after(pack_rows_f32_kernel<8>, nb, 256, 0, stream, true, a, b);
 }
 
 int launch_pack_pair(const float* a, uint64_t rows_a, uint64_t K_a, uint64_t ld_a, uint16_t* packed_a, const Packed& ga,
@@ -940,11 +946,8 @@ int launch_pack(const void* src, int dtype, bool trans, uint64_t rows, uint64_t 
         uint32_t* amax = packed_amax(packed, g);
         if (K <= 2048u) {
             const uint32_t nb = g.rowblocks * 8u;
-            if (K <= 512u) pack_cols_f32_kernel<2><<<nb, 512, 0, stream>>>(s, packed, amax, rows, K, ld, g.kblocks);
-            else if (K <= 1024u) pack_cols_f32_kernel<4><<<nb, 512, 0, stream>>>(s, packed, amax, rows, K, ld, g.kblocks);
-            else pack_cols_f32_kernel<8><<<nb, 512, 0, stream>>>(s, packed, amax, rows, K, ld, g.kblocks);
-            TB_CUDA(cudaGetLastError());
-            return TB_OK;
+            auto kern = K <= 512u ? pack_cols_f32_kernel<2> : K <= 1024u ? pack_cols_f32_kernel<4> : pack_cols_f32_kernel<8>;
+            return launch_after(kern, nb, 512, 0, stream, true, s, packed, amax, rows, K, ld, g.kblocks);
         }
         TB_CUDA(cudaMemsetAsync(amax, 0, (size_t)g.rowblocks * 128u * sizeof(uint32_t), stream));
         const uint32_t bx = (uint32_t)((rows + 255) / 256);
@@ -953,9 +956,11 @@ int launch_pack(const void* src, int dtype, bool trans, uint64_t rows, uint64_t 
         if (by > 65535) by = 65535;
         const uint64_t chunk = (K + by - 1) / by;
         amax_cols_kernel<<<dim3(bx, (uint32_t)((K + chunk - 1) / chunk)), 256, 0, stream>>>(s, amax, rows, K, ld, chunk);
+        TB_CUDA(cudaGetLastError());
         uint64_t tb = (uint64_t)g.rowblocks * g.kblocks;
         if (tb > (uint64_t)sm_count * 16) tb = (uint64_t)sm_count * 16;
-        pack_trans_f32_kernel<<<(uint32_t)tb, 256, 0, stream>>>(s, packed, amax, rows, K, ld, g.rowblocks, g.kblocks);
+        return launch_after(pack_trans_f32_kernel, (uint32_t)tb, 256, 0, stream, true, s, packed, amax, rows, K, ld, g.rowblocks,
+                            g.kblocks);
     } else {
         const uint64_t total = (uint64_t)g.rowblocks * g.kblocks * 512u;
         uint64_t blocks = (total + 255) / 256;
@@ -963,13 +968,9 @@ int launch_pack(const void* src, int dtype, bool trans, uint64_t rows, uint64_t 
         if (blocks > cap) blocks = cap;
         const uint32_t nb = (uint32_t)blocks;
         const uint16_t* s = static_cast<const uint16_t*>(src);
-        if (trans)
-            pack_kernel<true><<<nb, 256, 0, stream>>>(s, packed, rows, K, ld, g.rowblocks, g.kblocks);
-        else
-            pack_kernel<false><<<nb, 256, 0, stream>>>(s, packed, rows, K, ld, g.rowblocks, g.kblocks);
+        return launch_after(trans ? pack_kernel<true> : pack_kernel<false>, nb, 256, 0, stream, true, s, packed, rows, K, ld,
+                            g.rowblocks, g.kblocks);
     }
-    TB_CUDA(cudaGetLastError());
-    return TB_OK;
 }
 
 // element format of the planes: fp16 for fp16 inputs and for scaled fp32 operands, else bf16
@@ -1033,7 +1034,7 @@ GemmPlan plan_gemm(uint32_t npl, bool chunked, bool symmetric, int64_t M, int64_
 
 template <int NPL, int T>
 static int launch_gemm_nt(int device, const CUtensorMap& map_a, const CUtensorMap& map_b, GemmParams& p, uint32_t splits,
-                          cudaStream_t stream) {
+                          bool early, cudaStream_t stream) {
     constexpr uint32_t stage_bytes = 2u * T * NPL * GTILE_BYTES;
     // two CTAs of the small tile share an SM
     p.stages = ((T == 2 ? 200u : 100u) * 1024u) / stage_bytes;
@@ -1043,16 +1044,14 @@ static int launch_gemm_nt(int device, const CUtensorMap& map_a, const CUtensorMa
     auto kern = gemm_nt_kernel<NPL, T>;
     if (const int e = set_smem_limit((const void*)kern, device)) return e;
     const dim3 grid((p.N + 128u * T - 1) / (128u * T), (p.M + 128u * T - 1) / (128u * T), splits);
-    kern<<<grid, 384, smem, stream>>>(map_a, map_b, p);
-    TB_CUDA(cudaGetLastError());
-    return TB_OK;
+    return launch_after(kern, grid, 384, smem, stream, early, map_a, map_b, p);
 }
 
 // C[M x N] (+)= alpha * row_scale[m] * Apacked . Bpacked^T
 int launch_gemm(int device, cudaStream_t stream, const uint16_t* pa, const Packed& ga,
                 const uint16_t* pb, const Packed& gb, int dtype, int64_t M, int64_t N, float* C,
                 int64_t ldc, const float* row_scale, float alpha, int accumulate, int symmetric,
-                int chunked, float* partial, KRange range) {
+                int chunked, float* partial, KRange range, bool early) {
     CUtensorMap map_a, map_b;
     int rc = packed_tmap(&map_a, pa, ga, dtype);
     if (rc != TB_OK) return rc;
@@ -1096,20 +1095,19 @@ int launch_gemm(int device, cudaStream_t stream, const uint16_t* pa, const Packe
         const size_t smem = (size_t)CK_SLOTS * CK_SLOT_BYTES + 1024u;
         const dim3 grid((uint32_t)((N + 255) / 256), (uint32_t)((M + 127) / 128), pl.splits);
         if (const int e = set_smem_limit((const void*)gemm_nt_chunked_kernel, device)) return e;
-        gemm_nt_chunked_kernel<<<grid, 384, smem, stream>>>(map_a, map_b, p);
-        TB_CUDA(cudaGetLastError());
+        rc = launch_after(gemm_nt_chunked_kernel, grid, 384, smem, stream, early, map_a, map_b, p);
+        if (rc != TB_OK) return rc;
     } else if (pl.tile == 2) {
-        rc = ga.npl == 2 ? launch_gemm_nt<2, 2>(device, map_a, map_b, p, pl.splits, stream)
-                         : launch_gemm_nt<1, 2>(device, map_a, map_b, p, pl.splits, stream);
+        rc = ga.npl == 2 ? launch_gemm_nt<2, 2>(device, map_a, map_b, p, pl.splits, early, stream)
+                         : launch_gemm_nt<1, 2>(device, map_a, map_b, p, pl.splits, early, stream);
         if (rc != TB_OK) return rc;
     } else {
-        rc = ga.npl == 2 ? launch_gemm_nt<2, 1>(device, map_a, map_b, p, 1, stream) : launch_gemm_nt<1, 1>(device, map_a, map_b, p, 1, stream);
+        rc = ga.npl == 2 ? launch_gemm_nt<2, 1>(device, map_a, map_b, p, 1, early, stream) : launch_gemm_nt<1, 1>(device, map_a, map_b, p, 1, early, stream);
         if (rc != TB_OK) return rc;
     }
     if (pl.splits > 1) {
         const dim3 grid((uint32_t)((N + 31) / 32), (uint32_t)((M + 31) / 32), 1);
-        reduce_splits_kernel<<<grid, 256, 0, stream>>>(partial, pl.splits, whole);
-        TB_CUDA(cudaGetLastError());
+        return launch_after(reduce_splits_kernel, grid, 256, 0, stream, early, partial, pl.splits, whole);
     }
     return TB_OK;
 }

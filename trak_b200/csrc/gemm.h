@@ -53,10 +53,11 @@ enum KRange : int {
 
 // C[M x N] (+)= alpha * row_scale[m] * Apacked . Bpacked^T  (symmetric: A == B, mirrored stores;
 // chunked: scaled fp32 operands only -- the tensor core accumulates 64 k at a time and the chunks are
-// summed with rounded fp32 adds, for products whose error an inverse will amplify)
+// summed with rounded fp32 adds, for products whose error an inverse will amplify).  `early`: see launch_after; not where
+// another stream waits for the SMs that the launch would hold.
 int launch_gemm(int device, cudaStream_t stream, const uint16_t* pa, const Packed& ga, const uint16_t* pb,
                 const Packed& gb, int dtype, int64_t M, int64_t N, float* C, int64_t ldc,
                 const float* row_scale, float alpha, int accumulate, int symmetric, int chunked, float* partial,
-                KRange range = K_ALL);
+                KRange range = K_ALL, bool early = true);
 
 }  // namespace tb

@@ -61,6 +61,37 @@ __device__ __forceinline__ void publish_status(const uint32_t* status, const Sta
 }
 #endif
 
+#ifdef __CUDACC__
+// A launch that may begin while the one before it on the stream is still ending: its CTAs take the places that become
+// free, set up their barriers and tensor memory and start generating, and wait (cudaGridDependencySynchronize) where
+// they first need what the earlier launch wrote.  Worth 3 to 5 us a call; every kernel in front of such a launch lets it
+// begin at once.
+template <typename... Params, typename... Args>
+int launch_after(void (*kernel)(Params...), dim3 grid, uint32_t threads, size_t smem, cudaStream_t stream, bool early,
+                 Args&&... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = early ? 1 : 0;
+    TB_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
+    return TB_OK;
+}
+
+// First statement of a kernel between two such launches (or in front of its first use of global memory): what the earlier
+// launch wrote is there, and the next launch may take the places that become free.  Not before: a launch further on would
+// hold its shared memory through all of an earlier one that other streams' work should run beside.
+__device__ __forceinline__ void after_earlier_launch() {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+}
+#endif
+
 // Lets `kernel` use all of an SM's shared memory on `device` (the current one); once per kernel and device.
 constexpr int SMEM_PER_CTA = 227 * 1024;
 int set_smem_limit(const void* kernel, int device);

@@ -153,6 +153,7 @@ struct TileRegs {
 
 // A += lambda I, and zero for the counters that the block columns' CTAs meet at.
 __global__ void prepare_kernel(float* A, int64_t lda, int k, float lambda, uint32_t* counters, int n) {
+    after_earlier_launch();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < k && lambda != 0.0f) A[(int64_t)i * lda + i] += lambda;
     if (i < n) counters[i] = 0;
@@ -584,6 +585,7 @@ __device__ __forceinline__ bool rows_are_vec4(const float* A, int64_t lda, int k
 
 constexpr int RED_BLOCKS = 1024;
 __global__ void __launch_bounds__(256) abs_partial_kernel(const float* A, int64_t lda, int k, double* partial) {
+    after_earlier_launch();
     __shared__ double sh[256];
     double s = 0.0;
     const bool vec = rows_are_vec4(A, lda, k);
@@ -620,12 +622,14 @@ __device__ float mean_abs(const double* partial, int k) {
     return (float)(sh[0] / ((double)k * (double)k));
 }
 __global__ void __launch_bounds__(256) abs_final_kernel(const double* partial, int k, float* mean_out) {
+    after_earlier_launch();
     const float mean = mean_abs(partial, k);
     if (threadIdx.x == 0) *mean_out = mean;
 }
 // Every CTA sums the 8 KB of partial sums itself (about 1 us) instead of waiting for a launch that does.
 __global__ void __launch_bounds__(256) scale_by_inverse_kernel(float* A, int64_t lda, int k, const double* partial,
                                                                float* mean_out) {
+    after_earlier_launch();
     const float mean = mean_abs(partial, k), inv = 1.0f / mean;
     if (mean_out && blockIdx.x == 0 && threadIdx.x == 0) *mean_out = mean;
     const bool vec = rows_are_vec4(A, lda, k);
@@ -893,10 +897,10 @@ int tb_spd_inverse(int device, void* stream_, float* A, int64_t k, int64_t lda, 
                 const Packed gt = packed_tail(&tail, g, OUTER / 128);
                 float* partial_sums = reinterpret_cast<float*>(base + l.rest);
                 rc = launch_gemm(device, rest, tail, gt, L, g, TB_F32, r - d, d, A22 + d * lda, lda, nullptr, -1.0f, 1, 0, 1,
-                                 partial_sums);
+                                 partial_sums, K_ALL, false);
                 if (rc != TB_OK) return rc;
                 rc = launch_gemm(device, rest, tail, gt, tail, gt, TB_F32, r - d, r - d, A22 + d * lda + d, lda, nullptr,
-                                 -1.0f, 1, 1, 1, partial_sums);
+                                 -1.0f, 1, 1, 1, partial_sums, K_ALL, false);
                 if (rc != TB_OK) return rc;
                 if ((rc = record(side.s.updated, rest)) != TB_OK) return rc;
             }
@@ -925,13 +929,13 @@ int tb_spd_inverse(int device, void* stream_, float* A, int64_t k, int64_t lda, 
 
     // mean |entry| and the reference's rescale
     if (rescale_by_mean_abs || mean_abs_out) {
-        abs_partial_kernel<<<RED_BLOCKS, 256, 0, stream>>>(A, lda, K, partial);
-        if (rescale_by_mean_abs)
-            scale_by_inverse_kernel<<<std::min(K, sm_count * 8), 256, 0, stream>>>(A, lda, K, partial, mean_abs_out);
-        else
-            abs_final_kernel<<<1, 256, 0, stream>>>(partial, K, mean_abs_out);
+        rc = launch_after(abs_partial_kernel, RED_BLOCKS, 256, 0, stream, true, A, lda, K, partial);
+        if (rc != TB_OK) return rc;
+        rc = rescale_by_mean_abs ? launch_after(scale_by_inverse_kernel, std::min(K, sm_count * 8), 256, 0, stream, true, A, lda,
+                                                K, partial, mean_abs_out)
+                                 : launch_after(abs_final_kernel, 1, 256, 0, stream, true, partial, K, mean_abs_out);
+        if (rc != TB_OK) return rc;
     }
-    TB_CUDA(cudaGetLastError());
     return TB_OK;
 }
 
