@@ -379,6 +379,24 @@ __device__ void chol_block(const Tile& S, int jb, float* dinv, Tile& Dt, uint32_
     if (!ok) atomicCAS(status, 0u, (uint32_t)ST_NOT_SPD);
 }
 
+// Counters of a block column: `factored` tiles of the diagonal (CTA 0), and steps x CTAs finished by the others.
+struct BlockCounters {
+    uint32_t factored, finished;
+};
+// Waits until *counter has reached `target`; one thread.  Bounded.
+__device__ bool reached(const uint32_t* counter, uint32_t target, uint32_t* status) {
+    const uint64_t t0 = globaltimer_ns();
+    for (uint32_t n = 1;; ++n) {
+        uint32_t seen;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
+        if (seen >= target) return true;
+        if ((n & 255u) == 0 && globaltimer_ns() - t0 > WAIT_LIMIT_NS) {
+            if (atomicCAS(status, 0u, (uint32_t)ST_TIMEOUT_ACC) == 0u) status[1] = blockIdx.x;
+            return false;
+        }
+    }
+}
+
 // Step j of a block column's diagonal block (kb x kb, kb <= 512), in tiles of 64.  Before the step, rows i >= j hold
 // R[i, c] for c < j (what is left of the identity's elimination, W's future rows) and S[i, l] for l >= j (what is
 // left of A), and D = inv(chol(S[j, j])) is known.  The step makes row j of W final,
@@ -387,9 +405,10 @@ __device__ void chol_block(const Tile& S, int jb, float* dinv, Tile& Dt, uint32_
 //     S[i, l] -= P_i P_l^T (j < l <= i),   R[i, c] -= P_i W[j, c] (c < j),   R[i, j] = -P_i D.
 // One CTA per tile, each computing the P and W tiles it needs itself (three 64^3 products instead of another meeting point
 // and a trip through memory).  Rows i > j go from X to Y (tiles are read by many CTAs, so they are not updated in place);
-// W's rows go to `block`, the matrix itself, with zeros right of the diagonal.
-__device__ void block_tile(float* smem, const float* X, int64_t ldx, float* Y, float* block, int64_t lda, int kb,
-                           int j, int i, int c, const float* D) {
+// W's rows go to `block`, the matrix itself, with zeros right of the diagonal.  What a tile needs of X is fetched before D is
+// waited for (*factored > j), where a CTA spends a quarter of a step.  False when the wait ran out.
+__device__ bool block_tile(float* smem, const float* X, int64_t ldx, float* Y, float* block, int64_t lda, int kb, int j, int i,
+                           int c, const float* D, const uint32_t* factored, uint32_t* status, uint32_t* have_d) {
     Tile& Dt = *reinterpret_cast<Tile*>(smem);                // Dt[t][c] = D[c][t]
     Tile& T0 = *reinterpret_cast<Tile*>(smem + NB * TS);
     Tile& T1 = *reinterpret_cast<Tile*>(smem + 2 * NB * TS);
@@ -399,12 +418,20 @@ __device__ void block_tile(float* smem, const float* X, int64_t ldx, float* Y, f
     const int rows = min(NB, kb - i * NB), jw = min(NB, kb - j * NB), cols = min(NB, kb - c * NB);
     float acc[4][4];
     TileRegs<256> d, t1, t2;
+    auto wait_for_d = [&] {
+        if (tid == 0) *have_d = reached(factored, (uint32_t)j + 1u, status);
+        __syncthreads();
+        return *have_d != 0u;
+    };
     if (i == j) {  // row j of W
         if (c < j) {
-            d.fetch(tid, D, NB, NB, NB);
             t1.fetch(tid, X + (int64_t)j * NB * ldx + c * NB, ldx, rows, NB);
-            d.put<true>(tid, Dt);
             t1.put<false>(tid, T0);
+        }
+        if (!wait_for_d()) return false;
+        if (c < j) {
+            d.fetch(tid, D, NB, NB, NB);
+            d.put<true>(tid, Dt);
             __syncthreads();
             tile_mma(Dt, T0, exchange, acc);
         }
@@ -416,9 +443,8 @@ __device__ void block_tile(float* smem, const float* X, int64_t ldx, float* Y, f
                 if (r < rows && q < cols)
                     block[(int64_t)(j * NB + r) * lda + c * NB + q] = c < j ? acc[a][b] : c == j ? __ldcg(D + r * NB + q) : 0.0f;
             }
-        return;
+        return true;
     }
-    d.fetch(tid, D, NB, NB, NB);
     t1.fetch(tid, X + (int64_t)i * NB * ldx + j * NB, ldx, rows, jw);
     if (c > j && c != i)
         t2.fetch(tid, X + (int64_t)c * NB * ldx + j * NB, ldx, cols, jw);
@@ -438,15 +464,17 @@ __device__ void block_tile(float* smem, const float* X, int64_t ldx, float* Y, f
             for (int b = 0; b < 4; ++b) own[a][b] = (live && tx * 4 + b < cols) ? __ldcg(mine + a * ldx + b) : 0.0f;
         }
     }
-    d.put<true>(tid, Dt);
-    t1.put<true>(tid, T1);  // P_i^T = D S[i, j]^T, i.e. t-major, goes to T0
+    t1.put<true>(tid, T1);
     if (c > j && c != i)
         t2.put<true>(tid, T2);
     else if (c < j)
         t2.put<false>(tid, T2);
-    else if (c == j)
-        d.put<false>(tid, T2);
+    if (!wait_for_d()) return false;
+    d.fetch(tid, D, NB, NB, NB);
+    d.put<true>(tid, Dt);
+    if (c == j) d.put<false>(tid, T2);
     __syncthreads();
+    // P_i^T = D S[i, j]^T, i.e. P_i t-major
     tile_mma(Dt, T1, exchange, acc);
     put_piece(T0, ty, tx, acc);
     if (c != i && c != j) {  // the other operand, P_c^T or W[j, c], over T1 (the product above is done with it)
@@ -459,25 +487,9 @@ __device__ void block_tile(float* smem, const float* X, int64_t ldx, float* Y, f
     for (int a = 0; a < 4; ++a)
         *reinterpret_cast<float4*>(Y + (int64_t)(i * NB + ty * 4 + a) * OUTER + c * NB + tx * 4) =
             make_float4(own[a][0] - acc[a][0], own[a][1] - acc[a][1], own[a][2] - acc[a][2], own[a][3] - acc[a][3]);
+    return true;
 }
 
-// Counters of a block column: `factored` tiles of the diagonal (CTA 0), and steps x CTAs finished by the others.
-struct BlockCounters {
-    uint32_t factored, finished;
-};
-// Waits until *counter has reached `target`; one thread.  Bounded.
-__device__ bool reached(const uint32_t* counter, uint32_t target, uint32_t* status) {
-    const uint64_t t0 = globaltimer_ns();
-    for (uint32_t n = 1;; ++n) {
-        uint32_t seen;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
-        if (seen >= target) return true;
-        if ((n & 255u) == 0 && globaltimer_ns() - t0 > WAIT_LIMIT_NS) {
-            if (atomicCAS(status, 0u, (uint32_t)ST_TIMEOUT_ACC) == 0u) status[1] = blockIdx.x;
-            return false;
-        }
-    }
-}
 // What this CTA's threads have written, then the counter.  All threads; the next use of what they read needs no further
 // barrier.
 __device__ __forceinline__ void announce(uint32_t* counter) {
@@ -493,13 +505,14 @@ __device__ __forceinline__ void announce(uint32_t* counter) {
 // left them a step earlier) and goes on, without waiting for anyone unless the others fall behind.  They wait for a tile's
 // inverse, share the step's tiles and wait for one another.  A cooperative launch of about as many CTAs as the largest step
 // has tiles.  With one meeting point of all CTAs per step, CTA 0's tiles fetched behind it and the slower products and
-// factorisation of before, the 512-wide block took 126 us, 97 now.
+// factorisation of before, the 512-wide block took 126 us; 97 after that, and 88 with what a tile needs of the step before
+// fetched while its inverse is waited for.
 constexpr int STEP_THREADS = 256;
 constexpr size_t STEP_SMEM = (5 * NB * TS + EXCHANGE_FLOATS + CHOL_FLOATS) * sizeof(float);
 __global__ void __launch_bounds__(STEP_THREADS, 1) block_kernel(float* block, int64_t lda, int kb, float* blocks, float* dinv,
                                                                 BlockCounters* counters, uint32_t* status) {
     extern __shared__ __align__(16) float smem[];
-    __shared__ uint32_t proceed;
+    __shared__ uint32_t proceed, have_d;
     const int nt = (kb + NB - 1) / NB, tid = threadIdx.x;
     const uint32_t others = gridDim.x - 1;
     auto source = [&](int j) { return j == 0 ? block : blocks + (size_t)((j - 1) & 1) * OUTER * OUTER; };
@@ -554,9 +567,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) block_kernel(float* block, in
         }
     }
     for (int j = 0; j < nt; ++j) {
-        if (tid == 0)
-            proceed = reached(&counters->factored, (uint32_t)j + 1u, status) &&
-                      reached(&counters->finished, (uint32_t)j * others, status);
+        if (tid == 0) proceed = reached(&counters->finished, (uint32_t)j * others, status);
         __syncthreads();
         if (!proceed) return;
         float* Y = blocks + (size_t)(j & 1) * OUTER * OUTER;
@@ -570,7 +581,8 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) block_kernel(float* block, in
                 for (i = j + 1; c > i; ++i) c -= i + 1;
                 if (i == j + 1 && c == j + 1) continue;  // CTA 0's
             }
-            block_tile(smem, source(j), source_ld(j), Y, block, lda, kb, j, i, c, D);
+            if (!block_tile(smem, source(j), source_ld(j), Y, block, lda, kb, j, i, c, D, &counters->factored, status, &have_d))
+                return;
             __syncthreads();
         }
         announce(&counters->finished);
