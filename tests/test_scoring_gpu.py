@@ -261,6 +261,35 @@ def test_chained_launches_give_the_same_under_capture(cuda, n, k, m):
     assert all(torch.equal(a, b) for a, b in zip(first, out))
 
 
+def test_inverses_of_several_threads_at_once(cuda):
+    """Each launch of the diagonal block's kernel waits for its own CTAs only: more of them at once than the GPU holds."""
+    import threading
+    from trak_b200 import score_computers as sc
+    mats = []
+    for k in (512, 512, 300, 700, 1024, 512):
+        y = torch.randn(2 * k, k, device=cuda, generator=torch.Generator(device=cuda).manual_seed(k + len(mats)))
+        mats.append(y.T @ y / k)
+    refs = [sc.spd_inverse_(a.clone(), 1e-2) for a in mats]
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream(cuda)):
+                for _ in range(10):
+                    if not torch.equal(sc.spd_inverse_(mats[i].clone(), 1e-2), refs[i]):
+                        wrong.append(i)
+        except Exception as e:  # a bounded wait that ran out
+            wrong.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(mats))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 1, 1), (129, 257, 33), (300, 700, 95), (128, 256, 64), (513, 100, 4097)])
 def test_gram_and_gemm_at_ragged_sizes(cuda, M, N, K):
     """Tile, chunk (64 k) and slot (32 k) boundaries of both GEMM kernels, with accumulation into existing output."""
