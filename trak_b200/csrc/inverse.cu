@@ -540,6 +540,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) block_kernel(float* block, in
                 const int lane = tid & 31, id = (warp == 7 ? 32 : 0) + lane;
                 bool ok = lane != 0 || reached(&counters->finished, (uint32_t)j * others, status);
                 ok = __all_sync(0xffffffffu, ok);
+                __syncwarp();  // a vote orders no memory: this hands lane 0's acquire on to the lanes that read behind it
                 const float* at = source(j) + (int64_t)(j + 1) * NB * source_ld(j) + j * NB;
                 if (ok) {
                     TileRegs<64> t, u;
