@@ -263,6 +263,14 @@ int tb_project_static(int device, void *stream, const void *grads, int dtype, in
  * Zero over the whole 32-bit range is what keeps the matrix bit-identical to the reference's. */
 int tb_selftest_sqrt(int device, void *stream, uint64_t first, uint64_t count, uint64_t *mismatches_dev);
 
+/* The grid that tb_project lays over one pass of B rows (at most 512 of a Gaussian, 256 of a Rademacher projection) on a
+ * GPU of `sm_count` SMs, for tests and tuning; needs no device.  grid[0] output columns of a CTA, [1] generator groups of a
+ * CTA, [2] CTAs that an SM holds, [3] feature tiles, [4] feature tiles that a CTA walks at most, [5] CTAs beside one
+ * another along the features (of each of the N / grid[0] column tiles), [6] pipeline stages of a feature tile, [7] the most
+ * of them whose products are added up before the accumulators are read out. */
+int tb_project_grid(int64_t B, int64_t F, uint32_t N, uint32_t num_feature_tiles, int proj_type, int sm_count,
+                    uint32_t grid[8]);
+
 /* ---- pageable host memory (no counterpart in the reference) ---------------------
  * Copies between pageable host memory (numpy memmaps, host accumulators) and the device through a small pinned
  * ring per device and direction; several host threads share the host side, which runs under the PCIe copies: the

@@ -1,0 +1,42 @@
+"""The grids that the projection lays over its passes, computed without a device."""
+import ctypes
+
+import pytest
+
+from trak_b200 import _lib
+
+RAD, NOR = 0, 1
+
+
+def grid(B, F, N, T=148, p=RAD, sms=148):
+    out = (ctypes.c_uint32 * 8)()
+    rc = _lib.lib().tb_project_grid(B, F, N, T, p, sms, out)
+    assert rc == 0, rc
+    names = ("columns", "groups", "ctas_per_sm", "tiles", "tiles_per_cta", "bundles", "stages", "chain")
+    return dict(zip(names, out))
+
+
+def busiest_sm(g, N, sms=148):
+    """Column tiles x feature tiles that the busiest SM works through, CTAs handed out one by one."""
+    per_sm = [0.0] * (sms * g["ctas_per_sm"])
+    left = g["tiles"]
+    for _ in range(g["bundles"]):
+        walked = min(left, g["tiles_per_cta"])
+        left -= walked
+        for _ in range(N // g["columns"]):
+            i = per_sm.index(min(per_sm))
+            per_sm[i] += walked
+    assert left == 0
+    return max(per_sm)
+
+
+@pytest.mark.parametrize("T,sms", [(148, 148), (132, 132)])
+@pytest.mark.parametrize("F", [1_000_003, 11_173_962])
+@pytest.mark.parametrize("N", range(512, 4097, 512))
+@pytest.mark.parametrize("B", [65, 96, 128])
+def test_rademacher_batches_of_65_to_128_rows_fill_the_gpu(B, N, F, T, sms):
+    """These are bound by the MMAs: a pass takes as long as the tiles of its busiest SM, whose share must be near the mean
+    where the tiles are long.  Tiles of 256 columns cannot be shared: a whole one above the mean is allowed."""
+    g = grid(B, F, N, T, RAD, sms)
+    mean = g["tiles"] * (N // g["columns"]) / sms
+    assert busiest_sm(g, N, sms) <= max(1.16 * mean, -(-g["tiles"] * (N // g["columns"]) // sms))

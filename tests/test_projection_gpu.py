@@ -612,6 +612,41 @@ def test_accumulation_chains(cuda, p, B, F, T):
     assert rel_rows(stored.cpu().numpy()[:, cols][len(feats):], ref[len(feats):]) <= 1e-4
 
 
+PAIRED_SHAPES = [  # B, F, N, tiles, dtype, generator groups: Rademacher, 65 to 128 rows
+    (65, 9_472, 512, 148, "f16", 2),      # 64 features a tile: one stage, one chain
+    (128, 9_473, 512, 148, "bf16", 2),    # one feature more
+    (97, 20_011, 1536, 37, "f32", 2),     # a CTA with one tile beside those with two
+    (80, 100_003, 512, 3, "bf16", 2),     # 521 stages a tile: chains of 512 and 9
+    (128, 9_473, 1024, 148, "bf16", 4),
+    (66, 20_011, 2560, 148, "f16", 4),    # eleven tiles a CTA, five in the last
+    (65, 594_001, 4096, 36, "f16", 4),    # 258 stages a tile: a chain ends in the middle and at the end
+]
+
+
+@pytest.mark.parametrize("B,F,N,T,dt,groups", PAIRED_SHAPES)
+def test_rademacher_batches_of_65_to_128_rows(cuda, B, F, N, T, dt, groups):
+    """Both shapes of the CTA, at the edges of tiles, bundles and chains; one-hot rows are exact, the others within the
+    drift of the tensor core's truncating adds (chains of at most 4096 steps: below 5e-5)."""
+    import ctypes
+    from trak_b200 import _lib
+    grid = (ctypes.c_uint32 * 8)()
+    sms = torch.cuda.get_device_properties(cuda).multi_processor_count
+    assert _lib.lib().tb_project_grid(B, F, N, T, RAD, sms, grid) == 0
+    assert sms != 148 or (grid[0], grid[1]) == (256, groups)
+    g_cpu = (torch.randn(B, F, generator=torch.Generator().manual_seed(B + F)) * 0.1).to(DT[dt])
+    fts = o.feature_tile_size(F, T)
+    feats = [0, fts - 1, fts, F // 2, F - 1]
+    for r, f in enumerate(feats):
+        g_cpu[r].zero_()
+        g_cpu[r, f] = 1.0
+    out = ours(g_cpu.to(cuda), N, 31, T, RAD).cpu().numpy()
+    assert np.array_equal(out[:len(feats)], o.matrix_rows(RAD, F, N, 31, T, feats))
+    cols = [0, 9, N // 32 - 1]
+    ref = o.project_column_groups(RAD, as_numpy_input(g_cpu.half() if dt == "f32" else g_cpu), 31, T, cols)
+    got = np.concatenate([out[:, 32 * c:32 * c + 32] for c in cols], axis=1)
+    assert rel_rows(got[len(feats):], ref[len(feats):]) <= 1e-4
+
+
 STORED_SHAPES = [  # B, F, N, seed, tiles, dtype
     (16, 20011, 1024, 17, 148, "f16"),
     (130, 9473, 512, 5, 7, "f32"),
