@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(128) materialize_kernel(uint16_t* __restrict__
     const uint32_t q = threadIdx.x >> 5, lane = threadIdx.x & 31u, h = lane >> 4;
     const uint32_t stream_col = blockIdx.x * 128u + q * 32u + lane;
     const uint32_t by = blockIdx.y;
-    SignBases<BF16> bases;
+    SignBases<BF16, false> bases;
     if (PTYPE == TB_RADEMACHER) bases.load();
     Xw st;
     xw_seed(st, seed + 658105236u * stream_col + 359124577u * by);
@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(128) materialize_kernel(uint16_t* __restrict__
         for (uint32_t c = 0; c < 4; ++c) {
             uint32_t w[8];
             if constexpr (PTYPE == TB_RADEMACHER) {
-                gen_rademacher<BF16>(st, h, bases, w);
+                gen_rademacher(st, h, bases, w);
             } else {
                 uint32_t even[4], odd[4];
                 gen_normal<BF16>(st, even, odd);
