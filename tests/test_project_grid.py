@@ -40,3 +40,11 @@ def test_rademacher_batches_of_65_to_128_rows_fill_the_gpu(B, N, F, T, sms):
     g = grid(B, F, N, T, RAD, sms)
     mean = g["tiles"] * (N // g["columns"]) / sms
     assert busiest_sm(g, N, sms) <= max(1.16 * mean, -(-g["tiles"] * (N // g["columns"]) // sms))
+
+
+@pytest.mark.parametrize("F,stages,chain", [(9_472, 1, 1), (28_416, 3, 3), (28_417, 4, 2), (37_889, 5, 3), (100_003, 11, 6),
+                                            (1_000_003, 106, 53), (11_173_962, 1180, 256)])
+def test_four_groups_drain_in_mid_tile_only_where_the_tile_is_long(F, stages, chain):
+    """Chains of up to 48 MMA steps do not drift beyond the rounding of the sums; longer tiles take two chains or more."""
+    g = grid(128, F, 1024)
+    assert (g["groups"], g["stages"], g["chain"]) == (4, stages, chain)
