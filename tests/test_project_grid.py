@@ -48,3 +48,13 @@ def test_four_groups_drain_in_mid_tile_only_where_the_tile_is_long(F, stages, ch
     """Chains of up to 48 MMA steps do not drift beyond the rounding of the sums; longer tiles take two chains or more."""
     g = grid(128, F, 1024)
     assert (g["groups"], g["stages"], g["chain"]) == (4, stages, chain)
+
+
+@pytest.mark.parametrize("p", [RAD, NOR])
+@pytest.mark.parametrize("N", [512, 1024, 1536, 4096])
+@pytest.mark.parametrize("B", [1, 16, 64, 128])
+def test_a_grid_of_at_most_one_cta_per_sm_is_not_packed(B, N, p):
+    """The SMs that become free first would otherwise take two CTAs and the others none."""
+    g = grid(B, 1_000_003, N, 148, p)
+    assert g["ctas_per_sm"] == 1 or g["bundles"] * N // g["columns"] > 148
+    assert N != 512 or g["bundles"] * N // g["columns"] == 148
