@@ -984,6 +984,8 @@ static int packed_tmap(CUtensorMap* map, const uint16_t* packed, const Packed& g
                        2, packed, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
+constexpr uint32_t B200_SMS = 148;
+
 // Tile and number of slices of the contraction.  A 256 x 256 (or 128 x 256) tile per CTA leaves most of the 148 SMs
 // idle when the product is small: the Gram of 2048 columns is 36 such tiles however many rows it sums over.  The
 // choice minimises an estimate in microseconds: per wave of CTAs a fixed part (launch, first loads, epilogue) plus the
@@ -998,7 +1000,7 @@ static int packed_tmap(CUtensorMap* map, const uint16_t* packed, const Packed& g
 // The sizes alone decide, so that the workspace query, which names no device, agrees: every B200 has 148 SMs.  A product
 // that leaves out the k blocks where a triangular factor is zero (KRange) is planned like a whole one.
 GemmPlan plan_gemm(uint32_t npl, bool chunked, bool symmetric, int64_t M, int64_t N, uint32_t kblocks) {
-    constexpr double SMS = 148.0, SUM_FIXED = 7.0, SUM_BYTES_PER_US = 3.0e6;
+    constexpr double SMS = B200_SMS, SUM_FIXED = 7.0, SUM_BYTES_PER_US = 3.0e6;
     constexpr uint32_t MAX_SPLITS = 64;
     constexpr size_t MAX_PARTIAL = 256u << 20;
     constexpr double MAX_GRID_Y = 65535.0;  // tile rows of a launch, 32-row blocks of the sum
@@ -1036,14 +1038,18 @@ template <int NPL, int T>
 static int launch_gemm_nt(int device, const CUtensorMap& map_a, const CUtensorMap& map_b, GemmParams& p, uint32_t splits,
                           bool early, cudaStream_t stream) {
     constexpr uint32_t stage_bytes = 2u * T * NPL * GTILE_BYTES;
-    // two CTAs of the small tile share an SM
-    p.stages = ((T == 2 ? 200u : 100u) * 1024u) / stage_bytes;
+    const dim3 grid((p.N + 128u * T - 1) / (128u * T), (p.M + 128u * T - 1) / (128u * T), splits);
+    // Two CTAs of the small tile share an SM.  Launched while the packing still runs they would do so on the first SMs that
+    // become free, also where there is one for every SM and the others stay idle: such a grid takes all of the shared memory
+    // (fp32 2000 x 1000 x 1024 29.9 -> 21.9 us, 128 x 8192 x 2048 65.8 -> 47.7, 10,000 x 100 x 2048 71.6 -> 52.4; fp16
+    // 18,900 x 100 x 2048 61.9 -> 52.4).
+    const bool pairs = T == 1 && !(early && (uint64_t)grid.x * grid.y <= (uint64_t)B200_SMS);
+    p.stages = ((pairs ? 100u : 200u) * 1024u) / stage_bytes;
     if (p.stages > 8) p.stages = 8;
     const size_t smem = (size_t)p.stages * stage_bytes + 1024u;
     p.idesc = (p.idesc & 1u) ? idesc_f16(1u, 128u * T) : idesc_f16(0u, 128u * T);
     auto kern = gemm_nt_kernel<NPL, T>;
     if (const int e = set_smem_limit((const void*)kern, device)) return e;
-    const dim3 grid((p.N + 128u * T - 1) / (128u * T), (p.M + 128u * T - 1) / (128u * T), splits);
     return launch_after(kern, grid, 384, smem, stream, early, map_a, map_b, p);
 }
 
