@@ -905,6 +905,13 @@ static PackRows pack_rows_args(const void* src, uint64_t rows, uint64_t K, uint6
     return PackRows{static_cast<const float*>(src), packed, packed_amax(packed, g), rows, K, ld, g.rowblocks, g.kblocks};
 }
 
+// Whether the packing of so many operand elements is launched while the product before it on the stream still runs.  That
+// gains 2 us, but the CTAs of a large one then fill the SMs unevenly, around those of the product: 37,000 x 100 x 2048 in
+// a row took 110 us a product in fp16 and 174 in fp32 instead of 97 and 159, 20,000 x 100 x 2048 66 and 103 instead of 61
+// and 97; the two meet at about 20 million elements (fp16 25,000 x 100 x 512 21.8 early and 23.2, 10,000 x 100 x 2048 38.0
+// and 37.5; fp32 40,000 x 100 x 512 66.5 and 67.7, 60,000 x 100 x 512 81.6 and 80.7).
+static bool pack_early(uint64_t elements) { return elements < 25'000'000u; }
+
 // One or two fp32 operands (b.rowblocks = 0: one) whose rows are source rows.
 static int launch_pack_rows(const PackRows& a, const PackRows& b, int sm_count, cudaStream_t stream) {
     const uint64_t K = a.K > b.K ? a.K : b.K, rows = ((uint64_t)a.rowblocks + b.rowblocks) * 128u;
@@ -914,10 +921,11 @@ static int launch_pack_rows(const PackRows& a, const PackRows& b, int sm_count, 
     const uint64_t cap = (uint64_t)sm_count * 32;
     if (blocks > cap) blocks = cap;
     const uint32_t nb = (uint32_t)blocks;
-    if (w == 1) return launch_after(pack_rows_f32_kernel<1>, nb, 256, 0, stream, true, a, b);
-    if (w == 2) return launch_after(pack_rows_f32_kernel<2>, nb, 256, 0, stream, true, a, b);
-    if (w == 4) return launch_after(pack_rows_f32_kernel<4>, nb, 256, 0, stream, true, a, b);
-    return launch_after(pack_rows_f32_kernel<8>, nb, 256, 0, stream, true, a, b);
+    const bool early = pack_early(a.rows * a.K + b.rows * b.K);
+    if (w == 1) return launch_after(pack_rows_f32_kernel<1>, nb, 256, 0, stream, early, a, b);
+    if (w == 2) return launch_after(pack_rows_f32_kernel<2>, nb, 256, 0, stream, early, a, b);
+    if (w == 4) return launch_after(pack_rows_f32_kernel<4>, nb, 256, 0, stream, early, a, b);
+    return launch_after(pack_rows_f32_kernel<8>, nb, 256, 0, stream, early, a, b);
 }
 
 int launch_pack_pair(const float* a, uint64_t rows_a, uint64_t K_a, uint64_t ld_a, uint16_t* packed_a, const Packed& ga,
@@ -968,8 +976,8 @@ int launch_pack(const void* src, int dtype, bool trans, uint64_t rows, uint64_t 
         if (blocks > cap) blocks = cap;
         const uint32_t nb = (uint32_t)blocks;
         const uint16_t* s = static_cast<const uint16_t*>(src);
-        return launch_after(trans ? pack_kernel<true> : pack_kernel<false>, nb, 256, 0, stream, true, s, packed, rows, K, ld,
-                            g.rowblocks, g.kblocks);
+        return launch_after(trans ? pack_kernel<true> : pack_kernel<false>, nb, 256, 0, stream, trans || pack_early(rows * K), s,
+                            packed, rows, K, ld, g.rowblocks, g.kblocks);
     }
 }
 
