@@ -654,7 +654,9 @@ STORED_SHAPES = [  # B, F, N, seed, tiles, dtype
     (5, 16, 512, 9, 148, "f16"),          # fewer features than tiles
     (64, 4096, 1536, 4, 4, "f16"),        # tile size a multiple of 64
     (65, 70_001, 2048, 3, 1, "f16"),      # two column tiles a CTA with two sets of accumulators, three chains
-    (129, 3001, 512, 3, 5, "f16"),        # two column tiles a CTA, one set
+    (129, 3001, 512, 3, 5, "f16"),        # short tiles and an odd multiple of 512: one column tile a CTA
+    (129, 3001, 1024, 3, 5, "f16"),       # two column tiles a CTA, one set
+    (150, 20_485, 512, 3, 5, "f16"),      # the same, 64 stages a tile and one more feature
 ]
 
 
