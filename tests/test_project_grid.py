@@ -58,3 +58,10 @@ def test_a_grid_of_at_most_one_cta_per_sm_is_not_packed(B, N, p):
     g = grid(B, 1_000_003, N, 148, p)
     assert g["ctas_per_sm"] == 1 or g["bundles"] * N // g["columns"] > 148
     assert N != 512 or g["bundles"] * N // g["columns"] == 148
+
+
+def test_wide_grid_of_short_tiles_takes_fewer_ctas():
+    """Eight column tiles: two CTAs of four tiles to an SM where a tile is long, one of eight where the CTA itself costs more."""
+    for F, tiles, bundles in ((3_000, 8, 18), (9_472, 8, 19), (20_011, 8, 19), (1_000_003, 4, 37)):
+        g = grid(512, F, 1024, 148, NOR)
+        assert (g["tiles_per_cta"], g["bundles"]) == (tiles, bundles)
