@@ -129,7 +129,7 @@ int tb_project_segments(int device, void *stream, const tb_segment *segs, int32_
  * entries do not fit the GPUs it was written for.  On a B200 they can: the matrix of
  * (F, N, seed, num_feature_tiles, proj_type) takes tb_matrix_bytes(...) bytes (2 bytes per
  * entry, feature tiles padded to 64 features: 91.6 GB for F = 11,173,962, N = 4096), and
- * reading it from HBM is about three times faster than regenerating a Gaussian matrix.
+ * reading it from HBM is about twice as fast as regenerating a Gaussian matrix.
  * For a projector that serves many batches with one seed (TRAKer.featurize over a train
  * set):
  *

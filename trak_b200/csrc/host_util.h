@@ -64,9 +64,11 @@ __device__ __forceinline__ void publish_status(const uint32_t* status, const Sta
 #ifdef __CUDACC__
 // A launch that, where `early`, may begin while the one before it on the stream is still ending: its CTAs take the places
 // that become free, set up their barriers and tensor memory (and start generating), and wait
-// (cudaGridDependencySynchronize) where they first need what the earlier launch wrote.  Every kernel in front of such a
-// launch says when it may begin (cudaTriggerProgrammaticLaunchCompletion).  Worth about 1.5 us a launch: a projection 3 to
-// 5 us a call, scoring 1000 x 512 299 -> 270, the inverse of 2048 698 -> 640.
+// (cudaGridDependencySynchronize) where they first need what the earlier launch wrote.  A kernel in front of such a
+// launch says when it may begin (cudaTriggerProgrammaticLaunchCompletion); behind one that does not, like reduce_kernel, it
+// begins at that one's end.  Worth about 1.5 us a launch: a projection 3 to 5 us a call, scoring 1000 x 512 299 -> 270, the
+// inverse of 2048 698 -> 640.  The places become free unevenly, and an SM takes as many CTAs as fit: a grid of no more CTAs
+// than SMs asks for more than half of an SM's shared memory, or some SMs get two CTAs and others none.
 template <typename... Params, typename... Args>
 int launch_after(void (*kernel)(Params...), dim3 grid, uint32_t threads, size_t smem, cudaStream_t stream, bool early,
                  Args&&... args) {

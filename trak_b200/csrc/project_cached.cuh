@@ -2,8 +2,8 @@
 //
 // The reference never stores its projection matrix -- D x k entries do not fit the GPUs it was written for -- and
 // regenerates it in every call.  On a B200 the Gaussian matrix of the CIFAR ResNet-18 configuration (11.17M x 4096
-// fp16 = 91.6 GB) fits in HBM next to the gradients, and streaming it from HBM (14 ms at the measured 6.45 TB/s)
-// is three times faster than regenerating it (43 ms of XORWOW + Box-Muller instruction issue).  A projector that is
+// fp16 = 91.6 GB) fits in HBM next to the gradients, and streaming it from HBM (14 ms at the measured 6.54 TB/s)
+// takes less than half as long as regenerating it (32 ms of XORWOW + Box-Muller instruction issue).  A projector that is
 // used for many batches with one seed -- TRAKer.featurize over a whole train set -- can therefore generate the
 // matrix once (materialize_kernel: the very generator of project_kernel, writing to global memory) and project
 // every batch with a plain tcgen05 GEMM whose two operands both arrive by TMA (project_cached_kernel).  The matrix
@@ -71,8 +71,9 @@ __global__ void __launch_bounds__(128) materialize_kernel(uint16_t* __restrict__
 // (ProjParams::epoch) alternate between two sets of accumulators, so the MMA warp starts the next chain while the
 // epilogue warps add the finished one to the partial; two accumulators of more than 128 rows leave room for one set only.
 // Bound by the power limit at 256 rows (SM clock 0.9 GHz in a row of calls) and by the HBM stream of the matrix below.
-// With one column tile per CTA every gradient box crossed from the L2 twice as often (34 GB instead of 17 for 256 rows x
-// 2,097,169 features -> 4096, beside the 17 GB of the matrix): 4.98 -> 4.71 ms a call.
+// With one column tile per CTA every gradient box crosses from the L2 twice as often (34 GB instead of 17 for 256 rows x
+// 2,097,169 features -> 4096, beside the 17 GB of the matrix): 256 x 300,007 -> 4096, which ends before the power limit
+// bites, takes 769 us with one and 651 with two; at 2,097,169 features the two differ by less than a call from the next.
 template <uint32_t NACC>
 __global__ void __launch_bounds__(cached_threads(NACC), 1)
 project_cached_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,

@@ -67,7 +67,7 @@ class CudaProjector:
                  max_batch_size: int = 32, *args, store_matrix: bool = False, **kwargs) -> None:
         # store_matrix: keep the projection matrix of the current (seed, model_id) in device memory
         # (2 * proj_dim bytes per feature: 91.6 GB for a CIFAR ResNet-18 and proj_dim 4096) and read it
-        # instead of regenerating it in every call -- about three times faster for the Gaussian matrix
+        # instead of regenerating it in every call -- about twice as fast for the Gaussian matrix
         # when the same projector serves many batches, as TRAKer.featurize does.  Same matrix, same results
         # up to the order of the fp32 sums.
         self.store_matrix = bool(store_matrix)
