@@ -35,6 +35,9 @@ int project_dense(int device, void* stream, const void* grads, int dtype, int64_
                   int64_t ld_out, uint32_t N, uint32_t seed, uint32_t num_feature_tiles, int proj_type, float alpha,
                   int accumulate, void* ws, size_t ws_bytes, bool publish);
 
+// The least workspace that project_dense takes for these (valid) sizes; tb_project_workspace_bytes is what it wants.
+size_t project_least_bytes(int64_t B, int64_t F, uint32_t N, uint32_t num_feature_tiles);
+
 // Device address of the status word of `device` (valid after select_device).
 uint32_t* status_ptr(int device);
 

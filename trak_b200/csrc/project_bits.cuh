@@ -1,0 +1,585 @@
+// Rademacher projection of small batches on the integer tensor cores.
+//
+// Up to 16 rows the projection costs what its matrix costs to generate, and with a 16-bit operand most of that is not
+// XORWOW (7 instructions a draw) but turning 16 signs into 8 words of +-1.  Here the operand is made of bytes and the
+// draw's own bits are its values: one AND with 0x01010101 << i leaves four matrix entries as 0 or 2^i, and
+//     sum_f (+-1) q_f  =  2 sum_{f: bit set} q_f  -  sum_f q_f
+// makes a sign projection of it.  The gradients are integers too: a row is scaled by the power of two that brings its
+// largest magnitude below 2^28, rounded to q, and kept as four planes of signed base-256 digits, of which `kind::i8` adds up
+// every product exactly in 32 bits.  sum_f q_f comes from the staging.  Only the result of a CTA is rounded, once, to fp32.
+//
+//   * Exactness.  An fp16 (bf16) value has 11 (8) significant bits, so q is exact for every element within 2^-17 (2^-20) of
+//     its row's largest; below that an element is off by at most 2^-28 of the largest, which over n elements adds up to
+//     2^-29 sqrt(n) of the row's norm at most, whatever the distribution (6e-6 for 1e7 elements, all of them just wrong and
+//     one that outweighs the rest).  The fp32 accumulators of the 16-bit kernel drift by 2e-5 there on every input.
+//   * 2^i differs from word to word (bit 2j + h of a draw's byte: feature pair j, column parity h; two of the four j after
+//     a shift by four).  The column's factor 2^h is undone at the end, the features' 2^(2 (j & 1)) in the staging: even j are
+//     staged four times as large.
+//   * What bounds it: the integer pipe, 82 % busy with 11 instructions per 16 x 32 entries (4 of the 7 of a draw, 5 to spread
+//     it, 2 of hand-shakes; 35 instructions in all with a 16-bit operand, now 18), beside MMAs that keep the tensor pipe half
+//     busy.  16 rows, us a call, 16-bit operand -> this: 2,796,202 fp16 features -> 4096 1021 -> 639, 1,000,003 -> 8192
+//     732 -> 444, 40,000,001 bf16 -> 8192 27,750 -> 16,120; one row of 1,000,003 -> 2048 202 -> 131.  From 17 rows on the
+//     four planes make the MMAs the bound and the gain goes.
+//     Measured and dropped: four groups to a CTA (1.4 to 1.6 times as long: one warp issues 16 MMAs a round, each slot of
+//     which costs it 130 cycles of MMAs, 60 of waiting and 20 of commit), one slot a group (773 against 692 us), the next
+//     slots' barriers polled between MMAs (789), shifts as multiplications (no change; by the upper half of a product 3 %
+//     slower), the hand-over of a slot behind the next one's first chunk (no change).
+//   * A row with an infinity or a NaN (seen by absmax_kernel) is staged as the signs of its infinities; the CTA compares
+//     their signed sum with their number and writes what the sum of the row would be, +-inf or NaN.
+//
+// Included by project.cu after the generator definitions.
+#pragma once
+
+namespace tb {
+
+constexpr uint32_t BITS_K = 64;               // features per operand slot (a stage)
+constexpr uint32_t BITS_BOX_K = 128;          // features per box of the staged gradients (128 bytes a row)
+constexpr uint32_t BITS_PLANES = 4;           // base-256 digits of a staged gradient
+constexpr int BITS_NG = 2;                    // generator groups of a CTA
+constexpr uint32_t BITS_MAX_ROWS = 16;        // rows per launch
+constexpr uint32_t BITS_MAX_CHAIN = 32768;    // stages of a CTA: |digit| <= 128, A <= 8, so 2^31 / 1024 features
+constexpr uint32_t BITS_BATCH = 4;            // stages of gradients that arrive and are released together; a group has room for two
+constexpr uint32_t BITS_MAX_SLICES = 256;     // of a row in absmax_kernel
+constexpr int BITS_INF = 0x7ffffffe, BITS_NAN = 0x7fffffff;   // BitsParams::row_exp of a row that holds one
+
+struct BitsParams {
+    float* partials;            // [bundles][B][N]
+    uint32_t* status;
+    const long long* sums;      // [tiles][rows] sum of the rounded gradients q
+    const uint32_t* infs;       // [tiles][rows] infinities among them (rows of BITS_INF only)
+    const int* row_exp;         // [rows] 4 q is 2^row_exp times the gradient; or BITS_INF, BITS_NAN
+    uint32_t N, seed;
+    uint32_t B, rows;           // rows in this launch, and rounded up to 8
+    uint32_t nst;               // pipeline stages per feature tile, even
+    uint32_t tiles, tiles_per_bundle;
+    uint32_t idesc;
+};
+
+// 16 features of a pair of columns: byte b of word j is feature 2j + (b & 1) + 8 (b >> 1) of the 16, as the staging has them.
+__device__ __forceinline__ void gen_bits_pair(Xw& st0, Xw& st1, uint32_t* even, uint32_t* odd) {
+    const uint32_t d0 = xw_next(st0), d1 = xw_next(st1);
+    const uint32_t c = __byte_perm(d0, d1, 0x5140u), c4 = c >> 4;
+    even[0] = c & 0x01010101u;
+    odd[0] = c & 0x02020202u;
+    even[1] = c & 0x04040404u;
+    odd[1] = c & 0x08080808u;
+    even[2] = c4 & 0x01010101u;
+    odd[2] = c4 & 0x02020202u;
+    even[3] = c4 & 0x04040404u;
+    odd[3] = c4 & 0x08080808u;
+}
+
+// v 2^-e for any e: in two steps, each a power of two that fp32 has
+__device__ __forceinline__ float scale_by(float v, int e) {
+    const int a = e / 2, b = e - a;
+    return v * __int_as_float((127 + a) << 23) * __int_as_float((127 + b) << 23);
+}
+
+// One CTA: 256 output columns (two accumulators) x up to 16 rows x a bundle of feature tiles, two CTAs per SM.  Roles, rings
+// and hand-shakes are those of project_kernel with two accumulators; what differs is the operand, the digit planes beside one
+// another in the N dimension (rows x 4), and that the accumulators are read once, at the end.
+template <int NG>
+__global__ void __launch_bounds__((4 * NG + 2) * 32, 2)
+project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p) {
+    constexpr uint32_t GW = 4u, TMEM_COLS = 256u, SA = 2u;
+    constexpr uint32_t A_COL0 = 2u * BITS_PLANES * BITS_MAX_ROWS;   // accumulators, then the generated-operand ring
+    constexpr uint32_t SLOT = 2u * BITS_K / 4u;                     // tensor-memory columns of a slot
+    static_assert(A_COL0 + NG * SA * SLOT <= TMEM_COLS, "too many generator groups for the TMEM ring");
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ alignas(16) uint64_t bar_full_a[NG][SA];
+    __shared__ alignas(16) uint64_t bar_empty_a[NG][SA];
+    __shared__ uint64_t bar_full_b[NG][2];
+    __shared__ uint64_t bar_empty_b[NG][2];
+    __shared__ uint64_t bar_acc;
+    __shared__ uint32_t tmem_slot;
+    __shared__ uint32_t abort_word;
+    volatile uint32_t* abort_flag = &abort_word;
+
+    cudaTriggerProgrammaticLaunchCompletion();
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const uint32_t brows = BITS_PLANES * p.rows;   // N of the MMAs
+    const uint32_t box_bytes = brows * BITS_BOX_K;
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t tile0 = blockIdx.y * p.tiles_per_bundle;
+    const uint32_t ntile = min(p.tiles_per_bundle, p.tiles - tile0);
+
+    if (threadIdx.x == 0) {
+        for (int g = 0; g < NG; ++g)
+            for (uint32_t s = 0; s < 2u; ++s) {
+                mbar_init(smem_u32(&bar_full_a[g][s]), GW);
+                mbar_init(smem_u32(&bar_empty_a[g][s]), 1);
+                mbar_init(smem_u32(&bar_full_b[g][s]), 1);
+                mbar_init(smem_u32(&bar_empty_b[g][s]), 1);
+            }
+        mbar_init(smem_u32(&bar_acc), 1);
+        abort_word = 0;
+        fence_mbar_init();
+    }
+    if (warp == GW * NG + 1) {
+        tmem_alloc(smem_u32(&tmem_slot), TMEM_COLS);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = tmem_slot;
+
+    if (warp < GW * NG) {
+        // ------------------------- generators, then epilogue -------------------------
+        const uint32_t g = warp / GW, q = warp & 3u;
+        const uint32_t pair = q * 32u + lane;
+        const uint32_t stream_col = blockIdx.x * 256u + 2u * (pair & ~15u) + (pair & 15u);
+        const uint32_t lane_base = (q * 32u) << 16;
+        const uint32_t a_base = tmem_base + lane_base + A_COL0 + g * (SA * SLOT);
+        const uint32_t full = smem_u32(&bar_full_a[g][0]), empty = smem_u32(&bar_empty_a[g][0]);
+        bool ok = true;
+        uint32_t n = 0;  // slots this group has filled
+        for (uint32_t ti = g; ti < ntile && ok; ti += NG) {
+            Xw st0, st1;
+            xw_seed(st0, p.seed + 658105236u * stream_col + 359124577u * (tile0 + ti));
+            xw_seed(st1, p.seed + 658105236u * (stream_col + 16u) + 359124577u * (tile0 + ti));
+#pragma unroll 2
+            for (uint32_t s = 0; s < p.nst; ++s, ++n) {
+                const uint32_t slot = n & 1u, parity = (~n >> 1) & 1u;
+                // asked for before the generation and looked at behind it: the answer takes its time
+                const bool free = mbar_test_wait(empty + slot * 8u, parity);
+                uint32_t even[16], odd[16];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) gen_bits_pair(st0, st1, even + 4 * c, odd + 4 * c);
+                if (!__all_sync(0xffffffffu, free) && !mbar_wait_warp(empty + slot * 8u, parity, abort_flag)) {
+                    if (lane == 0) fail(p.status, abort_flag, ST_TIMEOUT_EMPTY, (g << 16) | s);
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                tmem_st_x16(a_base + slot * SLOT, even);
+                tmem_st_x16(a_base + slot * SLOT + SLOT / 2u, odd);
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full + slot * 8u);
+            }
+        }
+        // ---- the exact integer result of this CTA, as fp32 ----
+        if (ok && !mbar_wait_warp(smem_u32(&bar_acc), 0u, abort_flag)) {
+            if (lane == 0) fail(p.status, abort_flag, ST_TIMEOUT_ACC, g);
+            ok = false;
+        }
+        if (ok) {
+            cudaGridDependencySynchronize();  // the staging's sums and scales
+            tc_fence_after();
+            const uint32_t tmem_acc = tmem_base + lane_base;
+            const uint32_t n_out = blockIdx.x * 256u + 2u * pair;
+            float* dst = p.partials + (size_t)blockIdx.y * p.B * p.N + n_out;
+            for (uint32_t b4 = 4u * g; b4 < p.B; b4 += 4u * NG) {
+                // sums of four rows over the bundle's tiles: eight tiles at a time, row `lane & 3`
+                const uint32_t row = b4 + (lane & 3u);
+                long long sum = 0;
+                uint32_t ninf = 0;
+                const int exps = p.row_exp[row];
+                for (uint32_t t = lane >> 2; t < ntile; t += 8u) {
+                    sum += p.sums[(tile0 + t) * p.rows + row];
+                    ninf += p.infs[(tile0 + t) * p.rows + row];
+                }
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) {
+                    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                    ninf += __shfl_xor_sync(0xffffffffu, ninf, o);
+                }
+                uint32_t d[2][BITS_PLANES][4];
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int pl = 0; pl < (int)BITS_PLANES; ++pl)
+                        tmem_ld_x4(tmem_acc + h * brows + pl * p.rows + b4, d[h][pl]);
+                tmem_wait_ld();
+#pragma unroll
+                for (uint32_t j = 0; j < 4; ++j) {
+                    const uint32_t b = b4 + j;
+                    const long long total = __shfl_sync(0xffffffffu, sum, j);
+                    const uint32_t infs = __shfl_sync(0xffffffffu, ninf, j);
+                    const int e = __shfl_sync(0xffffffffu, exps, j);
+                    if (b >= p.B) break;
+                    float2 v;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        long long s = 0;  // 4 2^h times the sum of q over the set bits
+#pragma unroll
+                        for (int pl = (int)BITS_PLANES - 1; pl >= 0; --pl) s = s * 256 + (int)d[h][pl][j];
+                        s = (h == 0 ? 2 * s : s) - 4 * total;
+                        float r;
+                        if (e < BITS_INF)
+                            r = scale_by(__ll2float_rn(s), -e);
+                        else if (e == BITS_INF)
+                            r = infs == 0u ? 0.0f : s == (long long)infs * 4 ? INFINITY : s == -(long long)infs * 4 ? -INFINITY : NAN;
+                        else
+                            r = NAN;
+                        (h == 0 ? v.x : v.y) = r;
+                    }
+                    __stcg(reinterpret_cast<float2*>(dst + (size_t)b * p.N), v);
+                }
+            }
+        }
+    } else {
+        // stages of every group (cnt[] does not increase with g)
+        uint32_t cnt[NG];
+#pragma unroll
+        for (int g = 0; g < NG; ++g) cnt[g] = ntile > (uint32_t)g ? ((ntile - g + NG - 1) / NG) * p.nst : 0u;
+        const uint32_t maxcnt = cnt[0];
+        if (warp == GW * NG) {
+            // ------------------------------ TMA producer (one lane) ------------------------------
+            if (lane == 0) {
+                prefetch_tmap(&tmap);
+                cudaGridDependencySynchronize();  // the staged gradients; the generators need nothing and have begun
+                bool ok = true;
+                const uint32_t boxes = p.nst / 2u;   // per tile
+                uint32_t tile[NG], s[NG];
+#pragma unroll
+                for (int g = 0; g < NG; ++g) {
+                    tile[g] = tile0 + g;
+                    s[g] = 0;
+                }
+                for (uint32_t it = 0, n = 0; it < maxcnt && ok; it += BITS_BATCH, ++n) {
+                    const uint32_t slot = n & 1u, parity = (~n >> 1) & 1u;
+#pragma unroll
+                    for (int g = 0; g < NG; ++g) {
+                        if (it >= cnt[g]) continue;
+                        if (!mbar_wait(smem_u32(&bar_empty_b[g][slot]), parity, abort_flag)) {
+                            fail(p.status, abort_flag, ST_TIMEOUT_EMPTY, 0x8000u | (g << 16) | it);
+                            ok = false;
+                            break;
+                        }
+                        const uint32_t bar = smem_u32(&bar_full_b[g][slot]), loads = min(BITS_BATCH, cnt[g] - it) / 2u;
+                        mbar_expect_tx(bar, loads * box_bytes);
+                        for (uint32_t j = 0; j < loads; ++j) {
+                            tma_load_2d(smem_base + ((g * 2u + slot) * (BITS_BATCH / 2u) + j) * box_bytes, &tmap, 0,
+                                        (int)((tile[g] * boxes + s[g]) * brows), bar);
+                            if (++s[g] == boxes) {
+                                s[g] = 0;
+                                tile[g] += NG;
+                            }
+                        }
+                    }
+                }
+            }
+        } else {
+            // ------------------------------- MMA issuer -------------------------------
+            // Whole warp in the loop, one elected lane issues (operands stay in uniform registers).  The warp shares its
+            // scheduler with busy generators, so what counts is its instructions a slot: rings and parities are unrolled.
+            const bool leader = elect_one();
+            bool ok = true;
+            uint32_t started = 0;
+            for (uint32_t it = 0, n = 0; it < maxcnt && ok; it += BITS_BATCH, ++n) {
+                const uint32_t bslot = n & 1u, bparity = (n >> 1) & 1u;
+#pragma unroll
+                for (uint32_t j = 0; j < BITS_BATCH; ++j) {
+#pragma unroll
+                    for (int g = 0; g < NG; ++g) {
+                        if (it + j >= cnt[g] || !ok) continue;
+                        if (j == 0 && !mbar_wait_warp(smem_u32(&bar_full_b[g][bslot]), bparity, abort_flag)) {
+                            if (leader) fail(p.status, abort_flag, ST_TIMEOUT_FULL_B, (g << 16) | it);
+                            ok = false;
+                            continue;
+                        }
+                        if (!mbar_wait_warp(smem_u32(&bar_full_a[g][j & 1u]), (j >> 1) & 1u, abort_flag)) {
+                            if (leader) fail(p.status, abort_flag, ST_TIMEOUT_FULL_A, (g << 16) | it);
+                            ok = false;
+                            continue;
+                        }
+                        tc_fence_after();
+                        const uint32_t a_addr = tmem_base + A_COL0 + (g * SA + (j & 1u)) * SLOT;
+                        const uint64_t b_desc =
+                            smem_desc_k_sw128(smem_base + ((g * 2u + bslot) * (BITS_BATCH / 2u) + j / 2u) * box_bytes) + 4u * (j & 1u);
+                        if (leader) {
+                            umma_i8_ts(tmem_base, a_addr, b_desc, p.idesc, started);
+                            umma_i8_ts(tmem_base + brows, a_addr + SLOT / 2u, b_desc, p.idesc, started);
+                            // 32 features further: 8 TMEM columns, 32 bytes inside the swizzle row
+                            umma_i8_ts(tmem_base, a_addr + 8u, b_desc + 2u, p.idesc, 1u);
+                            umma_i8_ts(tmem_base + brows, a_addr + SLOT / 2u + 8u, b_desc + 2u, p.idesc, 1u);
+                            tc_commit(smem_u32(&bar_empty_a[g][j & 1u]));
+                            if (j + 1 == BITS_BATCH) tc_commit(smem_u32(&bar_empty_b[g][bslot]));
+                        }
+                        started = 1u;
+                    }
+                }
+            }
+            if (ok && leader) tc_commit(smem_u32(&bar_acc));
+        }
+    }
+
+    // ---------------------------------- teardown ----------------------------------
+    tc_fence_before();
+    __syncthreads();
+    if (*abort_flag) __nanosleep(200000);  // let copies and MMAs already in flight land
+    if (warp == GW * NG + 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, TMEM_COLS);
+    }
+}
+
+// ---- staging of the integer gradients ------------------------------------------------------------------------------
+enum class Elem { F32, F16, BF16 };
+template <Elem E>
+using elem_t = typename std::conditional<E == Elem::F32, float, uint16_t>::type;
+
+// Largest magnitude of slice blockIdx.x of row blockIdx.y, as the bits of the element type (monotonic, infinity above every
+// number and NaN above infinity); also clears the sums the staging adds to.  The ends of a parameter go element by element.
+// Bound by memory: 16 x 2,796,202 fp16 (89 MB) in 20 us.
+__device__ __forceinline__ uint32_t max_bits(uint32_t m, uint32_t w, bool wide) {
+    return wide ? max(m, w & 0x7fffffffu) : __vmaxu2(m, w & 0x7fff7fffu);
+}
+template <Elem E>
+__device__ __forceinline__ uint32_t max_bits_of_run(const elem_t<E>* src, uint64_t n, uint32_t m) {
+    constexpr bool WIDE = E == Elem::F32;
+    constexpr uint32_t V = 16u / sizeof(elem_t<E>);
+    auto one = [&](uint64_t i) {
+        m = max_bits(m, WIDE ? reinterpret_cast<const uint32_t*>(src)[i] : reinterpret_cast<const uint16_t*>(src)[i], WIDE);
+    };
+    const uint64_t head = min(n, (uint64_t)(((16u - (uint32_t)(reinterpret_cast<uintptr_t>(src) & 15u)) & 15u) / sizeof(elem_t<E>)));
+    const uint64_t vecs = (n - head) / V, tail = head + vecs * V;
+    if (threadIdx.x < head) one(threadIdx.x);
+    const uint4* vec = reinterpret_cast<const uint4*>(src + head);
+    uint64_t i = threadIdx.x;
+    for (; i + 3u * 256u < vecs; i += 4u * 256u) {
+        uint4 v[4];
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) v[j] = __ldg(vec + i + j * 256u);
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            m = max_bits(m, v[j].x, WIDE);
+            m = max_bits(m, v[j].y, WIDE);
+            m = max_bits(m, v[j].z, WIDE);
+            m = max_bits(m, v[j].w, WIDE);
+        }
+    }
+    for (; i < vecs; i += 256u) {
+        const uint4 v = __ldg(vec + i);
+        m = max_bits(m, v.x, WIDE);
+        m = max_bits(m, v.y, WIDE);
+        m = max_bits(m, v.z, WIDE);
+        m = max_bits(m, v.w, WIDE);
+    }
+    if (tail + threadIdx.x < n) one(tail + threadIdx.x);
+    return m;
+}
+
+template <Elem E, bool SEG>
+__global__ void __launch_bounds__(256)
+absmax_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ segs, uint32_t nsegs, uint64_t row0,
+              uint32_t* __restrict__ maxima, uint4* __restrict__ clear, uint32_t clear_n, uint64_t F, uint64_t ld,
+              uint64_t slice) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    __shared__ uint32_t part[8];
+    const uint32_t id = (blockIdx.y * gridDim.x + blockIdx.x) * 256u + threadIdx.x;
+    for (uint32_t i = id; i < clear_n; i += gridDim.x * gridDim.y * 256u) clear[i] = make_uint4(0u, 0u, 0u, 0u);
+    const uint64_t f0 = blockIdx.x * slice, f1 = min(F, f0 + slice);
+    uint32_t m = 0;
+    if (SEG) {
+        uint32_t lo = 0, hi = nsegs;  // last parameter whose start is <= f0
+        while (hi - lo > 1u) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (segs[mid].start <= f0)
+                lo = mid;
+            else
+                hi = mid;
+        }
+        for (uint64_t f = f0; f < f1; ++lo) {
+            const SegDev s = segs[lo];
+            const uint64_t end = min(f1, s.start + s.numel);
+            m = max_bits_of_run<E>(static_cast<const elem_t<E>*>(s.ptr) + (row0 + blockIdx.y) * s.stride + (f - s.start),
+                                   end - f, m);
+            f = end;
+        }
+    } else {
+        m = max_bits_of_run<E>(g + (uint64_t)blockIdx.y * ld + f0, f1 - f0, m);
+    }
+    if (E != Elem::F32) m = max(m & 0xffffu, m >> 16);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31u) == 0) part[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int w = 1; w < 8; ++w) m = max(m, part[w]);
+        maxima[blockIdx.y * gridDim.x + blockIdx.x] = m;
+    }
+}
+
+// The value the projection takes an element for: fp32 is rounded to fp16 as in stage_kernel.
+template <Elem E>
+__device__ __forceinline__ float staged_value(uint32_t bits) {
+    if (E == Elem::F32) return __half2float(__float2half_rn(__uint_as_float(bits)));
+    if (E == Elem::F16) return __half2float(__ushort_as_half((unsigned short)bits));
+    return __uint_as_float(bits << 16);
+}
+
+// Scale of a row from its largest element: the exponent e for which 2^e times every element is below 2^28, or what to do
+// with a row that is not finite.
+template <Elem E>
+__device__ __forceinline__ int row_exponent(uint32_t max_bits) {
+    const float m = staged_value<E>(max_bits);
+    if (m != m) return BITS_NAN;
+    if (m == INFINITY) return BITS_INF;
+    if (m == 0.0f) return 0;
+    int e;
+    frexpf(m, &e);  // m < 2^e
+    return 28 - e;
+}
+
+// stage_kernel for project_bits_kernel: staged[tile][128 features][plane][row].  A warp takes runs of 512 features of one
+// row, a lane 16 consecutive features, of which it makes the 16 bytes of every plane (gen_bits_pair says in which order).
+// Bound by memory, two bytes read (fp16) and four written an element, and next to that by 14 instructions an element:
+// 16 x 2,796,202 fp16 in 50 us.
+template <Elem E, bool SEG>
+__global__ void __launch_bounds__(256)
+stage_bits_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ segs, uint32_t nsegs, uint64_t row0,
+                  uint8_t* __restrict__ staged, const uint32_t* __restrict__ maxima, uint32_t slices,
+                  long long* __restrict__ sums, uint32_t* __restrict__ infs, int* __restrict__ row_exp, uint32_t B,
+                  uint32_t rows, uint64_t F, uint64_t ld, uint32_t fts, uint32_t nst, uint32_t tiles) {
+    using In = elem_t<E>;
+    cudaTriggerProgrammaticLaunchCompletion();  // see launch_after
+    constexpr uint32_t RUN = 512u, V = 16u / sizeof(In), LOADS = 16u / V;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t runs = (nst * BITS_K + RUN - 1u) / RUN, blocks = (runs + RUNS_PER_BLOCK - 1u) / RUNS_PER_BLOCK;
+    const uint32_t b_hi_n = rows / 8u;
+    const uint64_t total = (uint64_t)tiles * blocks * b_hi_n;
+    cudaGridDependencySynchronize();  // the maxima, and the cleared sums
+    uint32_t b_of = 0xffffffffu;
+    int e = 0;
+    float f1 = 1.0f, f2 = 1.0f;  // 2^e in two factors (bf16 reaches beyond one)
+    for (uint64_t i = blockIdx.x; i < total; i += gridDim.x) {
+        const uint64_t q = i / blocks;
+        const uint32_t run0 = (uint32_t)(i - q * blocks) * RUNS_PER_BLOCK;
+        const uint32_t tile = (uint32_t)(q / b_hi_n), b = ((uint32_t)q - tile * b_hi_n) * 8u + warp;
+        if (b != b_of) {
+            b_of = b;
+            uint32_t m = 0;
+            if (b < B)
+                for (uint32_t s = lane; s < slices; s += 32u) m = max(m, maxima[b * slices + s]);
+            e = row_exponent<E>(__reduce_max_sync(0xffffffffu, m));
+            const int a = e >= BITS_INF ? 0 : E == Elem::BF16 ? e / 2 : e, c = e < BITS_INF ? e - a : 0;
+            f1 = __int_as_float((127 + a) << 23);
+            f2 = __int_as_float((127 + c) << 23);
+        }
+        if (tile == 0 && run0 == 0 && lane == 0) row_exp[b] = e < BITS_INF ? e + 2 : e;
+        uint8_t* const out_tile = staged + (uint64_t)tile * nst * (BITS_PLANES * rows * BITS_K);
+        long long sum = 0;
+        uint32_t ninf = 0;
+        uint32_t seg = 0;
+        uint64_t s_start = 0, s_end = SEG ? 0 : F;
+        const In* s_row = SEG ? nullptr : g + (uint64_t)b * ld;
+        for (uint32_t run = run0; run < min(run0 + RUNS_PER_BLOCK, runs); ++run) {
+            const uint32_t t0 = run * RUN, t = t0 + lane * 16u;
+            const uint64_t f0 = (uint64_t)tile * fts + t0;
+            const bool live = b < B && f0 < F && t0 < fts;
+            if (SEG && live && f0 >= s_end) {
+                uint32_t lo = 0, hi = nsegs;  // last parameter whose start is <= f0
+                while (hi - lo > 1u) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (segs[mid].start <= f0)
+                        lo = mid;
+                    else
+                        hi = mid;
+                }
+                seg = lo;
+                s_start = segs[seg].start;
+                s_end = s_start + segs[seg].numel;
+                s_row = static_cast<const In*>(segs[seg].ptr) + (row0 + b) * segs[seg].stride;
+            }
+            const uint64_t at = f0 - s_start, left = s_end - f0;
+            const In* src = s_row + at;
+            const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 15u);
+            uint32_t x[16];  // bits of this lane's elements
+            if (live && t0 + RUN <= fts && RUN <= left && (off == 0u || (at >= V && RUN + V <= left))) {
+                // whole run inside the tile and one contiguous source, aligned vectors around it included
+                const uint4* vec = reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(src) - off) + LOADS * lane;
+                uint4 c[LOADS + 1];
+#pragma unroll
+                for (uint32_t j = 0; j < LOADS; ++j) c[j] = __ldg(vec + j);
+                if (off) {
+                    c[LOADS] = __ldg(vec + LOADS);
+#pragma unroll
+                    for (uint32_t j = 0; j < LOADS; ++j) c[j] = shift_words(c[j], c[j + 1], off);
+                }
+#pragma unroll
+                for (uint32_t j = 0; j < LOADS; ++j) {
+                    const uint32_t w[4] = {c[j].x, c[j].y, c[j].z, c[j].w};
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; ++k) {
+                        if constexpr (sizeof(In) == 4) {
+                            x[j * 4u + k] = w[k];
+                        } else {
+                            x[j * 8u + 2u * k] = w[k] & 0xffffu;
+                            x[j * 8u + 2u * k + 1u] = w[k] >> 16;
+                        }
+                    }
+                }
+            } else {
+                if (t >= nst * BITS_K) continue;
+                uint32_t si = seg;
+                uint64_t e_start = s_start, e_end = s_end;
+                const In* e_row = s_row;
+#pragma unroll
+                for (uint32_t k = 0; k < 16; ++k) {
+                    const uint64_t f = f0 + lane * 16u + k;
+                    x[k] = 0;
+                    if (b < B && t + k < fts && f < F) {
+                        while (SEG && f >= e_end) {
+                            ++si;
+                            e_start = e_end;
+                            e_end += segs[si].numel;
+                            e_row = static_cast<const In*>(segs[si].ptr) + (row0 + b) * segs[si].stride;
+                        }
+                        if constexpr (sizeof(In) == 4)
+                            x[k] = __float_as_uint(e_row[f - e_start]);
+                        else
+                            x[k] = e_row[f - e_start];
+                    }
+                }
+            }
+            // digits of 2^e x, features of even j four times as large (they meet A's 1 and 2, the others its 4 and 8)
+            uint32_t d[16];
+            int part[2] = {0, 0};  // eight values of less than 2^28 each
+#pragma unroll
+            for (uint32_t k = 0; k < 16; ++k) {
+                const bool four = ((k >> 1) & 1u) == 0u;
+                const float v = staged_value<E>(x[k]);
+                int qi;
+                if (e < BITS_INF) {
+                    qi = __float2int_rn(E == Elem::BF16 ? v * f1 * f2 : v * f1);
+                } else {
+                    qi = v == INFINITY ? 1 : v == -INFINITY ? -1 : 0;
+                    ninf += qi != 0;
+                }
+                part[k >> 3] += qi;
+                d[k] = (uint32_t)(four ? 4 * qi : qi) + 0x00808080u ^ 0x00808080u;  // bytes: balanced base-256 digits
+            }
+            sum += (long long)part[0] + part[1];
+            uint8_t* const dst = out_tile + ((size_t)(t / BITS_BOX_K) * (BITS_PLANES * rows) + b) * BITS_BOX_K + (t % BITS_BOX_K);
+            uint32_t o[BITS_PLANES][4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+                const uint32_t a0 = d[2u * j], a1 = d[2u * j + 1u], a2 = d[2u * j + 8u], a3 = d[2u * j + 9u];
+                const uint32_t l01 = __byte_perm(a0, a1, 0x5140u), h01 = __byte_perm(a0, a1, 0x7362u);
+                const uint32_t l23 = __byte_perm(a2, a3, 0x5140u), h23 = __byte_perm(a2, a3, 0x7362u);
+                o[0][j] = __byte_perm(l01, l23, 0x5410u);
+                o[1][j] = __byte_perm(l01, l23, 0x7632u);
+                o[2][j] = __byte_perm(h01, h23, 0x5410u);
+                o[3][j] = __byte_perm(h01, h23, 0x7632u);
+            }
+#pragma unroll
+            for (uint32_t pl = 0; pl < BITS_PLANES; ++pl)
+                *reinterpret_cast<uint4*>(dst + (size_t)pl * rows * BITS_BOX_K) = make_uint4(o[pl][0], o[pl][1], o[pl][2], o[pl][3]);
+        }
+        // one addition per warp to the tile's sum: integers, so their order does not matter
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0 && sum != 0)
+            atomicAdd(reinterpret_cast<unsigned long long*>(sums + (size_t)tile * rows + b), (unsigned long long)sum);
+        if (e == BITS_INF) {
+            ninf = __reduce_add_sync(0xffffffffu, ninf);
+            if (lane == 0 && ninf != 0) atomicAdd(infs + (size_t)tile * rows + b, ninf);
+        }
+    }
+}
+
+}  // namespace tb

@@ -55,7 +55,7 @@ extern "C" int tb_project_static(int device, void* stream, const void* grads, in
     int rc = tb::validate_project_args(grads, dtype, B, F, ld, out, ld_out, N, num_feature_tiles, proj_type);
     if (rc != TB_OK) return rc;
     // Shapes whose scratch does not fit the fixed array are refused up front.
-    const size_t need = tb_project_workspace_bytes(dtype, B, F, N, num_feature_tiles);
+    const size_t need = tb::project_least_bytes(B, F, N, num_feature_tiles);
     if (need > tb::STATIC_SCRATCH_BYTES) return TB_ERR_SCRATCH_LIMIT;
     // Makes `device` current and refuses anything that is not a B200-class GPU.
     rc = tb::select_device(device, nullptr);

@@ -69,6 +69,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
+// The same without the suspension that try_wait may take.
+__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // Bounded wait.  Returns false when the limit ran out or another role of the
 // CTA has already given up (abort_flag, in shared memory, non-zero).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
@@ -83,6 +96,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
             if (globaltimer_ns() - t0 > limit_ns) return false;
         }
     }
+}
+
+// The same by a converged warp, with the same answer in every lane.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    const bool got = mbar_wait(bar, parity, abort_flag);
+    return __all_sync(0xffffffffu, got);
 }
 
 // ---- TMA (plain tile loads; no cluster multicast anywhere) ------------------
@@ -142,6 +162,14 @@ __device__ __forceinline__ void tmem_st_x8(uint32_t taddr, const uint32_t (&r)[8
                  "r"(r[6]), "r"(r[7])
                  : "memory");
 }
+// The same for 16 columns.
+__device__ __forceinline__ void tmem_st_x16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+                 "%14, %15, %16};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                 "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+                 : "memory");
+}
 // One warp writes 8 consecutive 32-bit columns of 16 tensor-memory lanes: threads 0 to 15 the first four of lanes 0 to 15,
 // threads 16 to 31 the last four of the same lanes.
 __device__ __forceinline__ void tmem_st_halves_x4(uint32_t taddr, const uint32_t (&r)[4]) {
@@ -168,6 +196,14 @@ __device__ __forceinline__ void tmem_ld_x8(uint32_t taddr, uint32_t (&r)[8]) {
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
         : "r"(taddr)
         : "memory");
+}
+
+// One warp reads 4 consecutive 32-bit columns of its own 32 lanes.
+__device__ __forceinline__ void tmem_ld_x4(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr)
+                 : "memory");
 }
 
 // Fire-and-forget fp32 add (round to nearest) performed by the L2: no read comes back to the SM.
@@ -212,6 +248,16 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, ui
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// D[tmem] (+)= A[tmem] * B[smem descriptor], kind::i8 (signed bytes, exact 32-bit sums), K = 32.
+__device__ __forceinline__ void umma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                           uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
 // D[tmem] (+)= A[smem descriptor] * B[smem descriptor].
 __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                             uint32_t idesc, uint32_t accumulate) {
@@ -253,6 +299,11 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
 // K-major, M = 128, N = n (multiple of 16, 16..256).  fmt: 0 fp16, 1 bf16.
 __host__ __device__ inline uint32_t idesc_f16(uint32_t fmt, uint32_t n) {
     return (1u << 4) | (fmt << 7) | (fmt << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
+}
+
+// The same for kind::i8: signed bytes, 32-bit integer accumulation without saturation.
+__host__ __device__ inline uint32_t idesc_i8(uint32_t n) {
+    return (2u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
 
 }  // namespace tb
