@@ -603,15 +603,16 @@ struct PackRows {
     uint64_t rows, K, ld;
     uint32_t rowblocks, kblocks;
 };
-template <int W>
-__global__ void __launch_bounds__(256) pack_rows_f32_kernel(const PackRows a, const PackRows b) {
+template <int W, int THREADS = 256>
+__global__ void __launch_bounds__(THREADS) pack_rows_f32_kernel(const PackRows a, const PackRows b) {
     after_earlier_launch();
-    __shared__ uint32_t row_max[8];
+    constexpr uint32_t ROWS = THREADS / 32 / W;  // of a CTA
+    __shared__ uint32_t row_max[THREADS / 32];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, part = warp % W;
     constexpr uint32_t SPAN = W * 1024u;
     const uint64_t rows_a = (uint64_t)a.rowblocks * 128u, total = rows_a + (uint64_t)b.rowblocks * 128u;
-    for (uint64_t row0 = (uint64_t)blockIdx.x * (8u / W); row0 < total; row0 += (uint64_t)gridDim.x * (8u / W)) {
-        const uint64_t i = row0 + warp / W;  // 8 / W divides 128: a CTA's rows belong to one operand
+    for (uint64_t row0 = (uint64_t)blockIdx.x * ROWS; row0 < total; row0 += (uint64_t)gridDim.x * ROWS) {
+        const uint64_t i = row0 + warp / W;  // ROWS divides 128: a CTA's rows belong to one operand
         const bool first = i < rows_a;
         const PackRows& o = first ? a : b;
         const uint64_t R = first ? i : i - rows_a, span_k = (uint64_t)o.kblocks * 32u;
@@ -912,11 +913,27 @@ static PackRows pack_rows_args(const void* src, uint64_t rows, uint64_t K, uint6
 // and 37.5; fp32 40,000 x 100 x 512 66.5 and 67.7, 60,000 x 100 x 512 81.6 and 80.7).
 static bool pack_early(uint64_t elements) { return elements < 25'000'000u; }
 
+// A packing that runs beside an inverse (tb_gemm_nt_pack) leaves it half of the SMs: CTAs of 1024 threads, one to every
+// second SM, which still read 3.5 TB/s.  Spread over all of them it keeps the inverse's cooperative launch and its products,
+// which want whole SMs, waiting until it has ended.  get_x_xtx_inv of 50,000 x 2048 fp32 1671 -> 1638 us, 65,000 x 1024
+// 720 -> 704, 80,000 x 512 367 -> 356.
+constexpr int BESIDE_THREADS = 1024;
+static uint32_t beside_blocks(uint64_t blocks_of_256, int sm_count) {
+    return (uint32_t)std::min<uint64_t>((blocks_of_256 + 3) / 4, std::max(1, sm_count / 2));
+}
+
 // One or two fp32 operands (b.rowblocks = 0: one) whose rows are source rows.
-static int launch_pack_rows(const PackRows& a, const PackRows& b, int sm_count, cudaStream_t stream) {
+static int launch_pack_rows(const PackRows& a, const PackRows& b, int sm_count, cudaStream_t stream, bool beside = false) {
     const uint64_t K = a.K > b.K ? a.K : b.K, rows = ((uint64_t)a.rowblocks + b.rowblocks) * 128u;
     // warps per row: enough to hold it in registers, but not so many that most of their lanes idle
     const int w = K <= 1024u ? 1 : K <= 2048u ? 2 : K <= 4096u ? 4 : 8;
+    if (beside) {
+        auto kern = w == 1   ? pack_rows_f32_kernel<1, BESIDE_THREADS>
+                    : w == 2 ? pack_rows_f32_kernel<2, BESIDE_THREADS>
+                    : w == 4 ? pack_rows_f32_kernel<4, BESIDE_THREADS>
+                             : pack_rows_f32_kernel<8, BESIDE_THREADS>;
+        return launch_after(kern, beside_blocks((rows * w + 7) / 8, sm_count), BESIDE_THREADS, 0, stream, false, a, b);
+    }
     uint64_t blocks = (rows * w + 7) / 8;
     const uint64_t cap = (uint64_t)sm_count * 32;
     if (blocks > cap) blocks = cap;
@@ -946,9 +963,9 @@ Packed packed_tail(const uint16_t** packed, const Packed& g, uint32_t skip) {
 }
 
 int launch_pack(const void* src, int dtype, bool trans, uint64_t rows, uint64_t K, uint64_t ld,
-                uint16_t* packed, const Packed& g, int sm_count, cudaStream_t stream) {
+                uint16_t* packed, const Packed& g, int sm_count, cudaStream_t stream, bool beside) {
     if (dtype == TB_F32 && !trans)
-        return launch_pack_rows(pack_rows_args(src, rows, K, ld, packed, g), PackRows{}, sm_count, stream);
+        return launch_pack_rows(pack_rows_args(src, rows, K, ld, packed, g), PackRows{}, sm_count, stream, beside);
     if (dtype == TB_F32) {
         const float* s = static_cast<const float*>(src);
         uint32_t* amax = packed_amax(packed, g);
@@ -976,6 +993,9 @@ int launch_pack(const void* src, int dtype, bool trans, uint64_t rows, uint64_t 
         if (blocks > cap) blocks = cap;
         const uint32_t nb = (uint32_t)blocks;
         const uint16_t* s = static_cast<const uint16_t*>(src);
+        if (beside && !trans)
+            return launch_after(pack_kernel<false>, beside_blocks((total + 255) / 256, sm_count), BESIDE_THREADS, 0, stream, false,
+                                s, packed, rows, K, ld, g.rowblocks, g.kblocks);
         return launch_after(trans ? pack_kernel<true> : pack_kernel<false>, nb, 256, 0, stream, trans || pack_early(rows * K), s,
                             packed, rows, K, ld, g.rowblocks, g.kblocks);
     }
@@ -1162,7 +1182,7 @@ static int gemm_nt_parts(int device, void* stream_, const void* A, int64_t lda, 
         rc = launch_pack_rows(pack_rows_args(A, M, K, lda, pa, ga), pack_rows_args(B, N, K, ldb, pb, gb), sm_count, stream);
         if (rc != TB_OK) return rc;
     } else {
-        if (A && (rc = launch_pack(A, dtype, false, M, K, lda, pa, ga, sm_count, stream)) != TB_OK) return rc;
+        if (A && (rc = launch_pack(A, dtype, false, M, K, lda, pa, ga, sm_count, stream, !B)) != TB_OK) return rc;
         if (B && (rc = launch_pack(B, dtype, false, N, K, ldb, pb, gb, sm_count, stream)) != TB_OK) return rc;
     }
     if (!B) return TB_OK;

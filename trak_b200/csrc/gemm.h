@@ -21,9 +21,10 @@ inline uint32_t* packed_amax(const uint16_t* packed, const Packed& g) {
 
 Packed packed_geometry(int dtype, int64_t rows, int64_t K);
 
-// Packs `rows` x `K` operand elements from a row-major source (transposed when `trans`).
+// Packs `rows` x `K` operand elements from a row-major source (transposed when `trans`).  `beside`: on half of the SMs,
+// where the stream of an inverse waits for the others.
 int launch_pack(const void* src, int dtype, bool trans, uint64_t rows, uint64_t K, uint64_t ld,
-                uint16_t* packed, const Packed& g, int sm_count, cudaStream_t stream);
+                uint16_t* packed, const Packed& g, int sm_count, cudaStream_t stream, bool beside = false);
 
 // The same for two fp32 operands in one launch (neither transposed).
 int launch_pack_pair(const float* a, uint64_t rows_a, uint64_t K_a, uint64_t ld_a, uint16_t* packed_a, const Packed& ga,

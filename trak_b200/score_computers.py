@@ -303,7 +303,8 @@ class B200ScoreComputer:
                 with pair.stream(i):
                     blk = _as_device_matrix(block, self.device).to(inv.dtype)
                     pair.uses(blk)
-                    ready = (lambda: pair.after(inverted)) if apart else None
+                    # (a third block comes behind a product that has waited for the inverse)
+                    ready = (lambda: pair.after(inverted)) if apart and i < 2 else None
                     # the inverse is symmetric, so block @ inv == block @ inv.T
                     if result.dtype == torch.float32:
                         gemm_nt(blk, inv, out=result[rows], b_ready=ready)
