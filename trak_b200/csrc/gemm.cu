@@ -914,7 +914,7 @@ static PackRows pack_rows_args(const void* src, uint64_t rows, uint64_t K, uint6
 static bool pack_early(uint64_t elements) { return elements < 25'000'000u; }
 
 // A packing that runs beside an inverse (tb_gemm_nt_pack) leaves it half of the SMs: CTAs of 1024 threads, one to every
-// second SM, which still read 3.5 TB/s.  Spread over all of them it keeps the inverse's cooperative launch and its products,
+// second SM.  Spread over all of them it keeps the inverse's cooperative launch and its products,
 // which want whole SMs, waiting until it has ended.  get_x_xtx_inv of 50,000 x 2048 fp32 1671 -> 1638 us, 65,000 x 1024
 // 720 -> 704, 80,000 x 512 367 -> 356.
 constexpr int BESIDE_THREADS = 1024;

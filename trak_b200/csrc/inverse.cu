@@ -169,15 +169,19 @@ __global__ void prepare_kernel(float* A, int64_t lda, int k, float lambda, uint3
 //   1. the pivot warp has factored the block and published Ld^-1;
 //   2. O = Ld^-1 P: below the block the columns of L, in it and left of it the block's rows of W, final;
 //   3. the threads below update their pieces, x[i, j] -= sum_c O[c][i] O[c][j], and publish P of the next step.
-// Beside 3 the pivot warp takes the next diagonal block as it was before this step, updates it from O and factors it,
+// The pivot warp is a step ahead of the others: what it needs of step q for the next diagonal block are eight rows of O,
+// which it computes itself from P, and that block as it was before the step.  Then it factors it,
 // every lane for itself in registers (a lane then solves for one column of the inverse): a chain of eight reciprocal
-// square roots, 50 cycles each.
+// square roots, 50 cycles each.  So a step takes as long as the pivot warp's part or the others', not as both.
 // With four columns a step, a factor published instead of its inverse and substitutions by the threads of its pieces, a
-// tile took 12,500 cycles, 9,700 now (with 8 x 4 pieces in three warps 12,400:
-// half of it is stores and loads of shared memory, of which a warp gets one of 16 bytes every 14 cycles).
+// tile took 12,500 cycles (with 8 x 4 pieces in three warps 12,400: half of it is stores and loads of shared memory, of which
+// a warp gets one of 16 bytes every 14 cycles).  Every warp runs through straight code that no other warp of its scheduler
+// runs, so each piece of it is there once: with the hand-overs, the factorisation and the products of CTA 0 and of the others
+// expanded where they are used, the one-tile launch spent most of its time waiting for instructions (668 misses of the
+// instruction cache; 215 with one copy of each, and 15.3 -> 14.0 us with the pivot warp ahead).
 // Rows and columns beyond jb are an identity block.  `buf` is CHOL_FLOATS floats of shared memory outside S.
 constexpr int CW = 8;                                             // columns of a step
-constexpr int CHOL_FLOATS = 2 * CW * NB + 4 * CW * CW;
+constexpr int CHOL_FLOATS = 3 * CW * NB + 6 * CW * CW;
 static_assert(CHOL_FLOATS <= NB * TS, "a tile's worth of shared memory holds chol_block's buffers");
 constexpr int CHOL_THREADS = 192;  // warps 0 (pivot), 1, 2, 3, 5 and 6
 // 1 / sqrt(d) for a normal d; a subnormal one counts as not positive (the inverse would overflow)
@@ -207,13 +211,20 @@ __device__ __forceinline__ bool invert_block(float (&z)[CW][CW], int col, float 
     return ok;
 }
 __device__ void chol_block(const Tile& S, int jb, float* dinv, Tile& Dt, uint32_t* status, float* buf) {
-    auto sync = [] { asm volatile("barrier.cta.sync 1, %0;" ::"n"(CHOL_THREADS) : "memory"); };
+    // Barriers: 1 between the threads of the pieces; 2 and 3 (even and odd steps) hand them the step's Ld^-1, 4 and 5 hand
+    // the pivot warp the step's P.  Either side waits for the other's last hand-over before its next but one, so two of
+    // each, and two of the buffers behind them, are enough.
+    auto sync = [] { asm volatile("barrier.cta.sync 1, %0;" ::"n"(CHOL_THREADS - 32) : "memory"); };
+    auto take = [](int bar) { asm volatile("barrier.cta.sync %0, %1;" ::"r"(bar), "n"(CHOL_THREADS) : "memory"); };
+    auto give = [](int bar) { asm volatile("barrier.cta.arrive %0, %1;" ::"r"(bar), "n"(CHOL_THREADS) : "memory"); };
     const int tid = threadIdx.x, lane = tid & 31;
-    float (*P)[NB] = reinterpret_cast<float(*)[NB]>(buf);
-    float (*O)[NB] = reinterpret_cast<float(*)[NB]>(buf + CW * NB);
-    float (*inv)[CW] = reinterpret_cast<float(*)[CW]>(buf + 2 * CW * NB);  // Ld^-1 of the step
-    float* const before = buf + 2 * CW * NB + CW * CW;   // [2][CW][CW]: diagonal blocks as they were a step earlier
-    float (*now)[CW] = reinterpret_cast<float(*)[CW]>(before + 2 * CW * CW);
+    typedef float Panel[CW][NB];
+    typedef float Block[CW][CW];
+    Panel* const Ps = reinterpret_cast<Panel*>(buf);                         // P of even and odd steps
+    Panel& O = *reinterpret_cast<Panel*>(buf + 2 * CW * NB);
+    Block* const invs = reinterpret_cast<Block*>(buf + 3 * CW * NB);         // Ld^-1 of even and odd steps
+    Block* const before = invs + 2;                                          // diagonal blocks as they were a step earlier
+    Block &now = before[2], &rows_of_o = before[3];                          // the pivot warp's own
     const int warp = tid >> 5;
     const bool pivot = warp == 0;
     // piece (ty, tx) of the grid's threads, row by row: the first rows' warp, done early, shares a scheduler
@@ -239,6 +250,7 @@ __device__ void chol_block(const Tile& S, int jb, float* dinv, Tile& Dt, uint32_
     // P of step q, and the diagonal block of step q + 1 for the pivot warp
     auto publish = [&](int q) {
         const int r = ty - 2 * q, c = tx - 2 * q;  // piece row and column relative to the step's block
+        Panel& P = Ps[q & 1];
         if (c >= 0 && c < 2 && r >= 2) {
 #pragma unroll
             for (int b = 0; b < 4; ++b)
@@ -256,108 +268,123 @@ __device__ void chol_block(const Tile& S, int jb, float* dinv, Tile& Dt, uint32_
             }
         }
         if (r >= 2 && r < 4 && c >= 2) {
-            float (*d)[CW] = reinterpret_cast<float(*)[CW]>(before + ((q + 1) & 1) * CW * CW);
+            Block& d = before[(q + 1) & 1];
 #pragma unroll
             for (int a = 0; a < 4; ++a)
                 *reinterpret_cast<float4*>(&d[(r - 2) * 4 + a][(c - 2) * 4]) = make_float4(x[a][0], x[a][1], x[a][2], x[a][3]);
         }
     };
     bool ok = true;
-    float z[CW][CW], y[CW];
-    // factors z and publishes the inverse, one column per lane
-    auto factor = [&] {
-        ok = invert_block(z, lane & (CW - 1), y) && ok;
-        if (lane < CW) {
-#pragma unroll
-            for (int r = 0; r < CW; ++r) inv[r][lane] = r >= lane ? y[r] : 0.0f;
-        }
-    };
     if (pivot) {
+        float z[CW][CW], y[CW];
+        // factors z and publishes the inverse, one column per lane
+        auto factor = [&](int q) {
+            ok = invert_block(z, lane & (CW - 1), y) && ok;
+            if (lane < CW) {
 #pragma unroll
-        for (int i = 0; i < CW; ++i)
-#pragma unroll
-            for (int j = 0; j < CW; ++j) z[i][j] = j <= i ? entry(i, j) : 0.0f;
-        factor();
-    } else if (owner) {
-        publish(0);
-    }
-    for (int q = 0; q < steps; ++q) {
-        sync();
-        if (panel >= 0) {  // four entries of O each
-            const int at = panel & 63, c = (panel >> 6) * 4;
-            float o[4] = {}, v[4][CW];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                *reinterpret_cast<float4*>(&v[k][0]) = *reinterpret_cast<const float4*>(&inv[c + k][0]);
-                *reinterpret_cast<float4*>(&v[k][4]) = *reinterpret_cast<const float4*>(&inv[c + k][4]);
+                for (int r = 0; r < CW; ++r) invs[q & 1][r][lane] = r >= lane ? y[r] : 0.0f;
             }
+            __syncwarp();
+            give(2 + (q & 1));
+        };
+        for (int q = -1; q + 1 < steps; ++q) {
+            const int r = lane >> 2, c = (lane & 3) * 2, at = (q + 1) * CW;
+            float2 v = make_float2(c <= r ? entry(r, c) : 0.0f, c < r ? entry(r, c + 1) : 0.0f);
+            if (q >= 0) {
+                float w[CW];
 #pragma unroll
-            for (int d = 0; d < CW; ++d) {
-                const float p = P[d][at];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) o[k] = fmaf(v[k][d], p, o[k]);
-            }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) O[c + k][at] = o[k];
-        }
-        sync();
-        if (pivot) {
-            if (q + 1 < steps) {
-                const float (*d)[CW] = reinterpret_cast<const float(*)[CW]>(before + ((q + 1) & 1) * CW * CW);
-                const int r = lane >> 2, c = (lane & 3) * 2, at = (q + 1) * CW;
-                float2 v = *reinterpret_cast<const float2*>(&d[r][c]), m[CW];
+                for (int d = 0; d < CW; d += 4) {
+                    const float4 t = *reinterpret_cast<const float4*>(&invs[q & 1][r][d]);
+                    w[d] = t.x; w[d + 1] = t.y; w[d + 2] = t.z; w[d + 3] = t.w;
+                }
+                take(4 + (q & 1));
+                float2 o = make_float2(0.0f, 0.0f), m[CW];
                 float l[CW];
+                v = *reinterpret_cast<const float2*>(&before[(q + 1) & 1][r][c]);
+#pragma unroll
+                for (int d = 0; d < CW; ++d) {
+                    const float2 p = *reinterpret_cast<const float2*>(&Ps[q & 1][d][at + c]);
+                    o.x = fmaf(w[d], p.x, o.x);
+                    o.y = fmaf(w[d], p.y, o.y);
+                }
+                *reinterpret_cast<float2*>(&rows_of_o[r][c]) = o;
+                __syncwarp();
 #pragma unroll
                 for (int k = 0; k < CW; ++k) {
-                    l[k] = O[k][at + r];
-                    m[k] = *reinterpret_cast<const float2*>(&O[k][at + c]);
+                    l[k] = rows_of_o[k][r];
+                    m[k] = *reinterpret_cast<const float2*>(&rows_of_o[k][c]);
                 }
 #pragma unroll
                 for (int k = 0; k < CW; ++k) {
                     v.x = fmaf(-l[k], m[k].x, v.x);
                     v.y = fmaf(-l[k], m[k].y, v.y);
                 }
-                *reinterpret_cast<float2*>(&now[r][c]) = v;
-                __syncwarp();
+            }
+            *reinterpret_cast<float2*>(&now[r][c]) = v;
+            __syncwarp();
 #pragma unroll
-                for (int i = 0; i < CW; ++i)
+            for (int i = 0; i < CW; ++i)
 #pragma unroll
-                    for (int j = 0; j < CW; j += 4) {
-                        if (j > i) continue;
-                        const float4 w = *reinterpret_cast<const float4*>(&now[i][j]);
-                        z[i][j] = w.x; z[i][j + 1] = w.y; z[i][j + 2] = w.z; z[i][j + 3] = w.w;
+                for (int j = 0; j < CW; j += 4) {
+                    if (j > i) continue;
+                    const float4 t = *reinterpret_cast<const float4*>(&now[i][j]);
+                    z[i][j] = t.x; z[i][j + 1] = t.y; z[i][j + 2] = t.z; z[i][j + 3] = t.w;
+                }
+            factor(q + 1);
+        }
+    } else {
+        for (int q = 0; q < steps; ++q) {
+            if (owner) publish(q);
+            if (q + 1 < steps) give(4 + (q & 1));
+            take(2 + (q & 1));
+            if (panel >= 0) {  // four entries of O each
+                const Block& inv = invs[q & 1];
+                const Panel& P = Ps[q & 1];
+                const int at = panel & 63, c = (panel >> 6) * 4;
+                float o[4] = {}, v[4][CW];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    *reinterpret_cast<float4*>(&v[k][0]) = *reinterpret_cast<const float4*>(&inv[c + k][0]);
+                    *reinterpret_cast<float4*>(&v[k][4]) = *reinterpret_cast<const float4*>(&inv[c + k][4]);
+                }
+#pragma unroll
+                for (int d = 0; d < CW; ++d) {
+                    const float p = P[d][at];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) o[k] = fmaf(v[k][d], p, o[k]);
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) O[c + k][at] = o[k];
+            }
+            sync();
+            if (owner) {
+                const int r = ty - 2 * q, c = tx - 2 * q;
+                if (r >= 0 && r < 2) {  // the step's rows of W
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) {
+                        const float4 w = *reinterpret_cast<const float4*>(&O[r * 4 + a][tx * 4]);
+                        x[a][0] = w.x; x[a][1] = w.y; x[a][2] = w.z; x[a][3] = w.w;
                     }
-                factor();
-            }
-            continue;
-        }
-        if (!owner) continue;
-        const int r = ty - 2 * q, c = tx - 2 * q;
-        if (r >= 0 && r < 2) {  // the step's rows of W
+                } else if (r >= 2) {
+                    if (c >= 0 && c < 2) {  // from S, which has become L, to W
 #pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                const float4 w = *reinterpret_cast<const float4*>(&O[r * 4 + a][tx * 4]);
-                x[a][0] = w.x; x[a][1] = w.y; x[a][2] = w.z; x[a][3] = w.w;
-            }
-        } else if (r >= 2) {
-            if (c >= 0 && c < 2) {  // from S, which has become L, to W
+                        for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int a = 0; a < 4; ++a)
+                            for (int b = 0; b < 4; ++b) x[a][b] = 0.0f;
+                    }
 #pragma unroll
-                    for (int b = 0; b < 4; ++b) x[a][b] = 0.0f;
-            }
+                    for (int k = 0; k < CW; ++k) {
+                        const float4 l = *reinterpret_cast<const float4*>(&O[k][ty * 4]);
+                        const float4 o = *reinterpret_cast<const float4*>(&O[k][tx * 4]);
+                        const float lv[4] = {l.x, l.y, l.z, l.w}, ov[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
-            for (int k = 0; k < CW; ++k) {
-                const float4 l = *reinterpret_cast<const float4*>(&O[k][ty * 4]);
-                const float4 o = *reinterpret_cast<const float4*>(&O[k][tx * 4]);
-                const float lv[4] = {l.x, l.y, l.z, l.w}, ov[4] = {o.x, o.y, o.z, o.w};
+                        for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int a = 0; a < 4; ++a)
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) x[a][b] = fmaf(-lv[a], ov[b], x[a][b]);
+                            for (int b = 0; b < 4; ++b) x[a][b] = fmaf(-lv[a], ov[b], x[a][b]);
+                    }
+                }
             }
         }
-        if (q + 1 < steps) publish(q + 1);
     }
     if (owner) {
         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -474,15 +501,17 @@ __device__ bool block_tile(float* smem, const float* X, int64_t ldx, float* Y, f
     d.put<true>(tid, Dt);
     if (c == j) d.put<false>(tid, T2);
     __syncthreads();
-    // P_i^T = D S[i, j]^T, i.e. P_i t-major
-    tile_mma(Dt, T1, exchange, acc);
-    put_piece(T0, ty, tx, acc);
-    if (c != i && c != j) {  // the other operand, P_c^T or W[j, c], over T1 (the product above is done with it)
-        tile_mma(Dt, T2, exchange, acc);
-        put_piece(T1, ty, tx, acc);
+    // P_i^T = D S[i, j]^T, i.e. P_i t-major, into T0; the other operand, P_c^T or W[j, c], into T1 (the product before is done
+    // with it); then the product of the two
+    const int last = c != i && c != j ? 2 : 1;
+#pragma unroll 1
+    for (int product = 0;; ++product) {
+        tile_mma(product == last ? T0 : Dt,
+                 product == 0 ? T1 : product < last ? T2 : c == i ? T0 : c == j ? T2 : T1, exchange, acc);
+        if (product == last) break;
+        put_piece(product == 0 ? T0 : T1, ty, tx, acc);
+        __syncthreads();
     }
-    __syncthreads();
-    tile_mma(T0, c == i ? T0 : c == j ? T2 : T1, exchange, acc);
 #pragma unroll
     for (int a = 0; a < 4; ++a)
         *reinterpret_cast<float4*>(Y + (int64_t)(i * NB + ty * 4 + a) * OUTER + c * NB + tx * 4) =
@@ -505,8 +534,8 @@ __device__ __forceinline__ void announce(uint32_t* counter) {
 // left them a step earlier) and goes on, without waiting for anyone unless the others fall behind.  They wait for a tile's
 // inverse, share the step's tiles and wait for one another.  A cooperative launch of about as many CTAs as the largest step
 // has tiles.  With one meeting point of all CTAs per step, CTA 0's tiles fetched behind it and the slower products and
-// factorisation of before, the 512-wide block took 126 us; 97 after that, and 88 with what a tile needs of the step before
-// fetched while its inverse is waited for.
+// factorisation of before, the 512-wide block took 126 us; 97 after that, 89.3 with what a tile needs of the step before
+// fetched while its inverse is waited for, and 86.8 with one copy of the products' code and chol_block as it is.
 constexpr int STEP_THREADS = 256;
 constexpr size_t STEP_SMEM = (5 * NB * TS + EXCHANGE_FLOATS + CHOL_FLOATS) * sizeof(float);
 __global__ void __launch_bounds__(STEP_THREADS, 1) block_kernel(float* block, int64_t lda, int kb, float* blocks, float* dinv,
@@ -555,10 +584,12 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) block_kernel(float* block, in
             announce(&counters->factored);
             if (j + 1 == nt || !*const_cast<volatile uint32_t*>(&proceed)) return;
             float acc[4][4];
-            tile_mma(Dt, T1, exchange, acc);  // P^T
-            put_piece(T0, ty, tx, acc);
-            __syncthreads();
-            tile_mma(T0, T0, exchange, acc);
+#pragma unroll 1
+            for (int product = 0; product < 2; ++product) {  // P^T, then what it takes off
+                tile_mma(product ? T0 : Dt, product ? T0 : T1, exchange, acc);
+                if (product == 0) put_piece(T0, ty, tx, acc);
+                __syncthreads();
+            }
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
                 const float4 v = *reinterpret_cast<const float4*>(&next[ty * 4 + a][tx * 4]);
