@@ -232,7 +232,7 @@ int tb_finalize_scores(int device, void *stream, const float *score_sum, int64_t
  * e.g. a plugin in a process whose device memory already belongs to another
  * component's pool, or a serving loop that must avoid the device-wide
  * synchronisation of cudaMalloc / cudaFree.  The call allocates neither device nor
- * pinned host memory (the process's first tb_stream_status takes 8 KB of the latter).
+ * pinned host memory (the process's first tb_stream_status takes a page of the latter).
  *
  *   - shapes with tb_project_workspace_bytes(...) > TB_PROJECT_STATIC_SCRATCH_BYTES
  *     are refused with TB_ERR_SCRATCH_LIMIT

@@ -413,3 +413,17 @@ def test_empty_row_block_contributes_a_zero_gram(cuda):
     feats = sc.get_x_xtx_inv(X, gram)
     ref = br.x_xtx_inv(X.float(), br.xtx(X.float()), 1.0)
     assert feats.dtype == torch.float32 and rel(feats, ref) <= 1e-4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,N,K", [(1, 5, 31), (127, 64, 1024), (129, 200, 1025), (300, 130, 2049), (1000, 7, 4097), (20_000, 96, 100)])
+def test_operand_packed_beside_an_inverse_gives_the_bits_of_the_plain_product(cuda, M, N, K, dtype):
+    """b_ready lays a out with CTAs of 1024 threads: one, two, four and eight warps to a row, partial rows and row blocks."""
+    from trak_b200 import score_computers as scm
+    gen = torch.Generator().manual_seed(K)
+    a = torch.randn(M, K, generator=gen).to(dtype).to(cuda)
+    b = torch.randn(N, K, generator=gen).to(dtype).to(cuda)
+    called = []
+    got = scm.gemm_nt(a, b, b_ready=lambda: called.append(1))
+    assert called == [1] and torch.equal(got, scm.gemm_nt(a, b))

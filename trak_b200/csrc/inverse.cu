@@ -403,7 +403,7 @@ __device__ void chol_block(const Tile& S, int jb, float* dinv, Tile& Dt, uint32_
         for (int b = 0; b < 4; ++b)
             *reinterpret_cast<float4*>(&Dt[tx * 4 + b][ty * 4]) = make_float4(x[0][b], x[1][b], x[2][b], x[3][b]);
     }
-    if (!ok) atomicCAS(status, 0u, (uint32_t)ST_NOT_SPD);
+    if (!ok) record_status(status, (uint32_t)ST_NOT_SPD);
 }
 
 // Counters of a block column: `factored` tiles of the diagonal (CTA 0), and steps x CTAs finished by the others.
@@ -418,7 +418,7 @@ __device__ bool reached(const uint32_t* counter, uint32_t target, uint32_t* stat
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
         if (seen >= target) return true;
         if ((n & 255u) == 0 && globaltimer_ns() - t0 > WAIT_LIMIT_NS) {
-            if (atomicCAS(status, 0u, (uint32_t)ST_TIMEOUT_ACC) == 0u) status[1] = blockIdx.x;
+            if (record_status(status, (uint32_t)ST_TIMEOUT_ACC)) status[1] = blockIdx.x;
             return false;
         }
     }

@@ -67,7 +67,7 @@ extern "C" int tb_project_static(int device, void* stream, const void* grads, in
     // partial sums) is written earlier in the same call, so nothing has to start at zero
     // and the previous call's leftovers are harmless.
     // No status word is published: that takes a word of pinned host memory, and this call allocates none.  A
-    // tb_stream_status after it reads the word with a launch of its own.
+    // tb_stream_status after it reads what the kernels repeat to the host (record_status).
     return tb::project_dense(device, stream, grads, dtype, B, F, ld, out, ld_out, N, seed, num_feature_tiles,
                              proj_type, alpha, accumulate, scratch, tb::STATIC_SCRATCH_BYTES, false);
 }

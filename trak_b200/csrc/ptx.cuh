@@ -21,6 +21,20 @@ enum : uint32_t {
 
 constexpr uint64_t WAIT_LIMIT_NS = 4000000000ull;  // 4 s per wait
 
+// The status words of a device: [0] code, [1] CTA, [2] detail, and behind them the address of a word of mapped host memory
+// that repeats the code (0: there is none yet, see tb_stream_status).
+constexpr uint32_t STATUS_MIRROR = 4;  // a 64-bit address at this word
+constexpr uint32_t STATUS_LEN = 6;
+
+// Records `code`; true for the first since the words were cleared.
+__device__ __forceinline__ bool record_status(uint32_t* status, uint32_t code) {
+    const bool first = atomicCAS(status, 0u, code) == 0u;
+    __threadfence();  // whoever sets the address afterwards sees the code
+    const uint64_t mirror = *reinterpret_cast<const volatile uint64_t*>(status + STATUS_MIRROR);
+    if (mirror) *reinterpret_cast<volatile uint32_t*>(mirror) = code;
+    return first;
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
