@@ -86,10 +86,11 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
     constexpr uint32_t SLOT = 2u * BITS_K / 4u;                     // tensor-memory columns of a slot
     static_assert(A_COL0 + NG * SA * SLOT <= TMEM_COLS, "too many generator groups for the TMEM ring");
     extern __shared__ uint8_t smem_raw[];
-    __shared__ alignas(16) uint64_t bar_full_a[NG][SA];
-    __shared__ alignas(16) uint64_t bar_empty_a[NG][SA];
-    __shared__ uint64_t bar_full_b[NG][2];
-    __shared__ uint64_t bar_empty_b[NG][2];
+    // a slot of every group, and the boxes of every group, are handed over together
+    __shared__ alignas(16) uint64_t bar_full_a[SA];
+    __shared__ alignas(16) uint64_t bar_empty_a[SA];
+    __shared__ uint64_t bar_full_b[2];
+    __shared__ uint64_t bar_empty_b[2];
     __shared__ uint64_t bar_acc;
     __shared__ uint32_t tmem_slot;
     __shared__ uint32_t abort_word;
@@ -104,13 +105,12 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
     const uint32_t ntile = min(p.tiles_per_bundle, p.tiles - tile0);
 
     if (threadIdx.x == 0) {
-        for (int g = 0; g < NG; ++g)
-            for (uint32_t s = 0; s < 2u; ++s) {
-                mbar_init(smem_u32(&bar_full_a[g][s]), GW);
-                mbar_init(smem_u32(&bar_empty_a[g][s]), 1);
-                mbar_init(smem_u32(&bar_full_b[g][s]), 1);
-                mbar_init(smem_u32(&bar_empty_b[g][s]), 1);
-            }
+        for (uint32_t s = 0; s < 2u; ++s) {
+            mbar_init(smem_u32(&bar_full_a[s]), GW * NG);
+            mbar_init(smem_u32(&bar_empty_a[s]), 1);
+            mbar_init(smem_u32(&bar_full_b[s]), 1);
+            mbar_init(smem_u32(&bar_empty_b[s]), 1);
+        }
         mbar_init(smem_u32(&bar_acc), 1);
         abort_word = 0;
         fence_mbar_init();
@@ -131,7 +131,7 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
         const uint32_t stream_col = blockIdx.x * 256u + 2u * (pair & ~15u) + (pair & 15u);
         const uint32_t lane_base = (q * 32u) << 16;
         const uint32_t a_base = tmem_base + lane_base + A_COL0 + g * (SA * SLOT);
-        const uint32_t full = smem_u32(&bar_full_a[g][0]), empty = smem_u32(&bar_empty_a[g][0]);
+        const uint32_t full = smem_u32(&bar_full_a[0]), empty = smem_u32(&bar_empty_a[0]);
         bool ok = true;
         uint32_t n = 0;  // slots this group has filled
         for (uint32_t ti = g; ti < ntile && ok; ti += NG) {
@@ -159,6 +159,13 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
                 __syncwarp();
                 if (lane == 0) mbar_arrive(full + slot * 8u);
             }
+        }
+        // the rounds that the first groups still walk a tile in: the slots change hands without this one
+        for (const uint32_t all = ((ntile + NG - 1u) / NG) * p.nst; ok && n < all; ++n) {
+            const uint32_t slot = n & 1u;
+            ok = mbar_wait_warp(empty + slot * 8u, (~n >> 1) & 1u, abort_flag);
+            if (!ok && lane == 0) fail(p.status, abort_flag, ST_TIMEOUT_EMPTY, 0x4000u | (g << 16));
+            if (ok && lane == 0) mbar_arrive(full + slot * 8u);
         }
         // ---- the exact integer result of this CTA, as fp32 ----
         if (ok && !mbar_wait_warp(smem_u32(&bar_acc), 0u, abort_flag)) {
@@ -241,17 +248,19 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
                 }
                 for (uint32_t it = 0, n = 0; it < maxcnt && ok; it += BITS_BATCH, ++n) {
                     const uint32_t slot = n & 1u, parity = (~n >> 1) & 1u;
+                    if (!mbar_wait(smem_u32(&bar_empty_b[slot]), parity, abort_flag)) {
+                        fail(p.status, abort_flag, ST_TIMEOUT_EMPTY, 0x8000u | it);
+                        ok = false;
+                        break;
+                    }
+                    uint32_t loads = 0;
+#pragma unroll
+                    for (int g = 0; g < NG; ++g) loads += it < cnt[g] ? min(BITS_BATCH, cnt[g] - it) / 2u : 0u;
+                    const uint32_t bar = smem_u32(&bar_full_b[slot]);
+                    mbar_expect_tx(bar, loads * box_bytes);
 #pragma unroll
                     for (int g = 0; g < NG; ++g) {
-                        if (it >= cnt[g]) continue;
-                        if (!mbar_wait(smem_u32(&bar_empty_b[g][slot]), parity, abort_flag)) {
-                            fail(p.status, abort_flag, ST_TIMEOUT_EMPTY, 0x8000u | (g << 16) | it);
-                            ok = false;
-                            break;
-                        }
-                        const uint32_t bar = smem_u32(&bar_full_b[g][slot]), loads = min(BITS_BATCH, cnt[g] - it) / 2u;
-                        mbar_expect_tx(bar, loads * box_bytes);
-                        for (uint32_t j = 0; j < loads; ++j) {
+                        for (uint32_t j = 0; j < BITS_BATCH / 2u && it + 2u * j < cnt[g]; ++j) {
                             tma_load_2d(smem_base + ((g * 2u + slot) * (BITS_BATCH / 2u) + j) * box_bytes, &tmap, 0,
                                         (int)((tile[g] * boxes + s[g]) * brows), bar);
                             if (++s[g] == boxes) {
@@ -271,36 +280,38 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
             uint32_t started = 0;
             for (uint32_t it = 0, n = 0; it < maxcnt && ok; it += BITS_BATCH, ++n) {
                 const uint32_t bslot = n & 1u, bparity = (n >> 1) & 1u;
+                if (!mbar_wait_warp(smem_u32(&bar_full_b[bslot]), bparity, abort_flag)) {
+                    if (leader) fail(p.status, abort_flag, ST_TIMEOUT_FULL_B, it);
+                    ok = false;
+                    break;
+                }
 #pragma unroll
                 for (uint32_t j = 0; j < BITS_BATCH; ++j) {
+                    if (it + j >= maxcnt || !ok) continue;
+                    if (!mbar_wait_warp(smem_u32(&bar_full_a[j & 1u]), (j >> 1) & 1u, abort_flag)) {
+                        if (leader) fail(p.status, abort_flag, ST_TIMEOUT_FULL_A, it);
+                        ok = false;
+                        continue;
+                    }
+                    tc_fence_after();
+                    if (leader) {
 #pragma unroll
-                    for (int g = 0; g < NG; ++g) {
-                        if (it + j >= cnt[g] || !ok) continue;
-                        if (j == 0 && !mbar_wait_warp(smem_u32(&bar_full_b[g][bslot]), bparity, abort_flag)) {
-                            if (leader) fail(p.status, abort_flag, ST_TIMEOUT_FULL_B, (g << 16) | it);
-                            ok = false;
-                            continue;
-                        }
-                        if (!mbar_wait_warp(smem_u32(&bar_full_a[g][j & 1u]), (j >> 1) & 1u, abort_flag)) {
-                            if (leader) fail(p.status, abort_flag, ST_TIMEOUT_FULL_A, (g << 16) | it);
-                            ok = false;
-                            continue;
-                        }
-                        tc_fence_after();
-                        const uint32_t a_addr = tmem_base + A_COL0 + (g * SA + (j & 1u)) * SLOT;
-                        const uint64_t b_desc =
-                            smem_desc_k_sw128(smem_base + ((g * 2u + bslot) * (BITS_BATCH / 2u) + j / 2u) * box_bytes) + 4u * (j & 1u);
-                        if (leader) {
-                            umma_i8_ts(tmem_base, a_addr, b_desc, p.idesc, started);
-                            umma_i8_ts(tmem_base + brows, a_addr + SLOT / 2u, b_desc, p.idesc, started);
+                        for (int g = 0; g < NG; ++g) {
+                            if (it + j >= cnt[g]) continue;
+                            const uint32_t a_addr = tmem_base + A_COL0 + (g * SA + (j & 1u)) * SLOT;
+                            const uint64_t b_desc =
+                                smem_desc_k_sw128(smem_base + ((g * 2u + bslot) * (BITS_BATCH / 2u) + j / 2u) * box_bytes) + 4u * (j & 1u);
+                            const uint32_t acc = started | (uint32_t)(g > 0);
+                            umma_i8_ts(tmem_base, a_addr, b_desc, p.idesc, acc);
+                            umma_i8_ts(tmem_base + brows, a_addr + SLOT / 2u, b_desc, p.idesc, acc);
                             // 32 features further: 8 TMEM columns, 32 bytes inside the swizzle row
                             umma_i8_ts(tmem_base, a_addr + 8u, b_desc + 2u, p.idesc, 1u);
                             umma_i8_ts(tmem_base + brows, a_addr + SLOT / 2u + 8u, b_desc + 2u, p.idesc, 1u);
-                            tc_commit(smem_u32(&bar_empty_a[g][j & 1u]));
-                            if (j + 1 == BITS_BATCH) tc_commit(smem_u32(&bar_empty_b[g][bslot]));
                         }
-                        started = 1u;
+                        tc_commit(smem_u32(&bar_empty_a[j & 1u]));
+                        if (j + 1 == BITS_BATCH) tc_commit(smem_u32(&bar_empty_b[bslot]));
                     }
+                    started = 1u;
                 }
             }
             if (ok && leader) tc_commit(smem_u32(&bar_acc));
