@@ -1,4 +1,4 @@
-"""Rademacher batches of up to 16 rows on the integer tensor cores, against the fp64 oracle.
+"""Rademacher batches of up to 32 rows on the integer tensor cores, against the fp64 oracle.
 
 Their sums are exact up to one rounding per partial: at most 148 partials, each rounded to fp32 once and added up in fp32,
 are within (1 + sqrt(148)) * 2^-24 < 1e-6 of the row's norm.  Elements below 2^-17 of their row's largest are rounded to
@@ -51,6 +51,8 @@ def test_route_and_workspace():
     def bits(*a):  # an odd number of stages is rounded up only here
         return grid(*a)["stages"] % 2 == 0 and grid(*a)["chain"] == grid(*a)["stages"]
     assert bits(16, 592_003, 512) and bits(1, 592_003, 512)
+    assert bits(24, 330_003, 1536) and not bits(24, 310_003, 1536) and not bits(24, 990_003, 1024)
+    assert bits(32, 782_003, 1536) and not bits(32, 780_003, 1536) and not bits(33, 1_990_003, 1536)
     assert not bits(17, 592_003, 512) and not bits(16, 572_003, 512)
     assert bits(16, 64 * 32_767, 512, 1) and not bits(16, 64 * 32_769, 512, 1)
     for F, T in ((64 * 32_767, 1), (40_000_000, 20), (124_439_808, 148), (300_000_000, 148)):
@@ -73,6 +75,11 @@ def test_route_and_workspace():
     (5, 18_945, 16_384, 148),     # the last tile is short
     (16, 2_097_088, 512, 1),      # one tile, as long as 32-bit sums allow
     (3, 131, 2_300_416, 7),
+    (17, 330_003, 1536, 148),     # from here on four groups to a CTA, one CTA per SM
+    (24, 40_009, 12_800, 148),    # a box and a half per tile: the half is padding
+    (25, 782_003, 1536, 147),     # a last bundle of fewer tiles than groups
+    (32, 590_017, 2048, 3),       # fewer tiles than groups
+    (20, 219, 2_300_416, 7),
 ])
 def test_parity(cuda, B, F, N, T, dt):
     g = torch.randn(B, F, generator=torch.Generator().manual_seed(F)).mul_(1e-2).to(DT[dt])

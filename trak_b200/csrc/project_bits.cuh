@@ -1,6 +1,6 @@
 // Rademacher projection of small batches on the integer tensor cores.
 //
-// Up to 16 rows the projection costs what its matrix costs to generate, and with a 16-bit operand most of that is not
+// A small batch costs what its matrix costs to generate, and with a 16-bit operand most of that is not
 // XORWOW (7 instructions a draw) but turning 16 signs into 8 words of +-1.  Here the operand is made of bytes and the
 // draw's own bits are its values: one AND with 0x01010101 << i leaves four matrix entries as 0 or 2^i, and
 //     sum_f (+-1) q_f  =  2 sum_{f: bit set} q_f  -  sum_f q_f
@@ -15,15 +15,19 @@
 //   * 2^i differs from word to word (bit 2j + h of a draw's byte: feature pair j, column parity h; two of the four j after
 //     a shift by four).  The column's factor 2^h is undone at the end, the features' 2^(2 (j & 1)) in the staging: even j are
 //     staged four times as large.
-//   * What bounds it: the integer pipe, 82 % busy with 11 instructions per 16 x 32 entries (4 of the 7 of a draw, 5 to spread
-//     it, 2 of hand-shakes; 35 instructions in all with a 16-bit operand, now 18), beside MMAs that keep the tensor pipe half
-//     busy.  16 rows, us a call, 16-bit operand -> this: 2,796,202 fp16 features -> 4096 1021 -> 639, 1,000,003 -> 8192
-//     732 -> 444, 40,000,001 bf16 -> 8192 27,750 -> 16,120; one row of 1,000,003 -> 2048 202 -> 131.  From 17 rows on the
-//     four planes make the MMAs the bound and the gain goes.
-//     Measured and dropped: four groups to a CTA (1.4 to 1.6 times as long: one warp issues 16 MMAs a round, each slot of
-//     which costs it 130 cycles of MMAs, 60 of waiting and 20 of commit), one slot a group (773 against 692 us), the next
-//     slots' barriers polled between MMAs (789), shifts as multiplications (no change; by the upper half of a product 3 %
-//     slower), the hand-over of a slot behind the next one's first chunk (no change).
+//   * What bounds it.  Up to 16 rows the integer pipe, 90 % busy with 11 instructions per 16 x 32 entries (4 of the 7 of a draw,
+//     5 to spread it, 2 of hand-shakes; 35 instructions in all with a 16-bit operand, now 18): without its MMAs the kernel takes
+//     95 % of its time.  us a call, 16-bit operand -> this: 2,796,202 fp16 features -> 4096 1021 -> 625, 1,000,003 -> 8192
+//     732 -> 435, 40,000,001 bf16 -> 8192 27,750 -> 15,800; one row of 1,000,003 -> 2048 202 -> 128.
+//     From 17 to 32 rows the accumulators leave room for one CTA per SM, of four groups, and the digit planes' way from the L2
+//     bounds it (8 TB/s at 32 rows): 17 rows x 1,000,003 bf16 -> 8192 780 -> 567, 24 rows fp16 -> 2048 239 -> 202, 32 rows x
+//     2,796,202 -> 4096 1111 -> 930.
+//   * The groups' slots change hands together, and so do their boxes: one warp issues the MMAs beside busy generators, and a
+//     hand-over costs it some 300 cycles whatever it covers.  With barriers of each group's own 16 rows took 2 % longer (659
+//     us for 647), and four groups of 32-feature slots to a CTA 1023 us; with common ones 693, so two of 64 they stay.
+//     Measured and dropped: one slot a group (773 against 692 us), the next slots' barriers polled between MMAs (789), shifts
+//     as multiplications (no change; by the upper half of a product 3 % slower), the hand-over of a slot behind the next one's
+//     first chunk (no change), a loop over pairs of slots with fixed addresses (no change).
 //   * A row with an infinity or a NaN (seen by absmax_kernel) is staged as the signs of its infinities; the CTA compares
 //     their signed sum with their number and writes what the sum of the row would be, +-inf or NaN.
 //
@@ -35,10 +39,12 @@ namespace tb {
 constexpr uint32_t BITS_K = 64;               // features per operand slot (a stage)
 constexpr uint32_t BITS_BOX_K = 128;          // features per box of the staged gradients (128 bytes a row)
 constexpr uint32_t BITS_PLANES = 4;           // base-256 digits of a staged gradient
-constexpr int BITS_NG = 2;                    // generator groups of a CTA
-constexpr uint32_t BITS_MAX_ROWS = 16;        // rows per launch
+constexpr uint32_t BITS_MAX_ROWS = 32;        // rows per launch
 constexpr uint32_t BITS_MAX_CHAIN = 32768;    // stages of a CTA: |digit| <= 128, A <= 8, so 2^31 / 1024 features
-constexpr uint32_t BITS_BATCH = 4;            // stages of gradients that arrive and are released together; a group has room for two
+// The two shapes: up to 16 rows two groups to a CTA and two CTAs to an SM, up to 32 rows four groups and one; and the stages of
+// gradients that arrive and are released together, of which a group has room for two.
+__host__ __device__ constexpr uint32_t bits_groups(uint32_t rows) { return rows <= 16u ? 2u : 4u; }
+__host__ __device__ constexpr uint32_t bits_batch(uint32_t rows) { return rows <= 16u ? 4u : 2u; }
 constexpr uint32_t BITS_MAX_SLICES = 256;     // of a row in absmax_kernel
 constexpr int BITS_INF = 0x7ffffffe, BITS_NAN = 0x7fffffff;   // BitsParams::row_exp of a row that holds one
 
@@ -75,14 +81,16 @@ __device__ __forceinline__ float scale_by(float v, int e) {
     return v * __int_as_float((127 + a) << 23) * __int_as_float((127 + b) << 23);
 }
 
-// One CTA: 256 output columns (two accumulators) x up to 16 rows x a bundle of feature tiles, two CTAs per SM.  Roles, rings
-// and hand-shakes are those of project_kernel with two accumulators; what differs is the operand, the digit planes beside one
-// another in the N dimension (rows x 4), and that the accumulators are read once, at the end.
-template <int NG>
-__global__ void __launch_bounds__((4 * NG + 2) * 32, 2)
+// One CTA: 256 output columns (two accumulators) x up to ROWS rows x a bundle of feature tiles.  Roles and rings are those of
+// project_kernel with two accumulators; what differs is the operand, the digit planes beside one another in the N dimension
+// (rows x 4), the common hand-shakes, and that the accumulators are read once, at the end.
+template <uint32_t ROWS>
+__global__ void __launch_bounds__((4 * bits_groups(ROWS) + 2) * 32, ROWS <= 16 ? 2 : 1)
 project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p) {
-    constexpr uint32_t GW = 4u, TMEM_COLS = 256u, SA = 2u;
-    constexpr uint32_t A_COL0 = 2u * BITS_PLANES * BITS_MAX_ROWS;   // accumulators, then the generated-operand ring
+    constexpr int NG = bits_groups(ROWS);
+    constexpr uint32_t BATCH = bits_batch(ROWS);
+    constexpr uint32_t GW = 4u, TMEM_COLS = ROWS <= 16u ? 256u : 512u, SA = 2u;
+    constexpr uint32_t A_COL0 = 2u * BITS_PLANES * ROWS;            // accumulators, then the generated-operand ring
     constexpr uint32_t SLOT = 2u * BITS_K / 4u;                     // tensor-memory columns of a slot
     static_assert(A_COL0 + NG * SA * SLOT <= TMEM_COLS, "too many generator groups for the TMEM ring");
     extern __shared__ uint8_t smem_raw[];
@@ -246,7 +254,7 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
                     tile[g] = tile0 + g;
                     s[g] = 0;
                 }
-                for (uint32_t it = 0, n = 0; it < maxcnt && ok; it += BITS_BATCH, ++n) {
+                for (uint32_t it = 0, n = 0; it < maxcnt && ok; it += BATCH, ++n) {
                     const uint32_t slot = n & 1u, parity = (~n >> 1) & 1u;
                     if (!mbar_wait(smem_u32(&bar_empty_b[slot]), parity, abort_flag)) {
                         fail(p.status, abort_flag, ST_TIMEOUT_EMPTY, 0x8000u | it);
@@ -255,13 +263,13 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
                     }
                     uint32_t loads = 0;
 #pragma unroll
-                    for (int g = 0; g < NG; ++g) loads += it < cnt[g] ? min(BITS_BATCH, cnt[g] - it) / 2u : 0u;
+                    for (int g = 0; g < NG; ++g) loads += it < cnt[g] ? min(BATCH, cnt[g] - it) / 2u : 0u;
                     const uint32_t bar = smem_u32(&bar_full_b[slot]);
                     mbar_expect_tx(bar, loads * box_bytes);
 #pragma unroll
                     for (int g = 0; g < NG; ++g) {
-                        for (uint32_t j = 0; j < BITS_BATCH / 2u && it + 2u * j < cnt[g]; ++j) {
-                            tma_load_2d(smem_base + ((g * 2u + slot) * (BITS_BATCH / 2u) + j) * box_bytes, &tmap, 0,
+                        for (uint32_t j = 0; j < BATCH / 2u && it + 2u * j < cnt[g]; ++j) {
+                            tma_load_2d(smem_base + ((g * 2u + slot) * (BATCH / 2u) + j) * box_bytes, &tmap, 0,
                                         (int)((tile[g] * boxes + s[g]) * brows), bar);
                             if (++s[g] == boxes) {
                                 s[g] = 0;
@@ -278,7 +286,7 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
             const bool leader = elect_one();
             bool ok = true;
             uint32_t started = 0;
-            for (uint32_t it = 0, n = 0; it < maxcnt && ok; it += BITS_BATCH, ++n) {
+            for (uint32_t it = 0, n = 0; it < maxcnt && ok; it += BATCH, ++n) {
                 const uint32_t bslot = n & 1u, bparity = (n >> 1) & 1u;
                 if (!mbar_wait_warp(smem_u32(&bar_full_b[bslot]), bparity, abort_flag)) {
                     if (leader) fail(p.status, abort_flag, ST_TIMEOUT_FULL_B, it);
@@ -286,9 +294,9 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
                     break;
                 }
 #pragma unroll
-                for (uint32_t j = 0; j < BITS_BATCH; ++j) {
+                for (uint32_t j = 0; j < BATCH; ++j) {
                     if (it + j >= maxcnt || !ok) continue;
-                    if (!mbar_wait_warp(smem_u32(&bar_full_a[j & 1u]), (j >> 1) & 1u, abort_flag)) {
+                    if (!mbar_wait_warp(smem_u32(&bar_full_a[j & 1u]), ((it + j) >> 1) & 1u, abort_flag)) {
                         if (leader) fail(p.status, abort_flag, ST_TIMEOUT_FULL_A, it);
                         ok = false;
                         continue;
@@ -300,7 +308,7 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
                             if (it + j >= cnt[g]) continue;
                             const uint32_t a_addr = tmem_base + A_COL0 + (g * SA + (j & 1u)) * SLOT;
                             const uint64_t b_desc =
-                                smem_desc_k_sw128(smem_base + ((g * 2u + bslot) * (BITS_BATCH / 2u) + j / 2u) * box_bytes) + 4u * (j & 1u);
+                                smem_desc_k_sw128(smem_base + ((g * 2u + bslot) * (BATCH / 2u) + j / 2u) * box_bytes) + 4u * (j & 1u);
                             const uint32_t acc = started | (uint32_t)(g > 0);
                             umma_i8_ts(tmem_base, a_addr, b_desc, p.idesc, acc);
                             umma_i8_ts(tmem_base + brows, a_addr + SLOT / 2u, b_desc, p.idesc, acc);
@@ -309,7 +317,7 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
                             umma_i8_ts(tmem_base + brows, a_addr + SLOT / 2u + 8u, b_desc + 2u, p.idesc, 1u);
                         }
                         tc_commit(smem_u32(&bar_empty_a[j & 1u]));
-                        if (j + 1 == BITS_BATCH) tc_commit(smem_u32(&bar_empty_b[bslot]));
+                        if (j + 1 == BATCH) tc_commit(smem_u32(&bar_empty_b[bslot]));
                     }
                     started = 1u;
                 }
