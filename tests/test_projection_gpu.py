@@ -784,3 +784,23 @@ def test_generator_square_root_is_exact_on_every_possible_draw(cuda):
 def test_device_status_clean(cuda):
     from trak_b200 import _lib
     _lib.device_status(cuda.index)
+
+
+@pytest.mark.parametrize("dt", ["f16", "f32"])
+@pytest.mark.parametrize("B,F,N,T", [
+    (33, 7_690, 512, 148),      # one stage a tile
+    (48, 20_011, 1024, 148),    # the last stage is short
+    (64, 70_001, 512, 1),       # one tile of many stages, two chains
+    (33, 3_001, 1536, 5),       # an odd number of tiles, two groups
+    (64, 131, 512, 7),          # tiles of less than two chunks
+])
+def test_rademacher_33_to_64_rows_make_a_chunk_ahead_of_its_slot(cuda, dt, B, F, N, T):
+    """16-bit products summed in fp32 over up to 7e4 features: chains of at most 4096 steps drift by 1e-8 a step."""
+    g_cpu = torch.randn(B, F, generator=torch.Generator().manual_seed(B * F)).mul_(0.1).to(DT[dt])
+    feats = sorted({0, min(F - 1, 15), min(F - 1, 16), min(F - 1, 63), min(F - 1, 64), F - 1})
+    for i, f in enumerate(feats):
+        g_cpu[i].zero_()
+        g_cpu[i, f] = 1.0
+    out = ours(g_cpu.to(cuda), N, 13, T, RAD).cpu().numpy()
+    assert np.array_equal(out[:len(feats)], o.matrix_rows(RAD, F, N, 13, T, feats))
+    assert rel_rows(out, o.project(RAD, as_numpy_input(g_cpu), N, 13, T, round_f16=dt == "f32")) <= 5e-5
