@@ -427,3 +427,20 @@ def test_operand_packed_beside_an_inverse_gives_the_bits_of_the_plain_product(cu
     called = []
     got = scm.gemm_nt(a, b, b_ready=lambda: called.append(1))
     assert called == [1] and torch.equal(got, scm.gemm_nt(a, b))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k", [1, 64, 127, 128, 129, 255, 256, 257, 385])
+@pytest.mark.parametrize("n", [33, 64, 65, 1000])
+def test_gram_of_few_columns_at_the_edges_of_its_tiles(cuda, n, k):
+    """128-column tiles: short and odd contractions, sliced and not, on a column of the output that is not 16-byte aligned.
+    Both factors are within 2^-22 of their column's largest entry (fp16 pairs), sums within 2^-22 of the norms' product."""
+    from trak_b200 import score_computers as scm
+    x = torch.randn(n, k, generator=torch.Generator().manual_seed(n * 1000 + k), dtype=torch.float64).float()
+    wide = torch.full((k, k + 3), 7.0, device=cuda)
+    got = scm.gram(x.to(cuda), out=wide[:, 1:k + 1])
+    want = x.double().T @ x.double()
+    scale = x.double().norm(dim=0)
+    assert ((got.cpu().double() - want).abs() / (scale[:, None] * scale[None, :])).max() <= 2.0 ** -20
+    assert torch.equal(got, got.T)
+    assert (wide[:, 0] == 7).all() and (wide[:, k + 1:] == 7).all()

@@ -375,20 +375,29 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // (Issuing all small terms of a chunk before its large ones halves the truncation that is left,
 // a mean error of -2.3e-7 instead of -3.0e-7 on a Gram diagonal, but holds both slots until the
 // chunk's end, and with only four slots the loads then arrive late: 12.6 against 11.5 ms.)
-constexpr uint32_t CK_SLOTS = 4;
-constexpr uint32_t CK_SLOT_BYTES = 6 * GTILE_BYTES;  // A: hi, lo; B: [plane][two row blocks]  (48 KB per 32 k)
+// TN = 128 halves the columns of a tile, for products of so few tiles that SMs are left idle (plan_gemm): each entry of the
+// result comes of the same operations in the same order.
+template <uint32_t TN>
+struct Chunked {
+    static constexpr uint32_t BLOCKS = TN / 128u;                            // row blocks of B
+    static constexpr uint32_t SLOTS = TN == 256u ? 4u : 6u;
+    static constexpr uint32_t SLOT_BYTES = (2u + 2u * BLOCKS) * GTILE_BYTES;  // A: hi, lo; B: [plane][row block]  (per 32 k)
+};
 
+template <uint32_t TN>
 __global__ void __launch_bounds__(384, 1)
 gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                        const GemmParams p) {
+    constexpr uint32_t BLOCKS = Chunked<TN>::BLOCKS, SLOTS = Chunked<TN>::SLOTS, SLOT_BYTES = Chunked<TN>::SLOT_BYTES;
+    constexpr uint32_t COLS = TN / 2u;  // of an epilogue warp
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t bar_full[CK_SLOTS];
-    __shared__ uint64_t bar_empty[CK_SLOTS];
+    __shared__ uint64_t bar_full[SLOTS];
+    __shared__ uint64_t bar_empty[SLOTS];
     __shared__ uint64_t bar_acc_full[2];
     __shared__ uint64_t bar_acc_empty[2];
     __shared__ uint32_t tmem_slot;
     __shared__ uint32_t abort_word;
-    __shared__ float col_factor[256];
+    __shared__ float col_factor[TN];
     volatile uint32_t* abort_flag = &abort_word;
 
     // same L2-friendly numbering as gemm_nt_kernel, with 128-row tiles
@@ -402,22 +411,22 @@ gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     const uint32_t tile_n = (id % width) / gsize;
     if (p.range == K_TO_ROW) tile_m = tiles_m - 1u - tile_m;  // the longest contractions first
     // symmetric: a tile is needed when it holds some entry with n >= m
-    if (p.symmetric && tile_n < (tile_m >> 1)) return;
+    if (p.symmetric && tile_n < tile_m / BLOCKS) return;
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     // The k blocks of this tile, less those where an operand is zero (a triangular factor: a third of W^T W and half of
     // a merge is left), and of them this slice's.  Starts are multiples of 128 and slices even: whole chunks.
     uint32_t kb_lo = 0, kb_hi = p.kblocks;
-    if (p.range == K_FROM_ROW) kb_lo = min(p.kblocks, max(tile_m * 4u, p.symmetric ? tile_n * 8u : 0u));
+    if (p.range == K_FROM_ROW) kb_lo = min(p.kblocks, max(tile_m * 4u, p.symmetric ? tile_n * (4u * BLOCKS) : 0u));
     if (p.range == K_TO_ROW) kb_hi = min(p.kblocks, tile_m * 4u + 4u);
-    if (p.range == K_TO_COL) kb_hi = min(p.kblocks, tile_n * 8u + 8u);
+    if (p.range == K_TO_COL) kb_hi = min(p.kblocks, (tile_n + 1u) * (4u * BLOCKS));
     const uint32_t slice = ((kb_hi - kb_lo + gridDim.z - 1u) / gridDim.z + 1u) & ~1u;
     const uint32_t kb_first = min(kb_hi, kb_lo + blockIdx.z * slice), kb_end = min(kb_hi, kb_first + slice);
     const uint32_t nchunks = (kb_end - kb_first + 1u) >> 1;
 
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < CK_SLOTS; ++s) {
+        for (uint32_t s = 0; s < SLOTS; ++s) {
             mbar_init(smem_u32(&bar_full[s]), 1);
             mbar_init(smem_u32(&bar_empty[s]), 1);
         }
@@ -429,7 +438,7 @@ gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         fence_mbar_init();
     }
     if (warp == 1) {
-        tmem_alloc(smem_u32(&tmem_slot), 512);
+        tmem_alloc(smem_u32(&tmem_slot), 2u * TN);
         tmem_relinquish();
     }
     tc_fence_before();
@@ -455,17 +464,17 @@ gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                     break;
                 }
                 const uint32_t bar = smem_u32(&bar_full[slot]);
-                const uint32_t sa = smem_base + slot * CK_SLOT_BYTES, sb = sa + 2u * GTILE_BYTES;
-                mbar_expect_tx(bar, CK_SLOT_BYTES);
+                const uint32_t sa = smem_base + slot * SLOT_BYTES, sb = sa + 2u * GTILE_BYTES;
+                mbar_expect_tx(bar, SLOT_BYTES);
 #pragma unroll
                 for (uint32_t pl = 0; pl < 2; ++pl) {
                     tma_load_2d(sa + pl * GTILE_BYTES, &map_a, 0, (int)(((tile_m * p.kblocks + kb) * 2u + pl) * 128u), bar);
 #pragma unroll
-                    for (uint32_t h = 0; h < 2; ++h)
-                        tma_load_2d(sb + (pl * 2u + h) * GTILE_BYTES, &map_b, 0,
-                                    (int)((((tile_n * 2u + h) * p.kblocks + kb) * 2u + pl) * 128u), bar);
+                    for (uint32_t h = 0; h < BLOCKS; ++h)
+                        tma_load_2d(sb + (pl * BLOCKS + h) * GTILE_BYTES, &map_b, 0,
+                                    (int)((((tile_n * BLOCKS + h) * p.kblocks + kb) * 2u + pl) * 128u), bar);
                 }
-                if (++slot == CK_SLOTS) {
+                if (++slot == SLOTS) {
                     slot = 0;
                     ph ^= 1u;
                 }
@@ -486,7 +495,7 @@ gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                     break;
                 }
                 tc_fence_after();
-                const uint32_t d = tmem_base + set * 256u;
+                const uint32_t d = tmem_base + set * TN;
                 const uint32_t nkb = min(2u, kb_end - kb_first - 2u * c);
                 // per 32-k slot: its small terms first, then its large ones, and the slot is released
                 for (uint32_t j = 0; j < nkb; ++j) {
@@ -497,9 +506,9 @@ gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t sa = smem_base + (slot + j) * CK_SLOT_BYTES, sb = sa + 2u * GTILE_BYTES;
+                    const uint32_t sa = smem_base + (slot + j) * SLOT_BYTES, sb = sa + 2u * GTILE_BYTES;
                     const uint64_t a_hi = smem_desc_k_sw64(sa), a_lo = smem_desc_k_sw64(sa + GTILE_BYTES);
-                    const uint64_t b_hi = smem_desc_k_sw64(sb), b_lo = smem_desc_k_sw64(sb + 2u * GTILE_BYTES);
+                    const uint64_t b_hi = smem_desc_k_sw64(sb), b_lo = smem_desc_k_sw64(sb + BLOCKS * GTILE_BYTES);
                     if (leader) {
 #pragma unroll
                         for (uint32_t kk = 0; kk < 2; ++kk) {
@@ -514,7 +523,7 @@ gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 if (!ok) break;
                 if (leader) tc_commit(smem_u32(&bar_acc_full[set]));
                 slot += nkb;
-                if (slot >= CK_SLOTS) {
+                if (slot >= SLOTS) {
                     slot = 0;
                     ph ^= 1u;
                 }
@@ -525,14 +534,14 @@ gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         // ---------------------- running sums, then the epilogue ----------------------
         const uint32_t q = warp & 3u, chalf = (warp - 4u) >> 2;  // TMEM lane quarter, column half
         {
-            const uint32_t t = threadIdx.x - 128u, n = tile_n * 256u + t;
-            col_factor[t] = (p.amax_b && n < p.N) ? row_scale_down(p.amax_b[n]) : 1.0f;
+            const uint32_t t = threadIdx.x - 128u, n = tile_n * TN + t;
+            if (t < TN) col_factor[t] = (p.amax_b && n < p.N) ? row_scale_down(p.amax_b[n]) : 1.0f;
             asm volatile("bar.sync 1, 256;" ::: "memory");  // the eight epilogue warps only
         }
         const uint32_t lane_base = (q * 32u) << 16;
-        float sum[128];
+        float sum[COLS];
 #pragma unroll
-        for (int i = 0; i < 128; ++i) sum[i] = 0.0f;
+        for (int i = 0; i < (int)COLS; ++i) sum[i] = 0.0f;
         bool ok = true;
 #pragma unroll 1
         for (uint32_t c = 0; c < nchunks; ++c) {
@@ -545,9 +554,9 @@ gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 break;
             }
             tc_fence_after();
-            const uint32_t t0 = tmem_base + lane_base + set * 256u + chalf * 128u;
+            const uint32_t t0 = tmem_base + lane_base + set * TN + chalf * COLS;
 #pragma unroll
-            for (uint32_t cb = 0; cb < 8; cb += 4) {  // four loads in flight per wait
+            for (uint32_t cb = 0; cb < COLS / 16u; cb += 4) {  // four loads in flight per wait
                 uint32_t r[4][16];
 #pragma unroll
                 for (uint32_t u = 0; u < 4; ++u) tmem_ld_x16(t0 + (cb + u) * 16u, r[u]);
@@ -563,21 +572,21 @@ gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         }
         if (ok) {
             const uint32_t m = tile_m * 128u + q * 32u + lane;
-            const uint32_t n0 = tile_n * 256u + chalf * 128u;
+            const uint32_t n0 = tile_n * TN + chalf * COLS;
             const float rs = p.alpha * ((p.row_scale && m < p.M) ? p.row_scale[m] : 1.0f);
             const float fa = (p.amax_a && m < p.M) ? row_scale_down(p.amax_a[m]) : 1.0f;
 #pragma unroll
-            for (int i = 0; i < 128; ++i) sum[i] = ((sum[i] * fa) * col_factor[chalf * 128u + i]) * rs;
+            for (int i = 0; i < (int)COLS; ++i) sum[i] = ((sum[i] * fa) * col_factor[chalf * COLS + i]) * rs;
             // The pipeline buffers are idle by now (the last commit covered every MMA and every load
             // has been consumed), so each warp turns its 32 x 128 block around in its own slab of them.
             float* slab = reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw))) +
-                          (size_t)(warp - 4u) * (32u * slab_ld(128));
+                          (size_t)(warp - 4u) * (32u * slab_ld(COLS));
 #pragma unroll
-            for (int i = 0; i < 128; i += 4)
-                *reinterpret_cast<float4*>(slab + lane * slab_ld(128) + i) =
+            for (int i = 0; i < (int)COLS; i += 4)
+                *reinterpret_cast<float4*>(slab + lane * slab_ld(COLS) + i) =
                     make_float4(sum[i], sum[i + 1], sum[i + 2], sum[i + 3]);
             __syncwarp();
-            store_block_from_slab<128>(p, p.C + blockIdx.z * p.split_stride, slab, tile_m * 128u + q * 32u, n0, lane);
+            store_block_from_slab<COLS>(p, p.C + blockIdx.z * p.split_stride, slab, tile_m * 128u + q * 32u, n0, lane);
         }
     }
 
@@ -586,7 +595,7 @@ gemm_nt_chunked_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     if (*abort_flag) __nanosleep(200000);
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, 512);
+        tmem_dealloc(tmem_base, 2u * TN);
     }
 }
 
@@ -1014,7 +1023,7 @@ static int packed_tmap(CUtensorMap* map, const uint16_t* packed, const Packed& g
 
 constexpr uint32_t B200_SMS = 148;
 
-// Tile and number of slices of the contraction.  A 256 x 256 (or 128 x 256) tile per CTA leaves most of the 148 SMs
+// Tile and number of slices of the contraction.  A 256 x 256 (chunked: 128 x 256) tile per CTA leaves most of the 148 SMs
 // idle when the product is small: the Gram of 2048 columns is 36 such tiles however many rows it sums over.  The
 // choice minimises an estimate in microseconds: per wave of CTAs a fixed part (launch, first loads, epilogue) plus the
 // tensor-core time of its k blocks; slicing adds the kernel that sums the slices, which is bound by memory.
@@ -1025,6 +1034,11 @@ constexpr uint32_t B200_SMS = 148;
 // 200,000 x 128 x 2048 370 and 517, 200,000 x 512 x 512 341 and 298, 50,000 x 2048 x 2048 1113 and 931; fp16
 // 50,000 x 2048 x 512 214 and 171, 1000 x 1024 x 8192 83 and 48 (sliced).  Over those 284 products the choice is 0.3 % (mean)
 // and 15 % (worst) slower than the better of the two; with one wave length for both tiles it was 3 % and 72 %.
+// The chunked kernel's 128-column tile takes nearly as long per k block as the 256-column one -- with both operands from shared
+// memory an MMA of 128 x 128 reads as many bytes a cycle as that gives -- but starts and ends 3 us sooner and makes twice the
+// CTAs, so it is for products of one wave: inverse of 512 138 -> 134 us, 700 244 -> 226, 1024 301 -> 287, 2048 633 -> 589, 4096
+// 1412 -> 1340; Gram of 1000 x 512 48.8 -> 46.8, 2000 x 256 60.0 -> 56.4, 400 x 400 42.4 -> 37.2.  Taken for three waves it cost
+// 25 % (9000 x 3000 352 -> 440 us).
 // The sizes alone decide, so that the workspace query, which names no device, agrees: every B200 has 148 SMs.  A product
 // that leaves out the k blocks where a triangular factor is zero (KRange) is planned like a whole one.
 GemmPlan plan_gemm(uint32_t npl, bool chunked, bool symmetric, int64_t M, int64_t N, uint32_t kblocks) {
@@ -1044,19 +1058,22 @@ GemmPlan plan_gemm(uint32_t npl, bool chunked, bool symmetric, int64_t M, int64_
         best_t = rounds * pair + (rest > SMS ? pair : rest > 0 ? single : 0.0);
         best.tile = 1;
     }
-    const double tiles = chunked ? (symmetric ? tm2 * (tm2 + 1) : tm * tn2) : symmetric ? tm2 * (tm2 + 1) / 2 : tm2 * tn2;
-    const double per_kb = chunked ? 0.48 : npl == 2 ? 0.9 : 0.3;
-    for (uint32_t s = 1; s <= MAX_SPLITS && s <= kblocks; ++s) {
-        const uint32_t per = ((kblocks + s - 1) / s + 1u) & ~1u;  // whole 64-wide chunks
-        const uint32_t used = (kblocks + per - 1) / per;
-        const size_t bytes = used > 1 ? (size_t)used * M * N * sizeof(float) : 0;
-        if (used != s || bytes > MAX_PARTIAL || (s > 1 && M > 32 * MAX_GRID_Y)) continue;
-        const double waves = (double)(uint64_t)((tiles * s + SMS - 1) / SMS);
-        double t = waves * (8.0 + per * per_kb);
-        if (s > 1) t += SUM_FIXED + ((double)s * (symmetric ? 0.5 : 1.0) + 1.0) * M * N * 4.0 / SUM_BYTES_PER_US;
-        if (t < best_t) {
-            best_t = t;
-            best = GemmPlan{2, s, s > 1 ? per : kblocks, align_up(bytes, 1024)};
+    for (int tile = chunked ? 1 : 2; tile <= 2; ++tile) {
+        const double tiles = tile == 1 ? (symmetric ? tm * (tm + 1) / 2 : tm * (double)((N + 127) / 128))
+                             : chunked ? (symmetric ? tm2 * (tm2 + 1) : tm * tn2) : symmetric ? tm2 * (tm2 + 1) / 2 : tm2 * tn2;
+        const double per_kb = tile == 1 ? 0.43 : chunked ? 0.48 : npl == 2 ? 0.9 : 0.3, fixed = tile == 1 ? 5.0 : 8.0;
+        for (uint32_t s = 1; s <= MAX_SPLITS && s <= kblocks; ++s) {
+            const uint32_t per = ((kblocks + s - 1) / s + 1u) & ~1u;  // whole 64-wide chunks
+            const uint32_t used = (kblocks + per - 1) / per;
+            const size_t bytes = used > 1 ? (size_t)used * M * N * sizeof(float) : 0;
+            if (used != s || bytes > MAX_PARTIAL || (s > 1 && M > 32 * MAX_GRID_Y)) continue;
+            const double waves = (double)(uint64_t)((tiles * s + SMS - 1) / SMS);
+            double t = waves * (fixed + per * per_kb);
+            if (s > 1) t += SUM_FIXED + ((double)s * (symmetric ? 0.5 : 1.0) + 1.0) * M * N * 4.0 / SUM_BYTES_PER_US;
+            if (t < best_t) {
+                best_t = t;
+                best = GemmPlan{tile, s, s > 1 ? per : kblocks, align_up(bytes, 1024)};
+            }
         }
     }
     return best;
@@ -1124,12 +1141,14 @@ int launch_gemm(int device, cudaStream_t stream, const uint16_t* pa, const Packe
         p.split_stride = 0;
     }
     if (chunked) {
-        p.idesc = idesc_f16(p.idesc, 256);
-        p.stages = CK_SLOTS;
-        const size_t smem = (size_t)CK_SLOTS * CK_SLOT_BYTES + 1024u;
-        const dim3 grid((uint32_t)((N + 255) / 256), (uint32_t)((M + 127) / 128), pl.splits);
-        if (const int e = set_smem_limit((const void*)gemm_nt_chunked_kernel, device)) return e;
-        rc = launch_after(gemm_nt_chunked_kernel, grid, 384, smem, stream, early, map_a, map_b, p);
+        const uint32_t cols = 128u * (uint32_t)pl.tile;
+        p.idesc = idesc_f16(p.idesc, cols);
+        auto kern = pl.tile == 2 ? gemm_nt_chunked_kernel<256> : gemm_nt_chunked_kernel<128>;
+        const size_t smem = (pl.tile == 2 ? (size_t)Chunked<256>::SLOTS * Chunked<256>::SLOT_BYTES
+                                          : (size_t)Chunked<128>::SLOTS * Chunked<128>::SLOT_BYTES) + 1024u;
+        const dim3 grid((uint32_t)((N + cols - 1) / cols), (uint32_t)((M + 127) / 128), pl.splits);
+        if (const int e = set_smem_limit((const void*)kern, device)) return e;
+        rc = launch_after(kern, grid, 384, smem, stream, early, map_a, map_b, p);
         if (rc != TB_OK) return rc;
     } else if (pl.tile == 2) {
         rc = ga.npl == 2 ? launch_gemm_nt<2, 2>(device, map_a, map_b, p, pl.splits, early, stream)

@@ -34,7 +34,7 @@ int launch_pack_pair(const float* a, uint64_t rows_a, uint64_t K_a, uint64_t ld_
 // The packed operand without its first `skip` row blocks: moves `packed` and returns the geometry of what is left.
 Packed packed_tail(const uint16_t** packed, const Packed& g, uint32_t skip);
 
-// How launch_gemm computes a product: CTA tile (2: 256 wide, 1: 128 wide), slices of the contraction, and the bytes
+// How launch_gemm computes a product: CTA tile (2: 256 columns, 1: 128; as many rows, 128 where chunked), slices of the contraction, and the bytes
 // of the slices' partial products, which the caller provides as `partial`.
 struct GemmPlan {
     int tile;
