@@ -15,13 +15,13 @@
 //   * 2^i differs from word to word (bit 2j + h of a draw's byte: feature pair j, column parity h; two of the four j after
 //     a shift by four).  The column's factor 2^h is undone at the end, the features' 2^(2 (j & 1)) in the staging: even j are
 //     staged four times as large.
-//   * What bounds it.  Up to 16 rows the integer pipe, 90 % busy with 11 instructions per 16 x 32 entries (4 of the 7 of a draw,
+//   * What bounds it.  Up to 16 rows the integer pipe, 82 % busy with 11 instructions per 16 x 32 entries (4 of the 7 of a draw,
 //     5 to spread it, 2 of hand-shakes; 35 instructions in all with a 16-bit operand, now 18): without its MMAs the kernel takes
-//     95 % of its time.  us a call, 16-bit operand -> this: 2,796,202 fp16 features -> 4096 1021 -> 625, 1,000,003 -> 8192
-//     732 -> 435, 40,000,001 bf16 -> 8192 27,750 -> 15,800; one row of 1,000,003 -> 2048 202 -> 128.
-//     From 17 to 32 rows the accumulators leave room for one CTA per SM, of four groups, and the digit planes' way from the L2
-//     bounds it (8 TB/s at 32 rows): 17 rows x 1,000,003 bf16 -> 8192 780 -> 567, 24 rows fp16 -> 2048 239 -> 202, 32 rows x
-//     2,796,202 -> 4096 1111 -> 930.
+//     95 % of its time.  us a call, 16-bit operand -> this: 2,796,202 fp16 features -> 4096 1043 -> 647, 1,000,003 -> 8192
+//     753 -> 455, 10,000,001 bf16 -> 8192 7004 -> 4022; one row of 1,000,003 -> 2048 218 -> 142.
+//     From 17 to 32 rows the accumulators leave room for one CTA per SM, of four groups, and the MMAs bound it (tensor pipe
+//     75 % busy at 24 rows, 85 at 32, with 7 TB/s from the L2; without generating it takes as long): 17 rows x 1,000,003 bf16
+//     -> 8192 780 -> 559, 24 rows fp16 -> 2048 239 -> 200, 32 rows x 2,796,202 -> 4096 1111 -> 926.
 //   * The groups' slots change hands together, and so do their boxes: one warp issues the MMAs beside busy generators, and a
 //     hand-over costs it some 300 cycles whatever it covers.  With barriers of each group's own 16 rows took 2 % longer (659
 //     us for 647), and four groups of 32-feature slots to a CTA 1023 us; with common ones 693, so two of 64 they stay.
