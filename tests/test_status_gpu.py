@@ -127,3 +127,57 @@ def test_a_call_that_was_refused_does_not_vouch_for_the_device(cuda, job):
     assert rc == 8, lib.tb_strerror(rc)
     assert lib.tb_stream_status(cuda.index, stream.cuda_stream, None) == 7
     assert lib.tb_stream_status(cuda.index, stream.cuda_stream, None) == 0
+
+
+FIRST_READ = """
+import torch
+from trak_b200 import _lib
+lib, other = _lib.lib(), torch.cuda.Stream()
+stream = torch.cuda.current_stream().cuda_stream
+assert lib.tb_selftest_wait_timeout(0, stream, 20) == 0     # before there is a word for kernels to repeat a failure in
+assert lib.tb_stream_status(0, stream, None) == 7
+assert lib.tb_stream_status(0, stream, None) == 0
+for s in (stream, other.cuda_stream):                       # and with it, on either stream
+    assert lib.tb_selftest_wait_timeout(0, s, 20) == 0
+    assert lib.tb_stream_status(0, s, None) == 7
+    assert lib.tb_stream_status(0, stream, None) == 0
+    assert lib.tb_device_status(0, None) == 0
+assert lib.tb_selftest_wait_timeout(0, stream, 20) == 0
+assert lib.tb_device_status(0, None) == 7                   # read by the other call: nothing is left for the stream's
+assert lib.tb_stream_status(0, stream, None) == 0
+"""
+
+
+def test_a_failure_reaches_the_first_read_of_a_process_and_the_later_ones(cuda):
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    p = subprocess.run([sys.executable, "-c", FIRST_READ], cwd=root, capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr
+
+
+FIRST_READ_UNDER_A_CAPTURE = """
+import threading
+import torch
+from trak_b200 import _lib
+lib = _lib.lib()
+assert lib.tb_device_status(0, None) == 0   # the one-time set-up of the device
+x, side = torch.zeros(8, device="cuda"), torch.cuda.Stream()
+side.wait_stream(torch.cuda.current_stream())
+graph, codes = torch.cuda.CUDAGraph(), []
+torch.cuda.synchronize()
+with torch.cuda.graph(graph, capture_error_mode="thread_local"):   # "global" forbids any thread's wait for a stream
+    x.add_(1.0)
+    t = threading.Thread(target=lambda: codes.append(lib.tb_stream_status(0, side.cuda_stream, None)))
+    t.start()
+    t.join()
+    x.add_(1.0)
+graph.replay()
+torch.cuda.synchronize()
+assert codes == [0] and x.tolist() == [2.0] * 8, (codes, x)
+"""
+
+
+def test_the_first_read_beside_another_threads_capture(cuda):
+    """It makes its word on a stream of its own, so the capture goes on."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    p = subprocess.run([sys.executable, "-c", FIRST_READ_UNDER_A_CAPTURE], cwd=root, capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr

@@ -55,7 +55,7 @@ struct StatusNote {
 };
 int take_note(StatusNote* note);
 // To be called when the launch that stores `note` has been queued on `stream` as the last of its call: the thread's next
-// tb_stream_status on that stream then needs no launch of its own.
+// tb_stream_status on that stream then reads `note`.
 void arm_status(int device, cudaStream_t stream, const StatusNote& note);
 #ifdef __CUDACC__
 __device__ __forceinline__ void publish_status(const uint32_t* status, const StatusNote& note) {
