@@ -182,3 +182,34 @@ def test_one_hot_rows_last_pass_accumulation_and_small_workspaces(cuda):
     assert lib.tb_project_static(0, stream, big.data_ptr(), 0, 16, 600_011, 600_011, res.data_ptr(), N, N, 21, T, RAD,
                                  1.0, 0) == 0
     assert worst_row(res.cpu(), project(big, N, 21, T).cpu()) <= 1e-4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt", ["f16", "f32", "bf16"])
+@pytest.mark.parametrize("B,F,N", [(16, 592_003, 512), (24, 330_003, 1536)])
+def test_rows_that_few_elements_outweigh(cuda, B, F, N, dt):
+    """Elements of a step of the largest element's and less, up to the most that may outweigh the others, at both ends of the
+    exponents.  Rounding may take 2^-24 of the largest element and 2^-22 of the norm of the rest."""
+    gen = torch.Generator().manual_seed(6)
+    x = torch.randn(B, F, generator=gen, dtype=torch.float64)
+    u = torch.rand(F, generator=gen, dtype=torch.float64)
+    top = 1.0 if dt == "bf16" else 2.0 ** 15        # fp16: steps of its least number reach 2^39 below
+    x[0], x[0, 77] = (1 + u) * 2.0 ** -30 * top, top
+    x[1], x[1, F - 1] = 2.0 ** -28 * top, top       # half a step each
+    x[2], x[2, 5::50_021] = x[2] * 2.0 ** -16 * top, -top
+    x[3], x[3, 0::997] = x[3] * 2.0 ** -24 * top, 2.0 ** -8 * top
+    x[3, 40] = top
+    x[4] = torch.exp(3 * x[4]) * torch.randn(F, generator=gen, dtype=torch.float64)
+    x[4] *= top / x[4].abs().max()
+    x[5], x[5, 4000:4016] = x[5] * 2.0 ** -20 * top, top                       # all of one place of a tile
+    x[6], x[6, 9::8191] = torch.where(u < 0.01, x[6] * 2.0 ** -18 * top, torch.zeros(F, dtype=torch.float64)), top
+    if dt == "bf16":
+        x[7], x[7, 3] = (1 + u) * 2.0 ** 90, 2.0 ** 118
+        x[8], x[8, 3] = (1 + u) * 2.0 ** -125, 2.0 ** -97
+    g = x.to(DT[dt])
+    check(g, N, 23, 148, cuda, tol=TOL + 2.0 ** -24 + 2.0 ** -22)
+    # the parameters of a model, in the same bits
+    from trak_b200 import fast_jl
+    dense, cut = g.to(cuda), F // 3
+    parts = [dense[:, :1].contiguous(), dense[:, 1:cut].contiguous(), dense[:, cut:].contiguous()]
+    assert torch.equal(fast_jl.project_segments(parts, N, 23, 148, RAD), project(dense, N, 23, 148))

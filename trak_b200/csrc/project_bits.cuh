@@ -9,9 +9,18 @@
 // every product exactly in 32 bits.  sum_f q_f comes from the staging.  Only the result of a CTA is rounded, once, to fp32.
 //
 //   * Exactness.  An fp16 (bf16) value has 11 (8) significant bits, so q is exact for every element within 2^-17 (2^-20) of
-//     its row's largest; below that an element is off by at most 2^-28 of the largest, which over n elements adds up to
-//     2^-29 sqrt(n) of the row's norm at most, whatever the distribution (6e-6 for 1e7 elements, all of them just wrong and
-//     one that outweighs the rest).  The fp32 accumulators of the 16-bit kernel drift by 2e-5 there on every input.
+//     its row's largest.  Below that an element is off by at most half a step, 2^-28 of the largest: nothing on a row of like
+//     elements, ten times the error of the 16-bit kernel on one that a single element outweighs.  So the steps of a row are never
+//     coarser than its norm allows (row_exponent): rounding takes at most 2^-24 of its largest element and 2^-22 of the norm of
+//     the others.  The few elements that such steps put out of the planes' range are staged as zeros and listed by tile, and the
+//     CTAs that find one run the tile's streams once more (7 of the 18 instructions) and add them in 64 bits.
+//     Error against 64 bits over the row's norm, 16-bit kernel / steps by the largest element alone / this: 592,003 features
+//     beside one of 1 in bf16, N(0, 2^-8) 2.9e-7 / 7.6e-8 / 7.6e-8, N(0, 2^-16) 1.7e-5 / 4.4e-7 / 1.2e-7, uniform in 2^-30..2^-29
+//     1.7e-7 / 1.5e-6 / 1.3e-7, all of 2^-28 3.6e-7 / 3.8e-6 / 1.1e-7; 6,000,001 features, N(0, 2^-16) 9.0e-5 / 1.2e-6 / 8.6e-8,
+//     uniform 3.2e-7 / 3.9e-6 / 9.4e-8; N(0, 1) without the one 3.2e-6 / 7.4e-8 / 7.4e-8.
+//     us a call, the same three, one such element to a row: 16 x 1,000,003 bf16 -> 4096 371 / 237 / 249, 32 rows 400 / 350 / 384;
+//     without any, for the second reading of the rows' sums of squares, 16 x 2,796,202 fp16 -> 4096 1013 / 616 / 620, 16 x 40,001
+//     -> 8192 58 / 49 / 53, 32 x 1,048,576 -> 2048 225 / 219 / 224.
 //   * 2^i differs from word to word (bit 2j + h of a draw's byte: feature pair j, column parity h; two of the four j after
 //     a shift by four).  The column's factor 2^h is undone at the end, the features' 2^(2 (j & 1)) in the staging: even j are
 //     staged four times as large.
@@ -46,7 +55,15 @@ constexpr uint32_t BITS_MAX_CHAIN = 32768;    // stages of a CTA: |digit| <= 128
 __host__ __device__ constexpr uint32_t bits_groups(uint32_t rows) { return rows <= 16u ? 2u : 4u; }
 __host__ __device__ constexpr uint32_t bits_batch(uint32_t rows) { return rows <= 16u ? 4u : 2u; }
 constexpr uint32_t BITS_MAX_SLICES = 256;     // of a row in absmax_kernel
+constexpr float BITS_RANGE = 268435456.0f;     // 2^28: a rounded gradient stays below
 constexpr int BITS_INF = 0x7ffffffe, BITS_NAN = 0x7fffffff;   // BitsParams::row_exp of a row that holds one
+
+// 16 features of a row of which some are too large for the planes, in the list of their place in a tile (which of 16
+// features): 2^e times each of those, the others zero.
+struct Outliers {
+    uint32_t next, row;         // 1 + the index of the next record of the list, 0: the last
+    float q[16];
+};
 
 struct BitsParams {
     float* partials;            // [bundles][B][N]
@@ -54,6 +71,9 @@ struct BitsParams {
     const long long* sums;      // [tiles][rows] sum of the rounded gradients q
     const uint32_t* infs;       // [tiles][rows] infinities among them (rows of BITS_INF only)
     const int* row_exp;         // [rows] 4 q is 2^row_exp times the gradient; or BITS_INF, BITS_NAN
+    const uint32_t* last_out;   // [tiles] 1 + the last 16 features that have outliers, 0: none
+    const uint32_t* heads;      // [tiles][4 nst] 1 + their first record, 0: none
+    const Outliers* outliers;
     uint32_t N, seed;
     uint32_t B, rows;           // rows in this launch, and rounded up to 8
     uint32_t nst;               // pipeline stages per feature tile, even
@@ -61,10 +81,14 @@ struct BitsParams {
     uint32_t idesc;
 };
 
+// The two streams' signs of 16 features: bit 2j + h of byte b is feature 2j + (b & 1) + 8 (b >> 1) of the 16, column h of the pair.
+__device__ __forceinline__ uint32_t gen_bits(Xw& st0, Xw& st1) {
+    const uint32_t d0 = xw_next(st0), d1 = xw_next(st1);
+    return __byte_perm(d0, d1, 0x5140u);
+}
 // 16 features of a pair of columns: byte b of word j is feature 2j + (b & 1) + 8 (b >> 1) of the 16, as the staging has them.
 __device__ __forceinline__ void gen_bits_pair(Xw& st0, Xw& st1, uint32_t* even, uint32_t* odd) {
-    const uint32_t d0 = xw_next(st0), d1 = xw_next(st1);
-    const uint32_t c = __byte_perm(d0, d1, 0x5140u), c4 = c >> 4;
+    const uint32_t c = gen_bits(st0, st1), c4 = c >> 4;
     even[0] = c & 0x01010101u;
     odd[0] = c & 0x02020202u;
     even[1] = c & 0x04040404u;
@@ -100,6 +124,7 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
     __shared__ uint64_t bar_full_b[2];
     __shared__ uint64_t bar_empty_b[2];
     __shared__ uint64_t bar_acc;
+    __shared__ uint64_t bar_extra[2];  // between the generators
     __shared__ uint32_t tmem_slot;
     __shared__ uint32_t abort_word;
     volatile uint32_t* abort_flag = &abort_word;
@@ -120,6 +145,7 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
             mbar_init(smem_u32(&bar_empty_b[s]), 1);
         }
         mbar_init(smem_u32(&bar_acc), 1);
+        for (uint32_t s = 0; s < 2u; ++s) mbar_init(smem_u32(&bar_extra[s]), GW * NG);
         abort_word = 0;
         fence_mbar_init();
     }
@@ -175,32 +201,99 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
             if (!ok && lane == 0) fail(p.status, abort_flag, ST_TIMEOUT_EMPTY, 0x4000u | (g << 16));
             if (ok && lane == 0) mbar_arrive(full + slot * 8u);
         }
+        // What the staging knows of rows b4 to b4 + 3 over the bundle's tiles: eight tiles at a time, row `lane & 3`.
+        struct Rows {
+            long long sum;
+            uint32_t ninf;
+            int exps;
+        };
+        auto rows_from = [&](uint32_t b4) {
+            const uint32_t row = b4 + (lane & 3u);
+            Rows r = {0, 0u, p.row_exp[row]};
+            for (uint32_t t = lane >> 2; t < ntile; t += 8u) {
+                r.sum += p.sums[(tile0 + t) * p.rows + row];
+                r.ninf += p.infs[(tile0 + t) * p.rows + row];
+            }
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) {
+                r.sum += __shfl_xor_sync(0xffffffffu, r.sum, o);
+                r.ninf += __shfl_xor_sync(0xffffffffu, r.ninf, o);
+            }
+            return r;
+        };
+        // With one CTA to an SM nothing else runs at its end: they are fetched while the last products are made (17 rows x 70,001
+        // -> 8192 85 -> 80 us).  Beside another CTA it costs the generators registers and is not worth it (620 -> 643).
+        constexpr bool EARLY = ROWS > 16u;
+        Rows early[2];
+        static_assert(ROWS <= 8u * NG, "two turns of four rows to a group");
+        bool outside = false;  // some tile has elements that the planes do not hold; the same for every warp
+        if (ok) {
+            cudaGridDependencySynchronize();  // the staging's lists, sums and scales
+            for (uint32_t t = lane; t < ntile; t += 32u) outside |= p.last_out[tile0 + t] != 0u;
+            outside = __any_sync(0xffffffffu, outside);
+#pragma unroll
+            for (uint32_t turn = 0; turn < 2u; ++turn)
+                if (EARLY && 4u * (g + NG * turn) < p.B) early[turn] = rows_from(4u * (g + NG * turn));
+        }
         // ---- the exact integer result of this CTA, as fp32 ----
         if (ok && !mbar_wait_warp(smem_u32(&bar_acc), 0u, abort_flag)) {
             if (lane == 0) fail(p.status, abort_flag, ST_TIMEOUT_ACC, g);
             ok = false;
         }
         if (ok) {
-            cudaGridDependencySynchronize();  // the staging's sums and scales
             tc_fence_after();
             const uint32_t tmem_acc = tmem_base + lane_base;
             const uint32_t n_out = blockIdx.x * 256u + 2u * pair;
+            // What the planes do not hold: those tiles are generated once more, up to the last such element, and the signed
+            // sums kept in the boxes' place
+            long long(*const extra)[256] = reinterpret_cast<long long(*)[256]>(smem_raw + (smem_base - smem_u32(smem_raw)));
+            if (outside) {
+                auto meet = [&](int which) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&bar_extra[which]));
+                    if (ok && !mbar_wait_warp(smem_u32(&bar_extra[which]), 0u, abort_flag)) {
+                        if (lane == 0) fail(p.status, abort_flag, ST_TIMEOUT_ACC, 0x4000u | g);
+                        ok = false;
+                    }
+                };
+                for (uint32_t i = threadIdx.x; i < p.rows * 256u; i += GW * NG * 32u) extra[0][i] = 0;
+                meet(0);
+                for (uint32_t ti = g; ti < ntile && ok; ti += NG) {
+                    const uint32_t t = tile0 + ti, last = p.last_out[t];
+                    if (last == 0u) continue;
+                    Xw st0, st1;
+                    xw_seed(st0, p.seed + 658105236u * stream_col + 359124577u * t);
+                    xw_seed(st1, p.seed + 658105236u * (stream_col + 16u) + 359124577u * t);
+                    for (uint32_t k0 = 0; k0 < last; k0 += 32u) {
+                        const uint32_t k1 = min(32u, last - k0);
+                        const uint32_t first = lane < k1 ? p.heads[(size_t)t * p.nst * 4u + k0 + lane] : 0u;
+                        for (uint32_t k = 0; k < k1; ++k) {
+                            const uint32_t c = gen_bits(st0, st1);
+                            for (uint32_t r = __shfl_sync(0xffffffffu, first, k); r != 0u;) {
+                                const Outliers& o = p.outliers[r - 1u];
+                                long long v0 = 0, v1 = 0;
+                                for (uint32_t f = 0; f < 16u; ++f) {
+                                    const long long q = (long long)o.q[f];
+                                    const uint32_t at = 8u * ((f & 1u) | (f >> 3 << 1)) + 2u * ((f & 7u) >> 1);
+                                    v0 += c >> at & 1u ? q : -q;
+                                    v1 += c >> at & 2u ? q : -q;
+                                }
+                                unsigned long long* const sum = reinterpret_cast<unsigned long long*>(&extra[o.row][2u * pair]);
+                                atomicAdd(sum, (unsigned long long)v0);
+                                atomicAdd(sum + 1, (unsigned long long)v1);
+                                r = o.next;
+                            }
+                        }
+                    }
+                }
+                meet(1);
+            }
             float* dst = p.partials + (size_t)blockIdx.y * p.B * p.N + n_out;
-            for (uint32_t b4 = 4u * g; b4 < p.B; b4 += 4u * NG) {
-                // sums of four rows over the bundle's tiles: eight tiles at a time, row `lane & 3`
-                const uint32_t row = b4 + (lane & 3u);
-                long long sum = 0;
-                uint32_t ninf = 0;
-                const int exps = p.row_exp[row];
-                for (uint32_t t = lane >> 2; t < ntile; t += 8u) {
-                    sum += p.sums[(tile0 + t) * p.rows + row];
-                    ninf += p.infs[(tile0 + t) * p.rows + row];
-                }
-#pragma unroll
-                for (int o = 4; o < 32; o <<= 1) {
-                    sum += __shfl_xor_sync(0xffffffffu, sum, o);
-                    ninf += __shfl_xor_sync(0xffffffffu, ninf, o);
-                }
+#pragma unroll EARLY ? 2 : 1
+            for (uint32_t turn = 0; turn < 2u; ++turn) {
+                const uint32_t b4 = 4u * (g + NG * turn);
+                if (b4 >= p.B || !ok) break;
+                const Rows known = EARLY ? early[turn] : rows_from(b4);
                 uint32_t d[2][BITS_PLANES][4];
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
@@ -211,9 +304,9 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
 #pragma unroll
                 for (uint32_t j = 0; j < 4; ++j) {
                     const uint32_t b = b4 + j;
-                    const long long total = __shfl_sync(0xffffffffu, sum, j);
-                    const uint32_t infs = __shfl_sync(0xffffffffu, ninf, j);
-                    const int e = __shfl_sync(0xffffffffu, exps, j);
+                    const long long total = __shfl_sync(0xffffffffu, known.sum, j);
+                    const uint32_t infs = __shfl_sync(0xffffffffu, known.ninf, j);
+                    const int e = __shfl_sync(0xffffffffu, known.exps, j);
                     if (b >= p.B) break;
                     float2 v;
 #pragma unroll
@@ -222,6 +315,7 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
 #pragma unroll
                         for (int pl = (int)BITS_PLANES - 1; pl >= 0; --pl) s = s * 256 + (int)d[h][pl][j];
                         s = (h == 0 ? 2 * s : s) - 4 * total;
+                        if (outside) s += 4 * extra[b][2u * pair + h];
                         float r;
                         if (e < BITS_INF)
                             r = scale_by(__ll2float_rn(s), -e);
@@ -341,18 +435,55 @@ enum class Elem { F32, F16, BF16 };
 template <Elem E>
 using elem_t = typename std::conditional<E == Elem::F32, float, uint16_t>::type;
 
-// Largest magnitude of slice blockIdx.x of row blockIdx.y, as the bits of the element type (monotonic, infinity above every
-// number and NaN above infinity); also clears the sums the staging adds to.  The ends of a parameter go element by element.
-// Bound by memory: 16 x 2,796,202 fp16 (89 MB) in 20 us.
-__device__ __forceinline__ uint32_t max_bits(uint32_t m, uint32_t w, bool wide) {
-    return wide ? max(m, w & 0x7fffffffu) : __vmaxu2(m, w & 0x7fff7fffu);
-}
+// Largest magnitude and sum of squares of slice blockIdx.x of row blockIdx.y.  The former as the bits of the element type
+// (monotonic, infinity above every number and NaN above infinity); of the latter three for bf16, whose squares fp32 does not
+// hold: of the elements, and of 2^-90 and 2^90 times them.  Also clears what the staging adds to.  The ends of a parameter go
+// element by element.  Bound by memory: 16 x 2,796,202 fp16 (89 MB) in 20 us.
 template <Elem E>
-__device__ __forceinline__ uint32_t max_bits_of_run(const elem_t<E>* src, uint64_t n, uint32_t m) {
-    constexpr bool WIDE = E == Elem::F32;
+struct RowStats {
+    static constexpr uint32_t SUMS = E == Elem::BF16 ? 3u : 1u;
+    uint32_t max_bits;
+    float sums[SUMS];
+    __device__ __forceinline__ void square(float x) {
+        sums[0] = fmaf(x, x, sums[0]);
+        if constexpr (SUMS == 3u) {
+            const float low = x * 0x1p-90f, high = x * 0x1p90f;
+            sums[1] = fmaf(low, low, sums[1]);
+            sums[2] = fmaf(high, high, sums[2]);
+        }
+    }
+    __device__ __forceinline__ void add_one(uint32_t bits) {
+        max_bits = E == Elem::F32 ? max(max_bits, bits & 0x7fffffffu) : __vmaxu2(max_bits, bits & 0x7fffu);
+        square(E == Elem::F32 ? __uint_as_float(bits) : E == Elem::F16 ? __half2float(__ushort_as_half((unsigned short)bits))
+                                                                       : __uint_as_float(bits << 16));
+    }
+    __device__ __forceinline__ void add(uint32_t w) {  // 32 bits of elements
+        if constexpr (E == Elem::F32) {
+            add_one(w);
+        } else {
+            max_bits = __vmaxu2(max_bits, w & 0x7fff7fffu);
+            if constexpr (E == Elem::F16) {
+                const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w));
+                square(v.x);
+                square(v.y);
+            } else {
+                square(__uint_as_float(w << 16));
+                square(__uint_as_float(w & 0xffff0000u));
+            }
+        }
+    }
+    __device__ __forceinline__ void add(const uint4& v) {
+        add(v.x);
+        add(v.y);
+        add(v.z);
+        add(v.w);
+    }
+};
+template <Elem E>
+__device__ __forceinline__ void add_run(RowStats<E>& st, const elem_t<E>* src, uint64_t n) {
     constexpr uint32_t V = 16u / sizeof(elem_t<E>);
     auto one = [&](uint64_t i) {
-        m = max_bits(m, WIDE ? reinterpret_cast<const uint32_t*>(src)[i] : reinterpret_cast<const uint16_t*>(src)[i], WIDE);
+        st.add_one(E == Elem::F32 ? reinterpret_cast<const uint32_t*>(src)[i] : reinterpret_cast<const uint16_t*>(src)[i]);
     };
     const uint64_t head = min(n, (uint64_t)(((16u - (uint32_t)(reinterpret_cast<uintptr_t>(src) & 15u)) & 15u) / sizeof(elem_t<E>)));
     const uint64_t vecs = (n - head) / V, tail = head + vecs * V;
@@ -364,35 +495,24 @@ __device__ __forceinline__ uint32_t max_bits_of_run(const elem_t<E>* src, uint64
 #pragma unroll
         for (uint32_t j = 0; j < 4; ++j) v[j] = __ldg(vec + i + j * 256u);
 #pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) {
-            m = max_bits(m, v[j].x, WIDE);
-            m = max_bits(m, v[j].y, WIDE);
-            m = max_bits(m, v[j].z, WIDE);
-            m = max_bits(m, v[j].w, WIDE);
-        }
+        for (uint32_t j = 0; j < 4; ++j) st.add(v[j]);
     }
-    for (; i < vecs; i += 256u) {
-        const uint4 v = __ldg(vec + i);
-        m = max_bits(m, v.x, WIDE);
-        m = max_bits(m, v.y, WIDE);
-        m = max_bits(m, v.z, WIDE);
-        m = max_bits(m, v.w, WIDE);
-    }
+    for (; i < vecs; i += 256u) st.add(__ldg(vec + i));
     if (tail + threadIdx.x < n) one(tail + threadIdx.x);
-    return m;
 }
 
 template <Elem E, bool SEG>
 __global__ void __launch_bounds__(256)
 absmax_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ segs, uint32_t nsegs, uint64_t row0,
-              uint32_t* __restrict__ maxima, uint4* __restrict__ clear, uint32_t clear_n, uint64_t F, uint64_t ld,
-              uint64_t slice) {
+              uint32_t* __restrict__ maxima, float* __restrict__ squares, uint4* __restrict__ clear, uint32_t clear_n, uint64_t F,
+              uint64_t ld, uint64_t slice) {
     cudaTriggerProgrammaticLaunchCompletion();
-    __shared__ uint32_t part[8];
+    constexpr uint32_t SUMS = RowStats<E>::SUMS;
+    __shared__ RowStats<E> part[8];
     const uint32_t id = (blockIdx.y * gridDim.x + blockIdx.x) * 256u + threadIdx.x;
     for (uint32_t i = id; i < clear_n; i += gridDim.x * gridDim.y * 256u) clear[i] = make_uint4(0u, 0u, 0u, 0u);
     const uint64_t f0 = blockIdx.x * slice, f1 = min(F, f0 + slice);
-    uint32_t m = 0;
+    RowStats<E> st = {};
     if (SEG) {
         uint32_t lo = 0, hi = nsegs;  // last parameter whose start is <= f0
         while (hi - lo > 1u) {
@@ -405,21 +525,31 @@ absmax_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ segs, 
         for (uint64_t f = f0; f < f1; ++lo) {
             const SegDev s = segs[lo];
             const uint64_t end = min(f1, s.start + s.numel);
-            m = max_bits_of_run<E>(static_cast<const elem_t<E>*>(s.ptr) + (row0 + blockIdx.y) * s.stride + (f - s.start),
-                                   end - f, m);
+            add_run(st, static_cast<const elem_t<E>*>(s.ptr) + (row0 + blockIdx.y) * s.stride + (f - s.start), end - f);
             f = end;
         }
     } else {
-        m = max_bits_of_run<E>(g + (uint64_t)blockIdx.y * ld + f0, f1 - f0, m);
+        add_run(st, g + (uint64_t)blockIdx.y * ld + f0, f1 - f0);
     }
-    if (E != Elem::F32) m = max(m & 0xffffu, m >> 16);
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31u) == 0) part[threadIdx.x >> 5] = m;
+    if (E != Elem::F32) st.max_bits = max(st.max_bits & 0xffffu, st.max_bits >> 16);
+    st.max_bits = __reduce_max_sync(0xffffffffu, st.max_bits);
+#pragma unroll
+    for (uint32_t j = 0; j < SUMS; ++j)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) st.sums[j] += __shfl_xor_sync(0xffffffffu, st.sums[j], o);
+    if ((threadIdx.x & 31u) == 0) part[threadIdx.x >> 5] = st;
     __syncthreads();
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int w = 1; w < 8; ++w) m = max(m, part[w]);
-        maxima[blockIdx.y * gridDim.x + blockIdx.x] = m;
+        for (int w = 1; w < 8; ++w) {
+            st.max_bits = max(st.max_bits, part[w].max_bits);
+#pragma unroll
+            for (uint32_t j = 0; j < SUMS; ++j) st.sums[j] += part[w].sums[j];
+        }
+        const uint32_t at = blockIdx.y * gridDim.x + blockIdx.x;
+        maxima[at] = st.max_bits;
+#pragma unroll
+        for (uint32_t j = 0; j < SUMS; ++j) squares[at * SUMS + j] = st.sums[j];
     }
 }
 
@@ -431,17 +561,60 @@ __device__ __forceinline__ float staged_value(uint32_t bits) {
     return __uint_as_float(bits << 16);
 }
 
-// Scale of a row from its largest element: the exponent e for which 2^e times every element is below 2^28, or what to do
-// with a row that is not finite.
+// Scale of a row: the exponent e for which 2^e times every element is below 2^28, or what to do with a row that is not
+// finite.  Where that leaves steps so coarse that rounding could take more from the row than 2^-24 of its largest element and
+// 2^-22 of the norm of the rest, the exponent is the least that does not, and the elements that 2^e takes out of range go
+// beside the planes (`outside`): F / 4096 + 1 of them at most, since more would make that norm, and with it the steps, larger.
+// A number that comes as fp16 is a multiple of 2^-24: finer steps than that are never needed.
 template <Elem E>
-__device__ __forceinline__ int row_exponent(uint32_t max_bits) {
+__device__ __forceinline__ int row_exponent(uint32_t max_bits, const float (&sums)[RowStats<E>::SUMS], float half_sqrt_f, bool& outside) {
     const float m = staged_value<E>(max_bits);
+    outside = false;
     if (m != m) return BITS_NAN;
     if (m == INFINITY) return BITS_INF;
     if (m == 0.0f) return 0;
-    int e;
+    int e, by_norm;
     frexpf(m, &e);  // m < 2^e
-    return 28 - e;
+    const int by_max = 28 - e;
+    float square = sums[0], scaled = m;
+    int up = 0;     // `square` is of 2^up times the elements, and so is `scaled`
+    if constexpr (E == Elem::BF16) {
+        if (e > 40) {
+            square = sums[1];
+            up = -90;
+        } else if (e < -40) {
+            square = sums[2];
+            up = 90;
+        }
+        scaled = ldexpf(m, up);
+    }
+    const float rest = sqrtf(fmaxf(square - scaled * scaled, 0.0f));
+    by_norm = (int)(__float_as_uint(half_sqrt_f / (scaled * 0x1p-24f + rest * 0x1p-22f)) >> 23) - 126 + up;  // 2^by_norm above it
+    if (E != Elem::BF16) by_norm = min(by_norm, 24);
+    outside = by_norm > by_max;
+    return max(by_norm, by_max);
+}
+
+struct OutlierLists {
+    uint32_t *count, *last, *heads;  // records in use; BitsParams::last_out, heads
+    Outliers* outliers;
+    uint32_t most;
+};
+
+// Of 16 scaled elements of row b, place `place` of a tile, those that are too large for the planes, as a mask; they get a record.
+__device__ __noinline__ uint32_t keep_outliers(const OutlierLists& lists, const float (&v)[16], uint32_t b, uint32_t tile,
+                                               uint32_t places, uint32_t place) {
+    uint32_t taken = 0;
+    for (uint32_t k = 0; k < 16; ++k) taken |= (uint32_t)(fabsf(v[k]) >= BITS_RANGE) << k;
+    if (taken == 0u) return 0u;
+    const uint32_t r = atomicAdd(lists.count, 1u);
+    if (r >= lists.most) return 0u;  // never (row_exponent)
+    Outliers& o = lists.outliers[r];
+    o.row = b;
+    for (uint32_t k = 0; k < 16; ++k) o.q[k] = taken >> k & 1u ? v[k] : 0.0f;
+    o.next = atomicExch(lists.heads + (size_t)tile * places + place, r + 1u);
+    atomicMax(lists.last + tile, place + 1u);
+    return taken;
 }
 
 // stage_kernel for project_bits_kernel: staged[tile][128 features][plane][row].  A warp takes runs of 512 features of one
@@ -449,11 +622,11 @@ __device__ __forceinline__ int row_exponent(uint32_t max_bits) {
 // Bound by memory, two bytes read (fp16) and four written an element, and next to that by 14 instructions an element:
 // 16 x 2,796,202 fp16 in 50 us.
 template <Elem E, bool SEG>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, SEG ? 4 : 5)
 stage_bits_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ segs, uint32_t nsegs, uint64_t row0,
-                  uint8_t* __restrict__ staged, const uint32_t* __restrict__ maxima, uint32_t slices,
-                  long long* __restrict__ sums, uint32_t* __restrict__ infs, int* __restrict__ row_exp, uint32_t B,
-                  uint32_t rows, uint64_t F, uint64_t ld, uint32_t fts, uint32_t nst, uint32_t tiles) {
+                  uint8_t* __restrict__ staged, const uint32_t* __restrict__ maxima, const float* __restrict__ squares,
+                  uint32_t slices, long long* __restrict__ sums, uint32_t* __restrict__ infs, int* __restrict__ row_exp,
+                  const OutlierLists lists, float half_sqrt_f, uint32_t B, uint32_t rows, uint64_t F, uint64_t ld, uint32_t fts, uint32_t nst, uint32_t tiles) {
     using In = elem_t<E>;
     cudaTriggerProgrammaticLaunchCompletion();  // see launch_after
     constexpr uint32_t RUN = 512u, V = 16u / sizeof(In), LOADS = 16u / V;
@@ -464,6 +637,7 @@ stage_bits_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ se
     cudaGridDependencySynchronize();  // the maxima, and the cleared sums
     uint32_t b_of = 0xffffffffu;
     int e = 0;
+    bool outside = false;        // some elements of the row may be too large
     float f1 = 1.0f, f2 = 1.0f;  // 2^e in two factors (bf16 reaches beyond one)
     for (uint64_t i = blockIdx.x; i < total; i += gridDim.x) {
         const uint64_t q = i / blocks;
@@ -471,10 +645,19 @@ stage_bits_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ se
         const uint32_t tile = (uint32_t)(q / b_hi_n), b = ((uint32_t)q - tile * b_hi_n) * 8u + warp;
         if (b != b_of) {
             b_of = b;
-            uint32_t m = 0;
-            if (b < B)
-                for (uint32_t s = lane; s < slices; s += 32u) m = max(m, maxima[b * slices + s]);
-            e = row_exponent<E>(__reduce_max_sync(0xffffffffu, m));
+            RowStats<E> st = {};
+            if (b < B) {
+                for (uint32_t s = lane; s < slices; s += 32u) {
+                    st.max_bits = max(st.max_bits, maxima[b * slices + s]);
+#pragma unroll
+                    for (uint32_t j = 0; j < RowStats<E>::SUMS; ++j) st.sums[j] += squares[(b * slices + s) * RowStats<E>::SUMS + j];
+                }
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < RowStats<E>::SUMS; ++j)
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) st.sums[j] += __shfl_xor_sync(0xffffffffu, st.sums[j], o);
+            e = row_exponent<E>(__reduce_max_sync(0xffffffffu, st.max_bits), st.sums, half_sqrt_f, outside);
             const int a = e >= BITS_INF ? 0 : E == Elem::BF16 ? e / 2 : e, c = e < BITS_INF ? e - a : 0;
             f1 = __int_as_float((127 + a) << 23);
             f2 = __int_as_float((127 + c) << 23);
@@ -554,6 +737,14 @@ stage_bits_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ se
                             x[k] = e_row[f - e_start];
                     }
                 }
+            }
+            if (outside) {  // the planes hold zeros for what keep_outliers takes
+                float v[16];
+#pragma unroll
+                for (uint32_t k = 0; k < 16; ++k) v[k] = staged_value<E>(x[k]) * f1 * f2;
+                const uint32_t taken = keep_outliers(lists, v, b, tile, nst * 4u, t / 16u);
+#pragma unroll
+                for (uint32_t k = 0; k < 16; ++k) x[k] = taken >> k & 1u ? 0u : x[k];
             }
             // digits of 2^e x, features of even j four times as large (they meet A's 1 and 2, the others its 4 and 8)
             uint32_t d[16];
