@@ -18,19 +18,19 @@
 //     beside one of 1 in bf16, N(0, 2^-8) 2.9e-7 / 7.6e-8 / 7.6e-8, N(0, 2^-16) 1.7e-5 / 4.4e-7 / 1.2e-7, uniform in 2^-30..2^-29
 //     1.7e-7 / 1.5e-6 / 1.3e-7, all of 2^-28 3.6e-7 / 3.8e-6 / 1.1e-7; 6,000,001 features, N(0, 2^-16) 9.0e-5 / 1.2e-6 / 8.6e-8,
 //     uniform 3.2e-7 / 3.9e-6 / 9.4e-8; N(0, 1) without the one 3.2e-6 / 7.4e-8 / 7.4e-8.
-//     us a call, the same three, one such element to a row: 16 x 1,000,003 bf16 -> 4096 371 / 237 / 249, 32 rows 400 / 350 / 384;
-//     without any, for the second reading of the rows' sums of squares, 16 x 2,796,202 fp16 -> 4096 1013 / 616 / 620, 16 x 40,001
-//     -> 8192 58 / 49 / 53, 32 x 1,048,576 -> 2048 225 / 219 / 224.
+//     us a call, the same three, one such element to a row: 16 x 1,000,003 bf16 -> 4096 371 / 238 / 248, 32 rows 399 / 351 / 375,
+//     17 x 330,003 -> 1536 79 / 64 / 75; without any, 16 x 2,796,202 fp16 -> 4096 1013 / 617 / 625, 16 x 40,001 -> 8192
+//     58 / 49 / 52, 32 x 1,048,576 fp32 -> 2048 236 / 233 / 235.
 //   * 2^i differs from word to word (bit 2j + h of a draw's byte: feature pair j, column parity h; two of the four j after
 //     a shift by four).  The column's factor 2^h is undone at the end, the features' 2^(2 (j & 1)) in the staging: even j are
 //     staged four times as large.
 //   * What bounds it.  Up to 16 rows the integer pipe, 82 % busy with 11 instructions per 16 x 32 entries (4 of the 7 of a draw,
 //     5 to spread it, 2 of hand-shakes; 35 instructions in all with a 16-bit operand, now 18): without its MMAs the kernel takes
-//     95 % of its time.  us a call, 16-bit operand -> this: 2,796,202 fp16 features -> 4096 1043 -> 647, 1,000,003 -> 8192
-//     753 -> 455, 10,000,001 bf16 -> 8192 7004 -> 4022; one row of 1,000,003 -> 2048 218 -> 142.
+//     95 % of its time.  us a call, 16-bit operand -> this: 2,796,202 fp16 features -> 4096 1013 -> 625, 1,000,003 -> 8192
+//     721 -> 432, 10,000,001 bf16 -> 8192 6950 -> 4014; one row of 1,000,003 -> 2048 195 -> 120.
 //     From 17 to 32 rows the accumulators leave room for one CTA per SM, of four groups, and the MMAs bound it (tensor pipe
 //     75 % busy at 24 rows, 85 at 32, with 7 TB/s from the L2; without generating it takes as long): 17 rows x 1,000,003 bf16
-//     -> 8192 780 -> 559, 24 rows fp16 -> 2048 239 -> 200, 32 rows x 2,796,202 -> 4096 1111 -> 926.
+//     -> 8192 757 -> 543, 24 rows fp16 -> 2048 213 -> 180, 32 rows x 2,796,202 -> 4096 1102 -> 934.
 //   * The groups' slots change hands together, and so do their boxes: one warp issues the MMAs beside busy generators, and a
 //     hand-over costs it some 300 cycles whatever it covers.  With barriers of each group's own 16 rows took 2 % longer (659
 //     us for 647), and four groups of 32-feature slots to a CTA 1023 us; with common ones 693, so two of 64 they stay.
@@ -55,14 +55,15 @@ constexpr uint32_t BITS_MAX_CHAIN = 32768;    // stages of a CTA: |digit| <= 128
 __host__ __device__ constexpr uint32_t bits_groups(uint32_t rows) { return rows <= 16u ? 2u : 4u; }
 __host__ __device__ constexpr uint32_t bits_batch(uint32_t rows) { return rows <= 16u ? 4u : 2u; }
 constexpr uint32_t BITS_MAX_SLICES = 256;     // of a row in absmax_kernel
+constexpr uint32_t BITS_RUNS = 4;             // runs of 512 features that a warp of stage_bits_kernel takes at most
 constexpr float BITS_RANGE = 268435456.0f;     // 2^28: a rounded gradient stays below
 constexpr int BITS_INF = 0x7ffffffe, BITS_NAN = 0x7fffffff;   // BitsParams::row_exp of a row that holds one
 
-// 16 features of a row of which some are too large for the planes, in the list of their place in a tile (which of 16
-// features): 2^e times each of those, the others zero.
-struct Outliers {
-    uint32_t next, row;         // 1 + the index of the next record of the list, 0: the last
-    float q[16];
+// An element that is too large for the planes, in the list of its place in a tile (which of 16 features): 2^e times it.
+struct __align__(16) Outlier {
+    uint32_t next;              // 1 + the index of the next of the list, 0: the last
+    uint32_t row, feature;      // of the 16
+    float q;
 };
 
 struct BitsParams {
@@ -72,8 +73,8 @@ struct BitsParams {
     const uint32_t* infs;       // [tiles][rows] infinities among them (rows of BITS_INF only)
     const int* row_exp;         // [rows] 4 q is 2^row_exp times the gradient; or BITS_INF, BITS_NAN
     const uint32_t* last_out;   // [tiles] 1 + the last 16 features that have outliers, 0: none
-    const uint32_t* heads;      // [tiles][4 nst] 1 + their first record, 0: none
-    const Outliers* outliers;
+    const uint32_t* heads;      // [tiles][4 nst] 1 + the first of them, 0: none
+    const Outlier* outliers;
     uint32_t N, seed;
     uint32_t B, rows;           // rows in this launch, and rounded up to 8
     uint32_t nst;               // pipeline stages per feature tile, even
@@ -270,17 +271,12 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
                         for (uint32_t k = 0; k < k1; ++k) {
                             const uint32_t c = gen_bits(st0, st1);
                             for (uint32_t r = __shfl_sync(0xffffffffu, first, k); r != 0u;) {
-                                const Outliers& o = p.outliers[r - 1u];
-                                long long v0 = 0, v1 = 0;
-                                for (uint32_t f = 0; f < 16u; ++f) {
-                                    const long long q = (long long)o.q[f];
-                                    const uint32_t at = 8u * ((f & 1u) | (f >> 3 << 1)) + 2u * ((f & 7u) >> 1);
-                                    v0 += c >> at & 1u ? q : -q;
-                                    v1 += c >> at & 2u ? q : -q;
-                                }
+                                const Outlier o = p.outliers[r - 1u];
+                                const long long q = (long long)o.q;
+                                const uint32_t at = 8u * ((o.feature & 1u) | (o.feature >> 3 << 1)) + 2u * ((o.feature & 7u) >> 1);
                                 unsigned long long* const sum = reinterpret_cast<unsigned long long*>(&extra[o.row][2u * pair]);
-                                atomicAdd(sum, (unsigned long long)v0);
-                                atomicAdd(sum + 1, (unsigned long long)v1);
+                                atomicAdd(sum, (unsigned long long)(c >> at & 1u ? q : -q));
+                                atomicAdd(sum + 1, (unsigned long long)(c >> at & 2u ? q : -q));
                                 r = o.next;
                             }
                         }
@@ -289,45 +285,53 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
                 meet(1);
             }
             float* dst = p.partials + (size_t)blockIdx.y * p.B * p.N + n_out;
+            // twice: with the sums' additions in it the one loop takes 0.3 us longer (16 x 40,001 -> 8192, eight CTAs an SM's half
+            // one after another, 53.3 -> 51.3 us)
+            auto finish = [&](auto more) {
 #pragma unroll EARLY ? 2 : 1
-            for (uint32_t turn = 0; turn < 2u; ++turn) {
-                const uint32_t b4 = 4u * (g + NG * turn);
-                if (b4 >= p.B || !ok) break;
-                const Rows known = EARLY ? early[turn] : rows_from(b4);
-                uint32_t d[2][BITS_PLANES][4];
+                for (uint32_t turn = 0; turn < 2u; ++turn) {
+                    const uint32_t b4 = 4u * (g + NG * turn);
+                    if (b4 >= p.B || !ok) break;
+                    const Rows known = EARLY ? early[turn] : rows_from(b4);
+                    uint32_t d[2][BITS_PLANES][4];
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
+                    for (int h = 0; h < 2; ++h)
 #pragma unroll
-                    for (int pl = 0; pl < (int)BITS_PLANES; ++pl)
-                        tmem_ld_x4(tmem_acc + h * brows + pl * p.rows + b4, d[h][pl]);
-                tmem_wait_ld();
+                        for (int pl = 0; pl < (int)BITS_PLANES; ++pl)
+                            tmem_ld_x4(tmem_acc + h * brows + pl * p.rows + b4, d[h][pl]);
+                    tmem_wait_ld();
 #pragma unroll
-                for (uint32_t j = 0; j < 4; ++j) {
-                    const uint32_t b = b4 + j;
-                    const long long total = __shfl_sync(0xffffffffu, known.sum, j);
-                    const uint32_t infs = __shfl_sync(0xffffffffu, known.ninf, j);
-                    const int e = __shfl_sync(0xffffffffu, known.exps, j);
-                    if (b >= p.B) break;
-                    float2 v;
+                    for (uint32_t j = 0; j < 4; ++j) {
+                        const uint32_t b = b4 + j;
+                        const long long total = __shfl_sync(0xffffffffu, known.sum, j);
+                        const uint32_t infs = __shfl_sync(0xffffffffu, known.ninf, j);
+                        const int e = __shfl_sync(0xffffffffu, known.exps, j);
+                        if (b >= p.B) break;
+                        float2 v;
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        long long s = 0;  // 4 2^h times the sum of q over the set bits
+                        for (int h = 0; h < 2; ++h) {
+                            long long s = 0;  // 4 2^h times the sum of q over the set bits
 #pragma unroll
-                        for (int pl = (int)BITS_PLANES - 1; pl >= 0; --pl) s = s * 256 + (int)d[h][pl][j];
-                        s = (h == 0 ? 2 * s : s) - 4 * total;
-                        if (outside) s += 4 * extra[b][2u * pair + h];
-                        float r;
-                        if (e < BITS_INF)
-                            r = scale_by(__ll2float_rn(s), -e);
-                        else if (e == BITS_INF)
-                            r = infs == 0u ? 0.0f : s == (long long)infs * 4 ? INFINITY : s == -(long long)infs * 4 ? -INFINITY : NAN;
-                        else
-                            r = NAN;
-                        (h == 0 ? v.x : v.y) = r;
+                            for (int pl = (int)BITS_PLANES - 1; pl >= 0; --pl) s = s * 256 + (int)d[h][pl][j];
+                            s = (h == 0 ? 2 * s : s) - 4 * total;
+                            if constexpr (decltype(more)::value) s += 4 * extra[b][2u * pair + h];
+                            float r;
+                            if (e < BITS_INF)
+                                r = scale_by(__ll2float_rn(s), -e);
+                            else if (e == BITS_INF)
+                                r = infs == 0u ? 0.0f : s == (long long)infs * 4 ? INFINITY : s == -(long long)infs * 4 ? -INFINITY : NAN;
+                            else
+                                r = NAN;
+                            (h == 0 ? v.x : v.y) = r;
+                        }
+                        __stcg(reinterpret_cast<float2*>(dst + (size_t)b * p.N), v);
                     }
-                    __stcg(reinterpret_cast<float2*>(dst + (size_t)b * p.N), v);
                 }
-            }
+            };
+            if (outside)
+                finish(std::true_type{});
+            else
+                finish(std::false_type{});
         }
     } else {
         // stages of every group (cnt[] does not increase with g)
@@ -435,7 +439,7 @@ enum class Elem { F32, F16, BF16 };
 template <Elem E>
 using elem_t = typename std::conditional<E == Elem::F32, float, uint16_t>::type;
 
-// Largest magnitude and sum of squares of slice blockIdx.x of row blockIdx.y.  The former as the bits of the element type
+// Largest magnitude and sum of squares of a slice of row blockIdx.x.  The former as the bits of the element type
 // (monotonic, infinity above every number and NaN above infinity); of the latter three for bf16, whose squares fp32 does not
 // hold: of the elements, and of 2^-90 and 2^90 times them.  Also clears what the staging adds to.  The ends of a parameter go
 // element by element.  Bound by memory: 16 x 2,796,202 fp16 (89 MB) in 20 us.
@@ -509,9 +513,10 @@ absmax_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ segs, 
     cudaTriggerProgrammaticLaunchCompletion();
     constexpr uint32_t SUMS = RowStats<E>::SUMS;
     __shared__ RowStats<E> part[8];
+    const uint32_t row = blockIdx.x, part_of_row = gridDim.y - 1u - blockIdx.y;
     const uint32_t id = (blockIdx.y * gridDim.x + blockIdx.x) * 256u + threadIdx.x;
     for (uint32_t i = id; i < clear_n; i += gridDim.x * gridDim.y * 256u) clear[i] = make_uint4(0u, 0u, 0u, 0u);
-    const uint64_t f0 = blockIdx.x * slice, f1 = min(F, f0 + slice);
+    const uint64_t f0 = part_of_row * slice, f1 = min(F, f0 + slice);
     RowStats<E> st = {};
     if (SEG) {
         uint32_t lo = 0, hi = nsegs;  // last parameter whose start is <= f0
@@ -525,11 +530,11 @@ absmax_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ segs, 
         for (uint64_t f = f0; f < f1; ++lo) {
             const SegDev s = segs[lo];
             const uint64_t end = min(f1, s.start + s.numel);
-            add_run(st, static_cast<const elem_t<E>*>(s.ptr) + (row0 + blockIdx.y) * s.stride + (f - s.start), end - f);
+            add_run(st, static_cast<const elem_t<E>*>(s.ptr) + (row0 + row) * s.stride + (f - s.start), end - f);
             f = end;
         }
     } else {
-        add_run(st, g + (uint64_t)blockIdx.y * ld + f0, f1 - f0);
+        add_run(st, g + (uint64_t)row * ld + f0, f1 - f0);
     }
     if (E != Elem::F32) st.max_bits = max(st.max_bits & 0xffffu, st.max_bits >> 16);
     st.max_bits = __reduce_max_sync(0xffffffffu, st.max_bits);
@@ -546,7 +551,7 @@ absmax_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ segs, 
 #pragma unroll
             for (uint32_t j = 0; j < SUMS; ++j) st.sums[j] += part[w].sums[j];
         }
-        const uint32_t at = blockIdx.y * gridDim.x + blockIdx.x;
+        const uint32_t at = row * gridDim.y + part_of_row;
         maxima[at] = st.max_bits;
 #pragma unroll
         for (uint32_t j = 0; j < SUMS; ++j) squares[at * SUMS + j] = st.sums[j];
@@ -597,71 +602,53 @@ __device__ __forceinline__ int row_exponent(uint32_t max_bits, const float (&sum
 
 struct OutlierLists {
     uint32_t *count, *last, *heads;  // records in use; BitsParams::last_out, heads
-    Outliers* outliers;
+    Outlier* outliers;
     uint32_t most;
 };
-
-// Of 16 scaled elements of row b, place `place` of a tile, those that are too large for the planes, as a mask; they get a record.
-__device__ __noinline__ uint32_t keep_outliers(const OutlierLists& lists, const float (&v)[16], uint32_t b, uint32_t tile,
-                                               uint32_t places, uint32_t place) {
-    uint32_t taken = 0;
-    for (uint32_t k = 0; k < 16; ++k) taken |= (uint32_t)(fabsf(v[k]) >= BITS_RANGE) << k;
-    if (taken == 0u) return 0u;
-    const uint32_t r = atomicAdd(lists.count, 1u);
-    if (r >= lists.most) return 0u;  // never (row_exponent)
-    Outliers& o = lists.outliers[r];
-    o.row = b;
-    for (uint32_t k = 0; k < 16; ++k) o.q[k] = taken >> k & 1u ? v[k] : 0.0f;
-    o.next = atomicExch(lists.heads + (size_t)tile * places + place, r + 1u);
-    atomicMax(lists.last + tile, place + 1u);
-    return taken;
-}
 
 // stage_kernel for project_bits_kernel: staged[tile][128 features][plane][row].  A warp takes runs of 512 features of one
 // row, a lane 16 consecutive features, of which it makes the 16 bytes of every plane (gen_bits_pair says in which order).
 // Bound by memory, two bytes read (fp16) and four written an element, and next to that by 14 instructions an element:
-// 16 x 2,796,202 fp16 in 50 us.
+// 16 x 2,796,202 fp16 in 57 us.  A CTA takes the scale of its rows once and runs
+// of 512 features four at a time (16 x 592,003 fp16 14 us; 18 with eight runs to a CTA and the scale looked up for each).
 template <Elem E, bool SEG>
-__global__ void __launch_bounds__(256, SEG ? 4 : 5)
+__global__ void __launch_bounds__(256, !SEG && E == Elem::BF16 ? 5 : 4)
 stage_bits_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ segs, uint32_t nsegs, uint64_t row0,
                   uint8_t* __restrict__ staged, const uint32_t* __restrict__ maxima, const float* __restrict__ squares,
                   uint32_t slices, long long* __restrict__ sums, uint32_t* __restrict__ infs, int* __restrict__ row_exp,
-                  const OutlierLists lists, float half_sqrt_f, uint32_t B, uint32_t rows, uint64_t F, uint64_t ld, uint32_t fts, uint32_t nst, uint32_t tiles) {
+                  const OutlierLists lists, float half_sqrt_f, uint32_t B, uint32_t rows, uint64_t F, uint64_t ld,
+                  uint32_t fts, uint32_t nst, uint32_t tiles, uint32_t each) {
     using In = elem_t<E>;
     cudaTriggerProgrammaticLaunchCompletion();  // see launch_after
     constexpr uint32_t RUN = 512u, V = 16u / sizeof(In), LOADS = 16u / V;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t runs = (nst * BITS_K + RUN - 1u) / RUN, blocks = (runs + RUNS_PER_BLOCK - 1u) / RUNS_PER_BLOCK;
-    const uint32_t b_hi_n = rows / 8u;
-    const uint64_t total = (uint64_t)tiles * blocks * b_hi_n;
+    const uint32_t runs = (nst * BITS_K + RUN - 1u) / RUN, blocks = (runs + each - 1u) / each;
+    // a CTA stays with eight rows, of which it looks up the scale once
+    const uint32_t b_hi_n = rows / 8u, b = blockIdx.x % b_hi_n * 8u + warp;
+    const uint64_t total = (uint64_t)tiles * blocks;
     cudaGridDependencySynchronize();  // the maxima, and the cleared sums
-    uint32_t b_of = 0xffffffffu;
-    int e = 0;
-    bool outside = false;        // some elements of the row may be too large
-    float f1 = 1.0f, f2 = 1.0f;  // 2^e in two factors (bf16 reaches beyond one)
-    for (uint64_t i = blockIdx.x; i < total; i += gridDim.x) {
-        const uint64_t q = i / blocks;
-        const uint32_t run0 = (uint32_t)(i - q * blocks) * RUNS_PER_BLOCK;
-        const uint32_t tile = (uint32_t)(q / b_hi_n), b = ((uint32_t)q - tile * b_hi_n) * 8u + warp;
-        if (b != b_of) {
-            b_of = b;
-            RowStats<E> st = {};
-            if (b < B) {
-                for (uint32_t s = lane; s < slices; s += 32u) {
-                    st.max_bits = max(st.max_bits, maxima[b * slices + s]);
+    RowStats<E> st = {};
+    if (b < B) {
 #pragma unroll
-                    for (uint32_t j = 0; j < RowStats<E>::SUMS; ++j) st.sums[j] += squares[(b * slices + s) * RowStats<E>::SUMS + j];
-                }
-            }
+        for (uint32_t k = 0; k < BITS_MAX_SLICES / 32u; ++k) {  // all fetched at once
+            const uint32_t s = k * 32u + lane;
+            if (s >= slices) continue;
+            st.max_bits = max(st.max_bits, maxima[b * slices + s]);
 #pragma unroll
-            for (uint32_t j = 0; j < RowStats<E>::SUMS; ++j)
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) st.sums[j] += __shfl_xor_sync(0xffffffffu, st.sums[j], o);
-            e = row_exponent<E>(__reduce_max_sync(0xffffffffu, st.max_bits), st.sums, half_sqrt_f, outside);
-            const int a = e >= BITS_INF ? 0 : E == Elem::BF16 ? e / 2 : e, c = e < BITS_INF ? e - a : 0;
-            f1 = __int_as_float((127 + a) << 23);
-            f2 = __int_as_float((127 + c) << 23);
+            for (uint32_t j = 0; j < RowStats<E>::SUMS; ++j) st.sums[j] += squares[(b * slices + s) * RowStats<E>::SUMS + j];
         }
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < RowStats<E>::SUMS; ++j)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) st.sums[j] += __shfl_xor_sync(0xffffffffu, st.sums[j], o);
+    bool outside;  // some elements of the row may be too large
+    const int e = row_exponent<E>(__reduce_max_sync(0xffffffffu, st.max_bits), st.sums, half_sqrt_f, outside);
+    // 2^e in two factors (bf16 reaches beyond one)
+    const int e1 = e >= BITS_INF ? 0 : E == Elem::BF16 ? e / 2 : e, e2 = e < BITS_INF ? e - e1 : 0;
+    const float f1 = __int_as_float((127 + e1) << 23), f2 = __int_as_float((127 + e2) << 23);
+    for (uint64_t i = blockIdx.x / b_hi_n; i < total; i += gridDim.x / b_hi_n) {
+        const uint32_t tile = (uint32_t)(i / blocks), run0 = (uint32_t)(i - (uint64_t)tile * blocks) * each;
         if (tile == 0 && run0 == 0 && lane == 0) row_exp[b] = e < BITS_INF ? e + 2 : e;
         uint8_t* const out_tile = staged + (uint64_t)tile * nst * (BITS_PLANES * rows * BITS_K);
         long long sum = 0;
@@ -669,7 +656,7 @@ stage_bits_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ se
         uint32_t seg = 0;
         uint64_t s_start = 0, s_end = SEG ? 0 : F;
         const In* s_row = SEG ? nullptr : g + (uint64_t)b * ld;
-        for (uint32_t run = run0; run < min(run0 + RUNS_PER_BLOCK, runs); ++run) {
+        for (uint32_t run = run0; run < min(run0 + each, runs); ++run) {
             const uint32_t t0 = run * RUN, t = t0 + lane * 16u;
             const uint64_t f0 = (uint64_t)tile * fts + t0;
             const bool live = b < B && f0 < F && t0 < fts;
@@ -738,11 +725,22 @@ stage_bits_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ se
                     }
                 }
             }
-            if (outside) {  // the planes hold zeros for what keep_outliers takes
-                float v[16];
+            if (outside) {  // the planes hold zeros for what goes to the lists
+                auto scaled = [&](uint32_t bits) { return staged_value<E>(bits) * f1 * f2; };
+                uint32_t taken = 0;
 #pragma unroll
-                for (uint32_t k = 0; k < 16; ++k) v[k] = staged_value<E>(x[k]) * f1 * f2;
-                const uint32_t taken = keep_outliers(lists, v, b, tile, nst * 4u, t / 16u);
+                for (uint32_t k = 0; k < 16; ++k) taken |= (uint32_t)(fabsf(scaled(x[k])) >= BITS_RANGE) << k;
+                for (uint32_t left = taken; left != 0u; left &= left - 1u) {
+                    const uint32_t one = left & (0u - left);
+                    uint32_t bits = 0;
+#pragma unroll
+                    for (uint32_t k = 0; k < 16; ++k) bits |= one == 1u << k ? x[k] : 0u;
+                    const uint32_t r = atomicAdd(lists.count, 1u);
+                    if (r >= lists.most) break;  // never (row_exponent)
+                    uint32_t* const head = lists.heads + (size_t)tile * nst * 4u + t / 16u;
+                    lists.outliers[r] = {atomicExch(head, r + 1u), b, (uint32_t)__ffs((int)one) - 1u, scaled(bits)};
+                    atomicMax(lists.last + tile, t / 16u + 1u);
+                }
 #pragma unroll
                 for (uint32_t k = 0; k < 16; ++k) x[k] = taken >> k & 1u ? 0u : x[k];
             }
