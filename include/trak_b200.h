@@ -97,6 +97,12 @@ int tb_selftest_wait_timeout(int device, void *stream, uint32_t limit_ms);
 size_t tb_project_workspace_bytes(int dtype, int64_t B, int64_t F, uint32_t N,
                                   uint32_t num_feature_tiles);
 
+/* The least workspace that the projections below run in, of a gradient matrix (nsegs = 0) or of nsegs parameters.
+ * tb_project_workspace_bytes names no matrix type and asks for what a Rademacher matrix made on the fly can use: up to
+ * twice as much for up to 32 rows of many features.  A Gaussian or stored matrix never uses more than this. */
+size_t tb_project_least_workspace_bytes(int dtype, int64_t B, int64_t F, uint32_t N, uint32_t num_feature_tiles,
+                                        int32_t nsegs);
+
 int tb_project(int device, void *stream, const void *grads, int dtype, int64_t B, int64_t F,
                int64_t ld, float *out, int64_t ld_out, uint32_t N, uint32_t seed,
                uint32_t num_feature_tiles, int proj_type, float alpha, int accumulate, void *ws,

@@ -42,6 +42,7 @@ SIGNATURES = {
     "tb_selftest_wait_timeout": (_i, [_i, _vp, _u32]),
     "tb_selftest_sqrt": (_i, [_i, _vp, ctypes.c_uint64, ctypes.c_uint64, _vp]),
     "tb_project_workspace_bytes": (_sz, [_i, _i64, _i64, _u32, _u32]),
+    "tb_project_least_workspace_bytes": (_sz, [_i, _i64, _i64, _u32, _u32, _i32]),
     "tb_project_grid": (_i, [_i64, _i64, _u32, _u32, _i, _i, ctypes.POINTER(_u32)]),
     "tb_profile_events": (_i, [_vp, _vp]),
     "tb_project_segments_workspace_bytes": (_sz, [_i, _i64, _i64, _u32, _u32, _i32]),
@@ -168,11 +169,30 @@ class Workspaces:
     def __init__(self, most_kept: int = 8):   # per process; streams come and go, their buffers should not pile up
         self.most_kept, self.kept = most_kept, {}
 
-    def take(self, device: torch.device, stream: int, nbytes: int) -> torch.Tensor:
+    def take(self, device: torch.device, stream: int, nbytes: int, least=None) -> torch.Tensor:
+        """A buffer of ``nbytes``; of ``least()``, where that is given, when the device has no room for more."""
         ws = self.kept.pop((device.index, stream), None)
-        if ws is None or ws.numel() < nbytes:
+        size = 0 if ws is None else ws.numel()
+        if size < nbytes and least is not None and least() < nbytes:
+            if self.room(device) + size < nbytes:
+                nbytes = least()
+            else:
+                ws, size = None, 0   # given up before its successor is allocated
+                try:
+                    return torch.empty(nbytes, dtype=torch.uint8, device=device)
+                except torch.cuda.OutOfMemoryError:
+                    nbytes = least()
+        if size < nbytes:
+            ws = None
             ws = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
         return ws
+
+    @staticmethod
+    def room(device: torch.device) -> int:
+        """Bytes that can be allocated, fragmentation apart (which ``take`` finds out by trying)."""
+        if device.type != "cuda" or torch.cuda.is_current_stream_capturing():
+            return 1 << 62
+        return torch.cuda.mem_get_info(device)[0] + torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
 
     def give(self, device: torch.device, stream: int, ws: torch.Tensor) -> None:
         self.kept[(device.index, stream)] = ws  # most recently used last
