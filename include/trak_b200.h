@@ -87,8 +87,12 @@ int tb_selftest_wait_timeout(int device, void *stream, uint32_t limit_ms);
  *           fast_jl/fast_jl.cu:42
  *   alpha, accumulate   extras: fold 1/sqrt(D) and sum parameter chunks
  *           without another pass (trak/traker.py:426, trak/projectors.py:490)
- *   ws      workspace of at least tb_project_workspace_bytes(...) bytes,
- *           256-byte aligned; any B is accepted (no 8/16/32 variants).  The
+ *   ws      workspace of at least tb_project_least_workspace_bytes(...)
+ *           bytes, 256-byte aligned; any B is accepted (no 8/16/32 variants).
+ *           With tb_project_workspace_bytes(...) a last pass of up to 32
+ *           Rademacher rows may run on byte operands, faster and with a
+ *           smaller error; so ws_bytes can decide how a result is rounded
+ *           (the same sizes always give the same bits).  The
  *           batch is walked in passes that each regenerate the matrix once:
  *           up to 256 rows per pass for TB_RADEMACHER, up to 512 for
  *           TB_NORMAL (whose generation is what the projection costs), so
@@ -231,8 +235,10 @@ int tb_finalize_scores(int device, void *stream, const float *score_sum, int64_t
                        void *out, int out_dtype, int64_t ld_out);
 
 /* ---- projection without a caller-provided workspace ------------------------------
- * No counterpart in the reference.  Same arguments and result as tb_project, minus
- * `ws` / `ws_bytes`: the scratch lives in a fixed array inside the loaded library
+ * No counterpart in the reference.  Same arguments and result as tb_project with
+ * TB_PROJECT_STATIC_SCRATCH_BYTES of workspace (so up to 32 Rademacher rows that
+ * would need more than that for byte operands are rounded as with the least
+ * workspace): the scratch lives in a fixed array inside the loaded library
  * (TB_PROJECT_STATIC_SCRATCH_BYTES on every GPU that loads it, held until the
  * process exits).  Meant for hosts that cannot allocate device memory themselves,
  * e.g. a plugin in a process whose device memory already belongs to another
@@ -240,8 +246,8 @@ int tb_finalize_scores(int device, void *stream, const float *score_sum, int64_t
  * synchronisation of cudaMalloc / cudaFree.  The call allocates neither device nor
  * pinned host memory (the process's first tb_stream_status takes a page of the latter).
  *
- *   - shapes with tb_project_workspace_bytes(...) > TB_PROJECT_STATIC_SCRATCH_BYTES
- *     are refused with TB_ERR_SCRATCH_LIMIT
+ *   - shapes with tb_project_least_workspace_bytes(..., 0) >
+ *     TB_PROJECT_STATIC_SCRATCH_BYTES are refused with TB_ERR_SCRATCH_LIMIT
  *   - arguments are checked first, with tb_project's codes; a device that is not a
  *     B200-class GPU gives TB_ERR_UNSUPPORTED
  *   - the first call on a device looks up the array's device address (a one-time

@@ -109,3 +109,16 @@ def test_projections_ask_for_what_they_use(cuda, monkeypatch):
     # 16-bit operands: chains of 63 stages of 16-feature steps drift by less than 252 * 2^-24 of a sum
     worst = ((small_out - bytes_out).norm(dim=1) / bytes_out.norm(dim=1)).max()
     assert 0 < worst <= 2e-5
+
+
+def test_static_scratch_takes_what_fits_the_least_workspace():
+    """By the least size, not by the one with byte operands.  Device 63 does not exist, so nothing is launched."""
+    lib, limit, N, T = _lib.lib(), 32 << 20, 512, 148
+
+    def rc(B, F):
+        return lib.tb_project_static(63, None, 0x1000, 0, B, F, F, 0x2000, N, N, 0, T, 0, 1.0, 0)
+    for B, F in ((16, 600_011), (16, 870_000), (4, 592_003)):   # larger with byte operands than the scratch, or not
+        assert lib.tb_project_least_workspace_bytes(0, B, F, N, T, 0) <= limit and rc(B, F) not in (0, 9)
+    assert lib.tb_project_workspace_bytes(0, 16, 600_011, N, T) > limit
+    for B, F in ((16, 900_000), (128, 2_000_000)):
+        assert lib.tb_project_least_workspace_bytes(0, B, F, N, T, 0) > limit and rc(B, F) == 9
