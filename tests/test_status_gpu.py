@@ -181,3 +181,31 @@ def test_the_first_read_beside_another_threads_capture(cuda):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     p = subprocess.run([sys.executable, "-c", FIRST_READ_UNDER_A_CAPTURE], cwd=root, capture_output=True, text=True, timeout=300)
     assert p.returncode == 0, p.stderr
+
+
+def test_a_call_answers_for_itself_and_leaves_a_later_failure_to_its_own_caller(cuda, job):
+    """Thread A projects; then thread B's inverse, on a stream of its own, fails; A reads its status first."""
+    lib, g, out, ws = job
+    a, b = torch.cuda.Stream(cuda), torch.cuda.Stream(cuda)
+    assert lib.tb_stream_status(cuda.index, b.cuda_stream, None) == 0   # kernels repeat failures to the host from here on
+    indefinite = -torch.eye(64, device=cuda)
+    scratch = torch.empty(lib.tb_spd_inverse_workspace_bytes(64), dtype=torch.uint8, device=cuda)
+    torch.cuda.synchronize()
+    with ThreadPoolExecutor(1) as thread_a, ThreadPoolExecutor(1) as thread_b:
+        def project():
+            with torch.cuda.stream(a):
+                return _call(lib, cuda, "tb_project", g, out, ws)
+
+        def invert():
+            return lib.tb_spd_inverse(cuda.index, b.cuda_stream, indefinite.data_ptr(), 64, 64, 0.0, 0, None,
+                                      scratch.data_ptr(), scratch.numel())
+
+        def status(stream):
+            return lib.tb_stream_status(cuda.index, stream.cuda_stream, None)
+        assert thread_a.submit(project).result() == 0
+        a.synchronize()
+        assert thread_b.submit(invert).result() == 0
+        b.synchronize()
+        assert thread_a.submit(status, a).result() == 0
+        assert thread_b.submit(status, b).result() == 10   # TB_ERR_NOT_SPD
+        assert thread_b.submit(status, b).result() == 0

@@ -123,11 +123,12 @@ int take_note(StatusNote* note) {
     note->word = words + note->call % STATUS_WORDS;
     return TB_OK;
 }
-// After the kernel that stores it has ended: false where a later call has the word by now.
+// After the kernel that stores it has ended: false where a later call has the word by now, or may have (reads that need no word
+// take a number as well, so that an answer does not outlast a round of calls and reads).
 static bool read_note(const StatusNote& note, uint32_t* status) {
     const uint64_t v = *static_cast<volatile uint64_t*>(note.word);
     *status = (uint32_t)v;
-    return (uint32_t)(v >> 32) == note.call;
+    return (uint32_t)(v >> 32) == note.call && g_calls.load(std::memory_order_relaxed) - note.call < STATUS_WORDS;
 }
 
 // A word of mapped host memory per device that a kernel stores the code to beside the device's own (record_status), so that a
@@ -292,10 +293,15 @@ int tb_stream_status(int device, void* stream_, uint32_t* detail) {
     int rc = tb::select_device(device, nullptr);
     if (rc != TB_OK) return rc;
     const tb::StatusNote note = tb::t_armed.note;
-    uint32_t code = 0, *mirror = tb::g_mirror[device].load(std::memory_order_acquire);
-    if (!armed && (rc = tb::status_mirror(device, &mirror)) != TB_OK) return rc;
+    uint32_t code = 0, *mirror = nullptr;
+    if (!armed) {
+        if ((rc = tb::status_mirror(device, &mirror)) != TB_OK) return rc;
+        tb::g_calls.fetch_add(1, std::memory_order_relaxed);
+    }
     TB_CUDA(cudaStreamSynchronize(stream));
-    if ((armed && !tb::read_note(note, &code)) || code != 0 || (mirror && *static_cast<volatile uint32_t*>(mirror) != 0))
+    // A call that has published its status answers for itself: what another stream's kernels have recorded since is for their
+    // caller, and asking the device would take it from them.
+    if (armed ? !tb::read_note(note, &code) || code != 0 : *static_cast<volatile uint32_t*>(mirror) != 0)
         return tb_device_status(device, detail);
     if (detail) *detail = 0;
     return TB_OK;
