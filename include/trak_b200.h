@@ -210,9 +210,13 @@ int tb_gemm_nt(int device, void *stream, const void *A, int64_t lda, const void 
                int dtype, int64_t M, int64_t N, int64_t K, float *C, int64_t ldc,
                const float *row_scale, float alpha, int accumulate, void *ws, size_t ws_bytes);
 /* tb_gemm_nt in two steps, for a B that is not there yet: tb_gemm_nt_pack lays A out in the workspace, and
- * tb_gemm_nt_packed with the same workspace, type, M, N and K does the rest (ordered after it by the caller). */
+ * tb_gemm_nt_packed with the same workspace, type, M, N and K does the rest (ordered after it by the caller).
+ * tb_gemm_nt_pack_beside lays out the same on half of the SMs, for an A that would otherwise hold up what makes B on another
+ * stream (an inverse waits for whole SMs); it takes longer by itself. */
 int tb_gemm_nt_pack(int device, void *stream, const void *A, int64_t lda, int dtype, int64_t M, int64_t N, int64_t K,
                     void *ws, size_t ws_bytes);
+int tb_gemm_nt_pack_beside(int device, void *stream, const void *A, int64_t lda, int dtype, int64_t M, int64_t N, int64_t K,
+                           void *ws, size_t ws_bytes);
 int tb_gemm_nt_packed(int device, void *stream, const void *B, int64_t ldb, int dtype, int64_t M, int64_t N, int64_t K,
                       float *C, int64_t ldc, const float *row_scale, float alpha, int accumulate, void *ws,
                       size_t ws_bytes);

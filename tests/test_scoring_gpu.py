@@ -444,3 +444,31 @@ def test_gram_of_few_columns_at_the_edges_of_its_tiles(cuda, n, k):
     assert ((got.cpu().double() - want).abs() / (scale[:, None] * scale[None, :])).max() <= 2.0 ** -20
     assert torch.equal(got, got.T)
     assert (wide[:, 0] == 7).all() and (wide[:, k + 1:] == 7).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,K", [(129, 1025), (20_000, 512)])
+def test_packing_by_itself_takes_all_sms_and_beside_an_inverse_half_of_them(cuda, M, K, dtype):
+    """The launches' grids, as the profiler sees them; both leave the same operand."""
+    from torch.profiler import ProfilerActivity, profile
+    from trak_b200 import _lib
+    lib, N = _lib.lib(), 64
+    code = {torch.float16: 0, torch.bfloat16: 1, torch.float32: 2}[dtype]
+    a = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(dtype).to(cuda)
+    packed, launches = [], []
+    for name in ("tb_gemm_nt_pack", "tb_gemm_nt_pack_beside"):
+        ws = torch.zeros(lib.tb_gemm_nt_workspace_bytes(code, M, N, K), dtype=torch.uint8, device=cuda)
+        stream = torch.cuda.current_stream(cuda).cuda_stream
+
+        def call():
+            assert getattr(lib, name)(cuda.index, stream, a.data_ptr(), K, code, M, N, K, ws.data_ptr(), ws.numel()) == 0
+        call()
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            call()
+            torch.cuda.synchronize()
+        launches.append([e for e in prof.profiler.kineto_results.events() if "pack_" in e.name()])
+        packed.append(ws)
+    assert torch.equal(packed[0], packed[1])
+    threads = [[int("1024" in e.name()) for e in found] for found in launches]   # a template argument of the kernel's name
+    assert threads == [[0], [1]], [[e.name() for e in found] for found in launches]

@@ -54,6 +54,7 @@ SIGNATURES = {
     "tb_spd_inverse": (_i, [_i, _vp, _vp, _i64, _i64, _f, _i, _vp, _vp, _sz]),
     "tb_gemm_nt_workspace_bytes": (_sz, [_i, _i64, _i64, _i64]),
     "tb_gemm_nt_pack": (_i, [_i, _vp, _vp, _i64, _i, _i64, _i64, _i64, _vp, _sz]),
+    "tb_gemm_nt_pack_beside": (_i, [_i, _vp, _vp, _i64, _i, _i64, _i64, _i64, _vp, _sz]),
     "tb_gemm_nt_packed": (_i, [_i, _vp, _vp, _i64, _i, _i64, _i64, _i64, _vp, _i64, _vp, _f, _i, _vp, _sz]),
     "tb_gemm_nt": (_i, [_i, _vp, _vp, _i64, _vp, _i64, _i, _i64, _i64, _i64, _vp, _i64, _vp, _f, _i, _vp, _sz]),
     "tb_matrix_bytes": (_sz, [_i64, _u32, _u32]),

@@ -761,8 +761,8 @@ __global__ void __launch_bounds__(512) pack_cols_f32_kernel(const float* __restr
 //   value = src[R*ld + k]  (TRANS = false)  or  src[k*ld + R]  (TRANS = true: the operand is the
 //   transpose of the row-major source), zero outside [rows x K].
 // 16-bit types, copied as they are.
-template <bool TRANS>
-__global__ void pack_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ packed, uint64_t rows,
+template <bool TRANS, int THREADS = 256>
+__global__ void __launch_bounds__(THREADS) pack_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ packed, uint64_t rows,
                             uint64_t K, uint64_t ld, uint32_t rowblocks, uint32_t kblocks) {
     after_earlier_launch();
     // one thread = 8 consecutive k of one operand row (a 16-byte store)
@@ -922,7 +922,7 @@ static PackRows pack_rows_args(const void* src, uint64_t rows, uint64_t K, uint6
 // and 37.5; fp32 40,000 x 100 x 512 66.5 and 67.7, 60,000 x 100 x 512 81.6 and 80.7).
 static bool pack_early(uint64_t elements) { return elements < 25'000'000u; }
 
-// A packing that runs beside an inverse (tb_gemm_nt_pack) leaves it half of the SMs: CTAs of 1024 threads, one to every
+// A packing that runs beside an inverse (tb_gemm_nt_pack_beside) leaves it half of the SMs: CTAs of 1024 threads, one to every
 // second SM.  Spread over all of them it keeps the inverse's cooperative launch and its products,
 // which want whole SMs, waiting until it has ended.  get_x_xtx_inv of 50,000 x 2048 fp32 1671 -> 1638 us, 65,000 x 1024
 // 720 -> 704, 80,000 x 512 367 -> 356.
@@ -1003,8 +1003,8 @@ int launch_pack(const void* src, int dtype, bool trans, uint64_t rows, uint64_t 
         const uint32_t nb = (uint32_t)blocks;
         const uint16_t* s = static_cast<const uint16_t*>(src);
         if (beside && !trans)
-            return launch_after(pack_kernel<false>, beside_blocks((total + 255) / 256, sm_count), BESIDE_THREADS, 0, stream, false,
-                                s, packed, rows, K, ld, g.rowblocks, g.kblocks);
+            return launch_after(pack_kernel<false, BESIDE_THREADS>, beside_blocks((total + 255) / 256, sm_count), BESIDE_THREADS, 0,
+                                stream, false, s, packed, rows, K, ld, g.rowblocks, g.kblocks);
         return launch_after(trans ? pack_kernel<true> : pack_kernel<false>, nb, 256, 0, stream, trans || pack_early(rows * K), s,
                             packed, rows, K, ld, g.rowblocks, g.kblocks);
     }
@@ -1178,7 +1178,7 @@ size_t tb_gemm_nt_workspace_bytes(int dtype, int64_t M, int64_t N, int64_t K) {
 // The parts of tb_gemm_nt: A packed at the workspace's start, B packed behind it and the product.
 static int gemm_nt_parts(int device, void* stream_, const void* A, int64_t lda, const void* B, int64_t ldb, int dtype,
                          int64_t M, int64_t N, int64_t K, float* C, int64_t ldc, const float* row_scale, float alpha,
-                         int accumulate, void* ws, size_t ws_bytes) {
+                         int accumulate, void* ws, size_t ws_bytes, bool beside = false) {
     using namespace tb;
     if (dtype != TB_F16 && dtype != TB_BF16 && dtype != TB_F32) return TB_ERR_BAD_DTYPE;
     if (M <= 0 || N <= 0 || K <= 0 || lda < K || ldb < K || ldc < N || M > 0x7fffffff || N > 0x7fffffff)
@@ -1201,7 +1201,7 @@ static int gemm_nt_parts(int device, void* stream_, const void* A, int64_t lda, 
         rc = launch_pack_rows(pack_rows_args(A, M, K, lda, pa, ga), pack_rows_args(B, N, K, ldb, pb, gb), sm_count, stream);
         if (rc != TB_OK) return rc;
     } else {
-        if (A && (rc = launch_pack(A, dtype, false, M, K, lda, pa, ga, sm_count, stream, !B)) != TB_OK) return rc;
+        if (A && (rc = launch_pack(A, dtype, false, M, K, lda, pa, ga, sm_count, stream, beside)) != TB_OK) return rc;
         if (B && (rc = launch_pack(B, dtype, false, N, K, ldb, pb, gb, sm_count, stream)) != TB_OK) return rc;
     }
     if (!B) return TB_OK;
@@ -1219,6 +1219,11 @@ int tb_gemm_nt(int device, void* stream, const void* A, int64_t lda, const void*
 int tb_gemm_nt_pack(int device, void* stream, const void* A, int64_t lda, int dtype, int64_t M, int64_t N, int64_t K,
                     void* ws, size_t ws_bytes) {
     return gemm_nt_parts(device, stream, A, lda, nullptr, K, dtype, M, N, K, nullptr, N, nullptr, 1.0f, 0, ws, ws_bytes);
+}
+
+int tb_gemm_nt_pack_beside(int device, void* stream, const void* A, int64_t lda, int dtype, int64_t M, int64_t N, int64_t K,
+                           void* ws, size_t ws_bytes) {
+    return gemm_nt_parts(device, stream, A, lda, nullptr, K, dtype, M, N, K, nullptr, N, nullptr, 1.0f, 0, ws, ws_bytes, true);
 }
 
 int tb_gemm_nt_packed(int device, void* stream, const void* B, int64_t ldb, int dtype, int64_t M, int64_t N, int64_t K,

@@ -198,7 +198,8 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, row_scal
             alpha: float = 1.0, accumulate: bool = False, b_ready=None) -> torch.Tensor:
     """fp32 [M, N] = alpha * row_scale[:, None] * a @ b.T (+ out) for CUDA a [M, K], b [N, K].
 
-    ``b_ready`` makes the current stream wait for ``b``; it is called when ``a`` has been laid out for the product."""
+    ``b_ready`` makes the current stream wait for ``b``, which an inverse on another stream is making; it is called when
+    ``a`` has been laid out for the product, on half of the SMs."""
     if a.dtype != b.dtype:
         if b_ready is not None:
             b_ready()
@@ -227,7 +228,7 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, row_scal
         ws = _workspaces.take(dev, stream, lib.tb_gemm_nt_workspace_bytes(dt, M, N, K))
         scale = row_scale.data_ptr() if row_scale is not None else None
         if b_ready is not None:
-            _lib.check(lib.tb_gemm_nt_pack(dev.index, stream, a.data_ptr(), lda, dt, M, N, K, ws.data_ptr(), ws.numel()))
+            _lib.check(lib.tb_gemm_nt_pack_beside(dev.index, stream, a.data_ptr(), lda, dt, M, N, K, ws.data_ptr(), ws.numel()))
             b_ready()
             _lib.check(lib.tb_gemm_nt_packed(dev.index, stream, b.data_ptr(), ldb, dt, M, N, K, out.data_ptr(), ldc,
                                              scale, float(alpha), int(accumulate), ws.data_ptr(), ws.numel()))
