@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(256)
 absmax_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ segs, uint32_t nsegs, uint64_t row0,
               uint32_t* __restrict__ maxima, float* __restrict__ squares, uint4* __restrict__ clear, uint32_t clear_n, uint64_t F,
               uint64_t ld, uint64_t slice) {
-    cudaTriggerProgrammaticLaunchCompletion();
+    after_earlier_launch();
     constexpr uint32_t SUMS = RowStats<E>::SUMS;
     __shared__ RowStats<E> part[8];
     const uint32_t row = blockIdx.x, part_of_row = gridDim.y - 1u - blockIdx.y;
@@ -570,7 +570,8 @@ __device__ __forceinline__ float staged_value(uint32_t bits) {
 // finite.  Where that leaves steps so coarse that rounding could take more from the row than 2^-24 of its largest element and
 // 2^-22 of the norm of the rest, the exponent is the least that does not, and the elements that 2^e takes out of range go
 // beside the planes (`outside`): F / 4096 + 1 of them at most, since more would make that norm, and with it the steps, larger.
-// A number that comes as fp16 is a multiple of 2^-24: finer steps than that are never needed.
+// A number that comes as fp16 is a multiple of 2^-24: finer steps than that are never needed.  The last bits of the sums depend on
+// how a row is cut into parameters and aligned; a row whose bound they move across a power of two gets the next exponent.
 template <Elem E>
 __device__ __forceinline__ int row_exponent(uint32_t max_bits, const float (&sums)[RowStats<E>::SUMS], float half_sqrt_f, bool& outside) {
     const float m = staged_value<E>(max_bits);
