@@ -679,8 +679,9 @@ stage_bits_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ se
             const In* src = s_row + at;
             const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 15u);
             uint32_t x[16];  // bits of this lane's elements
-            if (live && t0 + RUN <= fts && RUN <= left && (off == 0u || (at >= V && RUN + V <= left))) {
-                // whole run inside the tile and one contiguous source, aligned vectors around it included
+            if (live && RUN <= left && (off == 0u || (at >= V && RUN + V <= left))) {
+                // whole run inside one contiguous source, aligned vectors around it included; a tile may end in it
+                if (t >= nst * BITS_K) continue;
                 const uint4* vec = reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(src) - off) + LOADS * lane;
                 uint4 c[LOADS + 1];
 #pragma unroll
@@ -702,6 +703,10 @@ stage_bits_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ se
                             x[j * 8u + 2u * k + 1u] = w[k] >> 16;
                         }
                     }
+                }
+                if (t0 + RUN > fts) {
+#pragma unroll
+                    for (uint32_t k = 0; k < 16; ++k) x[k] = t + k < fts ? x[k] : 0u;
                 }
             } else {
                 if (t >= nst * BITS_K) continue;
@@ -746,21 +751,28 @@ stage_bits_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ se
                 for (uint32_t k = 0; k < 16; ++k) x[k] = taken >> k & 1u ? 0u : x[k];
             }
             // digits of 2^e x, features of even j four times as large (they meet A's 1 and 2, the others its 4 and 8)
+            int q[16];
+            if (e < BITS_INF) {
+#pragma unroll
+                for (uint32_t k = 0; k < 16; ++k) {
+                    const float v = staged_value<E>(x[k]);
+                    q[k] = __float2int_rn(E == Elem::BF16 ? v * f1 * f2 : v * f1);
+                }
+            } else {
+#pragma unroll
+                for (uint32_t k = 0; k < 16; ++k) {
+                    const float v = staged_value<E>(x[k]);
+                    q[k] = v == INFINITY ? 1 : v == -INFINITY ? -1 : 0;
+                    ninf += q[k] != 0;
+                }
+            }
             uint32_t d[16];
             int part[2] = {0, 0};  // eight values of less than 2^28 each
 #pragma unroll
             for (uint32_t k = 0; k < 16; ++k) {
                 const bool four = ((k >> 1) & 1u) == 0u;
-                const float v = staged_value<E>(x[k]);
-                int qi;
-                if (e < BITS_INF) {
-                    qi = __float2int_rn(E == Elem::BF16 ? v * f1 * f2 : v * f1);
-                } else {
-                    qi = v == INFINITY ? 1 : v == -INFINITY ? -1 : 0;
-                    ninf += qi != 0;
-                }
-                part[k >> 3] += qi;
-                d[k] = (uint32_t)(four ? 4 * qi : qi) + 0x00808080u ^ 0x00808080u;  // bytes: balanced base-256 digits
+                part[k >> 3] += q[k];
+                d[k] = (uint32_t)(four ? 4 * q[k] : q[k]) + 0x00808080u ^ 0x00808080u;  // bytes: balanced base-256 digits
             }
             sum += (long long)part[0] + part[1];
             uint8_t* const dst = out_tile + ((size_t)(t / BITS_BOX_K) * (BITS_PLANES * rows) + b) * BITS_BOX_K + (t % BITS_BOX_K);
