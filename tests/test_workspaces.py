@@ -57,15 +57,15 @@ def test_least_workspace(shape, matrix, segments):
 
 def test_a_buffer_is_no_larger_than_there_is_room_for(monkeypatch):
     kept, cpu, empty = _lib.Workspaces(), torch.device("cpu"), torch.empty
-    assert kept.take(cpu, 1, 4000, lambda: 1000).numel() == 4000
-    assert kept.take(cpu, 1, 1000, lambda: 4000).numel() == 1000   # one size is asked for: `least` is not above it
+    assert kept.take(cpu, 1, 4000, (int, 1000)).numel() == 4000
+    assert kept.take(cpu, 1, 1000, (int, 4000)).numel() == 1000   # one size is asked for: `least` is not above it
     monkeypatch.setattr(_lib.Workspaces, "room", staticmethod(lambda device: 2500))
-    small = kept.take(cpu, 1, 4000, lambda: 1000)
+    small = kept.take(cpu, 1, 4000, (int, 1000))
     assert small.numel() == 1000
     kept.give(cpu, 1, small)
-    assert kept.take(cpu, 1, 4000, lambda: 1000) is small          # the least is there already
+    assert kept.take(cpu, 1, 4000, (int, 1000)) is small          # the least is there already
     kept.give(cpu, 1, empty(2000, dtype=torch.uint8))
-    assert kept.take(cpu, 1, 4000, lambda: 1000).numel() == 4000   # room once the kept one is given up
+    assert kept.take(cpu, 1, 4000, (int, 1000)).numel() == 4000   # room once the kept one is given up
 
     def fragmented(n, **kw):
         if n > 1000:
@@ -73,7 +73,7 @@ def test_a_buffer_is_no_larger_than_there_is_room_for(monkeypatch):
         return empty(n, **kw)
     monkeypatch.setattr(torch, "empty", fragmented)
     monkeypatch.setattr(_lib.Workspaces, "room", staticmethod(lambda device: 1 << 62))
-    assert kept.take(cpu, 1, 4000, lambda: 1000).numel() == 1000
+    assert kept.take(cpu, 1, 4000, (int, 1000)).numel() == 1000
     with pytest.raises(torch.cuda.OutOfMemoryError):
         kept.take(cpu, 1, 4000)
 

@@ -171,18 +171,22 @@ class Workspaces:
         self.most_kept, self.kept = most_kept, {}
 
     def take(self, device: torch.device, stream: int, nbytes: int, least=None) -> torch.Tensor:
-        """A buffer of ``nbytes``; of ``least()``, where that is given, when the device has no room for more."""
+        """A buffer of ``nbytes``; where the device has no room for that, of the smaller size that ``least``, a function
+        and its arguments, gives."""
         ws = self.kept.pop((device.index, stream), None)
+        if ws is not None and ws.numel() >= nbytes:
+            return ws
         size = 0 if ws is None else ws.numel()
-        if size < nbytes and least is not None and least() < nbytes:
+        smaller = nbytes if least is None else min(nbytes, least[0](*least[1:]))
+        if smaller < nbytes:
             if self.room(device) + size < nbytes:
-                nbytes = least()
+                nbytes = smaller
             else:
                 ws, size = None, 0   # given up before its successor is allocated
                 try:
                     return torch.empty(nbytes, dtype=torch.uint8, device=device)
                 except torch.cuda.OutOfMemoryError:
-                    nbytes = least()
+                    nbytes = smaller
         if size < nbytes:
             ws = None
             ws = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)

@@ -81,14 +81,6 @@ class StoredMatrix:
             elem == self.elem and input.device == self.device
 
 
-def _workspace(dev, stream, least, wanted, proj_type, matrix):
-    """Scratch for one projection: only a Rademacher matrix that is made on the fly has a use for more than the least
-    (byte operands for up to 32 rows), and does without where there is no room."""
-    if matrix is not None or int(proj_type) != _lib.TB_RADEMACHER:
-        return _workspaces.take(dev, stream, least())
-    return _workspaces.take(dev, stream, wanted(), least)
-
-
 def project(input, N, seed, num_feature_tiles, proj_type, *, alpha=1.0, out=None, accumulate=False,
             strict=None, allow_strided=False, matrix=None):
     """``alpha * input @ P`` with the fast_jl matrix P(seed, num_feature_tiles, proj_type).
@@ -131,8 +123,13 @@ def project(input, N, seed, num_feature_tiles, proj_type, *, alpha=1.0, out=None
     with _lib.on_device(dev):
         stream = _lib.current_stream(dev)
         tiles = max(num_feature_tiles, 1)
-        ws = _workspace(dev, stream, lambda: l.tb_project_least_workspace_bytes(dt, B, F, N, tiles, 0),
-                        lambda: l.tb_project_workspace_bytes(dt, B, F, N, tiles), proj_type, matrix)
+        # only a Rademacher matrix made on the fly has a use for more than the least (byte operands for up to 32 rows), and
+        # does without where there is no room
+        if matrix is None and proj_type == _lib.TB_RADEMACHER:
+            ws = _workspaces.take(dev, stream, l.tb_project_workspace_bytes(dt, B, F, N, tiles),
+                                  (l.tb_project_least_workspace_bytes, dt, B, F, N, tiles, 0))
+        else:
+            ws = _workspaces.take(dev, stream, l.tb_project_least_workspace_bytes(dt, B, F, N, tiles, 0))
         if matrix is not None:
             if not matrix.matches(input, N, num_feature_tiles) or matrix.seed != seed or \
                     matrix.proj_type != int(proj_type):
@@ -197,8 +194,11 @@ def project_segments(tensors, N, seed, num_feature_tiles, proj_type, *, alpha=1.
     with _lib.on_device(dev):
         stream = _lib.current_stream(dev)
         tiles = max(num_feature_tiles, 1)
-        ws = _workspace(dev, stream, lambda: l.tb_project_least_workspace_bytes(dt, B, F, N, tiles, len(tensors)),
-                        lambda: l.tb_project_segments_workspace_bytes(dt, B, F, N, tiles, len(tensors)), proj_type, matrix)
+        if matrix is None and proj_type == _lib.TB_RADEMACHER:   # as in project()
+            ws = _workspaces.take(dev, stream, l.tb_project_segments_workspace_bytes(dt, B, F, N, tiles, len(tensors)),
+                                  (l.tb_project_least_workspace_bytes, dt, B, F, N, tiles, len(tensors)))
+        else:
+            ws = _workspaces.take(dev, stream, l.tb_project_least_workspace_bytes(dt, B, F, N, tiles, len(tensors)))
         if matrix is not None:
             elem = _lib.TB_BF16 if dtype == torch.bfloat16 else _lib.TB_F16
             if (matrix.F, matrix.N, matrix.tiles, matrix.elem, matrix.device) != (F, N, num_feature_tiles, elem, dev) \
