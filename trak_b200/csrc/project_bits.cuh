@@ -13,24 +13,24 @@
 //     elements, ten times the error of the 16-bit kernel on one that a single element outweighs.  So the steps of a row are never
 //     coarser than its norm allows (row_exponent): rounding takes at most 2^-24 of its largest element and 2^-22 of the norm of
 //     the others.  The few elements that such steps put out of the planes' range are staged as zeros and listed by tile, and the
-//     CTAs that find one run the tile's streams once more (7 of the 18 instructions) and add them in 64 bits.
+//     CTAs that find one run the tile's streams once more (7 of the 17 instructions) and add them in 64 bits.
 //     Error against 64 bits over the row's norm, 16-bit kernel / steps by the largest element alone / this: 592,003 features
 //     beside one of 1 in bf16, N(0, 2^-8) 2.9e-7 / 7.6e-8 / 7.6e-8, N(0, 2^-16) 1.7e-5 / 4.4e-7 / 1.2e-7, uniform in 2^-30..2^-29
 //     1.7e-7 / 1.5e-6 / 1.3e-7, all of 2^-28 3.6e-7 / 3.8e-6 / 1.1e-7; 6,000,001 features, N(0, 2^-16) 9.0e-5 / 1.2e-6 / 8.6e-8,
 //     uniform 3.2e-7 / 3.9e-6 / 9.4e-8; N(0, 1) without the one 3.2e-6 / 7.4e-8 / 7.4e-8.
-//     us a call, the same three, one such element to a row: 16 x 1,000,003 bf16 -> 4096 371 / 238 / 248, 32 rows 399 / 351 / 375,
-//     17 x 330,003 -> 1536 79 / 64 / 75; without any, 16 x 2,796,202 fp16 -> 4096 1013 / 617 / 625, 16 x 40,001 -> 8192
-//     58 / 49 / 52, 32 x 1,048,576 fp32 -> 2048 236 / 233 / 235.
+//     us a call, the same three, one such element to a row: 16 x 1,000,003 bf16 -> 4096 370 / 237 / 242, 32 rows 400 / 350 / 368,
+//     17 x 330,003 -> 1536 79 / 64 / 72; without any, 16 x 2,796,202 fp16 -> 4096 1012 / 615 / 617, 32 x 2,796,202 1142 / 937 / 954,
+//     16 x 40,001 -> 8192 58 / 49 / 50, 32 x 1,048,576 fp32 -> 2048 239 / 235 / 231.
 //   * 2^i differs from word to word (bit 2j + h of a draw's byte: feature pair j, column parity h; two of the four j after
 //     a shift by four).  The column's factor 2^h is undone at the end, the features' 2^(2 (j & 1)) in the staging: even j are
 //     staged four times as large.
 //   * What bounds it.  Up to 16 rows the integer pipe, 82 % busy with 11 instructions per 16 x 32 entries (4 of the 7 of a draw,
-//     5 to spread it, 2 of hand-shakes; 35 instructions in all with a 16-bit operand, now 18): without its MMAs the kernel takes
-//     95 % of its time.  us a call, 16-bit operand -> this: 2,796,202 fp16 features -> 4096 1013 -> 625, 1,000,003 -> 8192
-//     721 -> 432, 10,000,001 bf16 -> 8192 6950 -> 4014; one row of 1,000,003 -> 2048 195 -> 120.
+//     5 to spread it, 2 of hand-shakes; 35 instructions in all with a 16-bit operand, now 17): without its MMAs the kernel takes
+//     95 % of its time.  us a call, 16-bit operand -> this: 2,796,202 fp16 features -> 4096 1012 -> 617, 1,000,003 -> 8192
+//     726 -> 425, 10,000,001 bf16 -> 8192 6951 -> 3991; one row of 1,000,003 -> 2048 195 -> 117.
 //     From 17 to 32 rows the accumulators leave room for one CTA per SM, of four groups, and the MMAs bound it (tensor pipe
 //     75 % busy at 24 rows, 85 at 32, with 7 TB/s from the L2; without generating it takes as long): 17 rows x 1,000,003 bf16
-//     -> 8192 757 -> 543, 24 rows fp16 -> 2048 213 -> 180, 32 rows x 2,796,202 -> 4096 1102 -> 934.
+//     -> 8192 757 -> 537, 24 rows fp16 -> 2048 213 -> 175, 32 rows x 2,796,202 -> 4096 1142 -> 954.
 //   * The groups' slots change hands together, and so do their boxes: one warp issues the MMAs beside busy generators, and a
 //     hand-over costs it some 300 cycles whatever it covers.  With barriers of each group's own 16 rows took 2 % longer (659
 //     us for 647), and four groups of 32-feature slots to a CTA 1023 us; with common ones 693, so two of 64 they stay.
@@ -285,8 +285,8 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
                 meet(1);
             }
             float* dst = p.partials + (size_t)blockIdx.y * p.B * p.N + n_out;
-            // twice: with the sums' additions in it the one loop takes 0.3 us longer (16 x 40,001 -> 8192, eight CTAs an SM's half
-            // one after another, 53.3 -> 51.3 us)
+            // twice: with these additions in it the one loop takes 0.3 us longer (16 x 40,001 -> 8192, where eight CTAs follow
+            // one another, 53.3 -> 51.3 us)
             auto finish = [&](auto more) {
 #pragma unroll EARLY ? 2 : 1
                 for (uint32_t turn = 0; turn < 2u; ++turn) {
@@ -609,9 +609,10 @@ struct OutlierLists {
 
 // stage_kernel for project_bits_kernel: staged[tile][128 features][plane][row].  A warp takes runs of 512 features of one
 // row, a lane 16 consecutive features, of which it makes the 16 bytes of every plane (gen_bits_pair says in which order).
-// Bound by memory, two bytes read (fp16) and four written an element, and next to that by 14 instructions an element:
-// 16 x 2,796,202 fp16 in 57 us.  A CTA takes the scale of its rows once and runs
-// of 512 features four at a time (16 x 592,003 fp16 14 us; 18 with eight runs to a CTA and the scale looked up for each).
+// Two bytes read (fp16) and four written an element at 4.8 TB/s, and 24 instructions an element, which take half of the issue
+// slots: with 32 warps to an SM it is the loads' latency that bounds it.  16 x 2,796,202 fp16 in 55 us, 32 x 1,048,576 fp32 in 47.
+// A CTA takes the scale of its rows once, and up to four runs of 512 features of a tile's even share (16 x 592,003 fp16 13 us;
+// 18 with eight runs to a CTA and the scale looked up for each).
 template <Elem E, bool SEG>
 __global__ void __launch_bounds__(256, !SEG && E == Elem::BF16 ? 5 : 4)
 stage_bits_kernel(const elem_t<E>* __restrict__ g, const SegDev* __restrict__ segs, uint32_t nsegs, uint64_t row0,
