@@ -106,6 +106,38 @@ __device__ __forceinline__ float scale_by(float v, int e) {
     return v * __int_as_float((127 + a) << 23) * __int_as_float((127 + b) << 23);
 }
 
+// Signed sums of the elements that the planes do not hold, of the tiles `tile`, `tile` + `step`, ... before `end`: those are
+// generated once more, up to the last such element.  `seed` is that of the thread's first stream in tile 0, `sums` its pair of
+// columns of row 0.  Not expanded where it is called, and without a pointer to the parameters: the loops in front of it keep
+// their registers.
+__device__ __noinline__ void add_outliers(const uint32_t* last_out, const uint32_t* heads, const Outlier* outliers, uint32_t nst,
+                                          long long* sums, uint32_t seed, uint32_t tile, uint32_t end, uint32_t step) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t t = tile; t < end; t += step) {
+        const uint32_t last = last_out[t];
+        if (last == 0u) continue;
+        Xw st0, st1;
+        xw_seed(st0, seed + 359124577u * t);
+        xw_seed(st1, seed + 658105236u * 16u + 359124577u * t);
+        for (uint32_t k0 = 0; k0 < last; k0 += 32u) {
+            const uint32_t k1 = min(32u, last - k0);
+            const uint32_t first = lane < k1 ? heads[(size_t)t * nst * 4u + k0 + lane] : 0u;
+            for (uint32_t k = 0; k < k1; ++k) {
+                const uint32_t c = gen_bits(st0, st1);
+                for (uint32_t r = __shfl_sync(0xffffffffu, first, k); r != 0u;) {
+                    const Outlier o = outliers[r - 1u];
+                    const long long q = (long long)o.q;
+                    const uint32_t at = 8u * ((o.feature & 1u) | (o.feature >> 3 << 1)) + 2u * ((o.feature & 7u) >> 1);
+                    unsigned long long* const sum = reinterpret_cast<unsigned long long*>(sums + o.row * 256u);
+                    atomicAdd(sum, (unsigned long long)(c >> at & 1u ? q : -q));
+                    atomicAdd(sum + 1, (unsigned long long)(c >> at & 2u ? q : -q));
+                    r = o.next;
+                }
+            }
+        }
+    }
+}
+
 // One CTA: 256 output columns (two accumulators) x up to ROWS rows x a bundle of feature tiles.  Roles and rings are those of
 // project_kernel with two accumulators; what differs is the operand, the digit planes beside one another in the N dimension
 // (rows x 4), the common hand-shakes, and that the accumulators are read once, at the end.
@@ -202,39 +234,11 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
             if (!ok && lane == 0) fail(p.status, abort_flag, ST_TIMEOUT_EMPTY, 0x4000u | (g << 16));
             if (ok && lane == 0) mbar_arrive(full + slot * 8u);
         }
-        // What the staging knows of rows b4 to b4 + 3 over the bundle's tiles: eight tiles at a time, row `lane & 3`.
-        struct Rows {
-            long long sum;
-            uint32_t ninf;
-            int exps;
-        };
-        auto rows_from = [&](uint32_t b4) {
-            const uint32_t row = b4 + (lane & 3u);
-            Rows r = {0, 0u, p.row_exp[row]};
-            for (uint32_t t = lane >> 2; t < ntile; t += 8u) {
-                r.sum += p.sums[(tile0 + t) * p.rows + row];
-                r.ninf += p.infs[(tile0 + t) * p.rows + row];
-            }
-#pragma unroll
-            for (int o = 4; o < 32; o <<= 1) {
-                r.sum += __shfl_xor_sync(0xffffffffu, r.sum, o);
-                r.ninf += __shfl_xor_sync(0xffffffffu, r.ninf, o);
-            }
-            return r;
-        };
-        // With one CTA to an SM nothing else runs at its end: they are fetched while the last products are made (17 rows x 70,001
-        // -> 8192 85 -> 80 us).  Beside another CTA it costs the generators registers and is not worth it (620 -> 643).
-        constexpr bool EARLY = ROWS > 16u;
-        Rows early[2];
-        static_assert(ROWS <= 8u * NG, "two turns of four rows to a group");
         bool outside = false;  // some tile has elements that the planes do not hold; the same for every warp
         if (ok) {
             cudaGridDependencySynchronize();  // the staging's lists, sums and scales
             for (uint32_t t = lane; t < ntile; t += 32u) outside |= p.last_out[tile0 + t] != 0u;
             outside = __any_sync(0xffffffffu, outside);
-#pragma unroll
-            for (uint32_t turn = 0; turn < 2u; ++turn)
-                if (EARLY && 4u * (g + NG * turn) < p.B) early[turn] = rows_from(4u * (g + NG * turn));
         }
         // ---- the exact integer result of this CTA, as fp32 ----
         if (ok && !mbar_wait_warp(smem_u32(&bar_acc), 0u, abort_flag)) {
@@ -259,40 +263,32 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
                 };
                 for (uint32_t i = threadIdx.x; i < p.rows * 256u; i += GW * NG * 32u) extra[0][i] = 0;
                 meet(0);
-                for (uint32_t ti = g; ti < ntile && ok; ti += NG) {
-                    const uint32_t t = tile0 + ti, last = p.last_out[t];
-                    if (last == 0u) continue;
-                    Xw st0, st1;
-                    xw_seed(st0, p.seed + 658105236u * stream_col + 359124577u * t);
-                    xw_seed(st1, p.seed + 658105236u * (stream_col + 16u) + 359124577u * t);
-                    for (uint32_t k0 = 0; k0 < last; k0 += 32u) {
-                        const uint32_t k1 = min(32u, last - k0);
-                        const uint32_t first = lane < k1 ? p.heads[(size_t)t * p.nst * 4u + k0 + lane] : 0u;
-                        for (uint32_t k = 0; k < k1; ++k) {
-                            const uint32_t c = gen_bits(st0, st1);
-                            for (uint32_t r = __shfl_sync(0xffffffffu, first, k); r != 0u;) {
-                                const Outlier o = p.outliers[r - 1u];
-                                const long long q = (long long)o.q;
-                                const uint32_t at = 8u * ((o.feature & 1u) | (o.feature >> 3 << 1)) + 2u * ((o.feature & 7u) >> 1);
-                                unsigned long long* const sum = reinterpret_cast<unsigned long long*>(&extra[o.row][2u * pair]);
-                                atomicAdd(sum, (unsigned long long)(c >> at & 1u ? q : -q));
-                                atomicAdd(sum + 1, (unsigned long long)(c >> at & 2u ? q : -q));
-                                r = o.next;
-                            }
-                        }
-                    }
-                }
+                if (ok)
+                    add_outliers(p.last_out, p.heads, p.outliers, p.nst, extra[0] + 2u * pair, p.seed + 658105236u * stream_col, tile0 + g,
+                                 tile0 + ntile, NG);
                 meet(1);
             }
             float* dst = p.partials + (size_t)blockIdx.y * p.B * p.N + n_out;
             // twice: with these additions in it the one loop takes 0.3 us longer (16 x 40,001 -> 8192, where eight CTAs follow
             // one another, 53.3 -> 51.3 us)
             auto finish = [&](auto more) {
-#pragma unroll EARLY ? 2 : 1
-                for (uint32_t turn = 0; turn < 2u; ++turn) {
-                    const uint32_t b4 = 4u * (g + NG * turn);
-                    if (b4 >= p.B || !ok) break;
-                    const Rows known = EARLY ? early[turn] : rows_from(b4);
+                for (uint32_t b4 = 4u * g; b4 < p.B && ok; b4 += 4u * NG) {
+                    // sums of four rows over the bundle's tiles: eight tiles at a time, row `lane & 3`.  (Fetched before the last
+                    // products are there 17 rows x 70,001 -> 8192 take 77 us for 80, but 32 x 11,173,962 -> 4096 3820 for 3740:
+                    // the generators' loop is allotted other registers.)
+                    const uint32_t row = b4 + (lane & 3u);
+                    long long sum = 0;
+                    uint32_t ninf = 0;
+                    const int exps = p.row_exp[row];
+                    for (uint32_t t = lane >> 2; t < ntile; t += 8u) {
+                        sum += p.sums[(tile0 + t) * p.rows + row];
+                        ninf += p.infs[(tile0 + t) * p.rows + row];
+                    }
+#pragma unroll
+                    for (int o = 4; o < 32; o <<= 1) {
+                        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                        ninf += __shfl_xor_sync(0xffffffffu, ninf, o);
+                    }
                     uint32_t d[2][BITS_PLANES][4];
 #pragma unroll
                     for (int h = 0; h < 2; ++h)
@@ -303,9 +299,9 @@ project_bits_kernel(const __grid_constant__ CUtensorMap tmap, const BitsParams p
 #pragma unroll
                     for (uint32_t j = 0; j < 4; ++j) {
                         const uint32_t b = b4 + j;
-                        const long long total = __shfl_sync(0xffffffffu, known.sum, j);
-                        const uint32_t infs = __shfl_sync(0xffffffffu, known.ninf, j);
-                        const int e = __shfl_sync(0xffffffffu, known.exps, j);
+                        const long long total = __shfl_sync(0xffffffffu, sum, j);
+                        const uint32_t infs = __shfl_sync(0xffffffffu, ninf, j);
+                        const int e = __shfl_sync(0xffffffffu, exps, j);
                         if (b >= p.B) break;
                         float2 v;
 #pragma unroll
