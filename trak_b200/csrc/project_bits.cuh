@@ -18,19 +18,19 @@
 //     beside one of 1 in bf16, N(0, 2^-8) 2.9e-7 / 7.6e-8 / 7.6e-8, N(0, 2^-16) 1.7e-5 / 4.4e-7 / 1.2e-7, uniform in 2^-30..2^-29
 //     1.7e-7 / 1.5e-6 / 1.3e-7, all of 2^-28 3.6e-7 / 3.8e-6 / 1.1e-7; 6,000,001 features, N(0, 2^-16) 9.0e-5 / 1.2e-6 / 8.6e-8,
 //     uniform 3.2e-7 / 3.9e-6 / 9.4e-8; N(0, 1) without the one 3.2e-6 / 7.4e-8 / 7.4e-8.
-//     us a call, the same three, one such element to a row: 16 x 1,000,003 bf16 -> 4096 370 / 237 / 242, 32 rows 400 / 350 / 368,
-//     17 x 330,003 -> 1536 79 / 64 / 72; without any, 16 x 2,796,202 fp16 -> 4096 1012 / 615 / 617, 32 x 2,796,202 1142 / 937 / 954,
-//     16 x 40,001 -> 8192 58 / 49 / 50, 32 x 1,048,576 fp32 -> 2048 239 / 235 / 231.
+//     us a call, the same three, one such element to a row: 16 x 1,000,003 bf16 -> 4096 371 / 238 / 241, 32 rows 400 / 351 / 365,
+//     17 x 330,003 -> 1536 79 / 64 / 72; without any, 16 x 2,796,202 fp16 -> 4096 1014 / 617 / 616, 32 x 2,796,202 1168 / 957 / 956,
+//     16 x 40,001 -> 8192 58 / 49 / 48, 32 x 1,048,576 fp32 -> 2048 240 / 236 / 231.
 //   * 2^i differs from word to word (bit 2j + h of a draw's byte: feature pair j, column parity h; two of the four j after
 //     a shift by four).  The column's factor 2^h is undone at the end, the features' 2^(2 (j & 1)) in the staging: even j are
 //     staged four times as large.
 //   * What bounds it.  Up to 16 rows the integer pipe, 82 % busy with 11 instructions per 16 x 32 entries (4 of the 7 of a draw,
 //     5 to spread it, 2 of hand-shakes; 35 instructions in all with a 16-bit operand, now 17): without its MMAs the kernel takes
-//     95 % of its time.  us a call, 16-bit operand -> this: 2,796,202 fp16 features -> 4096 1012 -> 617, 1,000,003 -> 8192
-//     726 -> 425, 10,000,001 bf16 -> 8192 6951 -> 3991; one row of 1,000,003 -> 2048 195 -> 117.
+//     95 % of its time.  us a call, 16-bit operand -> this: 2,796,202 fp16 features -> 4096 1014 -> 616, 1,000,003 -> 8192
+//     726 -> 425, 10,000,001 bf16 -> 8192 6970 -> 3989; one row of 1,000,003 -> 2048 196 -> 116.
 //     From 17 to 32 rows the accumulators leave room for one CTA per SM, of four groups, and the MMAs bound it (tensor pipe
 //     75 % busy at 24 rows, 85 at 32, with 7 TB/s from the L2; without generating it takes as long): 17 rows x 1,000,003 bf16
-//     -> 8192 757 -> 537, 24 rows fp16 -> 2048 213 -> 175, 32 rows x 2,796,202 -> 4096 1142 -> 954.
+//     -> 8192 757 -> 537, 24 rows fp16 -> 2048 213 -> 175, 32 rows x 2,796,202 -> 4096 1168 -> 956.
 //   * The groups' slots change hands together, and so do their boxes: one warp issues the MMAs beside busy generators, and a
 //     hand-over costs it some 300 cycles whatever it covers.  With barriers of each group's own 16 rows took 2 % longer (659
 //     us for 647), and four groups of 32-feature slots to a CTA 1023 us; with common ones 693, so two of 64 they stay.
